@@ -72,7 +72,6 @@ __device__ __forceinline__ DN operator-(DN a, DN b) { return DN(__dsub_rn(a.v, b
 __device__ __forceinline__ DN operator*(DN a, DN b) { return DN(__dmul_rn(a.v, b.v)); }
 __device__ __forceinline__ DN operator/(DN a, DN b) { return DN(__ddiv_rn(a.v, b.v)); }
 __device__ __forceinline__ DN operator-(DN a) { return DN(-a.v); }
-__device__ __forceinline__ DN &operator+=(DN &a, DN b) { return a = a + b; }
 __device__ __forceinline__ bool operator<(DN a, DN b) { return a.v < b.v; }
 __device__ __forceinline__ bool operator>(DN a, DN b) { return a.v > b.v; }
 __device__ __forceinline__ DN sqrt_(DN x) { return DN(__dsqrt_rn(x.v)); }
@@ -259,24 +258,6 @@ __device__ __forceinline__ double dist_exact(const BoxD &b, double4_32a u, doubl
 
 // ---- bonded terms: contributions per centre bead ----------------------------
 
-// harmonic bond (c, c+1): eval_tether_forces::iter tether.cpp:21-36,
-// harmonic::operator() harmonic.h:18-25.  Returns the force on c (the force on
-// c+1 is its negative).
-template <class T>
-__device__ __forceinline__ V3<T> tether_term(const TermP &p, double4_32a r1, double4_32a r2, T nat_dist, T *V) {
-    V3<T> r12 = diff<T>(r1, r2);
-    T r12_n = norm(r12);
-    T dr = r12_n - nat_dist, dr2 = dr * dr;
-    T H1 = tpar<T>(p.tether_H1, p.f.tether_H1), H2 = tpar<T>(p.tether_H2, p.f.tether_H2);
-    T V_ = T(0.5) * dr2 * (H1 + H2 * dr2);
-    T dV_dr = dr * (H1 + T(2) * H2 * dr2);
-    V_ = clampv<T>(V_, T(-1.0e3), T(1.0e3));
-    dV_dr = clampv<T>(dV_dr, T(-1.0e3), T(1.0e3));
-    *V = V_;
-    V3<T> u{r12.x / r12_n, r12.y / r12_n, r12.z / r12_n};
-    return dV_dr * u;
-}
-
 // ---- heuristic angles and dihedrals -----------------------------------------
 
 // Horner sums of V(theta) = sum_{d=0..6} a_d theta^d and its derivative, in
@@ -319,92 +300,11 @@ __device__ __noinline__ void heur_dih_nl(const T *hc, T s, T co, T *V, T *dV) {
     heur_dih_V<T>(c, s, co, V, dV);
 }
 
-// native angle (c-1, c, c+1): eval_native_angle_forces::iter
-// angle/native.cpp:13-39; or, with hc (the type's 7 coefficients), the
-// heuristic angle of eval_heurestic_angle_forces::iter
-// angle/heurestic.cpp:29-59, whose geometry is the same.  Writes the forces
-// on the three beads.
-template <class T>
-__device__ __forceinline__ void angle_term(const TermP &p, double4_32a q1, double4_32a q2, double4_32a q3, T nat_theta,
-                                           const double *hc, V3<T> *f1, V3<T> *f2, V3<T> *f3, T *V) {
-    V3<T> r12 = diff<T>(q1, q2), r23 = diff<T>(q2, q3);
-    V3<T> x12_23 = cross(r12, r23);
-    T r12_rn = ninv(r12), r23_rn = ninv(r23);
-    V3<T> d1 = r12_rn * unit(cross(r12, x12_23));
-    V3<T> d3 = r23_rn * unit(cross(r23, x12_23));
-    V3<T> d2 = (-d1) - d3;
-    T cos_theta = -dot(r12, r23) * r12_rn * r23_rn;
-    T theta = acos_c(cos_theta);
-    T dV;
-    if (hc) {
-        const double2 vd = heur_poly_nl(hc, (double)theta);
-        *V = (T)vd.x;
-        dV = (T)vd.y;
-    } else {
-        T dtheta = theta - nat_theta;
-        T k = T(p.nat_ang_k);
-        *V = T(0.5) * k * dtheta * dtheta;
-        dV = k * dtheta;
-    }
-    *f1 = -(dV * d1);
-    *f2 = -(dV * d2);
-    *f3 = -(dV * d3);
-}
-
-// native dihedral (c-1, c, c+1, c+2): eval_cnd_forces::iter
-// dihedral/complex_native.cpp:13-49 and eval_snd_forces::iter
-// dihedral/simple_native.cpp:13-45; or, with hc (the type's 6
-// coefficients), the heuristic dihedral of
-// eval_heurestic_dihedral_forces::iter dihedral/heurestic.cpp:29-70 with
-// phi = acos(cos_phi) [line 43 takes cos(cos_phi)], its energy in *Vc
-template <class T>
-__device__ __forceinline__ void dihedral_term(const TermP &p, double4_32a q1, double4_32a q2, double4_32a q3, double4_32a q4,
-                                              T nat_phi, bool cnd, bool snd, const T *hc, V3<T> *f, T *Vc, T *Vs) {
-    V3<T> r12 = diff<T>(q1, q2), r23 = diff<T>(q2, q3), r34 = diff<T>(q3, q4);
-    V3<T> x12_23 = cross(r12, r23), x23_34 = cross(r23, r34);
-    T x12_23_rn = ninv(x12_23), x23_34_rn = ninv(x23_34);
-    V3<T> x12_23_u = x12_23_rn * x12_23, x23_34_u = x23_34_rn * x23_34;
-    T cos_phi = dot(x12_23_u, x23_34_u);
-    T phi = acos_c(cos_phi);
-    if (dot(x12_23, r34) < T(0)) phi = -phi;
-    T diff_ = phi - nat_phi;
-    T dV = T(0);
-    *Vc = T(0);
-    *Vs = T(0);
-    if (hc) {
-        heur_dih_nl<T>(hc, sin(phi), cos_phi, Vc, &dV);
-    } else if (cnd) {
-        T sin_diff, cos_diff, sin_3diff, cos_3diff;
-        sincos_(diff_, &sin_diff, &cos_diff);
-        sincos_(T(3) * diff_, &sin_3diff, &cos_3diff);
-        T CDA = T(p.cnd_CDA), CDB = T(p.cnd_CDB);
-        *Vc = CDA * (T(1) - cos_diff) + CDB * (T(1) - cos_3diff);
-        dV += CDA * sin_diff + CDB * T(3) * sin_3diff;
-    }
-    if (snd && !hc) {
-        T CDH = T(p.snd_CDH);
-        *Vs = T(0.5) * CDH * diff_ * diff_;
-        dV += CDH * diff_;
-    }
-    T r23_n = norm(r23);
-    V3<T> d1 = x12_23_rn * (r23_n * (-x12_23_u));
-    V3<T> d4 = x23_34_rn * (r23_n * x23_34_u);
-    T k1 = dot(r12, r23), k4 = dot(r23, r34), den = r23_n * r23_n;
-    V3<T> df{(-d1.x * k1 + d4.x * k4) / den, (-d1.y * k1 + d4.y * k4) / den, (-d1.z * k1 + d4.z * k4) / den};
-    V3<T> d2 = (-d1) + df;
-    V3<T> d3 = (-d4) - df;
-    f[0] = -(dV * d1);
-    f[1] = -(dV * d2);
-    f[2] = -(dV * d3);
-    f[3] = -(dV * d4);
-}
-
 // chiral quad (c-1, c, c+1, c+2): eval_chiral_forces::iter chiral.cpp:15-37.
 // Writes the forces on the four beads.
 template <class T>
-__device__ __forceinline__ void chiral_term(const TermP &p, double4_32a q1, double4_32a q2, double4_32a q3,
-                                            double4_32a q4, T nat_factor, T nat_chir, V3<T> *f, T *V) {
-    V3<T> r12 = diff<T>(q1, q2), r23 = diff<T>(q2, q3), r34 = diff<T>(q3, q4);
+__device__ __forceinline__ void chiral_bonds(const TermP &p, V3<T> r12, V3<T> r23, V3<T> r34, T nat_factor, T nat_chir,
+                                             V3<T> *f, T *V) {
     V3<T> x12_23 = cross(r12, r23), x12_34 = cross(r12, r34), x23_34 = cross(r23, r34);
     T chir = dot(r12, x23_34) * nat_factor;
     T chir_diff = chir - nat_chir;
@@ -435,106 +335,6 @@ __device__ __forceinline__ void chiral_mixed(const TermP &p, V3<float> r12, V3<f
     f[3] = -(g * x12_23);
 }
 
-// ---- bonded terms of the mixed path -------------------------------------------
-// The reference formulation (acos of a clamped cosine; cross products of bond
-// vectors) loses all accuracy in FP32 near straight triples, where the stiff
-// starting chains live: the reference's own FP32 build misses by ~1e-3.  Here
-// the bond vectors, their cross products and the dihedral's triple product are
-// formed in FP64 and the angles are taken with atan2 in FP32:
-//   theta = atan2(|r12 x r23|, -r12.r23)                    (= acos of the cosine)
-//   phi   = atan2(|r23| (x12_23 . r34), x12_23 . x23_34)    (= +-acos, sign of
-//            x12_23 . r34 as in complex_native.cpp:27-28)
-// after which every FP32 operation is well conditioned.  Force expressions are
-// those of angle/native.cpp:25-38 and dihedral/complex_native.cpp:37-48.
-__device__ __forceinline__ V3<double> dsub(double4_32a u, double4_32a w) {
-    return V3<double>{w.x - u.x, w.y - u.y, w.z - u.z};
-}
-__device__ __forceinline__ V3<float> f3(V3<double> a) { return V3<float>{(float)a.x, (float)a.y, (float)a.z}; }
-
-// tether of the mixed path from the narrowed bond vector r12 = r2 - r1
-__device__ __forceinline__ V3<float> tether_vec(const TermP &p, V3<float> r12, float nat_dist, float *V) {
-    float r12_n = norm(r12);
-    float dr = r12_n - nat_dist, dr2 = dr * dr;
-    float H1 = p.f.tether_H1, H2 = p.f.tether_H2;
-    float V_ = 0.5f * dr2 * (H1 + H2 * dr2);
-    float dV_dr = dr * (H1 + 2.0f * H2 * dr2);
-    *V = clampv<float>(V_, -1.0e3f, 1.0e3f);
-    dV_dr = clampv<float>(dV_dr, -1.0e3f, 1.0e3f);
-    const float inv = 1.0f / r12_n;
-    return dV_dr * V3<float>{r12.x * inv, r12.y * inv, r12.z * inv};
-}
-
-// r12, r23: narrowed bond vectors; x12_23: narrowed FP64 cross product.
-// hc: heuristic angle coefficients (or null); their polynomial, whose terms
-// cancel to ~1e-5 of their size, is summed in FP64
-__device__ __forceinline__ void angle_mixed(const TermP &p, V3<float> r12, V3<float> r23, V3<float> x12_23,
-                                            float nat_theta, const double *hc, V3<float> *f1, V3<float> *f2,
-                                            V3<float> *f3o, float *V) {
-    float r12_rn = 1.0f / norm(r12), r23_rn = 1.0f / norm(r23);
-    V3<float> d1 = r12_rn * unit(cross(r12, x12_23));
-    V3<float> d3 = r23_rn * unit(cross(r23, x12_23));
-    V3<float> d2 = (-d1) - d3;
-    float theta = atan2f(norm(x12_23), -dot(r12, r23));
-    float dV;
-    if (hc) {
-        const double2 vd = heur_poly_nl(hc, (double)theta);
-        *V = (float)vd.x;
-        dV = (float)vd.y;
-    } else {
-        float dtheta = theta - nat_theta;
-        float k = p.f.nat_ang_k;
-        *V = 0.5f * k * dtheta * dtheta;
-        dV = k * dtheta;
-    }
-    *f1 = -(dV * d1);
-    *f2 = -(dV * d2);
-    *f3o = -(dV * d3);
-}
-
-// narrowed bond vectors and cross products; X = x12_23 . x23_34 and
-// T = x12_23 . r34 taken in FP64 by the caller
-// (hc: heuristic dihedral coefficients or null, as dihedral_term)
-__device__ __forceinline__ void dihedral_mixed(const TermP &p, V3<float> r12, V3<float> r23, V3<float> r34,
-                                               V3<float> x12_23, V3<float> x23_34, float X, float T,
-                                               float nat_phi, bool cnd, bool snd, const float *hc, V3<float> *f,
-                                               float *Vc, float *Vs) {
-    float r23_n = norm(r23);
-    float phi = atan2f(r23_n * T, X);
-    float diff_ = phi - nat_phi;
-    float dV = 0.0f;
-    *Vc = 0.0f;
-    *Vs = 0.0f;
-    if (hc) {
-        float sp, cp;
-        sincosf(phi, &sp, &cp);
-        heur_dih_nl<float>(hc, sp, cp, Vc, &dV);
-    } else if (cnd) {
-        float s1, c1, s3, c3;
-        sincosf(diff_, &s1, &c1);
-        sincosf(3.0f * diff_, &s3, &c3);
-        float CDA = p.f.cnd_CDA, CDB = p.f.cnd_CDB;
-        *Vc = CDA * (1.0f - c1) + CDB * (1.0f - c3);
-        dV += CDA * s1 + CDB * 3.0f * s3;
-    }
-    if (snd && !hc) {
-        float CDH = p.f.snd_CDH;
-        *Vs = 0.5f * CDH * diff_ * diff_;
-        dV += CDH * diff_;
-    }
-    float x12_23_rn = 1.0f / norm(x12_23), x23_34_rn = 1.0f / norm(x23_34);
-    V3<float> x12_23_u = x12_23_rn * x12_23, x23_34_u = x23_34_rn * x23_34;
-    V3<float> d1 = x12_23_rn * (r23_n * (-x12_23_u));
-    V3<float> d4 = x23_34_rn * (r23_n * x23_34_u);
-    float k1 = dot(r12, r23), k4 = dot(r23, r34), den = r23_n * r23_n;
-    V3<float> df{(-d1.x * k1 + d4.x * k4) / den, (-d1.y * k1 + d4.y * k4) / den, (-d1.z * k1 + d4.z * k4) / den};
-    V3<float> d2 = (-d1) + df;
-    V3<float> d3 = (-d4) - df;
-    f[0] = -(dV * d1);
-    f[1] = -(dV * d2);
-    f[2] = -(dV * d3);
-    f[3] = -(dV * d4);
-}
-
 // ---- pair terms: force on the first bead of r12 = r_uv(r_i, r_j) ------------
 
 // lj::operator(): primitives/lj.h:22-30
@@ -545,16 +345,6 @@ __device__ __forceinline__ void lj_eval(T depth, T r_min, T r_inv, T *V, T *dV) 
     T dV_dr = T(12) * depth * r_inv * (s6 - s12);
     *V = clampv<T>(V_, T(-1.0e3), T(1.0e3));
     *dV = clampv<T>(dV_dr, T(-1.0e3), T(1.0e3));
-}
-
-// Go contact: eval_go_forces::iter go.cpp:31-46
-template <class T>
-__device__ __forceinline__ V3<T> go_pair(const TermP &p, V3<T> r12, T nat_dist, T *V) {
-    T r12_rn = ninv(r12);
-    V3<T> u = r12_rn * r12;
-    T dV;
-    lj_eval<T>(tpar<T>(p.go_depth, p.f.go_depth), nat_dist, r12_rn, V, &dV);
-    return dV * u;
 }
 
 // native disulfide: eval_nat_ssbond_forces::iter native_ss.cpp:27-40,
@@ -570,39 +360,6 @@ __device__ __forceinline__ V3<T> ss_pair(const TermP &p, V3<T> r12, T *V) {
     dV_dr = clampv<T>(dV_dr, T(-1.0e3), T(1.0e3));
     const V3<T> u{r12.x / r12_n, r12.y / r12_n, r12.z / r12_n};
     return dV_dr * u;
-}
-
-// Pauli exclusion: eval_pauli_exclusion_forces::iter pauli.cpp:32-48,
-// shifted_lj::operator() shifted_lj.h:14-21
-template <class T>
-__device__ __forceinline__ V3<T> pauli_pair(const TermP &p, V3<T> r12, T *V) {
-    T r12_rn = ninv(r12);
-    T r_excl = tpar<T>(p.pauli_r_excl, p.f.pauli_r_excl);
-    if (T(1) < r12_rn * r_excl) {
-        V3<T> u = r12_rn * r12;
-        T depth = tpar<T>(p.pauli_depth, p.f.pauli_depth);
-        T s = r12_rn * r_excl, s6 = ipow6(s), s12 = s6 * s6;
-        T V_ = depth * (s12 - T(2) * s6 + T(1));
-        T dV_dr = T(12) * depth * r12_rn * (s6 - s12);
-        *V = clampv<T>(V_, T(-1.0e3), T(1.0e3));
-        dV_dr = clampv<T>(dV_dr, T(-1.0e3), T(1.0e3));
-        return dV_dr * u;
-    }
-    *V = T(0);
-    return V3<T>{T(0), T(0), T(0)};
-}
-
-// Debye-Hueckel: eval_const_es_forces::iter es/const.cpp:13-32 and
-// eval_relative_es_forces::iter es/relative.cpp:13-32
-template <class T>
-__device__ __forceinline__ V3<T> es_pair(const TermP &p, V3<T> r12, T q1_x_q2, T *V) {
-    T r12_n = norm(r12), r12_rn = T(1) / r12_n;
-    V3<T> u = r12_rn * r12;
-    T sdi = tpar<T>(p.es_sdi, p.f.es_sdi);
-    T Vij = tpar<T>(p.es_Vf, p.f.es_Vf) * q1_x_q2 * exp_(-r12_n * sdi) * r12_rn * r12_rn;
-    T dVij_dr = p.es_rel ? -Vij * (sdi + T(2) * r12_rn) : -Vij * (sdi + r12_rn);
-    *V = Vij;
-    return dVij_dr * u;
 }
 
 // sink_lj::operator(): primitives/sink_lj.h:24-33
@@ -682,29 +439,9 @@ __device__ __forceinline__ uint64_t gf2_apply(const uint64_t *__restrict__ col, 
     return y;
 }
 
-// ---- per-bead force accumulation and pair geometry, by path -------------------
-// FP64 path: FP64 sums in the reference's term order; r_uv in FP64.
-// Mixed path: FP32 terms summed per bead in float-float (each addition exact
-// to 2^-47 of the running sum, below the FP32 rounding of the terms by ~10^7)
-// and widened once; pair vectors from split positions in FP32 (the minimum
-// image subtracted in float-float), with no FP64 instruction per pair.
-template <class FT> struct Acc3;
-// FP64: every addition rounded on its own (never fused with the product that
-// formed the term), so the sums are the same bits whatever code shape the
-// compiler gives the loops
-template <> struct Acc3<double> {
-    double x = 0, y = 0, z = 0;
-    __device__ __forceinline__ void add(V3<double> f) { x = __dadd_rn(x, f.x); y = __dadd_rn(y, f.y); z = __dadd_rn(z, f.z); }
-    __device__ __forceinline__ void sub(V3<double> f) { x = __dadd_rn(x, -f.x); y = __dadd_rn(y, -f.y); z = __dadd_rn(z, -f.z); }
-    __device__ __forceinline__ V3<double> total() const { return V3<double>{x, y, z}; }
-};
-template <> struct Acc3<float> {
-    FF x{0.0f, 0.0f}, y{0.0f, 0.0f}, z{0.0f, 0.0f};
-    __device__ __forceinline__ void add(V3<float> f) { ff_acc(x, f.x); ff_acc(y, f.y); ff_acc(z, f.z); }
-    __device__ __forceinline__ void sub(V3<float> f) { ff_acc(x, -f.x); ff_acc(y, -f.y); ff_acc(z, -f.z); }
-    __device__ __forceinline__ V3<double> total() const { return V3<double>{ff_to_d(x), ff_to_d(y), ff_to_d(z)}; }
-};
-
+// ---- pair geometry of the mixed path ------------------------------------------
+// Pair vectors from split positions in FP32 (the minimum image subtracted in
+// float-float), with no FP64 instruction per pair.
 // w - u of split coordinates along one axis of length L = Lh + Ll (0 when open)
 __device__ __forceinline__ float mi_axis(F2 u, F2 w, float Lh, float Ll, float Linv, bool per) {
     if (!per) return __fadd_rn(__fsub_rn(w.h, u.h), __fsub_rn(w.l, u.l));
@@ -714,26 +451,7 @@ __device__ __forceinline__ float mi_axis(F2 u, F2 w, float Lh, float Ll, float L
     return __fadd_rn(q.h, __fsub_rn(q.l, __fmul_rn(n, Ll)));
 }
 
-// q_i q_j of the Debye-Hueckel pair (es_pair.cpp:17): an FP64 product on the
-// FP64 path; the charges are small integers, so the FP32 product of the
-// narrowed charges is the same value on the mixed path
-template <class FT> __device__ __forceinline__ FT charge_prod(double qi, double qj);
-template <> __device__ __forceinline__ double charge_prod<double>(double qi, double qj) { return qi * qj; }
-template <> __device__ __forceinline__ float charge_prod<float>(double qi, double qj) {
-    return __fmul_rn(narrow_f(qi), narrow_f(qj));
-}
-
 template <class FT> struct PairGeo;
-template <> struct PairGeo<double> {
-    BoxD bx;
-    bool per;
-    double4_32a pi;
-    __device__ __forceinline__ PairGeo(const BoxD &b, bool periodic, double4_32a p) : bx(b), per(periodic), pi(p) {}
-    __device__ __forceinline__ V3<double> to(double4_32a pj) const { return r_uv_p<double>(bx, per, pi, pj); }
-    __device__ __forceinline__ V3<double> between(double4_32a a, double4_32a b) const {
-        return r_uv_p<double>(bx, per, a, b);
-    }
-};
 template <> struct PairGeo<float> {
     float Lh[3], Ll[3], Li[3];
     bool per;

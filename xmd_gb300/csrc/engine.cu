@@ -44,7 +44,6 @@ std::string &last_error() {
                                      " at " #call);                                  \
     } while (0)
 
-constexpr int BLK_ON = 32;           // beads per granule of the force blocks' occupancy map
 constexpr int NL_MASK = 0x1FFFFFFF;
 constexpr int NL_PID = 1 << 29;
 constexpr int NL_PAULI = 1 << 30;
@@ -122,28 +121,12 @@ __device__ __forceinline__ unsigned long long warp_max_bits(unsigned long long v
     return v;
 }
 
-template <class FT>
-__device__ __forceinline__ void add3(double &fx, double &fy, double &fz, V3<FT> f) {
-    fx += (double)f.x;
-    fy += (double)f.y;
-    fz += (double)f.z;
-}
-
 // finiteness from the exponent bits (integer pipe)
 __device__ __forceinline__ bool finite_bits(double x) {
     return ((unsigned long long)__double_as_longlong(x) & 0x7ff0000000000000ull) != 0x7ff0000000000000ull;
 }
 
-// native distance of Go-list entry k in the path's type
-template <class FT> __device__ __forceinline__ FT nat_dist(const Dev &d, int k);
-template <> __device__ __forceinline__ double nat_dist<double>(const Dev &d, int k) { return d.nat_d[k]; }
-template <> __device__ __forceinline__ float nat_dist<float>(const Dev &d, int k) { return d.nat_df[k]; }
-
-// ---- force (+ integrate) kernel --------------------------------------------------
-// MODE 0: forces and per-term energies at pos[cur] (eval).
-// MODE 1: forces, then one Langevin predictor-corrector step (lang_pc.cpp:5-41)
-//         writing pos[cur^1], y1..y5, the generator state and the skin-test
-//         displacement (verify.cpp:10-15).
+// ---- external forces ---------------------------------------------------------------
 // Wall forces on one bead at its wrapped position rw.  ljw points at the bead's state for the first LJ attractive
 // wall (stride N); step = true advances the pair states.
 struct WallOut { double fx, fy, fz, vs, vl; };
@@ -389,631 +372,21 @@ __global__ void __launch_bounds__(128) k_pid(Dev d, TermP p, int cur) {
     if (MODE == 0 && Vsum != 0.0) atomicAdd(&d.Vrep[r * XMD_NUM_TERMS + XMD_TERM_PID], Vsum);
 }
 
-// Lanes of a bead in the step kernel.  A bead's pair entries (native
-// contacts, disulfides, Verlet row, quasi-adiabatic contacts) are dealt to
-// VL = 4 virtual lanes, entry k of a list to virtual lane k mod 4, each with
-// its own partial force; the partials are combined as ((v0 + v1) + (v2 + v3)).
-// The virtual lanes run on LPB = 1, 2 or 4 adjacent threads of one warp
-// (thread ln of a bead holds virtual lanes ln, ln + LPB, ...), a launch shape
-// chosen by the autotuner: the sums, and so the trajectory, are the same bits
-// for every LPB.  A bead's bonded centres are split in two tasks; its
-// integrator runs axis a on thread a mod LPB, with the generator, the new
-// position and the skin test on the last thread of the bead.
-constexpr int VL = 4;
+}  // namespace xmdg
+#include "step.cuh"
+namespace xmdg {
 
-template <int LPB> __device__ __forceinline__ unsigned bead_mask(int t) {
-    return ((1u << LPB) - 1u) << ((t & 31) & ~(LPB - 1));
-}
-__device__ __forceinline__ double vadd(double a, double b) { return __dadd_rn(a, b); }
-__device__ __forceinline__ FF vadd(FF a, FF b) { return ff_add(a, b); }
-__device__ __forceinline__ double xlane(unsigned m, double v, int o, int w) { return __shfl_xor_sync(m, v, o, w); }
-__device__ __forceinline__ FF xlane(unsigned m, FF v, int o, int w) {
-    return FF{__shfl_xor_sync(m, v.h, o, w), __shfl_xor_sync(m, v.l, o, w)};
-}
-// ((v0 + v1) + (v2 + v3)) of a bead's virtual lanes, the same bits on every
-// thread of the bead and for every LPB (each addition is commutative bit for
-// bit, for FP64 and for the float-float sum, so a thread may add its
-// partner's value to its own)
-template <int LPB, class T> __device__ __forceinline__ T vl_sum(unsigned m, const T (&a)[VL / LPB]) {
-    if constexpr (LPB == 4) {
-        const T s = vadd(a[0], xlane(m, a[0], 1, 4));
-        return vadd(s, xlane(m, s, 2, 4));
-    } else if constexpr (LPB == 2) {
-        // thread 0 holds v0 and v2, thread 1 v1 and v3
-        return vadd(vadd(a[0], xlane(m, a[0], 1, 2)), vadd(a[1], xlane(m, a[1], 1, 2)));
-    } else {
-        return vadd(vadd(a[0], a[1]), vadd(a[2], a[3]));
-    }
-}
-template <int LPB, class FT> __device__ __forceinline__ Acc3<FT> vl_sum3(unsigned m, const Acc3<FT> (&a)[VL / LPB]) {
-    constexpr int U = VL / LPB;
-    decltype(a[0].x) cx[U], cy[U], cz[U];
-#pragma unroll
-    for (int u = 0; u < U; ++u) { cx[u] = a[u].x; cy[u] = a[u].y; cz[u] = a[u].z; }
-    Acc3<FT> r;
-    r.x = vl_sum<LPB>(m, cx);
-    r.y = vl_sum<LPB>(m, cy);
-    r.z = vl_sum<LPB>(m, cz);
-    return r;
-}
-// sum over the threads of a bead (energies of the evaluation pass)
-template <int LPB> __device__ __forceinline__ double lane_sum(unsigned m, double v) {
-#pragma unroll
-    for (int o = 1; o < LPB; o <<= 1) v += __shfl_xor_sync(m, v, o, LPB);
-    return v;
-}
-// add f to the accumulator of the thread's m-th entry: virtual lane slot
-// m mod (VL / LPB)
-template <int LPB, class FT> __device__ __forceinline__ void acc_slot(Acc3<FT> (&acc)[VL / LPB], int m, V3<FT> f) {
-    if constexpr (LPB == 4) {
-        acc[0].add(f);
-    } else if constexpr (LPB == 2) {
-        if (m & 1) acc[1].add(f);
-        else acc[0].add(f);
-    } else {
-        switch (m & 3) {
-        case 0: acc[0].add(f); break;
-        case 1: acc[1].add(f); break;
-        case 2: acc[2].add(f); break;
-        default: acc[3].add(f); break;
-        }
-    }
-}
-__device__ __forceinline__ double comp3(double4_32a v, int a) { return a == 0 ? v.x : (a == 1 ? v.y : v.z); }
-
-// beads of a step-kernel block of FB bead slots (a block of FB - 3 beads,
-// whose bonded tasks would fill its threads exactly once, measured slower on
-// config 4: at one thread per bead its grid no longer fits one wave)
-template <int FB, int LPB> constexpr int force_beads() { return FB; }
-
-template <class FT, int MODE, int FB, int LPB>
-__device__ __forceinline__ void force_block(const Dev &d, const TermP &p, int cur) {
-    constexpr int NT = FB * LPB;
-    constexpr int FBT = force_beads<FB, LPB>();
-    constexpr int U = VL / LPB;                 // virtual lanes per thread
-    constexpr int AX = (3 + LPB - 1) / LPB;     // integrator axes per thread
-    const double4_32a *__restrict__ pin = d.pos[cur];
-    const int N = d.N, t = threadIdx.x, i0 = blockIdx.x * FBT;
-    const int bs = t / LPB, ln = t % LPB;   // bead slot in the block, thread of the bead
-    const int i = i0 + bs;
-    const unsigned qm = bead_mask<LPB>(t);  // the bead's threads in the warp
-    __shared__ double4_32a P[FBT + 6];
-    __shared__ V3<FT> Ct[FBT + 3], Ca[3][FBT + 3], Cd[4][FBT + 3];
-    // mixed path: every position of the tile split into float-float parts
-    // (integer operations); bond vectors e_k = P[k+1] - P[k] and cross
-    // products x_k = e_{k-1} x e_k formed once per tile slot in float-float
-    // arithmetic (~2^-44 relative, FP64-class where the FP32 forms lose
-    // everything: nearly straight triples) and shared by the tether, angle and
-    // dihedral centres that use them
-    constexpr int NE = sizeof(FT) == 4 ? FBT + 5 : 1;
-    __shared__ P2 S[sizeof(FT) == 4 ? FBT + 6 : 1];
-    __shared__ V3<FF> Eff[NE], Xff[NE];
-    __shared__ V3<float> Ef[NE], Xf[NE];
-    // quasi-adiabatic contact slots of each bead, in ascending order
-    __shared__ int Qs[FBT][QA_REF_CAP];
-
-    // mixed path: the integrator's per-bead state does not depend on the
-    // forces, so its loads are issued first and their latency passes under
-    // the force work (each thread the history of its axes, the last thread
-    // the generator and the list origin); the FP64 path is bound by its FP64
-    // pipe instead and loads them where they are used
-    constexpr bool EARLY = MODE == 1 && sizeof(FT) == 4;
-    const bool live = bs < FBT && i < N;
-    double yv[5 * AX];
-    uint64_t st0 = 0;
-    double4_32a o_i = make_double4_32a(0, 0, 0, 0);
-    int pf_n0 = 0, pf_n1 = 0, pf_cnt = 0;   // the pair loops' bounds, loaded first too
-    if (live) {
-        pf_n0 = d.nat_start[i];
-        pf_n1 = d.nat_end[i];
-        pf_cnt = d.nl_cnt[i];
-    }
-    const size_t Ns = (size_t)N;
-    if (EARLY && live) {
-#pragma unroll
-        for (int u = 0; u < AX; ++u) {
-            const int a = ln + LPB * u;
-            if (a < 3) {
-#pragma unroll
-                for (int q = 0; q < 5; ++q) yv[q * AX + u] = d.yh[(size_t)(q * 3 + a) * Ns + i];
-            }
-        }
-        if (ln == LPB - 1) {
-            st0 = d.rng[i];
-            o_i = d.orig[i];
-        }
-    }
-
-    for (int k = t; k < FBT + 6; k += NT) {
-        int idx = i0 - 3 + k;
-        P[k] = (idx >= 0 && idx < N) ? pin[idx] : make_double4_32a(0, 0, 0, 0);
-        if constexpr (sizeof(FT) == 4) S[k] = split_p(P[k]);
-    }
-    __syncthreads();
-    if constexpr (sizeof(FT) == 4) {
-        for (int k = t; k < NE; k += NT) {
-            const V3<FF> e{ff_diff(S[k].x, S[k + 1].x), ff_diff(S[k].y, S[k + 1].y), ff_diff(S[k].z, S[k + 1].z)};
-            Eff[k] = e;
-            Ef[k] = V3<float>{e.x.h, e.y.h, e.z.h};
-        }
-        __syncthreads();
-        for (int k = t + 1; k < NE; k += NT) {
-            const V3<FF> x = ff_cross(Eff[k - 1], Eff[k]);
-            Xff[k] = x;
-            Xf[k] = V3<float>{x.x.h, x.y.h, x.z.h};
-        }
-        __syncthreads();
-    }
-
-    // bonded contributions of centres c in [i0-2, i0+FBT].  A centre is two
-    // tasks, (tether, angle) and (dihedral, chirality).  With one thread per
-    // bead a thread takes both tasks of its centres; with more, the tasks are
-    // dealt so that the 32 threads of a warp take one task of 32 consecutive
-    // centres (no divergence between the two).
-    constexpr int NC = FBT + 3, NC32 = (NC + 31) / 32 * 32;
-    constexpr int NW = LPB == 1 ? NC : 2 * NC32;
-    auto bonded = [&](const int sc, const int task) {
-        const int c = i0 - 2 + sc;
-        const uint32_t fl = (c >= 0 && c < N) ? d.bflags[c] : 0u;
-        const V3<FT> z{FT(0), FT(0), FT(0)};
-        const int sp = c - (i0 - 3);
-        const bool own = (c >= i0 && c < i0 + FBT && c < N);
-        const int rc = own ? d.rep_of[c] : 0;
-        // a centre's angle and dihedral are native or heuristic (seq-file
-        // models: those without a native value); both kinds share one call
-        if (task == 0) {
-            V3<FT> ft = z, a1 = z, a2 = z, a3 = z;
-            if ((fl & BF_TETH) && p.on[XMD_TERM_TETHER]) {
-                FT V_;
-                if constexpr (sizeof(FT) == 4) ft = tether_vec(p, Ef[sp], d.bond_f[c].x, &V_);
-                else {
-                    DN Vn;
-                    ft = v3d(tether_term<DN>(p, P[sp], P[sp + 1], DN(d.teth_r0[c]), &Vn));
-                    V_ = (double)Vn;
-                }
-                if (MODE == 0 && own) atomicAdd(&d.Vrep[rc * XMD_NUM_TERMS + XMD_TERM_TETHER], (double)V_);
-            }
-            const bool h_ang = (fl & BF_HANG) && p.on[XMD_TERM_HEUR_ANG];
-            const bool do_ang = ((fl & BF_ANG) && p.on[XMD_TERM_NAT_ANG]) || h_ang;
-            const double *hac = h_ang ? d.heur_ang + 7 * ((fl >> BF_HANG_SHIFT) & 15u) : nullptr;
-            const int ang_slot = h_ang ? XMD_TERM_HEUR_ANG : XMD_TERM_NAT_ANG;
-            if (do_ang) {
-                double V_;
-                if constexpr (sizeof(FT) == 8) {
-                    // every operation rounded on its own (DN), as the
-                    // reference's uncontracted build: near-straight triples
-                    // make the bonded terms ill-conditioned
-                    V3<DN> b1, b2, b3;
-                    DN Vn;
-                    angle_term<DN>(p, P[sp - 1], P[sp], P[sp + 1], DN(d.ang_t0[c]), hac, &b1, &b2, &b3, &Vn);
-                    a1 = v3d(b1); a2 = v3d(b2); a3 = v3d(b3);
-                    V_ = (double)Vn;
-                } else {
-                    // mixed path: float-float bond vectors and cross products
-                    // (shared slots), FP32 forces
-                    float Vf;
-                    angle_mixed(p, Ef[sp - 1], Ef[sp], Xf[sp], d.bond_f[c].y, hac, &a1, &a2, &a3, &Vf);
-                    V_ = (double)Vf;
-                }
-                if (MODE == 0 && own) atomicAdd(&d.Vrep[rc * XMD_NUM_TERMS + ang_slot], V_);
-            }
-            Ct[sc] = ft;
-            Ca[0][sc] = a1; Ca[1][sc] = a2; Ca[2][sc] = a3;
-        } else {
-            V3<FT> q[4] = {z, z, z, z};
-            const bool h_dih = (fl & BF_HDIH) && p.on[XMD_TERM_HEUR_DIH];
-            const bool do_dih = ((fl & BF_DIH) && (p.on[XMD_TERM_CND] || p.on[XMD_TERM_SND])) || h_dih;
-            const int hdt = (int)((fl >> BF_HDIH_SHIFT) & 15u);
-            if (do_dih) {
-                double Vc, Vs;
-                if constexpr (sizeof(FT) == 8) {
-                    V3<DN> qn[4];
-                    DN Vcn, Vsn;
-                    dihedral_term<DN>(p, P[sp - 1], P[sp], P[sp + 1], P[sp + 2], DN(d.dih_p0[c]),
-                                      p.on[XMD_TERM_CND] != 0, p.on[XMD_TERM_SND] != 0,
-                                      h_dih ? reinterpret_cast<const DN *>(d.heur_dih) + 6 * hdt : nullptr, qn,
-                                      &Vcn, &Vsn);
-#pragma unroll
-                    for (int k = 0; k < 4; ++k) q[k] = v3d(qn[k]);
-                    Vc = (double)Vcn;
-                    Vs = (double)Vsn;
-                } else {
-                    float Vcf, Vsf;
-                    const float X = dot(Xf[sp], Xf[sp + 1]), T = ff_dot(Xff[sp], Eff[sp + 1]).h;
-                    dihedral_mixed(p, Ef[sp - 1], Ef[sp], Ef[sp + 1], Xf[sp], Xf[sp + 1], X, T, d.bond_f[c].z,
-                                   p.on[XMD_TERM_CND] != 0, p.on[XMD_TERM_SND] != 0,
-                                   h_dih ? d.heur_dih_f + 6 * hdt : nullptr, q, &Vcf, &Vsf);
-                    Vc = (double)Vcf;
-                    Vs = (double)Vsf;
-                }
-                if (MODE == 0 && own) {
-                    if (h_dih) atomicAdd(&d.Vrep[rc * XMD_NUM_TERMS + XMD_TERM_HEUR_DIH], Vc);
-                    else {
-                        if (p.on[XMD_TERM_CND]) atomicAdd(&d.Vrep[rc * XMD_NUM_TERMS + XMD_TERM_CND], Vc);
-                        if (p.on[XMD_TERM_SND]) atomicAdd(&d.Vrep[rc * XMD_NUM_TERMS + XMD_TERM_SND], Vs);
-                    }
-                }
-            }
-            // chirality of the quad (c-1, c, c+1, c+2): eval_chiral_forces::iter,
-            // chiral.cpp:15-37; its forces join the dihedral slots of the centre
-            if ((fl & BF_CHIR) && p.on[XMD_TERM_CHIR]) {
-                V3<FT> g[4];
-                double Vch;
-                if constexpr (sizeof(FT) == 8) {
-                    const double2 cp = d.chir[c];
-                    V3<DN> gn[4];
-                    DN Vn;
-                    chiral_term<DN>(p, P[sp - 1], P[sp], P[sp + 1], P[sp + 2], DN(cp.x), DN(cp.y), gn, &Vn);
-#pragma unroll
-                    for (int k = 0; k < 4; ++k) g[k] = v3d(gn[k]);
-                    Vch = (double)Vn;
-                } else {
-                    const float2 cp = d.chir_f32[c];
-                    // the triple product in float-float: planar quads are well conditioned
-                    const float tp = ff_dot(Eff[sp - 1], Xff[sp + 1]).h;
-                    float Vf;
-                    chiral_mixed(p, Ef[sp - 1], Ef[sp], Ef[sp + 1], Xf[sp], Xf[sp + 1], tp, cp.x, cp.y, g, &Vf);
-                    Vch = (double)Vf;
-                }
-#pragma unroll
-                for (int k = 0; k < 4; ++k) q[k] = q[k] + g[k];
-                if (MODE == 0 && own) atomicAdd(&d.Vrep[rc * XMD_NUM_TERMS + XMD_TERM_CHIR], Vch);
-            }
-            Cd[0][sc] = q[0]; Cd[1][sc] = q[1]; Cd[2][sc] = q[2]; Cd[3][sc] = q[3];
-        }
-    };
-    for (int w = t; w < NW; w += NT) {
-        if constexpr (LPB == 1) {
-            bonded(w, 0);
-            bonded(w, 1);
-        } else {
-            const int sc = ((w >> 6) << 5) | (w & 31);
-            if (sc < NC) bonded(sc, (w >> 5) & 1);
-        }
-    }
-    __syncthreads();
-
-    // from here on, the threads of a bead take the same branches
-    if (!live) return;
-    const int r = d.rep_of[i];
-    if (r < 0) return;     // free bead slot
-    if (MODE == 1 && d.rep[r].steps_left == 0) {
-        // the replica has taken its steps: it keeps its state (both buffers)
-        if (ln == LPB - 1) d.pos[cur ^ 1][i] = P[bs + 3];
-        return;
-    }
-    const int s = bs + 2;   // centre slot of bead i
-    // the partial forces of this thread's virtual lanes; virtual lane 0
-    // (thread 0, slot 0) starts from the bonded sum
-    Acc3<FT> acc[U];
-    if (ln == 0) {
-        Acc3<FT> &a0 = acc[0];
-        if constexpr (sizeof(FT) == 4) {
-            // the bonded contributions, computed in FP32, are summed in FP32
-            // and enter the float-float accumulator once
-            V3<float> bsum = Ct[s] - Ct[s - 1] + Ca[2][s - 1] + Ca[1][s] + Ca[0][s + 1] + Cd[0][s + 1] +
-                             Cd[1][s] + Cd[2][s - 1] + Cd[3][s - 2];
-            a0.add(bsum);
-        } else {
-            a0.add(Ct[s]);
-            a0.sub(Ct[s - 1]);
-            a0.add(Ca[2][s - 1]);
-            a0.add(Ca[1][s]);
-            a0.add(Ca[0][s + 1]);
-            a0.add(Cd[0][s + 1]);
-            a0.add(Cd[1][s]);
-            a0.add(Cd[2][s - 1]);
-            a0.add(Cd[3][s - 2]);
-        }
-    }
-
-    const double4_32a pi = P[bs + 3];
-    const BoxD bx = d.rep[r].box;
-    const bool per = (d.rep[r].per[0] | d.rep[r].per[1] | d.rep[r].per[2]) != 0;
-    const PairGeo<FT> geo(bx, per, pi);
-    double vgo = 0, vpa = 0, ves = 0;
-
-    // Thread ln takes entries k0 + ln, k0 + ln + LPB, ... of each list; its
-    // m-th entry goes to its virtual lane slot m mod U (the same slot on every
-    // active thread of the warp, so the slot switch does not diverge).  Each
-    // loop body appears once in the code; the loops are software-pipelined
-    // (the next entry's index data is loaded while this entry's partner is
-    // fetched).
-    if (p.on[XMD_TERM_GO]) {
-        const int k1 = pf_n1;
-        int k = pf_n0 + ln, m = 0;
-        int j = 0;
-        bool on = false;
-        FT nd = FT(0);
-        if (k < k1) {
-            j = d.nat_j[k];
-            on = d.nat_on[k] != 0;
-            nd = nat_dist<FT>(d, k);
-        }
-        for (; k < k1; k += LPB, ++m) {
-            int jn = 0;
-            bool onn = false;
-            FT ndn = FT(0);
-            if (k + LPB < k1) {
-                jn = d.nat_j[k + LPB];
-                onn = d.nat_on[k + LPB] != 0;
-                ndn = nat_dist<FT>(d, k + LPB);
-            }
-            if (on) {
-                FT V_;
-                const V3<FT> f = go_pair<FT>(p, geo.to(pin[j]), nd, &V_);
-                acc_slot<LPB>(acc, m, f);
-                if (MODE == 0 && i < j) vgo += (double)V_;
-            }
-            j = jn;
-            on = onn;
-            nd = ndn;
-        }
-    }
-    double vss = 0;
-    if (p.on[XMD_TERM_NAT_SS]) {
-        const int s1 = d.ss_end[i];
-        int m = 0;
-        for (int k = d.ss_start[i] + ln; k < s1; k += LPB, ++m) {
-            if (!d.ss_on[k]) continue;
-            const int j = d.ss_j[k];
-            FT V_;
-            const V3<FT> f = ss_pair<FT>(p, geo.to(pin[j]), &V_);
-            acc_slot<LPB>(acc, m, f);
-            if (MODE == 0 && i < j) vss += (double)V_;
-        }
-    }
-    {
-        const int cnt = pf_cnt;
-        int e_next = ln < cnt ? d.nl_row[(size_t)ln * N + i] : 0;
-        int m = 0;
-        for (int k = ln; k < cnt; k += LPB, ++m) {
-            const int e = e_next;
-            if (k + LPB < cnt) e_next = d.nl_row[(size_t)(k + LPB) * N + i];
-            const int j = e & NL_MASK;
-            const double4_32a pj = pin[j];
-            const V3<FT> r12 = geo.to(pj);
-            V3<FT> f{FT(0), FT(0), FT(0)};
-            bool any = false;
-            if (e & NL_PAULI) {
-                FT V_;
-                f = pauli_pair<FT>(p, r12, &V_);
-                any = true;
-                if (MODE == 0 && i < j) vpa += (double)V_;
-            }
-            if (e & NL_ES) {
-                FT V_;
-                const V3<FT> g = es_pair<FT>(p, r12, charge_prod<FT>(pi.w, pj.w), &V_);
-                // a pair on both lists adds its two forces one after the other
-                if (any) acc_slot<LPB>(acc, m, f);
-                f = g;
-                any = true;
-                if (MODE == 0 && i < j) ves += (double)V_;
-            }
-            if (any) acc_slot<LPB>(acc, m, f);
-        }
-    }
-
-    // quasi-adiabatic contacts: the force part of process_contacts::iter
-    // (process_contacts.cpp:25-40).  The bead's contact slots (at most
-    // QA_REF_CAP, held QA_REF_CAP / LPB per thread) are put in ascending order
-    // by rank and dealt to the virtual lanes like a list.
-    double vqa = 0;
-    if (d.qa_on && p.on[XMD_TERM_QA]) {
-        const QaDev &q = d.qa;
-        const int nref = min(q.ref_cnt[i], QA_REF_CAP);
-        constexpr int HOLD = QA_REF_CAP / LPB;
-        int v[HOLD], rk[HOLD];
-#pragma unroll
-        for (int u = 0; u < HOLD; ++u) {
-            const int k = u * LPB + ln;
-            v[u] = k < nref ? q.ref[(size_t)k * N + i] : INT_MAX;
-            rk[u] = 0;
-        }
-        for (int m = 0; m < nref; ++m) {
-            int x = 0;
-#pragma unroll
-            for (int u = 0; u < HOLD; ++u) {
-                const int y = __shfl_sync(qm, v[u], m % LPB, LPB);
-                if (m / LPB == u) x = y;
-            }
-#pragma unroll
-            for (int u = 0; u < HOLD; ++u) rk[u] += x < v[u];
-        }
-#pragma unroll
-        for (int u = 0; u < HOLD; ++u)
-            if (u * LPB + ln < nref) Qs[bs][rk[u]] = v[u];
-        __syncwarp(qm);
-        const double tnow = d.rep[r].t;
-        int m = 0;
-        for (int k = ln; k < nref; k += LPB, ++m) {
-            const int slot = Qs[bs][k];
-            int i1 = q.ct_i1[slot], i2 = q.ct_i2[slot];
-            V3<FT> r12 = geo.between(pin[i1], pin[i2]);
-            FT r12_rn = ninv(r12);
-            V3<FT> u = r12_rn * r12;
-            double sat = fmin(tnow - q.ct_ref[slot], p.qa_cycle) * p.qa_cycle_inv;
-            if (q.ct_status[slot] == QA_BREAKING) sat = 1.0 - sat;
-            double depth, rmin, rmax;
-            qa_lj(p, q, q.ct_type[slot], &depth, &rmin, &rmax);
-            FT V_, dV_;
-            sink_lj_eval<FT>((FT)depth, (FT)rmin, (FT)rmax, r12_rn * nsq(r12), r12_rn, &V_, &dV_);
-            V3<FT> f = ((FT)sat * dV_) * u;
-            acc_slot<LPB>(acc, m, i == i1 ? f : -f);
-            if (MODE == 0 && i == i1) vqa += sat * (double)V_;
-        }
-        if (MODE == 1 && ln == LPB - 1) {
-            // n and h at this step's positions (precompute_nh.cpp:12-20) to
-            // FP32 accuracy, for the sift's FP32 decisions (which recompute
-            // them in FP64 near a threshold)
-            V3<float> n{0.0f, 0.0f, 0.0f}, h{0.0f, 0.0f, 0.0f};
-            const uint32_t fl = d.bflags[i];
-            if ((fl & BF_PREV) && (fl & BF_NEXT)) qa_nh_f(P[bs + 2], P[bs + 3], P[bs + 4], &n, &h);
-            q.nh[i] = n.x; q.nh[Ns + i] = n.y; q.nh[2 * Ns + i] = n.z;
-            q.nh[3 * Ns + i] = h.x; q.nh[4 * Ns + i] = h.y; q.nh[5 * Ns + i] = h.z;
-        }
-    }
-
-    // the bead's force: its virtual lanes' partial sums combined (every
-    // thread of the bead holds it)
-    V3<double> ftot = vl_sum3<LPB>(qm, acc).total();
-    if (p.ext_on) {
-        // AFM pulls and walls, from k_ext (launched just before)
-        ftot = ftot + V3<double>{d.fext[3 * (size_t)i], d.fext[3 * (size_t)i + 1], d.fext[3 * (size_t)i + 2]};
-    }
-    if (p.on[XMD_TERM_PID]) {
-        // pseudo-improper dihedral bundles, from k_pid: the bead's own side,
-        // then the parts its chain neighbours' bundles put on it
-        const double *pf = d.pid_f;
-        const uint32_t fl = d.bflags[i];
-        V3<double> g{pf[3 * (size_t)i], pf[3 * (size_t)i + 1], pf[3 * (size_t)i + 2]};
-        if (fl & BF_PREV) {
-            const double *q = pf + 6 * Ns + 3 * (size_t)(i - 1);   // next-bead part of i - 1
-            g = g + V3<double>{q[0], q[1], q[2]};
-        }
-        if (fl & BF_NEXT) {
-            const double *q = pf + 3 * Ns + 3 * (size_t)(i + 1);   // previous-bead part of i + 1
-            g = g + V3<double>{q[0], q[1], q[2]};
-        }
-        ftot = ftot + g;
-    }
-    const double fx = ftot.x, fy = ftot.y, fz = ftot.z;
-    if (!(finite_bits(fx) && finite_bits(fy) && finite_bits(fz))) {
-        // the replica is frozen from the next step on (its skin check sets
-        // steps_left = 0); this bead keeps its state, so no non-finite
-        // position ever reaches a list build
-        if (ln == 0) atomicOr(d.status, ST_NONFINITE);
-        if (MODE == 1) {
-            if (ln == LPB - 1) {
-                d.rep[r].fault = 1;
-                d.pos[cur ^ 1][i] = pi;
-            }
-            return;
-        }
-    }
-
-    if (MODE == 0) {
-#pragma unroll
-        for (int u = 0; u < AX; ++u) {
-            const int a = ln + LPB * u;
-            if (a < 3) d.F[3 * (size_t)i + a] = a == 0 ? fx : (a == 1 ? fy : fz);
-        }
-        vgo = lane_sum<LPB>(qm, vgo);
-        vpa = lane_sum<LPB>(qm, vpa);
-        ves = lane_sum<LPB>(qm, ves);
-        vqa = lane_sum<LPB>(qm, vqa);
-        vss = lane_sum<LPB>(qm, vss);
-        if (ln == 0) {
-            double *Vr = d.Vrep + r * XMD_NUM_TERMS;
-            if (vgo != 0.0) atomicAdd(&Vr[XMD_TERM_GO], vgo);
-            if (vpa != 0.0) atomicAdd(&Vr[XMD_TERM_PAULI], vpa);
-            if (ves != 0.0) atomicAdd(&Vr[p.es_rel ? XMD_TERM_REL_ES : XMD_TERM_CONST_ES], ves);
-            if (vqa != 0.0) atomicAdd(&Vr[XMD_TERM_QA], vqa);
-            if (vss != 0.0) atomicAdd(&Vr[XMD_TERM_NAT_SS], vss);
-        }
-        return;
-    }
-
-    // ---- lang_pc_step::operator(), lang_pc.cpp:11-37, mass = 1 (main.cpp:156) ----
-    // the last thread of the bead: its four generator draws, three normals
-    double nz0 = 0.0, nz1 = 0.0, nz2 = 0.0;
-    if (ln == LPB - 1) {
-        if (!EARLY) {
-            st0 = d.rng[i];
-            o_i = d.orig[i];
-        }
-        uint64_t st = st0;
-        if constexpr (sizeof(FT) == 8) {
-            noise3(st, &nz0, &nz1, &nz2);
-        } else {
-            float a, b, c;
-            noise3m(st, &a, &b, &c);
-            nz0 = widen_f(a);
-            nz1 = widen_f(b);
-            nz2 = widen_f(c);
-        }
-        d.rng[i] = gf2_apply_nib(d.jump + JUMP_WORDS * r, st);
-    }
-    if constexpr (LPB > 1) {
-        nz0 = __shfl_sync(qm, nz0, LPB - 1, LPB);
-        nz1 = __shfl_sync(qm, nz1, LPB - 1, LPB);
-        nz2 = __shfl_sync(qm, nz2, LPB - 1, LPB);
-    }
-    // the Gear-5 corrector and predictor of the thread's axes
-    double y0a[AX];
-#pragma unroll
-    for (int u = 0; u < AX; ++u) {
-        const int a = ln + LPB * u;
-        y0a[u] = 0.0;
-        if (a >= 3) continue;
-        const double dt_inv = p.dt_inv, h = p.dt2_half;
-        const double gamma = p.gamma_factor * 1.0;
-        const double nsd = d.rep[r].noise_sd;
-        const double Fa = a == 0 ? fx : (a == 1 ? fy : fz);
-        const double nza = a == 0 ? nz0 : (a == 1 ? nz1 : nz2);
-        double *yh = d.yh;
-        double y0 = comp3(pi, a);
-        double y1, y2, y3, y4, y5;
-        if constexpr (EARLY) {
-            y1 = yv[0 * AX + u]; y2 = yv[1 * AX + u]; y3 = yv[2 * AX + u]; y4 = yv[3 * AX + u];
-            y5 = yv[4 * AX + u];
-        } else {
-            y1 = yh[(size_t)(0 * 3 + a) * Ns + i]; y2 = yh[(size_t)(1 * 3 + a) * Ns + i];
-            y3 = yh[(size_t)(2 * 3 + a) * Ns + i]; y4 = yh[(size_t)(3 * 3 + a) * Ns + i];
-            y5 = yh[(size_t)(4 * 3 + a) * Ns + i];
-        }
-        double v = y1 * dt_inv;
-        double a_ = Fa * 1.0 - gamma * v + nsd * nza;
-        double error = y2 - a_ * h;
-        y0 -= 3.0 / 16.0 * error;
-        y1 -= 251.0 / 360.0 * error;
-        y2 -= 1.0 * error;
-        y3 -= 11.0 / 18.0 * error;
-        y4 -= 1.0 / 6.0 * error;
-        y5 -= 1.0 / 60.0 * error;
-        y0 += y1 + y2 + y3 + y4 + y5;
-        y1 += 2.0 * y2 + 3.0 * y3 + 4.0 * y4 + 5.0 * y5;
-        y2 += 3.0 * y3 + 6.0 * y4 + 10.0 * y5;
-        y3 += 4.0 * y4 + 10.0 * y5;
-        y4 += 5.0 * y5;
-        yh[(size_t)(0 * 3 + a) * Ns + i] = y1;
-        yh[(size_t)(1 * 3 + a) * Ns + i] = y2;
-        yh[(size_t)(2 * 3 + a) * Ns + i] = y3;
-        yh[(size_t)(3 * 3 + a) * Ns + i] = y4;
-        yh[(size_t)(4 * 3 + a) * Ns + i] = y5;
-        y0a[u] = y0;
-    }
-    // the last thread: the new position (axis a from thread a mod LPB) and
-    // the skin-test displacement
-    const double px = __shfl_sync(qm, y0a[0 / LPB], 0 % LPB, LPB);
-    const double py = __shfl_sync(qm, y0a[1 / LPB], 1 % LPB, LPB);
-    const double pz = __shfl_sync(qm, y0a[2 / LPB], 2 % LPB, LPB);
-    double disp = 0.0;
-    if (ln == LPB - 1) {
-        const double4_32a pn = make_double4_32a(px, py, pz, pi.w);
-        d.pos[cur ^ 1][i] = pn;
-        // skin test displacement: norm(box->r_uv(r_, orig_r_)), verify.cpp:12-14
-        // squared; the check takes one square root of the maximum (sqrt is
-        // monotone and correctly rounded, so that equals the max of the norms)
-        if constexpr (sizeof(FT) == 4) {
-            // mixed path: the displacement from split positions (the FP64
-            // difference to FP32 accuracy), squared in FP32
-            const V3<float> e = geo.between(o_i, pn);
-            disp = widen_f(e.x * e.x + e.y * e.y + e.z * e.z);
-        } else {
-            // on open axes the wrap subtracts exactly zero: skipping it changes no bit
-            disp = per ? dist2_exact(bx, pn, o_i) : dist2_open(pn, o_i);
-        }
-    }
-    const unsigned lane = t & 31;
-    int r0 = __shfl_sync(0xffffffffu & __activemask(), r, 0);
-    unsigned mask = __activemask();
-    if (__all_sync(mask, r == r0) && mask == 0xffffffffu) {
-        const unsigned long long m = warp_max_bits((unsigned long long)__double_as_longlong(disp));
-        if (lane == 0) atomicMax(&d.rep[r].maxdisp, m);
-    } else if (ln == LPB - 1) {
-        atomicMax(&d.rep[r].maxdisp, (unsigned long long)__double_as_longlong(disp));
-    }
+// FP64 positions as float-float parts (mixed path).  The step kernel keeps
+// them up to date; the host may have placed, restored or uploaded positions
+// since, so every call that steps or evaluates starts with this pass (32 B
+// read, 32 B written per bead).
+__global__ void __launch_bounds__(256) k_split(Dev d, int cur) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= d.N) return;
+    const double4_32a q = d.pos[cur][i];
+    const P2 s = split_p(q);
+    d.spl[cur][2 * (size_t)i] = make_float4(s.x.h, s.y.h, s.z.h, narrow_f(q.w));
+    d.spl[cur][2 * (size_t)i + 1] = make_float4(s.x.l, s.y.l, s.z.l, 0.0f);
 }
 
 // ---- skin decision (nl::verify, verify.cpp:4-23) --------------------------------
@@ -1113,23 +486,21 @@ __global__ void __launch_bounds__(1024) k_qa_refree(Dev d, double dt, int check)
 // resident blocks the register allocation leaves room for: 16 warps per SM
 // (at most 128 registers) with one or two threads per bead, 28 (at most 73)
 // with four
-template <int FB, int LPB> constexpr int force_min_blocks() {
-    return LPB == 4 ? (896 / (FB * 4) > 0 ? 896 / (FB * 4) : 1) : 512 / (FB * LPB);
+template <class FT, int FB, int LPB> constexpr int force_min_blocks() {
+    return 65536 / (FB * LPB * (sizeof(FT) == 4 ? 64 : 80)) > 0 ? 65536 / (FB * LPB * (sizeof(FT) == 4 ? 64 : 80)) : 1;
 }
 enum : int { FUSE_NONE = 0, FUSE_CHECK = 1, FUSE_CHECK_GATE = 2, FUSE_GATE = 3 };
 template <class FT, int MODE, int FB, int LPB>
-__global__ void __launch_bounds__(FB * LPB, (force_min_blocks<FB, LPB>())) k_force(Dev d, TermP p, int cur,
+__global__ void __launch_bounds__(FB * LPB, (force_min_blocks<FT, FB, LPB>())) k_force(Dev d, TermP p, int cur,
                                                                                   int fuse) {
     __shared__ int last_s;
     static_assert(LPB == 1 || LPB == 2 || LPB == 4, "one, two or four threads per bead");
-    // uniform: the gate changes between launches
-    if (MODE == 1 && (fuse == FUSE_CHECK_GATE || fuse == FUSE_GATE) && d.gate[0]) return;
-    constexpr int FBT = force_beads<FB, LPB>();
-    // the block runs when an occupancy granule of its beads is on (uniform)
-    const int i0 = blockIdx.x * FBT, i1 = min(i0 + FBT, d.N) - 1;
-    bool on = false;
-    for (int g = i0 / BLK_ON; g <= i1 / BLK_ON; ++g) on |= d.blk_on[g] != 0;
-    if (on) force_block<FT, MODE, FB, LPB>(d, p, cur);
+    constexpr int FBT = step_beads<FB>();
+    const int i = blockIdx.x * FBT + threadIdx.x;
+    const int closed = MODE == 1 && (fuse == FUSE_CHECK_GATE || fuse == FUSE_GATE) ? d.gate[0] : 0;
+    const int r = threadIdx.x < FBT && i < d.N ? d.rep_of[i] : -1;   // on its way with the gate
+    if (closed) return;   // uniform: the gate changes between launches
+    force_block<FT, MODE, FB, LPB>(d, p, cur, r);
     if (MODE == 1 && (fuse == FUSE_CHECK || fuse == FUSE_CHECK_GATE)) {
         __syncthreads();
         if (threadIdx.x == 0) {
@@ -1417,6 +788,46 @@ __global__ void __launch_bounds__(CF_WARPS * 32) k_cell_finish(Dev d, int cur) {
 // offset (first occurrence of each key).  Quasi-adiabatic partners are ranked
 // by j within the warp at the end, so the free-pair source list is ordered as
 // update_free_pairs (free_pair.cpp:9-19) walks it.
+// Go-list membership of a native contact of length nd (r < T = 2 nd + pad,
+// go.cpp:11-22): by the FP32 squared distance d2 outside a band around T
+// (directed rounding, widened by the narrowing error of T and by mf, the
+// error bound of the FP32 distance), by the reference's test inside it
+__device__ __forceinline__ bool go_listed(const RepDev &rp, const BoxD &bx, float mf, double nd, float d2,
+                                          double4_32a pi, const double4_32a &pj) {
+    const double T = __dadd_rn(__dmul_rn(2.0, nd), rp.pad);
+    const float Tf = narrow_f(T);
+    const float mm = __fmaf_ru(Tf, 1.2e-7f, mf);
+    const float blo = __fsub_rd(Tf, mm), bhi = __fadd_ru(Tf, mm);
+    const Band B{blo > 0.0f ? __fmul_rd(blo, blo) : -1.0f, __fmul_ru(bhi, bhi)};
+    if (in_band(B, d2)) return dist_exact(bx, pi, pj) < T;
+    return d2 < B.lo;
+}
+// entry k of the natives [n0, n1) of the warp's bead: its list flag, and its
+// place in the bead's Go list, which keeps the order of the natives
+__device__ __forceinline__ void go_append(const Dev &d, int k, int n0, int n1, bool on, int j, double nd, int &ngo) {
+    const unsigned m = __ballot_sync(0xffffffffu, on);
+    if (k < n1) d.nat_on[k] = on;
+    if (on) {
+        const int at = n0 + ngo + __popc(m & ((1u << (threadIdx.x & 31)) - 1u));
+        d.act_j[at] = j;
+        d.act_d[at] = nd;
+    }
+    ngo += __popc(m);
+}
+// the Go list of beads [b, b + n) from the list flags (after a restore)
+__global__ void k_go_lists(Dev d, int b, int n) {
+    const int i = b + blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= b + n) return;
+    const int n0 = d.nat_start[i], n1 = d.nat_end[i];
+    int at = n0;
+    for (int k = n0; k < n1; ++k)
+        if (d.nat_on[k]) {
+            d.act_j[at] = d.nat_j[k];
+            d.act_d[at++] = d.nat_d[k];
+        }
+    d.go_cnt[i] = at - n0;
+}
+
 constexpr int NC_WARPS = 8;
 __global__ void __launch_bounds__(NC_WARPS * 32, 4) k_nl_cells(Dev d, TermP p, int cur) {
     const int lane = threadIdx.x & 31;
@@ -1436,19 +847,22 @@ __global__ void __launch_bounds__(NC_WARPS * 32, 4) k_nl_cells(Dev d, TermP p, i
     const float mf = rp.band_mf;
 
     // Go list: update_go_contacts, go.cpp:11-22 (lanes over the natives)
-    for (int k = n0 + lane; k < n1; k += 32) {
-        const double4_32a pj = pos[d.nat_j[k]];
-        const V3<float> e = geo.to(pj);
-        const float d2 = e.x * e.x + e.y * e.y + e.z * e.z;
-        // band around T = 2 r_nat + pad, as in the tile build (split
-        // differences carry <= 1 ulp, inside the margin)
-        const double T = d.nat_T[k];
-        const float Tf = narrow_f(T);
-        const float mm = __fmaf_ru(Tf, 1.2e-7f, mf);
-        const float blo = __fsub_rd(Tf, mm), bhi = __fadd_ru(Tf, mm);
-        const Band B{blo > 0.0f ? __fmul_rd(blo, blo) : -1.0f, __fmul_ru(bhi, bhi)};
-        d.nat_on[k] = in_band(B, d2) ? dist2_exact(bx, pi, pj) < d.nat_S[k] : d2 < B.lo;
+    int ngo = 0;
+    for (int k0 = n0; k0 < n1; k0 += 32) {
+        const int k = k0 + lane;
+        bool on = false;
+        int j = 0;
+        double nd = 0.0;
+        if (k < n1) {
+            j = d.nat_j[k];
+            nd = d.nat_d[k];
+            const double4_32a pj = pos[j];
+            const V3<float> e = geo.to(pj);
+            on = go_listed(rp, bx, mf, nd, e.x * e.x + e.y * e.y + e.z * e.z, pi, pj);
+        }
+        go_append(d, k, n0, n1, on, j, nd, ngo);
     }
+    if (lane == 0) d.go_cnt[i] = ngo;
 
     // neighbouring buckets: lane l < 27 takes offsets (l/9, l/3 % 3, l % 3) - 1
     int key = -1;
@@ -1799,29 +1213,27 @@ __device__ __forceinline__ void tl_chunk(const Dev &d, const TermP &p, int cur, 
         const bool pid_on = pid_term && (d.bflags[i] & (BF_PREV | BF_NEXT)) == (BF_PREV | BF_NEXT);
 
         // Go list: update_go_contacts, go.cpp:11-22
-        for (int k = n0 + lane; k < n1; k += 32) {
-            const int j = d.nat_j[k];
-            const float4 qj = sq[j - b];
-            float dx = qj.x - qi.x, dy = qj.y - qi.y, dz = qj.z - qi.z;
-            if (periodic) {
-                dx = min_image_f(dx, Lx);
-                dy = min_image_f(dy, Ly);
-                dz = min_image_f(dz, Lz);
+        int ngo = 0;
+        for (int k0 = n0; k0 < n1; k0 += 32) {
+            const int k = k0 + lane;
+            bool on = false;
+            int j = 0;
+            double nd = 0.0;
+            if (k < n1) {
+                j = d.nat_j[k];
+                nd = d.nat_d[k];
+                const float4 qj = sq[j - b];
+                float dx = qj.x - qi.x, dy = qj.y - qi.y, dz = qj.z - qi.z;
+                if (periodic) {
+                    dx = min_image_f(dx, Lx);
+                    dy = min_image_f(dy, Ly);
+                    dz = min_image_f(dz, Lz);
+                }
+                on = go_listed(rp, bx, mf, nd, dx * dx + dy * dy + dz * dz, pi, pos[j]);
             }
-            const float d2 = dx * dx + dy * dy + dz * dz;
-            // band around T = 2 r_nat + pad in FP32 with directed rounding,
-            // widened by the narrowing error of T: at least as wide as the
-            // FP64-formed band, so the exact test decides the same pairs
-            const double T = d.nat_T[k];
-            const float Tf = narrow_f(T);
-            const float mm = __fmaf_ru(Tf, 1.2e-7f, mf);
-            const float blo = __fsub_rd(Tf, mm), bhi = __fadd_ru(Tf, mm);
-            const Band B{blo > 0.0f ? __fmul_rd(blo, blo) : -1.0f, __fmul_ru(bhi, bhi)};
-            bool on;
-            if (in_band(B, d2)) on = dist2_exact(bx, pi, pos[j]) < d.nat_S[k];
-            else on = d2 < B.lo;
-            d.nat_on[k] = on;
+            go_append(d, k, n0, n1, on, j, nd, ngo);
         }
+        if (lane == 0) d.go_cnt[i] = ngo;
 
         // disulfide list: update_nat_ssbonds, native_ss.cpp:8-19 (exact test;
         // a bead has at most a few disulfides)
@@ -1970,7 +1382,12 @@ __global__ void __launch_bounds__(TL_THREADS, 4) k_nl_tile(Dev d, TermP p, int c
 // threads per bead, the shapes the autotuner chooses from); the evaluation
 // pass has one shape
 constexpr int EVAL_FB = 64, EVAL_LPB = 4;
-static int force_block_beads(int fb, int) { return fb; }
+static size_t force_smem(bool mixed, int mode, int fb, bool qa) {
+    if (mode == 0) fb = EVAL_FB;
+    if (mixed) return fb == 32 ? step_smem<float, 32>(qa) : fb == 64 ? step_smem<float, 64>(qa) : step_smem<float, 128>(qa);
+    return fb == 32 ? step_smem<double, 32>(qa) : fb == 64 ? step_smem<double, 64>(qa) : step_smem<double, 128>(qa);
+}
+static int force_blocks(int n, int fb) { return (n + fb - 6) / (fb - 5); }   // step_beads
 static void *force_kernel(bool mixed, int mode, int fb, int lpb) {
 #define XMD_FK(M, B, L) (mixed ? (void *)k_force<float, M, B, L> : (void *)k_force<double, M, B, L>)
     if (mode == 0) return XMD_FK(0, EVAL_FB, EVAL_LPB);
@@ -1998,11 +1415,20 @@ void Engine::launch_force(int mode, int c) {
         else k_pid<1><<<(d.N + 127) / 128, 128, 0, stream>>>(d, tp, c);
     }
     const int fb = mode == 0 ? EVAL_FB : tune.fb, lpb = mode == 0 ? EVAL_LPB : tune.lpb;
-    const int nb = (d.N + force_block_beads(fb, lpb) - 1) / force_block_beads(fb, lpb);
+    const int nb = force_blocks(d.N, fb);
     int fuse = FUSE_NONE;
     void *args[] = {&d, &tp, &c, &fuse};
-    CK(cudaLaunchKernel(force_kernel(params.precision == XMD_PREC_MIXED, mode, fb, lpb), dim3(nb), dim3(fb * lpb),
-                        args, 0, stream));
+    const bool mixed = params.precision == XMD_PREC_MIXED;
+    void *fk = force_kernel(mixed, mode, fb, lpb);
+    const size_t smem = force_smem(mixed, mode, fb, d.qa_on);
+    if (smem > 48 * 1024) CK(cudaFuncSetAttribute(fk, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    CK(cudaLaunchKernel(fk, dim3(nb), dim3(fb * lpb), args, smem, stream));
+}
+
+void Engine::split_positions() {
+    if (params.precision != XMD_PREC_MIXED) return;
+    k_split<<<(d.N + 255) / 256, 256, 0, stream>>>(d, cur);
+    ++launches;
 }
 
 Engine::Engine(const xmd_params &p) : params(p) {
@@ -2127,13 +1553,13 @@ void Engine::remove_replica(int rep) {
         CK(cudaMemsetAsync(d.rep_of + b, 0xff, sizeof(int32_t) * n, stream));
         CK(cudaMemsetAsync(d.bflags + b, 0, sizeof(uint32_t) * n, stream));
         CK(cudaMemsetAsync(d.nl_cnt + b, 0, sizeof(int32_t) * n, stream));
+        CK(cudaMemsetAsync(d.go_cnt + b, 0, sizeof(int32_t) * n, stream));
         if (r.nat_len) CK(cudaMemsetAsync(d.nat_on + r.nat_off, 0, r.nat_len, stream));
         if (r.chunk_len) CK(cudaMemsetAsync(d.chunks + r.chunk_off, 0xff, sizeof(int2) * r.chunk_len, stream));
         if (r.cell_len) CK(cudaMemsetAsync(d.cell_rep + r.cell_off, 0xff, sizeof(int32_t) * r.cell_len, stream));
         CK(cudaMemsetAsync(d.rep + rep, 0, sizeof(RepDev), stream));
         CK(cudaStreamSynchronize(stream));
         for (int i = 0; i < n; ++i) owner_h[b + i] = -1;
-        update_blocks(b, b + n);
         a_beads.release(b, n);
         a_nat.release(r.nat_off, r.nat_len);
         a_ss.release(r.ss_off, r.ss_len);
@@ -2190,7 +1616,6 @@ void Engine::activate_staged() {
                                cudaMemcpyHostToDevice, stream));
         CK(cudaMemcpyAsync(d.rep + st.k, &st.rd, sizeof(RepDev), cudaMemcpyHostToDevice, stream));
         for (int i = 0; i < r.n; ++i) owner_h[r.begin + i] = st.k;
-        update_blocks(r.begin, r.begin + r.n, false);
         r.staged = false;
         r.placed = true;
     }
@@ -2202,6 +1627,7 @@ void Engine::step_async(int nsteps) {
     ready();
     if (!params.langevin_on) throw std::invalid_argument("langevin: enabled is false; nothing integrates");
     ensure_nl();
+    split_positions();
     int s = 0;
     if (!timing && use_graphs) {
         const int gsteps = tune.graph_steps;
@@ -2518,6 +1944,16 @@ void Engine::derive_rep(int ri, RepDev &rd) {
         rd.box.cell[a] = r.cell[a];
         rd.box.cell_inv[a] = r.cell[a] != 0.0 ? 1.0 / r.cell[a] : 0.0;   // box.h:12-22
         rd.per[a] = r.cell[a] != 0.0;
+        rd.per_any |= rd.per[a];
+        // the length as h + l, h truncated as split_d's
+        uint64_t u;
+        std::memcpy(&u, &r.cell[a], 8);
+        u &= ~0x1fffffffull;
+        double h;
+        std::memcpy(&h, &u, 8);
+        rd.Lh[a] = (float)h;
+        rd.Ll[a] = (float)(r.cell[a] - h);
+        rd.Li[a] = (float)rd.box.cell_inv[a];
     }
     // max_cutoff: main.cpp:500, 545-551, 628-630, 642-644, 742-746
     double mc = 0.0;
@@ -2601,6 +2037,8 @@ void Engine::allocate() {
     const size_t NN = (size_t)std::max(1, cap.nat);
     d.pos[0] = (double4_32a *)dalloc(sizeof(double4_32a) * N);
     d.pos[1] = (double4_32a *)dalloc(sizeof(double4_32a) * N);
+    d.spl[0] = (float4 *)dalloc(2 * sizeof(float4) * N);
+    d.spl[1] = (float4 *)dalloc(2 * sizeof(float4) * N);
     d.yh = (double *)dalloc(sizeof(double) * 15 * (size_t)N);
     d.orig = (double4_32a *)dalloc(sizeof(double4_32a) * N);
     d.F = (double *)dalloc(sizeof(double) * 3 * (size_t)N);
@@ -2614,15 +2052,16 @@ void Engine::allocate() {
     d.teth_r0 = (double *)dalloc(sizeof(double) * N);
     d.ang_t0 = (double *)dalloc(sizeof(double) * N);
     d.dih_p0 = (double *)dalloc(sizeof(double) * N);
+    d.dih_cs = (double2 *)dalloc(sizeof(double2) * N);
     d.bond_f = (float4 *)dalloc(sizeof(float4) * N);
     d.nat_start = (int32_t *)dalloc(sizeof(int32_t) * N);
     d.nat_end = (int32_t *)dalloc(sizeof(int32_t) * N);
     d.nat_j = (int32_t *)dalloc(sizeof(int32_t) * NN);
     d.nat_d = (double *)dalloc(sizeof(double) * NN);
-    d.nat_df = (float *)dalloc(sizeof(float) * NN);
-    d.nat_T = (double *)dalloc(sizeof(double) * NN);
-    d.nat_S = (double *)dalloc(sizeof(double) * NN);
     d.nat_on = (uint8_t *)dalloc(NN);
+    d.act_j = (int32_t *)dalloc(sizeof(int32_t) * NN);
+    d.act_d = (double *)dalloc(sizeof(double) * NN);
+    d.go_cnt = (int32_t *)dalloc(sizeof(int32_t) * N);
     {
         const size_t SS = (size_t)std::max(1, cap.ss);
         d.ss_start = (int32_t *)dalloc(sizeof(int32_t) * N);
@@ -2632,8 +2071,10 @@ void Engine::allocate() {
         d.ss_j = (int32_t *)dalloc(sizeof(int32_t) * SS);
         d.ss_on = (uint8_t *)dalloc(SS);
         CK(cudaMemsetAsync(d.ss_on, 0, SS, stream));
-        d.chir = (double2 *)dalloc(sizeof(double2) * N);
-        d.chir_f32 = (float2 *)dalloc(sizeof(float2) * N);
+        if (p.on[XMD_TERM_CHIR]) {
+            d.chir = (double2 *)dalloc(sizeof(double2) * N);
+            d.chir_f32 = (float2 *)dalloc(sizeof(float2) * N);
+        }
         d.afm = (AfmTip *)dalloc(sizeof(AfmTip) * (size_t)std::max(1, cap.afm));
         // wall planes, and the state of every (bead, LJ attractive wall) pair
         double wt[2 * XMD_MAX_WALLS * 6] = {0};
@@ -2642,7 +2083,6 @@ void Engine::allocate() {
         d.wall = (double *)dalloc(sizeof(wt));
         CK(cudaMemcpyAsync(d.wall, wt, sizeof(wt), cudaMemcpyHostToDevice, stream));
         const size_t nlj = walls[1].size() / 6;
-        d.fext = (double *)dalloc(sizeof(double) * 3 * N);
         d.ljw = (LjWallState *)dalloc(sizeof(LjWallState) * std::max<size_t>(1, nlj * N));
         CK(cudaMemsetAsync(d.ljw, 0, sizeof(LjWallState) * std::max<size_t>(1, nlj * N), stream));
         CK(cudaStreamSynchronize(stream));
@@ -2686,8 +2126,6 @@ void Engine::allocate() {
     d.nwork = (int *)dalloc(sizeof(int));
     CK(cudaMemsetAsync(d.nwork, 0, sizeof(int), stream));
     CK(cudaMemsetAsync(d.chunks, 0xff, sizeof(int2) * d.nchunks, stream));
-    d.blk_on = (uint8_t *)dalloc((N + BLK_ON - 1) / BLK_ON + 8);
-    CK(cudaMemsetAsync(d.blk_on, 0, (N + BLK_ON - 1) / BLK_ON + 8, stream));
     owner_h.assign(N, -1);
     a_beads.init(N);
     a_nat.init(cap.nat);
@@ -2754,6 +2192,7 @@ void Engine::allocate() {
     tp.vel_afm_H2 = p.vel_afm_H2;
     tp.ext_on = (cap.afm > 0 && (p.on[XMD_TERM_VEL_AFM] || p.on[XMD_TERM_FORCE_AFM])) ||
                 (p.on[XMD_TERM_SOLID_WALL] && !walls[0].empty()) || (p.on[XMD_TERM_LJ_WALL] && !walls[1].empty());
+    if (tp.ext_on) d.fext = (double *)dalloc(sizeof(double) * 3 * N);
     tp.n_solid = p.on[XMD_TERM_SOLID_WALL] ? (int)walls[0].size() / 6 : 0;
     tp.n_ljw = p.on[XMD_TERM_LJ_WALL] ? (int)walls[1].size() / 6 : 0;
     tp.solid_eps = p.solid_wall_depth;
@@ -2896,19 +2335,6 @@ void Engine::place_pending() {
         }
 }
 
-// occupancy granules [b0/BLK_ON, (b1-1)/BLK_ON] on when any bead slot in them
-// is placed (a force block runs when any of its granules is on)
-void Engine::update_blocks(int b0, int b1, bool wait) {
-    if (b1 <= b0) return;
-    const int k0 = b0 / BLK_ON, k1 = (b1 - 1) / BLK_ON;
-    std::vector<uint8_t> on(k1 - k0 + 1, 0);
-    for (int k = k0; k <= k1; ++k)
-        for (int i = k * BLK_ON; i < std::min(cap.beads, (k + 1) * BLK_ON); ++i)
-            if (owner_h[i] >= 0) { on[k - k0] = 1; break; }
-    CK(cudaMemcpyAsync(d.blk_on + k0, on.data(), on.size(), cudaMemcpyHostToDevice, stream));
-    if (wait) CK(cudaStreamSynchronize(stream));
-}
-
 // static data, lists and state of replica slot k onto the device.  With st
 // (staged placement) every upload goes on the side stream, after the last
 // removal's clears, and the activation data (bead and bucket owners, the
@@ -3012,8 +2438,10 @@ void Engine::place(int k, Staged *st) {
             ch[i] = make_double2(on ? r.chir_f[i] : 0.0, on ? r.chir_n[i] : 0.0);
             chf[i] = make_float2((float)ch[i].x, (float)ch[i].y);
         }
-        up(d.chir + b, ch.data(), sizeof(double2) * n);
-        up(d.chir_f32 + b, chf.data(), sizeof(float2) * n);
+        if (d.chir) {
+            up(d.chir + b, ch.data(), sizeof(double2) * n);
+            up(d.chir_f32 + b, chf.data(), sizeof(float2) * n);
+        }
         // disulfide partners per bead, both directions, ordered by partner
         std::vector<std::vector<int>> sp(n);
         for (size_t q = 0; q < r.ss_i1.size(); ++q) {
@@ -3033,16 +2461,20 @@ void Engine::place(int k, Staged *st) {
         if (nss) CK(cudaMemsetAsync(d.ss_on + so, 0, nss, us));
     }
     std::vector<float4> bf(n);
-    for (int i = 0; i < n; ++i) bf[i] = make_float4((float)tr[i], (float)ar[i], (float)dr[i], 0.0f);
+    std::vector<double2> dcs(n);
+    for (int i = 0; i < n; ++i) {
+        dcs[i] = make_double2(std::cos(dr[i]), std::sin(dr[i]));
+        bf[i] = make_float4(0.0f, (float)ar[i], (float)dcs[i].x, (float)dcs[i].y);
+    }
+    up(d.dih_cs + b, dcs.data(), sizeof(double2) * n);
     up(d.bond_f + b, bf.data(), sizeof(float4) * n);
     up(d.nat_start + b, ns.data(), sizeof(int32_t) * n);
     up(d.nat_end + b, ne.data(), sizeof(int32_t) * n);
     up(d.nat_j + no, nj.data(), sizeof(int32_t) * nj.size());
     up(d.nat_d + no, nd.data(), sizeof(double) * nd.size());
-    std::vector<float> ndf(nd.begin(), nd.end());
-    up(d.nat_df + no, ndf.data(), sizeof(float) * ndf.size());
     CK(cudaMemsetAsync(d.nat_on + no, 0, nnat, us));
     CK(cudaMemsetAsync(d.nl_cnt + b, 0, sizeof(int32_t) * n, us));
+    CK(cudaMemsetAsync(d.go_cnt + b, 0, sizeof(int32_t) * n, us));
     if (ncell) {
         std::vector<int32_t> cr(ncell, k);
         if (st) st->cell_rep = cr;
@@ -3054,14 +2486,6 @@ void Engine::place(int k, Staged *st) {
 
     RepDev rd;
     derive_rep(k, rd);
-    {
-        std::vector<double> nT(nd.size());
-        for (size_t q = 0; q < nd.size(); ++q) nT[q] = 2.0 * nd[q] + rd.pad;   // 2 r_nat is exact
-        up(d.nat_T + no, nT.data(), sizeof(double) * nT.size());
-        std::vector<double> nS(nT.size());
-        for (size_t q = 0; q < nT.size(); ++q) nS[q] = sq_below(nT[q]);
-        up(d.nat_S + no, nS.data(), sizeof(double) * nS.size());
-    }
     rd.cell_off = co;
     rd.cell_budget = ncell;
     rd.tile = tile;
@@ -3145,7 +2569,6 @@ void Engine::place(int k, Staged *st) {
     }
     CK(cudaStreamSynchronize(stream));
     for (int i = 0; i < n; ++i) owner_h[b + i] = k;
-    update_blocks(b, b + n);
     r.placed = true;
     upload_state(k);
 }
@@ -3418,6 +2841,7 @@ size_t Engine::snapshot_io(int rep, unsigned char *buf, size_t bytes, bool save,
         rd.fp_n = sr.fp_n; rd.ct_n = sr.ct_n; rd.steps_left = sr.steps_left;
         rd.maxdisp = sr.maxdisp; rd.rebuilds = sr.rebuilds;
         CK(cudaMemcpy(d.rep + rep, &rd, sizeof(RepDev), cudaMemcpyHostToDevice));
+        k_go_lists<<<(n + 127) / 128, 128, 0, stream>>>(d, b, n);
         h.steps_left = sr.steps_left;
     }
     return off;
@@ -3665,8 +3089,11 @@ cudaGraphExec_t Engine::graph_for(int start_cur, bool gated, int len) {
     cudaGraph_t g;
     CK(cudaGraphCreate(&g, 0));
     cudaGraphNode_t prev = nullptr;
-    const int nb = (d.N + force_block_beads(tune.fb, tune.lpb) - 1) / force_block_beads(tune.fb, tune.lpb);
-    void *fk = force_kernel(params.precision == XMD_PREC_MIXED, 1, tune.fb, tune.lpb);
+    const int nb = force_blocks(d.N, tune.fb);
+    const bool mixed = params.precision == XMD_PREC_MIXED;
+    void *fk = force_kernel(mixed, 1, tune.fb, tune.lpb);
+    const size_t fsmem = force_smem(mixed, 1, tune.fb, d.qa_on);
+    if (fsmem > 48 * 1024) CK(cudaFuncSetAttribute(fk, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fsmem));
     double dt = params.dt;
     // without the quasi-adiabatic term the step kernel takes the skin
     // decision itself (its last block) where no IF node needs it; with it,
@@ -3686,6 +3113,7 @@ cudaGraphExec_t Engine::graph_for(int start_cur, bool gated, int len) {
         kf.func = fk;
         kf.gridDim = dim3(nb);
         kf.blockDim = dim3(tune.fb * tune.lpb);
+        kf.sharedMemBytes = (unsigned)fsmem;
         kf.kernelParams = fargs;
         cudaGraphNode_t nf, nc, ncond;
         void *eargs[] = {&d, &tp, &c};
@@ -3884,6 +3312,7 @@ void Engine::eval_forces(int rep, double *F, double *V) {
     check_rep(reps, rep);
     ready();
     ensure_nl();
+    split_positions();
     CK(cudaMemsetAsync(d.Vrep, 0, sizeof(double) * XMD_NUM_TERMS * d.R, stream));
     launch_force(0, cur);
     const RepHost &h = reps[rep];

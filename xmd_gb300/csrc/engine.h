@@ -57,6 +57,8 @@ struct RepDev {
     int begin, n;
     int cell_off, cell_budget;
     int per[3];
+    int per_any;             // some axis is periodic
+    float Lh[3], Ll[3], Li[3];   // mixed path: cell as h + l, and its inverse (0 on open axes)
     int dims[3];             // cells along periodic axes
     double lo[3], cs[3];     // bounding-box minimum and 1/cell edge along open axes
     int hashed;              // cells hashed into the bucket budget
@@ -125,6 +127,7 @@ struct Dev {
     int N, R, nl_cap;
     double4_32a *pos[2];        // x, y, z, charge; double-buffered
     double *yh;             // [15][N]: y1x y1y y1z y2x ... y5z
+    float4 *spl[2];         // mixed path: positions split per axis, [2 i] = (hx, hy, hz, charge), [2 i + 1] = (lx, ly, lz, 0)
     double4_32a *orig;          // positions at the last list rebuild
     double *F;              // [3N] force output of eval
     double *Vrep;           // [R][XMD_NUM_TERMS] energies of eval
@@ -133,6 +136,7 @@ struct Dev {
     int32_t *chain, *seq;
     uint8_t *atype;
     double *teth_r0, *ang_t0, *dih_p0;
+    double2 *dih_cs;        // (cos, sin) of dih_p0
     double2 *chir;          // (nat_factor, nat_chir) per centre i2 of a chiral quad
     float2 *chir_f32;       // the same in FP32 (mixed path)
     const double *heur_ang;     // [9][7] heuristic angle coefficients a0..a6
@@ -144,13 +148,13 @@ struct Dev {
     double *fext;           // [3N] external force of the step (k_ext: AFM, walls)
     int32_t *ss_start, *ss_end, *ss_j;   // native disulfide partners per bead (CSR, both directions)
     uint8_t *ss_on;         // in the list of the last rebuild (update_nat_ssbonds, native_ss.cpp:8-19)
-    float4 *bond_f;         // (r0, theta0, phi0) in FP32 for the mixed path
+    float4 *bond_f;         // (0, theta0, cos phi0, sin phi0) in FP32 for the mixed path
     int32_t *nat_start, *nat_end, *nat_j;   // natives of bead i: [nat_start[i], nat_end[i])
     double *nat_d;
-    float *nat_df;          // nat_d in FP32 for the mixed path
-    double *nat_T;          // Go-list threshold 2 r_nat + pad of each entry (go.cpp:11-22)
-    double *nat_S;          // its squared form: s < nat_S <=> sqrt(s) < nat_T
-    uint8_t *nat_on;
+    uint8_t *nat_on;        // in the Go list of the last rebuild (update_go_contacts, go.cpp:11-22)
+    int32_t *act_j;         // the Go list of bead i: go_cnt[i] entries from nat_start[i], in nat_j's order
+    double *act_d;
+    int32_t *go_cnt;
     int32_t *nl_row, *nl_cnt;
     int32_t *cell_cnt, *cell_start, *cell_fill, *cell_items, *bead_cell;
     float4 *cell_pos;       // bucket-sorted FP32 coordinates (+ bead index bits)
@@ -172,7 +176,6 @@ struct Dev {
     int *work;              // chunks of the replicas flagged at the last skin check
     int *nwork;             // number of entries in `work`
     int any_cell;           // some replica uses the cell-grid build
-    uint8_t *blk_on;        // force blocks (FB beads) holding at least one placed bead
     int qa_on;
     QaDev qa;
     // pseudo-improper dihedral potential: per bead its bundles' forces on
@@ -367,6 +370,7 @@ private:
     bool timing = false;
     bool isolate_faults = false;
     void launch_force(int mode, int c);
+    void split_positions();
     int tile_sms = 1, tile_max_per_sm = 1;     // for the tile build's resident grid
     // the QA sift's fixed grid: four blocks per SM, each taking at most
     // QA_SIFT groups of free-pair slots
@@ -432,7 +436,6 @@ private:
     void place_pending();
     void ready();                              // allocated, every replica placed
     void ready_alloc();
-    void update_blocks(int b0, int b1, bool wait = true);
     void *dalloc(size_t bytes);
     void finalize();
     void release();

@@ -1,0 +1,896 @@
+// step.cuh - the block of the step kernel (included by engine.cu).
+//
+// A block of FB bead slots takes FBT = FB - 5 beads, so that everything it
+// derives from the chain geometry is one full round of FB lanes: FB bonds and
+// cross products, FB - 2 bonded centres (the beads' own and three of the
+// neighbours').  The work passes through shared memory in phases, each dealt
+// so that whole warps do one thing with every lane busy (GB300 issues an FP64
+// warp instruction over 16 cycles of the SM's FP64 pipe however few lanes
+// are active, and the mixed path is bound by latency and issue):
+//   A  the tile's positions; per bead its list lengths (prefix sum)
+//   B  per slot: bond vector, cross product, their inverse lengths, once for
+//      every term that uses them; beside it the beads' noise
+//   D  per centre: tether + angle, and dihedral + chirality, on separate warps
+//   E  pair entries: the lists of all beads of the block as one sequence,
+//      one thread per entry whatever bead it belongs to, forces to shared
+//      memory.  Warps without a part in B and D start here at once; every
+//      warp takes the next 32 entries until none is left
+//   F  one thread per (axis, bead): the bead's force summed in a fixed order,
+//      then the integrator; G  new positions, skin test
+// A bead's entries are its active native contacts, its Verlet row and its
+// quasi-adiabatic contacts, summed in that order after the bonded forces: the
+// trajectory is the same bits for every launch shape.
+//
+// What it measured, 256 chains of 50-800 beads (66,007), us per MD step at 64
+// slots x 4 threads, against a block whose threads kept to one bead each from
+// list loops to integrator (bonded geometry formed per term, a third of the
+// bonded warps with 3 live lanes, noise and skin test on a quarter of the
+// lanes): FP64 456 -> 156 (its FP64 pipe 81 % active), mixed 65 -> 44 (27.5 M
+// -> 11.6 M warp instructions).  One chain of 100 beads in FP64: 55 -> 24.
+#pragma once
+
+namespace xmdg {
+
+template <int FB> constexpr int step_beads() { return FB - 5; }
+
+// one term into the running force: FP64 rounded on its own; FP32 terms into a
+// float-float sum whose low part collects the exact errors of the high part
+__device__ __forceinline__ void sum_acc(double &a, double v) { a = __dadd_rn(a, v); }
+__device__ __forceinline__ void sum_acc(FF &a, float v) {
+    const FF s = two_sum(a.h, v);
+    a.h = s.h;
+    a.l = __fadd_rn(a.l, s.l);
+}
+__device__ __forceinline__ double sum_total(double a) { return a; }
+__device__ __forceinline__ double sum_total(FF a) { return ff_to_d(a); }
+template <class FT> struct StepSum { using T = double; };
+template <> struct StepSum<float> { using T = FF; };
+
+// dot and cross products with the contractions written out, so that every
+// instantiation of the block rounds alike
+template <class T> __device__ __forceinline__ T fma_(T a, T b, T c);
+template <> __device__ __forceinline__ double fma_(double a, double b, double c) { return __fma_rn(a, b, c); }
+template <> __device__ __forceinline__ float fma_(float a, float b, float c) { return __fmaf_rn(a, b, c); }
+__device__ __forceinline__ double mul_(double a, double b) { return __dmul_rn(a, b); }
+__device__ __forceinline__ float mul_(float a, float b) { return __fmul_rn(a, b); }
+__device__ __forceinline__ double add_(double a, double b) { return __dadd_rn(a, b); }
+__device__ __forceinline__ float add_(float a, float b) { return __fadd_rn(a, b); }
+template <class T> __device__ __forceinline__ T fdot(V3<T> a, V3<T> b) {
+    return fma_<T>(a.x, b.x, fma_<T>(a.y, b.y, mul_(a.z, b.z)));
+}
+template <class T> __device__ __forceinline__ V3<T> fcross(V3<T> a, V3<T> b) {
+    return V3<T>{fma_<T>(a.y, b.z, -mul_(a.z, b.y)), fma_<T>(a.z, b.x, -mul_(a.x, b.z)),
+                 fma_<T>(a.x, b.y, -mul_(a.y, b.x))};
+}
+template <class T> __device__ __forceinline__ V3<T> fscl(T s, V3<T> a) {
+    return V3<T>{mul_(s, a.x), mul_(s, a.y), mul_(s, a.z)};
+}
+
+// 1 / sqrt(x).  FP32: the hardware estimate and one Newton step (3
+// instructions, within 1 ulp), where 1 / sqrtf(x) takes about twenty; zero
+// and infinity as the estimate gives them.
+__device__ __forceinline__ double rsq(double x) { return rsqrt(x); }
+__device__ __forceinline__ float rsq(float x) {
+    const float y = rsqrtf(x);
+    const float r = __fmaf_rn(-__fmul_rn(x, y), y, 1.0f);
+    const float z = __fmaf_rn(__fmul_rn(0.5f, y), r, y);
+    return x > 0.0f && y > 0.0f ? z : y;
+}
+
+// ---- geometry slots -------------------------------------------------------------
+// FP64: bond e (3), unit cross product u (3), |e|, 1/|e|, 1/|x|.  Bonds, cross
+// products, lengths and units are formed with every operation rounded on its
+// own, as the reference's uncontracted build forms them: on extended starts
+// triples are straight to ~1e-6 rad, where a contracted cross product moves
+// a dihedral force by 1e-10 of itself.
+// Mixed: bond and cross product in float-float (6 + 6), 1/|e|, 1/|x|.
+enum : int { GE = 0, GU = 3, GLEN = 6, GRN = 7, GRX = 8, GN64 = 9 };
+enum : int { MEH = 0, MEL = 3, MXH = 6, MXL = 9, MRN = 12, MRX = 13, GN32 = 16 };
+
+// energies of the evaluation pass: per thread for the block's first replica,
+// reduced over the warp at the end; other replicas at once
+enum : int { EV_N = XMD_NUM_TERMS };
+template <int MODE> struct Ener {
+    __device__ __forceinline__ void add(const Dev &, int, int, double) {}
+    __device__ __forceinline__ void flush(const Dev &) {}
+    __device__ __forceinline__ void start(int) {}
+};
+template <> struct Ener<0> {
+    double v[EV_N];
+    int r0;
+    __device__ __forceinline__ void start(int r) {
+        r0 = r;
+#pragma unroll
+        for (int k = 0; k < EV_N; ++k) v[k] = 0.0;
+    }
+    __device__ __forceinline__ void add(const Dev &d, int r, int term, double e) {
+        if (r == r0) {
+#pragma unroll
+            for (int k = 0; k < EV_N; ++k)
+                if (k == term) v[k] += e;
+        } else {
+            atomicAdd(&d.Vrep[r * XMD_NUM_TERMS + term], e);
+        }
+    }
+    __device__ __forceinline__ void flush(const Dev &d) {
+        if (r0 < 0) return;
+#pragma unroll
+        for (int k = 0; k < EV_N; ++k) {
+            double e = v[k];
+            if (!__any_sync(0xffffffffu, e != 0.0)) continue;
+            for (int o = 16; o; o >>= 1) e += __shfl_xor_sync(0xffffffffu, e, o);
+            if ((threadIdx.x & 31) == 0) atomicAdd(&d.Vrep[r0 * XMD_NUM_TERMS + k], e);
+        }
+    }
+};
+
+// ---- bonded centres ----------------------------------------------------------------
+// a centre's parameters: bond length (mixed: with its low part), angle, cosine
+// and sine of the dihedral
+template <class FT> struct CentreP { FT r0, t0, c0, s0, r0l; };
+
+// sp: the centre's position slot.  g: geometry slots [.][FB].
+
+// tether (c, c+1), angle (c-1, c, c+1): the force on c from its bond, the
+// angle's forces on c-1 and c+1 (on c: minus their sum)
+template <class FT, int MODE, int FB>
+__device__ __forceinline__ void bond_angle(const Dev &d, const TermP &p, const FT (*g)[FB], int sp, uint32_t fl,
+                                           const CentreP<FT> &cp, bool own, int rc, Ener<MODE> &en, V3<FT> *ft,
+                                           V3<FT> *a1, V3<FT> *a2, V3<FT> *a3) {
+    constexpr bool MIX = sizeof(FT) == 4;
+    const bool h_ang = (fl & BF_HANG) && p.on[XMD_TERM_HEUR_ANG];
+    const bool do_ang = ((fl & BF_ANG) && p.on[XMD_TERM_NAT_ANG]) || h_ang;
+    const double *hac = h_ang ? d.heur_ang + 7 * ((fl >> BF_HANG_SHIFT) & 15u) : nullptr;
+    const V3<FT> e1{g[0][sp - 1], g[1][sp - 1], g[2][sp - 1]}, e2{g[0][sp], g[1][sp], g[2][sp]};
+    const FT rn1 = g[MIX ? MRN : GRN][sp - 1], rn2 = g[MIX ? MRN : GRN][sp];
+    if ((fl & BF_TETH) && p.on[XMD_TERM_TETHER]) {
+        // eval_tether_forces::iter tether.cpp:21-36, harmonic.h:18-25
+        FT dr;
+        if constexpr (MIX) {
+            // the bond length in float-float: its stiffness (2500 eps per unit
+            // squared) makes an FP32 length the largest error of the force
+            const FF px = two_prod(e2.x, e2.x), py = two_prod(e2.y, e2.y), pz = two_prod(e2.z, e2.z);
+            const FF s1 = two_sum(px.h, py.h), s2 = two_sum(s1.h, pz.h);
+            float low = __fadd_rn(__fadd_rn(px.l, py.l), __fadd_rn(pz.l, __fadd_rn(s1.l, s2.l)));
+            const V3<float> el{g[MEL][sp], g[MEL + 1][sp], g[MEL + 2][sp]};
+            low = __fmaf_rn(2.0f, fdot(e2, el), low);
+            const float l0 = __fmul_rn(s2.h, rn2);
+            const float rest = __fadd_rn(__fmaf_rn(-l0, l0, s2.h), low);
+            dr = __fadd_rn(__fsub_rn(l0, cp.r0), __fmaf_rn(__fmul_rn(0.5f, rn2), rest, -cp.r0l));
+        } else {
+            dr = g[GLEN][sp] - cp.r0;
+        }
+        const FT dr2 = mul_(dr, dr);
+        const FT H1 = tpar<FT>(p.tether_H1, p.f.tether_H1), H2 = tpar<FT>(p.tether_H2, p.f.tether_H2);
+        FT dV = mul_(dr, fma_<FT>(mul_(FT(2), H2), dr2, H1));
+        dV = clampv<FT>(dV, FT(-1.0e3), FT(1.0e3));
+        *ft = fscl<FT>(mul_(dV, rn2), e2);
+        if (MODE == 0 && own)
+            en.add(d, rc, XMD_TERM_TETHER,
+                   (double)clampv<FT>(mul_(mul_(FT(0.5), dr2), fma_<FT>(H2, dr2, H1)), FT(-1.0e3), FT(1.0e3)));
+    }
+    if (do_ang) {
+        // eval_native_angle_forces::iter angle/native.cpp:13-39.  The cross
+        // products of the bonds with the plane's normal have lengths |r12| and
+        // |r23| (the bonds lie in the plane), so the reference's unit vectors
+        // along them need no further square root.
+        V3<FT> u;   // the plane's unit normal
+        double V_ = 0.0;
+        FT dV, theta;
+        if constexpr (MIX) {
+            const V3<float> x{g[MXH][sp], g[MXH + 1][sp], g[MXH + 2][sp]};
+            u = fscl<float>(g[MRX][sp], x);
+            theta = atan2f(__fmul_rn(fdot(x, x), g[MRX][sp]), -fdot(e1, e2));
+        } else {
+            u = V3<double>{g[GU][sp], g[GU + 1][sp], g[GU + 2][sp]};
+            const V3<DN> b1{e1.x, e1.y, e1.z}, b2{e2.x, e2.y, e2.z};
+            theta = acos_c<DN>(-dot(b1, b2) * DN(rn1) * DN(rn2)).v;
+        }
+        if (hac) {
+            const double2 vd = heur_poly_nl(hac, (double)theta);
+            V_ = vd.x;
+            dV = (FT)vd.y;
+        } else {
+            const FT dt = theta - cp.t0;
+            dV = mul_(tpar<FT>(p.nat_ang_k, p.f.nat_ang_k), dt);
+            if (MODE == 0) V_ = (double)mul_(FT(0.5), mul_(dV, dt));
+        }
+        if (MODE == 0 && own) en.add(d, rc, h_ang ? XMD_TERM_HEUR_ANG : XMD_TERM_NAT_ANG, V_);
+        *a1 = fscl<FT>(-mul_(dV, mul_(rn1, rn1)), fcross(e1, u));
+        *a3 = fscl<FT>(-mul_(dV, mul_(rn2, rn2)), fcross(e2, u));
+        *a2 = V3<FT>{-add_(a1->x, a3->x), -add_(a1->y, a3->y), -add_(a1->z, a3->z)};
+    }
+}
+
+// dihedral and chirality of (c-1, c, c+1, c+2): forces on the four beads
+template <class FT, int MODE, int FB>
+__device__ __forceinline__ void dihedral_chiral(const Dev &d, const TermP &p, const FT (*g)[FB], int c, int sp,
+                                                uint32_t fl, const CentreP<FT> &cp, bool own, int rc, Ener<MODE> &en,
+                                                V3<FT> *q) {
+    constexpr bool MIX = sizeof(FT) == 4;
+    const bool h_dih = (fl & BF_HDIH) && p.on[XMD_TERM_HEUR_DIH];
+    const bool do_dih = ((fl & BF_DIH) && (p.on[XMD_TERM_CND] || p.on[XMD_TERM_SND])) || h_dih;
+    const int hdt = (int)((fl >> BF_HDIH_SHIFT) & 15u);
+    const V3<FT> e1{g[0][sp - 1], g[1][sp - 1], g[2][sp - 1]}, e2{g[0][sp], g[1][sp], g[2][sp]},
+        e3{g[0][sp + 1], g[1][sp + 1], g[2][sp + 1]};
+    if (do_dih) {
+        // eval_cnd_forces::iter dihedral/complex_native.cpp:13-49,
+        // eval_snd_forces::iter dihedral/simple_native.cpp:13-45.  Sine and
+        // cosine of phi come from the geometry, those of phi - phi0 and
+        // 3 (phi - phi0) by the addition theorems: no arc cosine and no
+        // sine of an angle, except for the terms that need phi itself.
+        V3<FT> u1, u2;
+        FT rx1, rx2, rn2, len2, cphi, sphi, tsign;
+        if constexpr (MIX) {
+            rx1 = g[MRX][sp]; rx2 = g[MRX][sp + 1]; rn2 = g[MRN][sp];
+            const V3<float> x1{g[MXH][sp], g[MXH + 1][sp], g[MXH + 2][sp]},
+                x2{g[MXH][sp + 1], g[MXH + 1][sp + 1], g[MXH + 2][sp + 1]};
+            u1 = fscl<float>(rx1, x1);
+            u2 = fscl<float>(rx2, x2);
+            len2 = __fmul_rn(fdot(e2, e2), rn2);
+            // the triple product in float-float: small against its factors
+            // for flat quads
+            const V3<FF> xf{FF{x1.x, g[MXL][sp]}, FF{x1.y, g[MXL + 1][sp]}, FF{x1.z, g[MXL + 2][sp]}};
+            const V3<FF> ef{FF{e3.x, g[MEL][sp + 1]}, FF{e3.y, g[MEL + 1][sp + 1]}, FF{e3.z, g[MEL + 2][sp + 1]}};
+            tsign = ff_dot(xf, ef).h;
+            sphi = __fmul_rn(__fmul_rn(__fmul_rn(len2, tsign), rx1), rx2);
+            cphi = __fmul_rn(__fmul_rn(fdot(x1, x2), rx1), rx2);
+        } else {
+            rx1 = g[GRX][sp]; rx2 = g[GRX][sp + 1]; rn2 = g[GRN][sp];
+            len2 = g[GLEN][sp];
+            u1 = V3<double>{g[GU][sp], g[GU + 1][sp], g[GU + 2][sp]};
+            u2 = V3<double>{g[GU][sp + 1], g[GU + 1][sp + 1], g[GU + 2][sp + 1]};
+            // the cosine as the reference rounds it, clamped; the sine of its
+            // arc cosine is sqrt((1 - c)(1 + c))
+            const V3<DN> a{u1.x, u1.y, u1.z}, b{u2.x, u2.y, u2.z};
+            cphi = clampv<double>(dot(a, b).v, -1.0, 1.0);
+            const double s2 = __dmul_rn(__dsub_rn(1.0, cphi), __dadd_rn(1.0, cphi));
+            sphi = s2 > 0.0 ? __dmul_rn(s2, rsqrt(s2)) : s2;
+            tsign = fdot(u1, e3);
+            if (tsign < 0.0) sphi = -sphi;
+        }
+        FT dV = FT(0);
+        double Vc = 0.0, Vs = 0.0;
+        if (h_dih) {
+            FT V_;
+            if constexpr (MIX) heur_dih_nl<float>(d.heur_dih_f + 6 * hdt, sphi, cphi, &V_, &dV);
+            else heur_dih_nl<double>(d.heur_dih + 6 * hdt, sphi, cphi, &V_, &dV);
+            Vc = (double)V_;
+        } else if (p.on[XMD_TERM_CND]) {
+            const FT c0 = cp.c0, s0 = cp.s0;
+            const FT CDA = tpar<FT>(p.cnd_CDA, p.f.cnd_CDA), CDB = tpar<FT>(p.cnd_CDB, p.f.cnd_CDB);
+            const FT sd = fma_<FT>(sphi, c0, -mul_(cphi, s0));
+            const FT sd2 = mul_(sd, sd);
+            // sin 3x = sin x (3 - 4 sin^2 x), cos 3x = cos x (1 - 4 sin^2 x)
+            const FT s3 = mul_(sd, fma_<FT>(FT(-4), sd2, FT(3)));
+            dV = fma_<FT>(mul_(FT(3), CDB), s3, mul_(CDA, sd));
+            if (MODE == 0) {
+                const FT cd = fma_<FT>(cphi, c0, mul_(sphi, s0));
+                const FT c3 = mul_(cd, fma_<FT>(FT(-4), sd2, FT(1)));
+                // 1 - cos x = sin^2 x / (1 + cos x), without cancellation at the minimum
+                const FT v1 = cd > FT(0) ? sd2 / (FT(1) + cd) : FT(1) - cd;
+                const FT v3 = c3 > FT(0) ? s3 * s3 / (FT(1) + c3) : FT(1) - c3;
+                Vc = (double)(CDA * v1 + CDB * v3);
+            }
+        }
+        if (p.on[XMD_TERM_SND] && !h_dih) {
+            FT phi, CDH, p0;
+            if constexpr (MIX) {
+                phi = atan2f(sphi, cphi);
+                CDH = p.f.snd_CDH;
+                p0 = narrow_f(d.dih_p0[c]);
+            } else {
+                phi = acos(cphi);
+                if (tsign < 0.0) phi = -phi;
+                CDH = p.snd_CDH;
+                p0 = d.dih_p0[c];
+            }
+            const FT df = phi - p0;
+            dV = fma_<FT>(CDH, df, dV);
+            Vs = 0.5 * (double)CDH * (double)df * (double)df;
+        }
+        if (MODE == 0 && own) {
+            if (h_dih) en.add(d, rc, XMD_TERM_HEUR_DIH, Vc);
+            else {
+                if (p.on[XMD_TERM_CND]) en.add(d, rc, XMD_TERM_CND, Vc);
+                if (p.on[XMD_TERM_SND]) en.add(d, rc, XMD_TERM_SND, Vs);
+            }
+        }
+        const FT k = mul_(dV, len2), iden = mul_(rn2, rn2);
+        q[0] = fscl<FT>(mul_(k, rx1), u1);
+        q[3] = fscl<FT>(-mul_(k, rx2), u2);
+        const FT k1 = mul_(fdot(e1, e2), iden), k4 = mul_(fdot(e2, e3), iden);
+        const V3<FT> w{fma_<FT>(q[0].x, k1, -mul_(q[3].x, k4)), fma_<FT>(q[0].y, k1, -mul_(q[3].y, k4)),
+                       fma_<FT>(q[0].z, k1, -mul_(q[3].z, k4))};
+        q[1] = V3<FT>{-add_(q[0].x, w.x), -add_(q[0].y, w.y), -add_(q[0].z, w.z)};
+        q[2] = V3<FT>{add_(w.x, -q[3].x), add_(w.y, -q[3].y), add_(w.z, -q[3].z)};
+    }
+    if ((fl & BF_CHIR) && p.on[XMD_TERM_CHIR]) {
+        // eval_chiral_forces::iter chiral.cpp:15-37
+        V3<FT> h[4];
+        double Vch;
+        if constexpr (MIX) {
+            const float2 ch = d.chir_f32[c];
+            const V3<float> x1{g[MXH][sp], g[MXH + 1][sp], g[MXH + 2][sp]},
+                x2{g[MXH][sp + 1], g[MXH + 1][sp + 1], g[MXH + 2][sp + 1]};
+            const V3<FF> ef{FF{e1.x, g[MEL][sp - 1]}, FF{e1.y, g[MEL + 1][sp - 1]}, FF{e1.z, g[MEL + 2][sp - 1]}};
+            const V3<FF> xf{FF{x2.x, g[MXL][sp + 1]}, FF{x2.y, g[MXL + 1][sp + 1]}, FF{x2.z, g[MXL + 2][sp + 1]}};
+            float Vf;
+            chiral_mixed(p, e1, e2, e3, x1, x2, ff_dot(ef, xf).h, ch.x, ch.y, h, &Vf);
+            Vch = (double)Vf;
+        } else {
+            const double2 ch = d.chir[c];
+            V3<DN> gn[4];
+            DN Vn;
+            const V3<DN> b1{e1.x, e1.y, e1.z}, b2{e2.x, e2.y, e2.z}, b3{e3.x, e3.y, e3.z};
+            chiral_bonds<DN>(p, b1, b2, b3, DN(ch.x), DN(ch.y), gn, &Vn);
+#pragma unroll
+            for (int k = 0; k < 4; ++k) h[k] = v3d(gn[k]);
+            Vch = (double)Vn;
+        }
+#pragma unroll
+        for (int k = 0; k < 4; ++k) q[k] = q[k] + h[k];
+        if (MODE == 0 && own) en.add(d, rc, XMD_TERM_CHIR, Vch);
+    }
+}
+
+// ---- pair vectors -------------------------------------------------------------------
+// mixed: from split positions; the minimum image leaves the short form unless
+// a pair actually lies across the box
+__device__ __forceinline__ V3<float> pair_vec(const RepDev &rp, const F2 (&a)[3], const F2 (&b)[3]) {
+    float v[3];
+#pragma unroll
+    for (int k = 0; k < 3; ++k) v[k] = __fadd_rn(__fsub_rn(b[k].h, a[k].h), __fsub_rn(b[k].l, a[k].l));
+    if (rp.per_any) {
+#pragma unroll
+        for (int k = 0; k < 3; ++k)
+            if (rintf(__fmul_rn(v[k], rp.Li[k])) != 0.0f)
+                v[k] = mi_axis(a[k], b[k], rp.Lh[k], rp.Ll[k], rp.Li[k], true);
+    }
+    return V3<float>{v[0], v[1], v[2]};
+}
+__device__ __forceinline__ void spl_load(const float4 *spl, int j, F2 (&b)[3]) {
+    const float4 h = spl[2 * (size_t)j], l = spl[2 * (size_t)j + 1];
+    b[0] = F2{h.x, l.x}; b[1] = F2{h.y, l.y}; b[2] = F2{h.z, l.z};
+}
+
+// ---- the block ----------------------------------------------------------------------
+template <class FT, int FB> struct StepSh {
+    static constexpr bool MIX = sizeof(FT) == 4;
+    // pair forces held at once; a block with more entries takes several passes
+    static constexpr int FCAP = 8 * FB;
+    double F[3][FB];                  // new positions
+    uint64_t rng[FB];                 // generator states after the step
+    FT p[MIX ? 7 : 4][FB + 4];        // positions; mixed: h, l per axis, charge; FP64: x, y, z, charge
+    FT g[MIX ? (int)GN32 : (int)GN64][FB];   // geometry
+    FT c[24][FB];                     // centre forces: tether, angle on c-1, c, c+1, dihedral on c-1 .. c+2
+    FT f[3][FCAP];                    // pair forces
+    FT n[3][FB];                      // noise
+    FT e[3][FB];                      // squared skin-test displacement per axis
+    int off[FB + 4], ng[FB], nl[FB], nat0[FB], rep[FB], state[FB], ws[4], next;
+    // followed, in contexts with the quasi-adiabatic term, by the beads'
+    // contact slots in ascending order, int [FB][QA_REF_CAP]
+};
+template <class FT, int FB> constexpr size_t step_smem(bool qa) {
+    return (sizeof(StepSh<FT, FB>) + 15) / 16 * 16 + (qa ? sizeof(int) * QA_REF_CAP * FB : 0);
+}
+
+// force of pair entry e of the block on its bead
+template <class FT, int MODE, int FB>
+__device__ __forceinline__ V3<FT> pair_entry(const Dev &d, const TermP &p, int cur, const StepSh<FT, FB> &s,
+                                             const int (*s_q)[QA_REF_CAP], int i0, int e, Ener<MODE> &en) {
+    constexpr bool MIX = sizeof(FT) == 4;
+    // the entry's bead: the last one that starts at or before it
+    int lo = 0;
+#pragma unroll
+    for (int h = FB / 2; h; h >>= 1)
+        if (s.off[lo + h] <= e) lo += h;
+    const int i = i0 + lo, ng = s.ng[lo];
+    int m = e - s.off[lo];
+    int j = -1, slot = -1, ent = 0;
+    FT rm = FT(0);
+    if (m < ng) {
+        const int q = s.nat0[lo] + m;
+        j = d.act_j[q];
+        if constexpr (MIX) rm = narrow_f(d.act_d[q]);
+        else rm = d.act_d[q];
+    } else if ((m -= ng) < s.nl[lo]) {
+        ent = d.nl_row[(size_t)m * d.N + i];
+        if (ent & (NL_PAULI | NL_ES)) j = ent & NL_MASK;
+        rm = tpar<FT>(p.pauli_r_excl, p.f.pauli_r_excl);
+    } else {
+        slot = s_q[lo][m - s.nl[lo]];
+        const int x = d.qa.ct_i1[slot];
+        j = x == i ? d.qa.ct_i2[slot] : x;
+    }
+    if (j < 0) return V3<FT>{FT(0), FT(0), FT(0)};   // a PID bundle only
+    const int r = s.rep[lo];
+    const RepDev &rp = d.rep[r];
+    V3<FT> r12;
+    FT qj;
+    if constexpr (MIX) {
+        const F2 pa[3] = {{s.p[0][lo + 3], s.p[3][lo + 3]}, {s.p[1][lo + 3], s.p[4][lo + 3]},
+                          {s.p[2][lo + 3], s.p[5][lo + 3]}};
+        const float4 h = d.spl[cur][2 * (size_t)j], l = d.spl[cur][2 * (size_t)j + 1];
+        const F2 pb[3] = {{h.x, l.x}, {h.y, l.y}, {h.z, l.z}};
+        r12 = pair_vec(rp, pa, pb);
+        qj = h.w;
+    } else {
+        const double4_32a pj = d.pos[cur][j];
+        const double4_32a pi = make_double4_32a(s.p[0][lo + 3], s.p[1][lo + 3], s.p[2][lo + 3], 0.0);
+        r12 = r_uv_p<double>(rp.box, rp.per_any != 0, pi, pj);
+        qj = pj.w;
+    }
+    const FT s2 = fdot(r12, r12), rn = rsq(s2);
+    FT dV = FT(0);
+    if (slot >= 0) {
+        // quasi-adiabatic contact: the force part of process_contacts::iter
+        // (process_contacts.cpp:25-40)
+        double sat = fmin(rp.t - d.qa.ct_ref[slot], p.qa_cycle) * p.qa_cycle_inv;
+        if (d.qa.ct_status[slot] == QA_BREAKING) sat = 1.0 - sat;
+        double depth, rmin, rmax;
+        qa_lj(p, d.qa, d.qa.ct_type[slot], &depth, &rmin, &rmax);
+        FT V_, dq;
+        sink_lj_eval<FT>((FT)depth, (FT)rmin, (FT)rmax, mul_(rn, s2), rn, &V_, &dq);
+        dV = mul_((FT)sat, dq);
+        if (MODE == 0 && i < j) en.add(d, r, XMD_TERM_QA, sat * (double)V_);
+    } else {
+        // Go (go.cpp:31-46, lj.h:22-30) and Pauli (pauli.cpp:32-48,
+        // shifted_lj.h:14-21) have one force law, Pauli inside r_excl only
+        const bool go = ent == 0;
+        const FT x = mul_(rn, rm);
+        if (go || ((ent & NL_PAULI) && FT(1) < x)) {
+            const FT depth = go ? tpar<FT>(p.go_depth, p.f.go_depth) : tpar<FT>(p.pauli_depth, p.f.pauli_depth);
+            const FT x2 = mul_(x, x), x3 = mul_(x2, x), s6 = mul_(x3, x3);
+            // s6 - s12 = s6 (1 - s6)
+            dV = mul_(mul_(mul_(FT(12), depth), rn), mul_(s6, add_(FT(1), -s6)));
+            dV = clampv<FT>(dV, FT(-1.0e3), FT(1.0e3));
+            if (MODE == 0 && i < j) {
+                FT V_ = mul_(depth, add_(mul_(s6, add_(s6, FT(-2))), go ? FT(0) : FT(1)));
+                V_ = clampv<FT>(V_, FT(-1.0e3), FT(1.0e3));
+                en.add(d, r, go ? XMD_TERM_GO : XMD_TERM_PAULI, (double)V_);
+            }
+        }
+        if (ent & NL_ES) {
+            // eval_const_es_forces::iter es/const.cpp:13-32,
+            // eval_relative_es_forces::iter es/relative.cpp:13-32
+            const FT sdi = tpar<FT>(p.es_sdi, p.f.es_sdi);
+            const FT V_ = mul_(mul_(mul_(tpar<FT>(p.es_Vf, p.f.es_Vf), mul_(s.p[MIX ? 6 : 3][lo + 3], qj)),
+                                    exp_(-mul_(mul_(s2, rn), sdi))),
+                               mul_(rn, rn));
+            dV = fma_<FT>(-V_, fma_<FT>(p.es_rel ? FT(2) : FT(1), rn, sdi), dV);
+            if (MODE == 0 && i < j) en.add(d, r, p.es_rel ? XMD_TERM_REL_ES : XMD_TERM_CONST_ES, (double)V_);
+        }
+    }
+    return fscl<FT>(mul_(dV, rn), r12);
+}
+
+// MODE 0: forces and per-term energies at pos[cur] (eval).
+// MODE 1: forces, then one Langevin predictor-corrector step (lang_pc.cpp:5-41)
+//         writing pos[cur^1], y1..y5, the generator state and the skin-test
+//         displacement (verify.cpp:10-15).
+// r: replica of the block's bead t (threads t < FBT), -1 where there is none.
+template <class FT, int MODE, int FB, int LPB>
+__device__ __forceinline__ void force_block(const Dev &d, const TermP &p, int cur, int r) {
+    constexpr bool MIX = sizeof(FT) == 4;
+    constexpr int NT = FB * LPB, FBT = step_beads<FB>(), NP = FB + 1, NC = FBT + 3;
+    constexpr int TT = (3 * FBT + NT - 1) / NT;   // (axis, bead) tasks per thread
+    constexpr int FCAP = StepSh<FT, FB>::FCAP;
+    using ST = typename StepSum<FT>::T;
+    extern __shared__ __align__(16) unsigned char step_mem[];
+    StepSh<FT, FB> &s = *reinterpret_cast<StepSh<FT, FB> *>(step_mem);
+    int(*const s_q)[QA_REF_CAP] = reinterpret_cast<int(*)[QA_REF_CAP]>(step_mem + step_smem<FT, FB>(false));
+    const int N = d.N, t = threadIdx.x, i0 = blockIdx.x * FBT, lane = t & 31;
+    const size_t Ns = (size_t)N;
+    const bool qa = d.qa_on && p.on[XMD_TERM_QA];
+
+    // ---- A: tile and list lengths.  What later phases load from memory
+    // without needing a result is loaded here, so that its latency passes
+    // once: the centre's parameters, the generator state
+    for (int k = t; k < NP; k += NT) {
+        const int idx = i0 - 3 + k;
+        const bool ok = idx >= 0 && idx < N;
+        if constexpr (MIX) {
+            const float4 z = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            const float4 h = ok ? d.spl[cur][2 * (size_t)idx] : z, l = ok ? d.spl[cur][2 * (size_t)idx + 1] : z;
+            s.p[0][k] = h.x; s.p[1][k] = h.y; s.p[2][k] = h.z;
+            s.p[3][k] = l.x; s.p[4][k] = l.y; s.p[5][k] = l.z;
+            s.p[6][k] = h.w;
+        } else {
+            const double4_32a q = ok ? d.pos[cur][idx] : make_double4_32a(0, 0, 0, 0);
+            s.p[0][k] = q.x; s.p[1][k] = q.y; s.p[2][k] = q.z; s.p[3][k] = q.w;
+        }
+    }
+    const int sc = t & (FB - 1), c = i0 - 2 + sc;   // the thread's centre (t < 2 FB)
+    uint32_t fl = 0;
+    CentreP<FT> cp{FT(0), FT(0), FT(0), FT(0), FT(0)};
+    if (t < 2 * FB && sc < NC && c >= 0 && c < N) {
+        fl = d.bflags[c];
+        if constexpr (MIX) {
+            const float4 q = d.bond_f[c];
+            const F2 r0 = split_d(d.teth_r0[c]);
+            cp = CentreP<float>{r0.h, q.y, q.z, q.w, r0.l};
+        } else {
+            if (LPB == 1 || t < FB) { cp.r0 = d.teth_r0[c]; cp.t0 = d.ang_t0[c]; }
+            if (LPB == 1 || t >= FB) { const double2 q = d.dih_cs[c]; cp.c0 = q.x; cp.s0 = q.y; }
+        }
+    }
+    const int bn = LPB == 1 ? t : t - FB;           // the bead whose noise this thread draws
+    const bool draws = MODE == 1 && bn >= 0 && bn < FBT && i0 + bn < N;
+    uint64_t st0 = 0;
+    if (draws) st0 = d.rng[i0 + bn];
+    int scan = 0, cnt = 0;
+    if (t < FB) {
+        const int i = i0 + t;
+        int ng = 0, nl = 0, nq = 0, nat0 = 0;
+        if (r >= 0) {
+            nl = d.nl_cnt[i];
+            if (p.on[XMD_TERM_GO]) {
+                nat0 = d.nat_start[i];
+                ng = d.go_cnt[i];
+            }
+            if (qa) nq = min(d.qa.ref_cnt[i], QA_REF_CAP);
+        }
+        scan = cnt = ng + nl + nq;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int y = __shfl_up_sync(0xffffffffu, scan, o);
+            if (lane >= o) scan += y;
+        }
+        if (lane == 31) s.ws[t >> 5] = scan;
+        s.ng[t] = ng; s.nl[t] = nl; s.nat0[t] = nat0; s.rep[t] = r;
+        // a replica that has taken its steps keeps its state
+        if (MODE == 0) s.state[t] = r >= 0 ? 1 : -1;
+    }
+    if (t == 0) s.next = 0;
+    if (!__syncthreads_or(r >= 0)) return;   // no bead slot of the block is in use
+    int T = 0;
+#pragma unroll
+    for (int k = 0; k < FB / 32; ++k) T += s.ws[k];
+    if (t < FB) {
+        int base = 0;
+        for (int k = 0; k < (t >> 5); ++k) base += s.ws[k];
+        s.off[t] = base + scan - cnt;
+        if (t == FB - 1) s.off[FB] = T;
+        if (MODE == 1) s.state[t] = r < 0 ? -1 : (d.rep[r].steps_left == 0 ? 0 : 1);
+    }
+    __syncthreads();
+    if (qa) {
+        // the beads' contact slots (at most QA_REF_CAP, held QA_REF_CAP / LPB
+        // per thread of the bead) in ascending order, by rank
+        const int b = t / LPB, ln = t % LPB;
+        const unsigned qm = ((1u << LPB) - 1u) << (lane & ~(LPB - 1));
+        const int nref = s.off[b + 1] - s.off[b] - s.ng[b] - s.nl[b];
+        constexpr int HOLD = QA_REF_CAP / LPB;
+        int v[HOLD], rk[HOLD];
+#pragma unroll
+        for (int u = 0; u < HOLD; ++u) {
+            const int k = u * LPB + ln;
+            v[u] = k < nref ? d.qa.ref[(size_t)k * N + i0 + b] : INT_MAX;
+            rk[u] = 0;
+        }
+        for (int m = 0; m < nref; ++m) {
+            int x = 0;
+#pragma unroll
+            for (int u = 0; u < HOLD; ++u) {
+                const int y = __shfl_sync(qm, v[u], m % LPB, LPB);
+                if (m / LPB == u) x = y;
+            }
+#pragma unroll
+            for (int u = 0; u < HOLD; ++u) rk[u] += x < v[u];
+        }
+#pragma unroll
+        for (int u = 0; u < HOLD; ++u)
+            if (u * LPB + ln < nref) s_q[b][rk[u]] = v[u];
+        __syncthreads();
+    }
+
+    Ener<MODE> en;
+    en.start(s.rep[0]);
+    const V3<FT> z{FT(0), FT(0), FT(0)};
+    if (t < 2 * FB) {
+        // ---- B: bonds, cross products; noise
+        if (t < FB) {
+            const int k = t;
+            if constexpr (MIX) {
+                auto bond = [&](int a) {
+                    return V3<FF>{ff_diff(F2{s.p[0][a], s.p[3][a]}, F2{s.p[0][a + 1], s.p[3][a + 1]}),
+                                  ff_diff(F2{s.p[1][a], s.p[4][a]}, F2{s.p[1][a + 1], s.p[4][a + 1]}),
+                                  ff_diff(F2{s.p[2][a], s.p[5][a]}, F2{s.p[2][a + 1], s.p[5][a + 1]})};
+                };
+                const V3<FF> e = bond(k);
+                s.g[MEH][k] = e.x.h; s.g[MEH + 1][k] = e.y.h; s.g[MEH + 2][k] = e.z.h;
+                s.g[MEL][k] = e.x.l; s.g[MEL + 1][k] = e.y.l; s.g[MEL + 2][k] = e.z.l;
+                const V3<float> ef{e.x.h, e.y.h, e.z.h};
+                s.g[MRN][k] = rsq(fdot(ef, ef));
+                if (k > 0) {
+                    const V3<FF> x = ff_cross(bond(k - 1), e);
+                    s.g[MXH][k] = x.x.h; s.g[MXH + 1][k] = x.y.h; s.g[MXH + 2][k] = x.z.h;
+                    s.g[MXL][k] = x.x.l; s.g[MXL + 1][k] = x.y.l; s.g[MXL + 2][k] = x.z.l;
+                    const V3<float> xf{x.x.h, x.y.h, x.z.h};
+                    s.g[MRX][k] = rsq(fdot(xf, xf));
+                }
+            } else {
+                auto bond = [&](int a) {
+                    return V3<DN>{DN(s.p[0][a + 1]) - DN(s.p[0][a]), DN(s.p[1][a + 1]) - DN(s.p[1][a]),
+                                  DN(s.p[2][a + 1]) - DN(s.p[2][a])};
+                };
+                const V3<DN> e = bond(k);
+                const DN len = norm(e);
+                s.g[GE][k] = e.x.v; s.g[GE + 1][k] = e.y.v; s.g[GE + 2][k] = e.z.v;
+                s.g[GLEN][k] = len.v;
+                s.g[GRN][k] = (DN(1.0) / len).v;
+                if (k > 0) {
+                    const V3<DN> x = cross(bond(k - 1), e);
+                    const DN rx = ninv(x);
+                    s.g[GRX][k] = rx.v;
+                    s.g[GU][k] = (rx * x.x).v; s.g[GU + 1][k] = (rx * x.y).v; s.g[GU + 2][k] = (rx * x.z).v;
+                }
+            }
+        }
+        if (draws) {
+            // four draws per bead (normal_x2 then normal, lang_pc.cpp:15-16)
+            FT a, b, g;
+            if constexpr (MIX) noise3m(st0, &a, &b, &g);
+            else noise3(st0, &a, &b, &g);
+            s.n[0][bn] = a; s.n[1][bn] = b; s.n[2][bn] = g;
+            const int rb = s.rep[bn];
+            s.rng[bn] = rb >= 0 ? gf2_apply_nib(d.jump + JUMP_WORDS * rb, st0) : 0;
+        }
+        // the geometry is read by the warps of this part only
+        if constexpr (LPB == 4) asm volatile("bar.sync 1, %0;" ::"n"(2 * FB) : "memory");
+        else __syncthreads();
+
+        // ---- D: bonded centres
+        const int sp = sc + 1;
+        const bool own = MODE == 0 && c >= i0 && c < i0 + FBT && c < N;
+        const int rc = own ? s.rep[c - i0] : 0;
+        if (sc < NC && (LPB == 1 || t < FB)) {
+            V3<FT> ft = z, a1 = z, a2 = z, a3 = z;
+            bond_angle<FT, MODE, FB>(d, p, s.g, sp, fl, cp, own, rc, en, &ft, &a1, &a2, &a3);
+            s.c[0][sc] = ft.x; s.c[1][sc] = ft.y; s.c[2][sc] = ft.z;
+            s.c[3][sc] = a1.x; s.c[4][sc] = a1.y; s.c[5][sc] = a1.z;
+            s.c[6][sc] = a2.x; s.c[7][sc] = a2.y; s.c[8][sc] = a2.z;
+            s.c[9][sc] = a3.x; s.c[10][sc] = a3.y; s.c[11][sc] = a3.z;
+        }
+        if (sc < NC && (LPB == 1 || t >= FB)) {
+            V3<FT> q[4] = {z, z, z, z};
+            dihedral_chiral<FT, MODE, FB>(d, p, s.g, c, sp, fl, cp, own, rc, en, q);
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                s.c[12 + 3 * k][sc] = q[k].x; s.c[13 + 3 * k][sc] = q[k].y; s.c[14 + 3 * k][sc] = q[k].z;
+            }
+        }
+        if (MODE == 1 && qa && t < FBT && r >= 0) {
+            // n and h at this step's positions (precompute_nh.cpp:12-20) to
+            // FP32 accuracy, for the sift's FP32 decisions (which recompute
+            // them in FP64 near a threshold)
+            const int i = i0 + t;
+            const uint32_t fb = d.bflags[i];
+            V3<float> n{0.0f, 0.0f, 0.0f}, h{0.0f, 0.0f, 0.0f};
+            if ((fb & BF_PREV) && (fb & BF_NEXT)) {
+                const int s1 = t + 2, s2 = t + 3;    // bonds to the bead and from it
+                float dv[3];
+#pragma unroll
+                for (int a = 0; a < 3; ++a) {
+                    if constexpr (MIX) {
+                        const FF x1{s.g[MEH + a][s1], s.g[MEL + a][s1]}, x2{s.g[MEH + a][s2], s.g[MEL + a][s2]};
+                        dv[a] = ff_sub(x2, x1).h;
+                    } else {
+                        dv[a] = narrow_f(__dsub_rn(s.g[GE + a][s2], s.g[GE + a][s1]));
+                    }
+                }
+                n = unit_f(V3<float>{dv[0], dv[1], dv[2]});
+                if constexpr (MIX) {
+                    h = -unit_f(V3<float>{s.g[MXH][s2], s.g[MXH + 1][s2], s.g[MXH + 2][s2]});
+                } else {
+                    h = V3<float>{-narrow_f(s.g[GU][s2]), -narrow_f(s.g[GU + 1][s2]), -narrow_f(s.g[GU + 2][s2])};
+                }
+            }
+            float *nh = d.qa.nh;
+            nh[i] = n.x; nh[Ns + i] = n.y; nh[2 * Ns + i] = n.z;
+            nh[3 * Ns + i] = h.x; nh[4 * Ns + i] = h.y; nh[5 * Ns + i] = h.z;
+        }
+    }
+
+    // ---- E: pair entries, FCAP at a time; between the passes every (axis,
+    // bead) thread adds its bead's forces
+    ST acc[TT];
+    double y[TT][6], o[TT], sd[TT];
+    for (int p0 = 0;; p0 += FCAP) {
+        const int pe = min(T - p0, FCAP);
+        for (;;) {
+            int at = 0;
+            if (lane == 0) at = atomicAdd(&s.next, 32);
+            at = __shfl_sync(0xffffffffu, at, 0);
+            if (at >= pe) break;
+            if (at + lane < pe) {
+                const V3<FT> f = pair_entry<FT, MODE, FB>(d, p, cur, s, s_q, i0, p0 + at + lane, en);
+                s.f[0][at + lane] = f.x; s.f[1][at + lane] = f.y; s.f[2][at + lane] = f.z;
+            }
+        }
+        if (MODE == 1 && p0 == 0) {
+            // the integrator's state, on its way while the last entries finish
+#pragma unroll
+            for (int u = 0; u < TT; ++u) {
+                const int w = t + u * NT, a = w / FBT, b = w - a * FBT, i = i0 + b;
+                if (w >= 3 * FBT || i >= N || s.rep[b] < 0) continue;
+                y[u][0] = reinterpret_cast<const double *>(d.pos[cur] + i)[a];
+#pragma unroll
+                for (int q = 0; q < 5; ++q) y[u][q + 1] = d.yh[(size_t)(q * 3 + a) * Ns + i];
+                o[u] = reinterpret_cast<const double *>(d.orig + i)[a];
+                sd[u] = d.rep[s.rep[b]].noise_sd;
+            }
+        }
+        __syncthreads();
+#pragma unroll
+        for (int u = 0; u < TT; ++u) {
+            const int w = t + u * NT, a = w / FBT, b = w - a * FBT;
+            if (w >= 3 * FBT) continue;
+            if (p0 == 0) {
+                const int k = b + 2;   // centre slot of the bead
+                const FT v[9] = {s.c[a][k], -s.c[a][k - 1], s.c[9 + a][k - 1], s.c[6 + a][k], s.c[3 + a][k + 1],
+                                 s.c[12 + a][k + 1], s.c[15 + a][k], s.c[18 + a][k - 1], s.c[21 + a][k - 2]};
+                acc[u] = ST{};
+                if constexpr (MIX) {
+                    // FP32 contributions are summed in FP32 and enter once
+                    float x = v[0];
+#pragma unroll
+                    for (int q = 1; q < 9; ++q) x = __fadd_rn(x, v[q]);
+                    sum_acc(acc[u], x);
+                } else {
+#pragma unroll
+                    for (int q = 0; q < 9; ++q) sum_acc(acc[u], v[q]);
+                }
+            }
+            const int e1 = min(s.off[b + 1] - p0, FCAP);
+            for (int q = max(s.off[b] - p0, 0); q < e1; ++q) sum_acc(acc[u], s.f[a][q]);
+        }
+        if (p0 + FCAP >= T) break;
+        __syncthreads();
+        if (t == 0) s.next = 0;
+        __syncthreads();
+    }
+
+    // the rest of the bead's force: native disulfides, AFM pulls and walls
+    // (k_ext), pseudo-improper dihedral bundles (k_pid: the bead's own side
+    // and its chain neighbours' parts for it)
+    double F[TT];
+#pragma unroll
+    for (int u = 0; u < TT; ++u) {
+        const int w = t + u * NT, a = w / FBT, b = w - a * FBT, i = i0 + b;
+        F[u] = 0.0;
+        if (w >= 3 * FBT || s.state[b] != 1) continue;
+        if (p.on[XMD_TERM_NAT_SS]) {
+            const int s1 = d.ss_end[i];
+            for (int k = d.ss_start[i]; k < s1; ++k) {
+                if (!d.ss_on[k]) continue;
+                const int j = d.ss_j[k], rb = s.rep[b];
+                V3<FT> r12;
+                if constexpr (MIX) {
+                    F2 pa[3], pb[3];
+                    spl_load(d.spl[cur], i, pa);
+                    spl_load(d.spl[cur], j, pb);
+                    r12 = pair_vec(d.rep[rb], pa, pb);
+                } else {
+                    r12 = r_uv_p<double>(d.rep[rb].box, d.rep[rb].per_any != 0, d.pos[cur][i], d.pos[cur][j]);
+                }
+                FT V_;
+                const V3<FT> f = ss_pair<FT>(p, r12, &V_);
+                sum_acc(acc[u], a == 0 ? f.x : (a == 1 ? f.y : f.z));
+                if (MODE == 0 && i < j && a == 0) en.add(d, rb, XMD_TERM_NAT_SS, (double)V_);
+            }
+        }
+        F[u] = sum_total(acc[u]);
+        if (p.ext_on) F[u] += d.fext[3 * (size_t)i + a];
+        if (p.on[XMD_TERM_PID]) {
+            const double *pf = d.pid_f;
+            const uint32_t fb = d.bflags[i];
+            double g = pf[3 * (size_t)i + a];
+            if (fb & BF_PREV) g += pf[6 * Ns + 3 * (size_t)(i - 1) + a];   // next-bead part of i - 1
+            if (fb & BF_NEXT) g += pf[3 * Ns + 3 * (size_t)(i + 1) + a];   // previous-bead part of i + 1
+            F[u] += g;
+        }
+        if constexpr (MODE == 0) d.F[3 * (size_t)i + a] = F[u];
+        // a non-finite force: the replica is frozen from the next step on (its
+        // skin check sets steps_left = 0); this bead keeps its state, so no
+        // non-finite position ever reaches a list build
+        if (!finite_bits(F[u])) {
+            atomicOr(d.status, ST_NONFINITE);
+            if (MODE == 1) s.state[b] = 2;
+        }
+    }
+    if constexpr (MODE == 0) {
+        en.flush(d);
+    } else {
+        // ---- F: lang_pc_step::operator(), lang_pc.cpp:11-37, mass = 1
+        // (main.cpp:156): Gear-5 corrector, then the predictor's Taylor shift by
+        // repeated addition (15 additions)
+        __syncthreads();
+#pragma unroll
+        for (int u = 0; u < TT; ++u) {
+            const int w = t + u * NT, a = w / FBT, b = w - a * FBT, i = i0 + b;
+            if (w >= 3 * FBT || s.state[b] != 1) continue;
+            double nz;
+            if constexpr (MIX) nz = widen_f(s.n[a][b]);
+            else nz = s.n[a][b];
+            double(&q)[6] = y[u];
+            const double v = __dmul_rn(q[1], p.dt_inv);
+            const double acl = __fma_rn(sd[u], nz, __fma_rn(-p.gamma_factor, v, F[u]));
+            const double err = __fma_rn(-acl, p.dt2_half, q[2]);
+            q[0] = __fma_rn(-(3.0 / 16.0), err, q[0]);
+            q[1] = __fma_rn(-(251.0 / 360.0), err, q[1]);
+            q[2] = __dsub_rn(q[2], err);
+            q[3] = __fma_rn(-(11.0 / 18.0), err, q[3]);
+            q[4] = __fma_rn(-(1.0 / 6.0), err, q[4]);
+            q[5] = __fma_rn(-(1.0 / 60.0), err, q[5]);
+#pragma unroll
+            for (int m = 0; m < 5; ++m)
+#pragma unroll
+                for (int k = 4; k >= m; --k) q[k] = __dadd_rn(q[k], q[k + 1]);
+#pragma unroll
+            for (int k = 0; k < 5; ++k) d.yh[(size_t)(k * 3 + a) * Ns + i] = q[k + 1];
+            s.F[a][b] = q[0];
+            // skin test: norm(box->r_uv(r_, orig_r_)), verify.cpp:12-14, squared;
+            // the check takes one square root of the maximum (sqrt is monotone
+            // and correctly rounded, so that equals the max of the norms).
+            // Open axes wrap by exactly zero.  The mixed path squares the FP64
+            // difference in FP32.
+            double e = __dsub_rn(o[u], q[0]);
+            const RepDev &rp = d.rep[s.rep[b]];
+            if (rp.per_any)
+                e = __dsub_rn(e, __dmul_rn(rp.box.cell[a], rint(__dmul_rn(e, rp.box.cell_inv[a]))));
+            if constexpr (MIX) {
+                const float ef = narrow_f(e);
+                s.e[a][b] = __fmul_rn(ef, ef);
+            } else {
+                s.e[a][b] = __dmul_rn(e, e);
+            }
+        }
+        __syncthreads();
+
+        // ---- G: new positions, generator, skin-test displacement
+        if (t < FB) {
+            const int i = i0 + t, st = s.state[t];
+            double disp = 0.0;
+            if (st == 0 || st == 2) {
+                // the replica has taken its steps, or the bead keeps its state
+                if (st == 2) d.rep[r].fault = 1;
+                d.pos[cur ^ 1][i] = d.pos[cur][i];
+                if constexpr (MIX) {
+                    d.spl[cur ^ 1][2 * (size_t)i] = d.spl[cur][2 * (size_t)i];
+                    d.spl[cur ^ 1][2 * (size_t)i + 1] = d.spl[cur][2 * (size_t)i + 1];
+                }
+            } else if (st == 1) {
+                const FT q = s.p[MIX ? 6 : 3][t + 3];
+                double4_32a pn = make_double4_32a(s.F[0][t], s.F[1][t], s.F[2][t], 0.0);
+                if constexpr (MIX) {
+                    const P2 x = split_p(pn);
+                    pn.w = widen_f(q);
+                    d.spl[cur ^ 1][2 * (size_t)i] = make_float4(x.x.h, x.y.h, x.z.h, q);
+                    d.spl[cur ^ 1][2 * (size_t)i + 1] = make_float4(x.x.l, x.y.l, x.z.l, 0.0f);
+                    disp = widen_f(__fadd_rn(__fadd_rn(s.e[0][t], s.e[1][t]), s.e[2][t]));
+                } else {
+                    pn.w = q;
+                    disp = __dadd_rn(__dadd_rn(s.e[0][t], s.e[1][t]), s.e[2][t]);
+                }
+                d.pos[cur ^ 1][i] = pn;
+                d.rng[i] = s.rng[t];
+            }
+            // one atomic per warp where its beads are of one replica
+            const unsigned act = __ballot_sync(0xffffffffu, st == 1);
+            if (act) {
+                const int r0 = __shfl_sync(0xffffffffu, r, __ffs(act) - 1);
+                const unsigned long long db = (unsigned long long)__double_as_longlong(disp);
+                if (__all_sync(0xffffffffu, st != 1 || r == r0)) {
+                    const unsigned long long m = warp_max_bits(db);
+                    if (lane == 0) atomicMax(&d.rep[r0].maxdisp, m);
+                } else if (st == 1) {
+                    atomicMax(&d.rep[r].maxdisp, db);
+                }
+            }
+        }
+    }
+}
+
+}  // namespace xmdg
