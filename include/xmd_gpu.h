@@ -421,8 +421,8 @@ int xmd_gpu_server_destroy(xmd_gpu_server *srv);
  * (i, j) order, at most `cap` pairs; *d_count receives the number found.
  * When that number exceeds cap, d_pairs holds the first cap pairs of the
  * full (i, j)-ordered list.  d_r = positions [3n], d_chain / d_seq = [n];
- * cell = host array, 0 = open along that axis.  Each bead's row is kept sorted
- * by insertion in one thread, O(m^2) for m partners: meant for Verlet-list
+ * cell = host array, 0 = open along that axis.  Rows of more than 512 partners
+ * are put in order by insertion, O(m^2) for m partners: meant for Verlet-list
  * densities, slow when most beads lie within the cutoff of most others.
  *
  * The first call on a device looks up the scratch's device address (once per

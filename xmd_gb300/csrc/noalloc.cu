@@ -15,15 +15,26 @@
 // The search itself is the one the engine runs at every Verlet rebuild:
 // pairs i < j, not in the same chain with |seq_i - seq_j| < 3
 // (legacy_update.cpp:24-26), whose minimum-image distance is below the
-// cutoff (legacy_update.cpp:28-29), in (i, j) order.  Cells of the cutoff's
-// edge are hashed into n buckets, which bounds the scratch by the bead count.
-// One thread builds one bead's row and keeps it sorted by insertion, so a row
-// of m partners costs O(m^2): cheap at Verlet-list densities (tens to a few
-// hundred partners), slow when most beads are within the cutoff of most
-// others (a periodic box under two cutoffs wide, a cluster much denser than
-// a protein).
+// cutoff (legacy_update.cpp:28-29), in (i, j) order.
+//
+// Eight launches, all over the whole grid: bounds and grid, bucket counts,
+// their scan, the bucket sort (with FP32 coordinates beside the indices), row
+// counts, their scan, the rows.  Rows are bound by instruction issue: one warp
+// takes one bead, in bucket order, and its lanes the candidates of the
+// neighbouring buckets 32 at a time, so a bead's latency chain is a few
+// rounds instead of one candidate after another.  A candidate is decided in
+// FP32 unless its distance lies in the FP32 error band around the cutoff,
+// where the FP64 test decides (GB300 runs an FP64 warp instruction over 16
+// cycles; FP64 throughout would make the search FP64-bound).  A row of up to
+// NA_ROW partners is put in order by rank in shared memory; a longer one by
+// insertion in global memory, O(m^2) for m partners (a periodic box under two
+// cutoffs wide, a cluster much denser than a protein).
+//
+// 30,720 beads at 1e-3 A^-3, cutoff 20 A: 3,200 us -> 122 us (one block for
+// the grid took 250 us of it, and one thread per row, twice, 1,500 us each).
 #include <cuda_runtime.h>
 
+#include <climits>
 #include <cstdint>
 #include <mutex>
 #include <stdexcept>
@@ -36,19 +47,25 @@ namespace xmdg {
 namespace {
 
 constexpr int NA_MAX = XMD_NOALLOC_MAX_BEADS;   // beads, and buckets
-constexpr int NA_BLOCK = 1024;
+constexpr int NA_SCAN = 1024;                   // elements per scan block
+constexpr int NA_PARTS = NA_MAX / NA_SCAN;
+constexpr int NA_ROW = 512;                     // partners of a row ordered in shared memory
+constexpr int NA_WARPS = 8;
+constexpr int NA_PACK = 1023;                   // cell coordinates that fit the packed form
 
-struct NaScratch {
-    int bucket_cnt[NA_MAX];
-    int bucket_start[NA_MAX];
-    int bucket_fill[NA_MAX];
-    int items[NA_MAX];
-    int bead_bucket[NA_MAX];
-    int row_cnt[NA_MAX];
-    int row_off[NA_MAX];
+struct __align__(16) NaScratch {
+    int start[NA_MAX];     // bucket counts, then starts within their scan block
+    int row[NA_MAX];       // sort cursors per bucket; then row counts, then row offsets within their scan block
+    float4 items[NA_MAX];  // beads in bucket order: FP32 coordinates and the bead's index
+    int cell[NA_MAX];      // packed cell coordinates of each bead (or its bucket, when they do not fit)
+    int start_base[NA_PARTS], row_base[NA_PARTS], part[NA_PARTS];
+    unsigned long long lo_key[3], hi_key[3];
+    unsigned done[3];
     // grid of the current call
-    int per[3], dims[3], nbuckets;
-    double lo[3], inv_edge, cell[3], cell_inv[3];
+    int per[3], dims[3], nbuckets, direct, packed;
+    int far;               // some bead lies so many boxes away that its wrapped FP32 coordinate is off
+    double lo[3], inv_edge, box[3], box_inv[3];
+    float blo, bhi, L[3];  // FP32 decision band of the squared distance; box lengths
 };
 
 // The scratch.  Every call reuses it and leaves its contents behind; each
@@ -57,9 +74,18 @@ struct NaScratch {
 // race on it.
 static __device__ __align__(256) NaScratch g_na_scratch;
 
+// doubles as unsigned integers of the same order
+__device__ __forceinline__ unsigned long long na_key_of(double x) {
+    const unsigned long long u = (unsigned long long)__double_as_longlong(x);
+    return (u >> 63) ? ~u : u | 0x8000000000000000ull;
+}
+__device__ __forceinline__ double na_of_key(unsigned long long k) {
+    return __longlong_as_double((long long)((k >> 63) ? k & 0x7fffffffffffffffull : ~k));
+}
+
 __device__ __forceinline__ int na_coord(const NaScratch &s, int a, double x) {
     if (s.per[a]) {
-        double f = x * s.cell_inv[a];
+        double f = x * s.box_inv[a];
         f -= floor(f);
         int k = (int)(f * s.dims[a]);
         return k < 0 ? 0 : (k >= s.dims[a] ? s.dims[a] - 1 : k);
@@ -67,171 +93,341 @@ __device__ __forceinline__ int na_coord(const NaScratch &s, int a, double x) {
     int k = (int)floor((x - s.lo[a]) * s.inv_edge);
     return k < 0 ? 0 : k;
 }
-__device__ __forceinline__ int na_key(const NaScratch &s, int cx, int cy, int cz) {
+// bucket of a cell: the cell itself on a grid that is periodic along every
+// axis and fits, hashed otherwise
+__device__ __forceinline__ int na_bucket(const NaScratch &s, int cx, int cy, int cz) {
+    if (s.direct) return (cz * s.dims[1] + cy) * s.dims[0] + cx;
     uint32_t h = (uint32_t)cx * 73856093u ^ (uint32_t)cy * 19349663u ^ (uint32_t)cz * 83492791u;
-    return (int)(h % (uint32_t)s.nbuckets);
+    h ^= h >> 15;
+    return (int)(h & (uint32_t)(s.nbuckets - 1));
 }
 __device__ __forceinline__ double na_dist(const NaScratch &s, const double *r, int i, int j) {
     double d[3];
 #pragma unroll
     for (int a = 0; a < 3; ++a) {
         double x = __dsub_rn(r[3 * j + a], r[3 * i + a]);
-        d[a] = __dsub_rn(x, __dmul_rn(s.cell[a], rint(__dmul_rn(x, s.cell_inv[a]))));
+        d[a] = __dsub_rn(x, __dmul_rn(s.box[a], rint(__dmul_rn(x, s.box_inv[a]))));
     }
     return __dsqrt_rn(__dadd_rn(__dadd_rn(__dmul_rn(d[0], d[0]), __dmul_rn(d[1], d[1])), __dmul_rn(d[2], d[2])));
 }
+__device__ __forceinline__ float na_image(float d, float L) {
+    const float h = 0.5f * L;
+    d = d > h ? d - L : d;
+    return d < -h ? d + L : d;
+}
 
-// grid, bucket counts, scan, fill and in-bucket order: one block
-__global__ void __launch_bounds__(NA_BLOCK) k_na_grid(NaScratch *s, const double *__restrict__ r, int n,
-                                                      double c0, double c1, double c2, double cutoff) {
-    const int t = threadIdx.x, lane = t & 31, w = t >> 5;
-    __shared__ double red[6][32];
-    __shared__ int scan_s[NA_BLOCK];
-    const double cellv[3] = {c0, c1, c2};
-    double lo[3] = {1e300, 1e300, 1e300};
-    for (int i = t; i < n; i += NA_BLOCK)
-        for (int a = 0; a < 3; ++a) lo[a] = fmin(lo[a], r[3 * i + a]);
+__global__ void __launch_bounds__(256) k_na_clear(NaScratch *s) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < NA_MAX) {
+        s->start[i] = 0;
+        s->row[i] = 0;
+    }
+    if (i == 0) s->far = 0;
+    if (i < 3) {
+        s->lo_key[i] = ~0ull;
+        s->hi_key[i] = 0ull;
+        s->done[i] = 0u;
+    }
+}
+
+// bounds along the open axes; the last block sets the grid and the FP32 band
+__global__ void __launch_bounds__(256) k_na_grid(NaScratch *s, const double *__restrict__ r, int n, double c0,
+                                                 double c1, double c2, double cutoff) {
+    const double cell[3] = {c0, c1, c2};
+    const int t = threadIdx.x, lane = t & 31;
+    __shared__ int last;
     for (int a = 0; a < 3; ++a) {
-        for (int o = 16; o; o >>= 1) lo[a] = fmin(lo[a], __shfl_xor_sync(0xffffffffu, lo[a], o));
-        if (lane == 0) red[a][w] = lo[a];
+        if (cell[a] != 0.0) continue;
+        double lo = 1e300, hi = -1e300;
+        for (int i = blockIdx.x * 256 + t; i < n; i += gridDim.x * 256) {
+            const double x = r[3 * i + a];
+            lo = fmin(lo, x);
+            hi = fmax(hi, x);
+        }
+        for (int o = 16; o; o >>= 1) {
+            lo = fmin(lo, __shfl_xor_sync(0xffffffffu, lo, o));
+            hi = fmax(hi, __shfl_xor_sync(0xffffffffu, hi, o));
+        }
+        if (lane == 0) {
+            atomicMin(&s->lo_key[a], na_key_of(lo));
+            atomicMax(&s->hi_key[a], na_key_of(hi));
+        }
     }
     __syncthreads();
     if (t == 0) {
-        const double edge = cutoff * (1.0 + 1e-9);
-        for (int a = 0; a < 3; ++a) {
-            double l = 1e300;
-            for (int q = 0; q < NA_BLOCK / 32; ++q) l = fmin(l, red[a][q]);
-            s->cell[a] = cellv[a];
-            s->cell_inv[a] = cellv[a] != 0.0 ? 1.0 / cellv[a] : 0.0;
-            s->per[a] = cellv[a] != 0.0;
-            int dm = s->per[a] ? (int)floor(cellv[a] / edge) : 0;
-            s->dims[a] = dm < 1 ? 1 : dm;
-            s->lo[a] = l;
+        __threadfence();
+        last = atomicAdd(&s->done[0], 1u) == gridDim.x - 1;
+    }
+    __syncthreads();
+    if (!last || t != 0) return;
+    __threadfence();
+    const double edge = cutoff * (1.0 + 1e-9);
+    double ext = cutoff;
+    bool direct = true, packed = true;
+    long long total = 1;
+    for (int a = 0; a < 3; ++a) {
+        s->box[a] = cell[a];
+        s->box_inv[a] = cell[a] != 0.0 ? 1.0 / cell[a] : 0.0;
+        s->per[a] = cell[a] != 0.0;
+        s->L[a] = (float)cell[a];
+        int dm = 1;
+        if (cell[a] != 0.0) {
+            const double q = floor(cell[a] / edge);
+            dm = q < 1.0 ? 1 : (q > 1e9 ? 1000000000 : (int)q);
+            ext = fmax(ext, cell[a]);
+            s->lo[a] = 0.0;
+        } else {
+            direct = false;
+            const double lo = na_of_key(*(volatile unsigned long long *)&s->lo_key[a]);
+            const double hi = na_of_key(*(volatile unsigned long long *)&s->hi_key[a]);
+            s->lo[a] = lo;
+            ext = fmax(ext, hi - lo);
+            packed = packed && (hi - lo) / edge < (double)(NA_PACK - 1);
         }
-        s->inv_edge = 1.0 / edge;
-        s->nbuckets = n > 0 ? n : 1;
+        packed = packed && dm <= NA_PACK;
+        s->dims[a] = dm;
+        total = total > NA_MAX ? total : total * dm;
     }
-    __syncthreads();
-    const int nb = s->nbuckets;
-    for (int c = t; c < nb; c += NA_BLOCK) {
-        s->bucket_cnt[c] = 0;
-        s->bucket_fill[c] = 0;
-    }
-    __syncthreads();
-    for (int i = t; i < n; i += NA_BLOCK) {
-        int k = na_key(*s, na_coord(*s, 0, r[3 * i]), na_coord(*s, 1, r[3 * i + 1]), na_coord(*s, 2, r[3 * i + 2]));
-        s->bead_bucket[i] = k;
-        atomicAdd(&s->bucket_cnt[k], 1);
-    }
-    __syncthreads();
-    const int chunk = (nb + NA_BLOCK - 1) / NA_BLOCK;
-    const int b0 = t * chunk, b1 = min(nb, b0 + chunk);
-    int sum = 0;
-    for (int c = b0; c < b1; ++c) sum += s->bucket_cnt[c];
-    scan_s[t] = sum;
-    __syncthreads();
-    for (int o = 1; o < NA_BLOCK; o <<= 1) {
-        int v = t >= o ? scan_s[t - o] : 0;
-        __syncthreads();
-        scan_s[t] += v;
-        __syncthreads();
-    }
-    int run = scan_s[t] - sum;
-    for (int c = b0; c < b1; ++c) {
-        s->bucket_start[c] = run;
-        run += s->bucket_cnt[c];
-    }
-    __syncthreads();
-    // the order inside a bucket is free: each row is ordered by j below
-    for (int i = t; i < n; i += NA_BLOCK) {
-        int k = s->bead_bucket[i];
-        s->items[s->bucket_start[k] + atomicAdd(&s->bucket_fill[k], 1)] = i;
-    }
+    s->inv_edge = 1.0 / edge;
+    s->direct = direct && total <= NA_MAX;
+    s->packed = packed;
+    int nb = 1024;
+    while (nb < 2 * n && nb < NA_MAX) nb *= 2;
+    s->nbuckets = s->direct ? (int)total : nb;
+    // FP32 coordinates of magnitude <= ext, each rounded once, give distances
+    // within 5e-7 ext (three axes, at most four roundings each, and the
+    // squares' three); the band is three times that.  Outside the range in
+    // which FP32 squares neither overflow nor vanish, the exact test decides
+    // every candidate.
+    const double m = 1.5e-6 * ext, a = cutoff - m, b = cutoff + m;
+    const bool in_range = ext < 1e15 && cutoff > 1e-12;
+    s->blo = in_range && a > 0.0 ? __double2float_rd(a * a) : -1.0f;
+    s->bhi = in_range ? __double2float_ru(b * b) : __int_as_float(0x7f800000);
 }
 
-// partners j > i of bead i; pass 0 counts, pass 1 writes then orders by j
-__global__ void __launch_bounds__(128) k_na_rows(NaScratch *s, const double *__restrict__ r,
-                                                 const int32_t *__restrict__ chain, const int32_t *__restrict__ seq,
-                                                 int n, double cutoff, int pass, int32_t *pairs, int cap) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+__device__ __forceinline__ int na_bucket_of(const NaScratch &s, int v) {
+    return s.packed ? na_bucket(s, v & 1023, (v >> 10) & 1023, (v >> 20) & 1023) : v;
+}
+__global__ void __launch_bounds__(256) k_na_count(NaScratch *s, const double *__restrict__ r, int n) {
+    const int i = blockIdx.x * 256 + threadIdx.x;
     if (i >= n) return;
-    int cc[3];
-    for (int a = 0; a < 3; ++a) cc[a] = na_coord(*s, a, r[3 * i + a]);
-    int keys[27], nk = 0;
-    for (int dz = -1; dz <= 1; ++dz)
-        for (int dy = -1; dy <= 1; ++dy)
-            for (int dx = -1; dx <= 1; ++dx) {
-                int c[3] = {cc[0] + dx, cc[1] + dy, cc[2] + dz};
-                bool skip = false;
-                for (int a = 0; a < 3; ++a) {
-                    if (s->per[a]) c[a] = ((c[a] % s->dims[a]) + s->dims[a]) % s->dims[a];
-                    else if (c[a] < 0) skip = true;
-                }
-                if (skip) continue;
-                int key = na_key(*s, c[0], c[1], c[2]);
-                bool dup = false;
-                for (int q = 0; q < nk; ++q) dup |= keys[q] == key;
-                if (!dup) keys[nk++] = key;
-            }
-    const int ci = chain[i], si = seq[i];
-    int cnt = 0;
-    // pass 1: the row's m smallest partners (m = what fits below cap: all of
-    // them, except in the row that straddles cap), kept sorted by j with
-    // insertion as they are found, so the output is always the (i, j)-ordered
-    // prefix of the full list
-    const int base = pass ? s->row_off[i] : 0;
-    const int m = pass ? min(s->row_cnt[i], max(0, cap - base)) : 0;
-    int32_t *row = pairs + 2 * (size_t)base;
-    int kept = 0;
-    for (int kk = 0; kk < nk; ++kk) {
-        const int q0 = s->bucket_start[keys[kk]], q1 = q0 + s->bucket_cnt[keys[kk]];
-        for (int q = q0; q < q1; ++q) {
-            int j = s->items[q];
-            if (j <= i) continue;
-            int sj = seq[j];
-            int df = si > sj ? si - sj : sj - si;
-            if (chain[j] == ci && df < 3) continue;
-            if (!(na_dist(*s, r, i, j) < cutoff)) continue;
-            ++cnt;
-            if (m == 0 || (kept == m && j >= row[2 * (m - 1) + 1])) continue;
-            int y = kept < m ? kept : m - 1;   // the slot that opens (the largest drops out when full)
-            while (y > 0 && row[2 * (y - 1) + 1] > j) {
-                row[2 * y + 1] = row[2 * (y - 1) + 1];
-                --y;
-            }
-            row[2 * y + 1] = j;
-            if (kept < m) ++kept;
-        }
+    const int cx = na_coord(*s, 0, r[3 * i]), cy = na_coord(*s, 1, r[3 * i + 1]), cz = na_coord(*s, 2, r[3 * i + 2]);
+    const int b = na_bucket(*s, cx, cy, cz);
+    s->cell[i] = s->packed ? (cx & 1023) | (cy & 1023) << 10 | (cz & 1023) << 20 : b;
+    atomicAdd(&s->start[b], 1);
+    bool far = false;
+#pragma unroll
+    for (int a = 0; a < 3; ++a) far |= fabs(r[3 * i + a] * s->box_inv[a]) > 1e6;
+    if (far) s->far = 1;
+}
+
+// exclusive scan of v[0..m) within blocks of NA_SCAN elements; the last block
+// to finish scans the blocks' totals into base (and writes the grand total)
+__global__ void __launch_bounds__(256) k_na_scan(NaScratch *s, int rows, int m, int32_t *count) {
+    int *v = rows ? s->row : s->start, *base = rows ? s->row_base : s->start_base;
+    const int t = threadIdx.x, lane = t & 31, w = t >> 5;
+    __shared__ int ws[8], last;
+    const int e = blockIdx.x * NA_SCAN + 4 * t;
+    int q[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) q[k] = e + k < m ? v[e + k] : 0;
+    const int sum = q[0] + q[1] + q[2] + q[3];
+    int x = sum;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int y = __shfl_up_sync(0xffffffffu, x, o);
+        if (lane >= o) x += y;
     }
-    if (!pass) {
-        s->row_cnt[i] = cnt;
+    if (lane == 31) ws[w] = x;
+    __syncthreads();
+    int before = x - sum;
+    for (int k = 0; k < w; ++k) before += ws[k];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        if (e + k < m) v[e + k] = before;
+        before += q[k];
+    }
+    if (t == 255) s->part[blockIdx.x] = before;
+    __syncthreads();
+    if (t == 0) {
+        __threadfence();
+        last = atomicAdd(&s->done[1 + rows], 1u) == gridDim.x - 1;
+    }
+    __syncthreads();
+    if (!last || w != 0) return;
+    __threadfence();
+    int run = 0;
+    for (int k0 = 0; k0 < (int)gridDim.x; k0 += 32) {
+        const int k = k0 + lane;
+        const int p = k < (int)gridDim.x ? *(volatile int *)&s->part[k] : 0;
+        int y = p;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int u = __shfl_up_sync(0xffffffffu, y, o);
+            if (lane >= o) y += u;
+        }
+        if (k < (int)gridDim.x) base[k] = run + y - p;
+        run += __shfl_sync(0xffffffffu, y, 31);
+    }
+    if (lane == 0 && count) *count = run;
+}
+
+__device__ __forceinline__ int na_start(const NaScratch &s, int b) { return s.start[b] + s.start_base[b / NA_SCAN]; }
+
+// the order inside a bucket is free: each row is ordered by j below
+__global__ void __launch_bounds__(256) k_na_sort(NaScratch *s, const double *__restrict__ r, int n) {
+    const int i = blockIdx.x * 256 + threadIdx.x;
+    if (i >= n) return;
+    const int b = na_bucket_of(*s, s->cell[i]);
+    const int at = na_start(*s, b) + atomicAdd(&s->row[b], 1);
+    float f[3];
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+        const double x = r[3 * i + a];
+        f[a] = (float)(s->per[a] ? x - s->box[a] * floor(x * s->box_inv[a]) : x - s->lo[a]);
+    }
+    s->items[at] = make_float4(f[0], f[1], f[2], __int_as_float(i));
+}
+
+// partners j > i, one warp per bead; pass 0 counts, pass 1 writes the row in
+// order of j (its m smallest partners, m = what fits below cap, so that the
+// output is always the (i, j)-ordered prefix of the full list)
+template <int PASS>
+__global__ void __launch_bounds__(NA_WARPS * 32) k_na_rows(NaScratch *s, const double *__restrict__ r,
+                                                           const int32_t *__restrict__ chain,
+                                                           const int32_t *__restrict__ seq, int n, double cutoff,
+                                                           int32_t *pairs, int cap, const int32_t *count) {
+    const unsigned FULL = 0xffffffffu;
+    const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5;
+    const int slot = blockIdx.x * NA_WARPS + wp;
+    if (slot >= n) return;   // warp-uniform exits
+    __shared__ int buf[PASS ? NA_WARPS : 1][PASS ? NA_ROW : 1];
+    const float4 me = s->items[slot];
+    const int i = __float_as_int(me.w);
+    int base = 0, m = 0, rows = 0;
+    if (PASS) {
+        base = s->row[i] + s->row_base[i / NA_SCAN];
+        rows = (i + 1 < n ? s->row[i + 1] + s->row_base[(i + 1) / NA_SCAN] : *count) - base;
+        m = min(rows, max(0, cap - base));
+        if (m == 0) return;
+    }
+    const bool per = (s->per[0] | s->per[1] | s->per[2]) != 0;
+    const float Lx = s->L[0], Ly = s->L[1], Lz = s->L[2];
+    const float blo = s->far ? -1.0f : s->blo, bhi = s->far ? __int_as_float(0x7f800000) : s->bhi;
+    int cc[3];
+    if (s->packed) {
+        const int v = s->cell[i];
+        cc[0] = v & 1023; cc[1] = (v >> 10) & 1023; cc[2] = (v >> 20) & 1023;
+    } else {
+        for (int a = 0; a < 3; ++a) cc[a] = na_coord(*s, a, r[3 * i + a]);
+    }
+    // neighbouring buckets: lane l < 27 takes offsets (l % 3, l / 3 % 3, l / 9) - 1,
+    // the first lane of each bucket its range
+    int key = -1;
+    if (lane < 27) {
+        const int off[3] = {lane % 3 - 1, lane / 3 % 3 - 1, lane / 9 - 1};
+        bool ok = true;
+#pragma unroll
+        for (int a = 0; a < 3; ++a) {
+            int k = cc[a] + off[a];
+            if (s->per[a]) {
+                const int dm = s->dims[a];
+                k = k < 0 ? k + dm : (k >= dm ? k - dm : k);
+            } else if (k < 0) {
+                ok = false;
+            }
+            cc[a] = k;
+        }
+        if (ok) key = na_bucket(*s, cc[0], cc[1], cc[2]);
+    }
+    const unsigned same = __match_any_sync(FULL, key);
+    int q0 = 0, len = 0;
+    if (key >= 0 && (same & ((1u << lane) - 1u)) == 0u) {
+        q0 = na_start(*s, key);
+        len = (key + 1 < s->nbuckets ? na_start(*s, key + 1) : n) - q0;
+    }
+    int pre = len;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int y = __shfl_up_sync(FULL, pre, o);
+        if (lane >= o) pre += y;
+    }
+    const int total = __shfl_sync(FULL, pre, 31);
+    pre -= len;
+    q0 -= pre;
+    const int ci = chain[i], si = seq[i];
+    int32_t *const row = pairs + 2 * (size_t)base;
+    const bool long_row = PASS && rows > NA_ROW;
+    int cnt = 0, kept = 0;
+    for (int g0 = 0; g0 < total; g0 += 32) {
+        // candidate g lies in the bucket of the last lane that starts at or before it
+        const int g = g0 + lane;
+        int lo = 0;
+#pragma unroll
+        for (int h = 16; h; h >>= 1) {
+            const int pm = __shfl_sync(FULL, pre, lo + h);
+            if (pm <= g) lo += h;
+        }
+        const int q = __shfl_sync(FULL, q0, lo) + g;
+        bool hit = false;
+        int j = -1;
+        if (g < total) {
+            const float4 f = s->items[q];
+            j = __float_as_int(f.w);
+            if (j > i) {
+                float dx = f.x - me.x, dy = f.y - me.y, dz = f.z - me.z;
+                if (per) {
+                    dx = na_image(dx, Lx);
+                    dy = na_image(dy, Ly);
+                    dz = na_image(dz, Lz);
+                }
+                const float d2 = dx * dx + dy * dy + dz * dz;
+                if (!(d2 > bhi)) {
+                    const int sj = seq[j], df = si > sj ? si - sj : sj - si;
+                    if (!(chain[j] == ci && df < 3)) hit = d2 < blo || na_dist(*s, r, i, j) < cutoff;
+                }
+            }
+        }
+        unsigned bm = __ballot_sync(FULL, hit);
+        if (PASS && !long_row) {
+            if (hit) buf[wp][cnt + __popc(bm & ((1u << lane) - 1u))] = j;
+        } else if (PASS) {
+            // insertion, the row's m smallest kept in order
+            for (; bm; bm &= bm - 1) {
+                const int jj = __shfl_sync(FULL, j, __ffs(bm) - 1);
+                if (lane != 0) continue;
+                if (kept == m && jj >= row[2 * (m - 1) + 1]) continue;
+                int y = kept < m ? kept : m - 1;
+                while (y > 0 && row[2 * (y - 1) + 1] > jj) {
+                    row[2 * y + 1] = row[2 * (y - 1) + 1];
+                    --y;
+                }
+                row[2 * y + 1] = jj;
+                if (kept < m) ++kept;
+            }
+            continue;
+        }
+        cnt += __popc(bm);
+    }
+    if (!PASS) {
+        if (lane == 0) s->row[i] = cnt;
         return;
     }
-    for (int x = 0; x < m; ++x) row[2 * x] = i;
-}
-
-// exclusive scan of the row counts; total to the caller's counter
-__global__ void __launch_bounds__(NA_BLOCK) k_na_scan(NaScratch *s, int n, int32_t *count) {
-    const int t = threadIdx.x;
-    __shared__ int scan_s[NA_BLOCK];
-    const int chunk = (n + NA_BLOCK - 1) / NA_BLOCK;
-    const int i0 = t * chunk, i1 = min(n, i0 + chunk);
-    int sum = 0;
-    for (int i = i0; i < i1; ++i) sum += s->row_cnt[i];
-    scan_s[t] = sum;
-    __syncthreads();
-    for (int o = 1; o < NA_BLOCK; o <<= 1) {
-        int v = t >= o ? scan_s[t - o] : 0;
-        __syncthreads();
-        scan_s[t] += v;
-        __syncthreads();
+    __syncwarp();
+    if (long_row) {
+        for (int k = lane; k < m; k += 32) row[2 * k] = i;
+        return;
     }
-    int run = scan_s[t] - sum;
-    for (int i = i0; i < i1; ++i) {
-        s->row_off[i] = run;
-        run += s->row_cnt[i];
+    // each partner's rank among the row's is its place
+    for (int k0 = 0; k0 < cnt; k0 += 32) {
+        const int k = k0 + lane, v = k < cnt ? buf[wp][k] : INT_MAX;
+        int rank = 0;
+        for (int u = 0; u < cnt; ++u) rank += buf[wp][u] < v;
+        if (k < cnt && rank < m) {
+            row[2 * rank] = i;
+            row[2 * rank + 1] = v;
+        }
     }
-    if (t == NA_BLOCK - 1) *count = scan_s[t];
 }
 
 // Device address of the scratch, looked up once per device with that device
@@ -268,11 +464,16 @@ int verlet_pairs_noalloc(const double *d_r, const int32_t *d_chain, const int32_
         if (e != cudaSuccess) throw std::runtime_error(std::string("CUDA error ") + cudaGetErrorString(e));
         return XMD_OK;
     }
-    k_na_grid<<<1, NA_BLOCK, 0, st>>>(s, d_r, n, cell[0], cell[1], cell[2], cutoff);
-    const int nb = (n + 127) / 128;
-    k_na_rows<<<nb, 128, 0, st>>>(s, d_r, d_chain, d_seq, n, cutoff, 0, d_pairs, cap);
-    k_na_scan<<<1, NA_BLOCK, 0, st>>>(s, n, d_count);
-    k_na_rows<<<nb, 128, 0, st>>>(s, d_r, d_chain, d_seq, n, cutoff, 1, d_pairs, cap);
+    const int nb = (n + 255) / 256, nw = (n + NA_WARPS - 1) / NA_WARPS;
+    const bool open = cell[0] == 0.0 || cell[1] == 0.0 || cell[2] == 0.0;
+    k_na_clear<<<NA_MAX / 256, 256, 0, st>>>(s);
+    k_na_grid<<<open ? nb : 1, 256, 0, st>>>(s, d_r, n, cell[0], cell[1], cell[2], cutoff);
+    k_na_count<<<nb, 256, 0, st>>>(s, d_r, n);
+    k_na_scan<<<NA_PARTS, 256, 0, st>>>(s, 0, NA_MAX, nullptr);
+    k_na_sort<<<nb, 256, 0, st>>>(s, d_r, n);
+    k_na_rows<0><<<nw, NA_WARPS * 32, 0, st>>>(s, d_r, d_chain, d_seq, n, cutoff, d_pairs, cap, d_count);
+    k_na_scan<<<(n + NA_SCAN - 1) / NA_SCAN, 256, 0, st>>>(s, 1, n, d_count);
+    k_na_rows<1><<<nw, NA_WARPS * 32, 0, st>>>(s, d_r, d_chain, d_seq, n, cutoff, d_pairs, cap, d_count);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) throw std::runtime_error(std::string("CUDA error ") + cudaGetErrorString(e));
     return XMD_OK;
