@@ -428,6 +428,10 @@ __device__ __forceinline__ void nl_check_block(const Dev &d, int advance, double
         if (advance && left == 0 && !first) rb = 0;   // no further step uses a list
         rp.rebuild = rb;
         any |= rb;
+        if (rb && !tile) {   // the cell build's bounding box starts empty
+#pragma unroll
+            for (int a = 0; a < 3; ++a) { rp.lo_key[a] = 0xffffffffu; rp.hi_key[a] = 0u; }
+        }
         // the tile build's work list: every chunk of the flagged replicas
         // (order is free: each chunk writes its own rows)
         if (rb && tile) {
@@ -553,241 +557,278 @@ __device__ __forceinline__ Band make_band(double T, double m) {
 }
 __device__ __forceinline__ bool in_band(const Band &B, float d2) { return d2 >= B.lo && d2 <= B.hi; }
 
-// ---- cell lists: one block per flagged replica -----------------------------------
-// Cells have an edge of at least the Verlet radius.  Periodic axes are cut
-// into dims = floor(L / r) cells (wrapped); open axes count cells from the
-// bounding-box minimum without bound.  When every axis is periodic and the
-// grid fits the replica's bucket budget, a cell IS a bucket; otherwise cells
-// are hashed into the budget (chains in open space occupy few of their
+// ---- cell lists of the flagged replicas ---------------------------------------------
+// Two grids per replica.  The near grid holds every bead, with cells of at
+// least the largest radius of the terms that act between any two beads
+// (Pauli, quasi-adiabatic, PID; each with the pad).  The far grid holds the
+// charged beads, with cells of at least the electrostatic radius: only pairs of
+// charged beads are kept beyond the near radius.  One grid at the list radius
+// would give every bead the candidates of 27 cells of 25 A, ten times as many
+// as the two grids do at 1e-3 beads per A^3 and a fifth of the beads charged.
+//
+// Periodic axes are cut into dims = floor(L / r) cells (wrapped); open axes
+// count cells from the bounding-box minimum without bound.  When every axis is
+// periodic and the grid fits its bucket budget, a cell IS a bucket; otherwise
+// cells are hashed into the budget (chains in open space occupy few of their
 // bounding box's cells).  Buckets are visited once each, so collisions only
 // add candidates; the exact distance test decides.
-__device__ __forceinline__ int cell_coord(const RepDev &rp, int a, double x) {
+enum : int { CG_NEAR = 0, CG_FAR = 1 };
+constexpr int CELL_PACK = 1023;   // cell coordinates that fit the packed form
+constexpr int CELL_SCAN = 1024;   // buckets per block of the scan
+constexpr int CELL_CHARGED = 1 << 31;
+
+__device__ __forceinline__ int cell_coord(const RepDev &rp, int g, int a, double x) {
     if (rp.per[a]) {
         double f = x * rp.box.cell_inv[a];
         f -= floor(f);
-        int k = (int)(f * rp.dims[a]);
-        return k < 0 ? 0 : (k >= rp.dims[a] ? rp.dims[a] - 1 : k);
+        int k = (int)(f * rp.dims[g][a]);
+        return k < 0 ? 0 : (k >= rp.dims[g][a] ? rp.dims[g][a] - 1 : k);
     }
-    int k = (int)floor((x - rp.lo[a]) * rp.cs[a]);   // cs holds 1 / cell edge on open axes
+    int k = (int)floor((x - rp.lo[a]) * rp.cs[g]);   // cs holds 1 / cell edge on open axes
     return k < 0 ? 0 : k;
 }
-__device__ __forceinline__ int cell_key(const RepDev &rp, int cx, int cy, int cz) {
-    if (!rp.hashed) return (cz * rp.dims[1] + cy) * rp.dims[0] + cx;
+// bucket of a cell in the pool: the near grids of all replicas first, then the
+// far grids, each half the size
+__device__ __forceinline__ int cell_bucket(const Dev &d, const RepDev &rp, int g, int cx, int cy, int cz) {
+    const int off = g == CG_NEAR ? rp.cell_off : d.ncells_near + rp.cell_off / 2;
+    if (!rp.hashed[g]) return off + (cz * rp.dims[g][1] + cy) * rp.dims[g][0] + cx;
     uint32_t h = (uint32_t)cx * 73856093u ^ (uint32_t)cy * 19349663u ^ (uint32_t)cz * 83492791u;
-    return (int)(h % (uint32_t)rp.cell_budget);
+    h = (h ^ (h >> 15)) * 0x9e3779b1u;
+    return off + (int)__umulhi(h, (uint32_t)(g == CG_NEAR ? rp.cell_budget : rp.cell_budget / 2));
 }
-// FP32 coordinate for the pre-filter: wrapped into [0, L) or taken from the
-// bounding-box minimum
-__device__ __forceinline__ float rel_coord(const RepDev &rp, int a, double x) {
-    if (rp.per[a]) return (float)(x - rp.box.cell[a] * floor(x * rp.box.cell_inv[a]));
-    return (float)(x - rp.lo[a]);
-}
-__device__ __forceinline__ double comp(double4_32a v, int a) { return a == 0 ? v.x : (a == 1 ? v.y : v.z); }
-
-constexpr int CB = 1024;
-__global__ void __launch_bounds__(CB) k_cells(Dev d, int cur) {
-    const int r = blockIdx.x;
-    if (r == 0 && threadIdx.x == 0) atomicAdd(d.ctr, 1ull);
-    RepDev &rp = d.rep[r];
-    if (!rp.active || !rp.rebuild || rp.tile) return;
-    const double4_32a *pos = d.pos[cur];
-    const int b = rp.begin, n = rp.n, off = rp.cell_off, bud = rp.cell_budget;
-    __shared__ double red_lo[3][32], red_hi[3][32];
-    const int t = threadIdx.x, lane = t & 31, w = t >> 5;
-
-    // bounding box along open axes (none in a fully periodic box); four
-    // loads in flight per thread
-    double lo[3] = {1e300, 1e300, 1e300}, hi[3] = {-1e300, -1e300, -1e300};
-    const bool any_open = !(rp.per[0] && rp.per[1] && rp.per[2]);
-    for (int i0 = b + t; any_open && i0 < b + n; i0 += 4 * CB) {
-        double4_32a q[4];
-#pragma unroll
-        for (int u = 0; u < 4; ++u) q[u] = pos[min(i0 + u * CB, b + n - 1)];   // repeats are harmless
-#pragma unroll
-        for (int u = 0; u < 4; ++u)
-            for (int a = 0; a < 3; ++a) {
-                lo[a] = fmin(lo[a], comp(q[u], a));
-                hi[a] = fmax(hi[a], comp(q[u], a));
-            }
-    }
-    for (int a = 0; a < 3; ++a) {
-        for (int o = 16; o; o >>= 1) {
-            lo[a] = fmin(lo[a], __shfl_xor_sync(0xffffffffu, lo[a], o));
-            hi[a] = fmax(hi[a], __shfl_xor_sync(0xffffffffu, hi[a], o));
-        }
-        if (lane == 0) { red_lo[a][w] = lo[a]; red_hi[a][w] = hi[a]; }
-    }
-    __syncthreads();
-    if (t == 0) {
-        const double rr = rp.req_r * (1.0 + 1e-9);
-        long total = 1;
-        bool all_per = true;
-        double ext = 0.0;
-        for (int a = 0; a < 3; ++a) {
-            double l = 1e300, hh = -1e300;
-            for (int q = 0; q < CB / 32; ++q) { l = fmin(l, red_lo[a][q]); hh = fmax(hh, red_hi[a][q]); }
-            if (rp.per[a]) {
-                int dm = (int)floor(rp.box.cell[a] / rr);
-                dm = dm < 1 ? 1 : (dm > 4096 ? 4096 : dm);
-                rp.dims[a] = dm;
-                rp.lo[a] = 0.0;
-                rp.cs[a] = 0.0;
-                total *= dm;
-                ext = fmax(ext, rp.box.cell[a]);
-            } else {
-                all_per = false;
-                rp.dims[a] = 0;
-                rp.lo[a] = l;
-                rp.cs[a] = 1.0 / rr;
-                ext = fmax(ext, hh - l);
-            }
-        }
-        rp.hashed = !(all_per && total <= bud);
-        // FP32 error bound of a distance (see band_margin); the pre-filter
-        // radius req_r + m never rejects a pair inside req_r
-        rp.band_m = band_margin(fmax(ext, rp.req_r));
-        double m = rp.req_r + rp.band_m;
-        rp.pre2 = __double2float_ru(m * m);
-        const double T[5] = {rp.req_r, 1.0 / rp.pauli_min_inv, 1.0 / rp.es_min_inv, 1.0 / rp.qa_min_inv,
-                             1.0 / rp.pid_min_inv};
-        for (int k = 0; k < 5; ++k) {
-            const Band B = make_band(T[k], rp.band_m);
-            rp.band_lo[k] = B.lo;
-            rp.band_hi[k] = B.hi;
-        }
-        rp.band_mf = __double2float_ru(rp.band_m);
-        rp.first = 0;
-        rp.rebuilds += 1;
-    }
-    __syncthreads();
-    const int ncell = rp.hashed ? bud : rp.dims[0] * rp.dims[1] * rp.dims[2];
-    for (int c = t; c < ncell; c += CB) {
-        d.cell_cnt[off + c] = 0;
-        d.cell_fill[off + c] = 0;
-    }
-}
-
-// The bucket sort of the flagged replicas, over the whole grid: count, scan
-// (one block per replica, over its buckets), scatter, then per bucket a
-// deterministic order (ascending bead index) and the FP32 coordinates.
 __device__ __forceinline__ bool cell_flagged(const Dev &d, int r) {
     if (r < 0) return false;
     const RepDev &rp = d.rep[r];
     return rp.active && rp.rebuild && !rp.tile;
 }
-__global__ void k_cell_count(Dev d, int cur) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+__device__ __forceinline__ int cell_start(const Dev &d, int c) { return d.cell_start[c] + d.cell_base[c / CELL_SCAN]; }
+// floats as unsigned integers of the same order
+__device__ __forceinline__ unsigned f_key(float x) {
+    const unsigned u = __float_as_uint(x);
+    return (u >> 31) ? ~u : u | 0x80000000u;
+}
+__device__ __forceinline__ float f_of_key(unsigned k) { return __uint_as_float((k >> 31) ? k & 0x7fffffffu : ~k); }
+
+// Bounding boxes along open axes, over the whole grid (in FP32: the minimum is
+// only the origin of the cells and of the FP32 coordinates, and coordinates
+// below it fall into cell 0); the last block then sets the grids and FP32
+// bands of the flagged replicas.  One block per replica took 138 us for one of
+// 54,744 beads.
+__global__ void __launch_bounds__(256) k_cells(Dev d, int cur) {
+    const int i = blockIdx.x * 256 + threadIdx.x;
+    __shared__ int last_s;
+    const int r = i < d.N ? d.rep_of[i] : -1;
+    const bool on = cell_flagged(d, r) && !(d.rep[r].per[0] && d.rep[r].per[1] && d.rep[r].per[2]);
+    const unsigned act = __ballot_sync(0xffffffffu, on);
+    if (on) {
+        const double4_32a q = d.pos[cur][i];
+        const unsigned m = __match_any_sync(act, r);
+        const bool lead = (threadIdx.x & 31) == __ffs(m) - 1;
+        const float x[3] = {narrow_f(q.x), narrow_f(q.y), narrow_f(q.z)};
+#pragma unroll
+        for (int a = 0; a < 3; ++a) {
+            const unsigned lo = __reduce_min_sync(m, f_key(x[a])), hi = __reduce_max_sync(m, f_key(x[a]));
+            if (lead) {
+                atomicMin(&d.rep[r].lo_key[a], lo);
+                atomicMax(&d.rep[r].hi_key[a], hi);
+            }
+        }
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        __threadfence();
+        last_s = atomicAdd(&d.ctr[3], 1ull) == (unsigned long long)(gridDim.x - 1);
+    }
+    __syncthreads();
+    if (!last_s) return;
+    __threadfence();
+    if (threadIdx.x == 0) {
+        d.ctr[3] = 0ull;
+        atomicAdd(d.ctr, 1ull);
+    }
+    for (int k = threadIdx.x; k < d.R; k += 256) {
+        if (!cell_flagged(d, k)) continue;
+        RepDev &rp = d.rep[k];
+        bool all_per = true;
+        double ext = 0.0, span[3];
+        for (int a = 0; a < 3; ++a) {
+            span[a] = rp.box.cell[a];
+            if (!rp.per[a]) {
+                all_per = false;
+                const float lo = f_of_key(*(volatile unsigned *)&rp.lo_key[a]);
+                rp.lo[a] = (double)lo;
+                span[a] = (double)f_of_key(*(volatile unsigned *)&rp.hi_key[a]) - (double)lo;
+            } else {
+                rp.lo[a] = 0.0;
+            }
+            ext = fmax(ext, span[a]);
+        }
+        for (int g = 0; g < 2; ++g) {
+            const double rr = (g == CG_NEAR ? rp.r_near : rp.r_far) * (1.0 + 1e-9);
+            const int bud = g == CG_NEAR ? rp.cell_budget : rp.cell_budget / 2;
+            long long total = 1;
+            bool packed = true;
+            for (int a = 0; a < 3; ++a) {
+                int dm = 1;
+                if (rp.per[a]) {
+                    const double q = floor(rp.box.cell[a] / rr);
+                    dm = q < 1.0 ? 1 : (q > 4096.0 ? 4096 : (int)q);
+                    packed = packed && dm <= CELL_PACK;
+                } else {
+                    packed = packed && span[a] / rr < (double)(CELL_PACK - 2);
+                }
+                rp.dims[g][a] = dm;
+                total *= dm;
+            }
+            rp.cs[g] = 1.0 / rr;
+            rp.hashed[g] = !(all_per && total <= bud);
+            rp.packed[g] = packed;
+        }
+        // FP32 error bound of a distance (see band_margin)
+        rp.band_m = band_margin(fmax(ext * (1.0 + 1e-6), rp.req_r));
+        const double T[5] = {rp.req_r, 1.0 / rp.pauli_min_inv, 1.0 / rp.es_min_inv, 1.0 / rp.qa_min_inv,
+                             1.0 / rp.pid_min_inv};
+        for (int q = 0; q < 5; ++q) {
+            const Band B = make_band(T[q], rp.band_m);
+            rp.band_lo[q] = B.lo;
+            rp.band_hi[q] = B.hi;
+        }
+        const Band B = make_band(rp.s_near > 0.0 ? rp.r_near : 0.0, rp.band_m);
+        rp.near_lo = B.lo;
+        rp.near_hi = B.hi;
+        rp.band_mf = __double2float_ru(rp.band_m);
+        rp.first = 0;
+        rp.rebuilds += 1;
+    }
+}
+
+// bucket counts of both grids; cell_key keeps a bead's packed cell
+// coordinates (or its bucket, where they do not fit), -1 where it is in no cell
+__global__ void __launch_bounds__(256) k_cell_count(Dev d, int cur) {
+    const int i = blockIdx.x * 256 + threadIdx.x;
     if (i >= d.N) return;
     const int r = d.rep_of[i];
-    if (!cell_flagged(d, r)) return;
-    const RepDev &rp = d.rep[r];
-    const double4_32a q = d.pos[cur][i];
-    const int c = rp.cell_off + cell_key(rp, cell_coord(rp, 0, q.x), cell_coord(rp, 1, q.y), cell_coord(rp, 2, q.z));
-    d.bead_cell[i] = c;
-    atomicAdd(&d.cell_cnt[c], 1);
+    const bool on = cell_flagged(d, r);
+    int key[2] = {-1, -1};
+    if (on) {
+        const RepDev &rp = d.rep[r];
+        const double4_32a q = d.pos[cur][i];
+        for (int g = 0; g < 2; ++g) {
+            if (g == CG_FAR && !(rp.far && q.w != 0.0)) continue;
+            const int cx = cell_coord(rp, g, 0, q.x), cy = cell_coord(rp, g, 1, q.y), cz = cell_coord(rp, g, 2, q.z);
+            const int b = cell_bucket(d, rp, g, cx, cy, cz);
+            key[g] = rp.packed[g] ? cx | cy << 10 | cz << 20 : b;
+            atomicAdd(&d.cell_cnt[b], 1);
+        }
+    }
+    d.cell_key[i] = key[0];
+    d.cell_key[d.N + i] = key[1];
 }
-__global__ void __launch_bounds__(CB) k_cell_scan(Dev d) {
-    const int r = blockIdx.x;
-    if (!cell_flagged(d, r)) return;
-    const RepDev &rp = d.rep[r];
-    __shared__ int scan_s[CB];
-    const int t = threadIdx.x, off = rp.cell_off;
-    const int ncell = rp.hashed ? rp.cell_budget : rp.dims[0] * rp.dims[1] * rp.dims[2];
-    // exclusive scan of the counts, contiguous chunk per thread
-    const int chunk = (ncell + CB - 1) / CB;
-    const int c0 = t * chunk, c1 = min(ncell, c0 + chunk);
-    int sum = 0;
-    for (int c = c0; c < c1; ++c) sum += d.cell_cnt[off + c];
-    scan_s[t] = sum;
+// exclusive scan of the bucket counts within blocks of CELL_SCAN; the last
+// block to finish scans the blocks' totals into cell_base
+__global__ void __launch_bounds__(256) k_cell_scan(Dev d) {
+    const int t = threadIdx.x, lane = t & 31, w = t >> 5;
+    __shared__ int ws[8], last_s;
+    const int e = blockIdx.x * CELL_SCAN + 4 * t;
+    int q[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) q[k] = e + k < d.ncells ? d.cell_cnt[e + k] : 0;
+    const int sum = q[0] + q[1] + q[2] + q[3];
+    int x = sum;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int y = __shfl_up_sync(0xffffffffu, x, o);
+        if (lane >= o) x += y;
+    }
+    if (lane == 31) ws[w] = x;
     __syncthreads();
-    for (int o = 1; o < CB; o <<= 1) {
-        int v = t >= o ? scan_s[t - o] : 0;
-        __syncthreads();
-        scan_s[t] += v;
-        __syncthreads();
+    int before = x - sum;
+    for (int k = 0; k < w; ++k) before += ws[k];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        if (e + k < d.ncells) d.cell_start[e + k] = before;
+        before += q[k];
     }
-    int run = rp.begin + scan_s[t] - sum;
-    for (int c = c0; c < c1; ++c) {
-        d.cell_start[off + c] = run;
-        run += d.cell_cnt[off + c];
+    if (t == 255) d.cell_base[blockIdx.x] = before;
+    __syncthreads();
+    if (t == 0) {
+        __threadfence();
+        last_s = atomicAdd(&d.ctr[3], 1ull) == (unsigned long long)(gridDim.x - 1);
     }
+    __syncthreads();
+    if (!last_s || w != 0) return;
+    __threadfence();
+    if (t == 0) d.ctr[3] = 0ull;
+    int run = 0;
+    for (int k0 = 0; k0 < (int)gridDim.x; k0 += 32) {
+        const int k = k0 + lane;
+        const int p = k < (int)gridDim.x ? *(volatile int *)&d.cell_base[k] : 0;
+        int y = p;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int u = __shfl_up_sync(0xffffffffu, y, o);
+            if (lane >= o) y += u;
+        }
+        if (k < (int)gridDim.x) d.cell_base[k] = run + y - p;
+        run += __shfl_sync(0xffffffffu, y, 31);
+    }
+    if (lane == 0) d.cell_base[gridDim.x] = run;
 }
-__global__ void k_cell_scatter(Dev d) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+__device__ __forceinline__ int cell_bucket_of(const Dev &d, const RepDev &rp, int g, int key) {
+    return rp.packed[g] ? cell_bucket(d, rp, g, key & 1023, (key >> 10) & 1023, (key >> 20) & 1023) : key;
+}
+// the sort leaves every count at zero, for the next build
+__global__ void __launch_bounds__(256) k_cell_scatter(Dev d) {
+    const int i = blockIdx.x * 256 + threadIdx.x;
     if (i >= d.N) return;
-    if (!cell_flagged(d, d.rep_of[i])) return;
-    const int c = d.bead_cell[i];
-    const int slot = atomicAdd(&d.cell_fill[c], 1);
-    d.cell_items[d.cell_start[c] + slot] = i;
-}
-// one warp per bucket of the pool: the bucket's beads put in ascending index
-// order (each item's rank among the bucket's items; buckets of more than
-// 8 x 32 beads are sorted by one lane), then their FP32 coordinates
-constexpr int CF_WARPS = 8, CF_HOLD = 8;
-__global__ void __launch_bounds__(CF_WARPS * 32) k_cell_finish(Dev d, int cur) {
-    const int lane = threadIdx.x & 31;
-    const int c = blockIdx.x * CF_WARPS + (threadIdx.x >> 5);
-    if (c >= d.ncells) return;   // warp-uniform exits
-    const int r = d.cell_rep[c];
-    if (!cell_flagged(d, r)) return;
-    const RepDev &rp = d.rep[r];
-    const int ncell = rp.hashed ? rp.cell_budget : rp.dims[0] * rp.dims[1] * rp.dims[2];
-    if (c - rp.cell_off >= ncell) return;
-    const int s0 = d.cell_start[c], m = d.cell_cnt[c];
-    int *it = d.cell_items + s0;
-    const unsigned FULL = 0xffffffffu;
-    if (m <= 32 * CF_HOLD) {
-        int v[CF_HOLD], rk[CF_HOLD];
-#pragma unroll
-        for (int u = 0; u < CF_HOLD; ++u) {
-            v[u] = u * 32 + lane < m ? it[u * 32 + lane] : 0x7fffffff;
-            rk[u] = 0;
-        }
-        for (int k = 0; k < m; ++k) {
-            int x = 0;
-#pragma unroll
-            for (int u = 0; u < CF_HOLD; ++u)
-                if ((k >> 5) == u) x = __shfl_sync(FULL, v[u], k & 31);
-#pragma unroll
-            for (int u = 0; u < CF_HOLD; ++u) rk[u] += x < v[u];
-        }
-        __syncwarp();
-#pragma unroll
-        for (int u = 0; u < CF_HOLD; ++u)
-            if (u * 32 + lane < m) it[rk[u]] = v[u];
-    } else if (lane == 0) {
-        for (int x = 1; x < m; ++x) {
-            int vv = it[x], y = x - 1;
-            while (y >= 0 && it[y] > vv) { it[y + 1] = it[y]; --y; }
-            it[y + 1] = vv;
-        }
-    }
-    __syncwarp();
-    const double4_32a *pos = d.pos[cur];
-    for (int k = s0 + lane; k < s0 + m; k += 32) {
-        const int i = d.cell_items[k];
-        const double4_32a q = pos[i];
-        d.cell_pos[k] = make_float4(rel_coord(rp, 0, q.x), rel_coord(rp, 1, q.y), rel_coord(rp, 2, q.z),
-                                    __int_as_float(i));
-        d.cell_cs[k] = make_int2(d.chain[i], d.seq[i]);
-        d.bead_slot[i] = k;
+    for (int g = 0; g < 2; ++g) {
+        const int key = d.cell_key[(size_t)g * d.N + i];
+        if (key == -1) continue;
+        const int b = cell_bucket_of(d, d.rep[d.rep_of[i]], g, key);
+        d.cell_items[cell_start(d, b) + atomicSub(&d.cell_cnt[b], 1) - 1] = i;
     }
 }
-
-// ---- Verlet rows (legacy_update.cpp:16-62 + the update_* filters) ---------------
+// slots of a bucket
+__device__ __forceinline__ int cell_slots(const Dev &d) { return d.cell_base[(d.ncells + CELL_SCAN - 1) / CELL_SCAN]; }
+__device__ __forceinline__ int2 cell_range(const Dev &d, int b) {
+    return make_int2(cell_start(d, b), b + 1 < d.ncells ? cell_start(d, b + 1) : cell_slots(d));
+}
+// one thread per slot: the bead's rank among its bucket's is its place there
+// (a deterministic order), with its FP32 coordinates, wrapped into [0, L) or
+// taken from the bounding-box minimum
+__global__ void __launch_bounds__(256) k_cell_finish(Dev d, int cur) {
+    const int k = blockIdx.x * 256 + threadIdx.x;
+    if (k >= cell_slots(d)) return;
+    const int i = d.cell_items[k];
+    const RepDev &rp = d.rep[d.rep_of[i]];
+    // the near slots come first
+    const int g = k < cell_start(d, d.ncells_near) ? CG_NEAR : CG_FAR;
+    const int2 s = cell_range(d, cell_bucket_of(d, rp, g, d.cell_key[(size_t)g * d.N + i]));
+    int rank = 0;
+    for (int u = s.x; u < s.y; ++u) rank += d.cell_items[u] < i;
+    const double4_32a q = d.pos[cur][i];
+    const double x[3] = {q.x, q.y, q.z};
+    float f[3];
+#pragma unroll
+    for (int a = 0; a < 3; ++a)
+        f[a] = (float)(rp.per[a] ? x[a] - rp.box.cell[a] * floor(x[a] * rp.box.cell_inv[a]) : x[a] - rp.lo[a]);
+    d.cell_pos[s.x + rank] = make_float4(f[0], f[1], f[2], __int_as_float(q.w != 0.0 ? i | CELL_CHARGED : i));
+}
 
 // ---- Verlet rows of the cell build (legacy_update.cpp:16-62 + the update_*
-// filters), one warp per bead i --------------------------------------------------
+// filters), one warp per bead i, beads in bucket order ------------------------------
 // A pair is decided in FP32 when its FP32 distance is outside the bands of
 // the replica (k_cells: the list radius, r_excl + pad, 2D + pad, the QA
 // formation radius + pad, each widened by the FP32 error bound), and by the
-// exact FP64 test inside them.  The candidates of each neighbouring bucket
-// are taken 32 at a time by the lanes: loads of a bucket are contiguous, the
-// row is compacted by ballot, and the bead's latency chain is one bucket deep
-// instead of one candidate deep.  Buckets are visited z, then y, then x
-// offset (first occurrence of each key).  Quasi-adiabatic partners are ranked
-// by j within the warp at the end, so the free-pair source list is ordered as
-// update_free_pairs (free_pair.cpp:9-19) walks it.
+// exact FP64 test inside them.  The candidates of the neighbouring buckets are
+// taken 32 at a time by the lanes: the row is compacted by ballot, and the
+// bead's latency chain is a few rounds deep instead of one candidate deep.
+// The near grid gives every pair within the near radius, all its flags with it;
+// the far grid then, for a charged bead, the pairs beyond that radius.
+// Buckets are visited z, then y, then x offset (first occurrence of each
+// bucket).  Quasi-adiabatic partners are ranked by j within the warp at the
+// end, so the free-pair source list is ordered as update_free_pairs
+// (free_pair.cpp:9-19) walks it.
 // Go-list membership of a native contact of length nd (r < T = 2 nd + pad,
 // go.cpp:11-22): by the FP32 squared distance d2 outside a band around T
 // (directed rounding, widened by the narrowing error of T and by mf, the
@@ -831,77 +872,49 @@ __global__ void k_go_lists(Dev d, int b, int n) {
 constexpr int NC_WARPS = 8;
 __global__ void __launch_bounds__(NC_WARPS * 32, 4) k_nl_cells(Dev d, TermP p, int cur) {
     const int lane = threadIdx.x & 31;
-    const int i = blockIdx.x * NC_WARPS + (threadIdx.x >> 5);
-    if (i >= d.N) return;   // warp-uniform exits
-    const int r = d.rep_of[i];
-    if (r < 0) return;
-    const RepDev &rp = d.rep[r];
-    if (!rp.rebuild || rp.tile) return;
+    const int slot = blockIdx.x * NC_WARPS + (threadIdx.x >> 5);
+    if (slot >= cell_start(d, d.ncells_near)) return;   // warp-uniform: the near slots
+    const float4 me = d.cell_pos[slot];
+    const int i = __float_as_int(me.w) & ~CELL_CHARGED;
+    const bool charged = __float_as_int(me.w) < 0;
+    const RepDev &rp = d.rep[d.rep_of[i]];
     const double4_32a *pos = d.pos[cur];
     const double4_32a pi = pos[i];
-    const BoxD bx = rp.box;
     const int ci = d.chain[i], si = d.seq[i];
     const int n0 = d.nat_start[i], n1 = d.nat_end[i];
     const unsigned FULL = 0xffffffffu, lt = (1u << lane) - 1u;
-    const PairGeo<float> geo(bx, (rp.per[0] | rp.per[1] | rp.per[2]) != 0, pi);
-    const float mf = rp.band_mf;
+    const bool periodic = rp.per_any != 0;
 
     // Go list: update_go_contacts, go.cpp:11-22 (lanes over the natives)
     int ngo = 0;
-    for (int k0 = n0; k0 < n1; k0 += 32) {
-        const int k = k0 + lane;
-        bool on = false;
-        int j = 0;
-        double nd = 0.0;
-        if (k < n1) {
-            j = d.nat_j[k];
-            nd = d.nat_d[k];
-            const double4_32a pj = pos[j];
-            const V3<float> e = geo.to(pj);
-            on = go_listed(rp, bx, mf, nd, e.x * e.x + e.y * e.y + e.z * e.z, pi, pj);
+    if (n0 < n1) {
+        const PairGeo<float> geo(rp.box, periodic, pi);
+        for (int k0 = n0; k0 < n1; k0 += 32) {
+            const int k = k0 + lane;
+            bool on = false;
+            int j = 0;
+            double nd = 0.0;
+            if (k < n1) {
+                j = d.nat_j[k];
+                nd = d.nat_d[k];
+                const double4_32a pj = pos[j];
+                const V3<float> e = geo.to(pj);
+                on = go_listed(rp, rp.box, rp.band_mf, nd, e.x * e.x + e.y * e.y + e.z * e.z, pi, pj);
+            }
+            go_append(d, k, n0, n1, on, j, nd, ngo);
         }
-        go_append(d, k, n0, n1, on, j, nd, ngo);
     }
     if (lane == 0) d.go_cnt[i] = ngo;
 
-    // neighbouring buckets: lane l < 27 takes offsets (l/9, l/3 % 3, l % 3) - 1
-    int key = -1;
-    if (lane < 27) {
-        const int off[3] = {lane % 3 - 1, (lane / 3) % 3 - 1, lane / 9 - 1};
-        int cc[3];
-        bool ok = true;
-        for (int a = 0; a < 3; ++a) {
-            int k = cell_coord(rp, a, a == 0 ? pi.x : (a == 1 ? pi.y : pi.z)) + off[a];
-            if (rp.per[a]) k = ((k % rp.dims[a]) + rp.dims[a]) % rp.dims[a];
-            else if (k < 0) ok = false;
-            cc[a] = k;
-        }
-        if (ok) key = cell_key(rp, cc[0], cc[1], cc[2]);
-    }
-    // first occurrence of each key in lane order
-    const unsigned same = __match_any_sync(FULL, key);
-    const bool lead = key >= 0 && (same & lt) == 0u;
-    // each lead lane fetches its bucket's range up front
-    int kq0 = 0, kq1 = 0;
-    if (lead) {
-        const int c = rp.cell_off + key;
-        kq0 = d.cell_start[c];
-        kq1 = kq0 + d.cell_cnt[c];
-    }
-
-    const float4 me = d.cell_pos[d.bead_slot[i]];
-    const float mx = me.x, my = me.y, mz = me.z;
-    const float Lx = narrow_f(bx.cell[0]), Ly = narrow_f(bx.cell[1]), Lz = narrow_f(bx.cell[2]);
-    const bool periodic = (rp.per[0] | rp.per[1] | rp.per[2]) != 0;
-    const float pre2 = rp.pre2;
+    const float Lx = narrow_f(rp.box.cell[0]), Ly = narrow_f(rp.box.cell[1]), Lz = narrow_f(rp.box.cell[2]);
     const Band Breq{rp.band_lo[0], rp.band_hi[0]}, Bpa{rp.band_lo[1], rp.band_hi[1]};
     const Band Bes{rp.band_lo[2], rp.band_hi[2]}, Bqa{rp.band_lo[3], rp.band_hi[3]};
-    const Band Bpid{rp.band_lo[4], rp.band_hi[4]};
+    const Band Bpid{rp.band_lo[4], rp.band_hi[4]}, Bnear{rp.near_lo, rp.near_hi};
     const bool pauli_on = p.on[XMD_TERM_PAULI] != 0;
     // PID bundles join beads that both have their chain neighbours
     const bool pid_on = p.on[XMD_TERM_PID] != 0 && (d.bflags[i] & (BF_PREV | BF_NEXT)) == (BF_PREV | BF_NEXT);
     const bool go_on = p.on[XMD_TERM_GO] != 0;
-    const bool es_on = (p.on[XMD_TERM_CONST_ES] || p.on[XMD_TERM_REL_ES]);
+    const bool es_on = charged && (p.on[XMD_TERM_CONST_ES] || p.on[XMD_TERM_REL_ES]);
     const bool qa_on = d.qa_on && p.on[XMD_TERM_QA];
     const int nref = qa_on ? min(d.qa.ref_cnt[i], QA_REF_CAP) : 0;
     const int nnat = n1 - n0;
@@ -911,7 +924,7 @@ __global__ void __launch_bounds__(NC_WARPS * 32, 4) k_nl_cells(Dev d, TermP p, i
     const int ss0 = d.ss_start[i], ss1 = d.ss_end[i];
     if (ss_on)
         for (int k = ss0 + lane; k < ss1; k += 32)
-            d.ss_on[k] = dist2_exact(bx, pi, pos[d.ss_j[k]]) < rp.s_ss;
+            d.ss_on[k] = dist2_exact(rp.box, pi, pos[d.ss_j[k]]) < rp.s_ss;
     const int nss = ss_on ? ss1 - ss0 : 0;
     const int my_ss = lane < nss ? d.ss_j[ss0 + lane] : -1;
     int my_qa = -1;
@@ -919,69 +932,107 @@ __global__ void __launch_bounds__(NC_WARPS * 32, 4) k_nl_cells(Dev d, TermP p, i
         const int s = d.qa.ref[(size_t)lane * d.N + i];
         my_qa = d.qa.ct_i1[s] == i ? d.qa.ct_i2[s] : d.qa.ct_i1[s];
     }
-    const float qi_w = narrow_f(pi.w);
     const int cap = d.nl_cap;
     int cnt = 0, tcnt = 0;
-    // the buckets' candidates as one sequence (lead lanes in lane order, each
-    // bucket in its ascending bead order), taken 32 at a time: lane l takes
-    // entry g = base + l, which lies in the bucket of the last lane whose
-    // exclusive prefix of bucket sizes is <= g
-    const int csz = kq1 - kq0;
-    int pre = csz;
+    for (int g = 0; g < 2; ++g) {
+        if (g == CG_NEAR ? rp.s_near <= 0.0 : !(es_on && rp.far)) continue;
+        // neighbouring buckets: lane l < 27 takes offsets (l % 3, l / 3 % 3, l / 9) - 1,
+        // the first lane of each bucket its range of slots
+        int key = -1;
+        if (lane < 27) {
+            int cc[3];
+            if (rp.packed[g]) {
+                const int v = d.cell_key[(size_t)g * d.N + i];
+                cc[0] = v & 1023; cc[1] = (v >> 10) & 1023; cc[2] = (v >> 20) & 1023;
+            } else {
+                cc[0] = cell_coord(rp, g, 0, pi.x);
+                cc[1] = cell_coord(rp, g, 1, pi.y);
+                cc[2] = cell_coord(rp, g, 2, pi.z);
+            }
+            const int off[3] = {lane % 3 - 1, (lane / 3) % 3 - 1, lane / 9 - 1};
+            bool ok = true;
 #pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        const int y = __shfl_up_sync(FULL, pre, o);
-        if (lane >= o) pre += y;
-    }
-    const int total = __shfl_sync(FULL, pre, 31);
-    pre -= csz;   // exclusive
-    for (int base = 0; base < total; base += 32) {
-        {
-            const int g = base + lane;
+            for (int a = 0; a < 3; ++a) {
+                int k = cc[a] + off[a];
+                if (rp.per[a]) {
+                    const int dm = rp.dims[g][a];
+                    k = k < 0 ? k + dm : (k >= dm ? k - dm : k);
+                } else if (k < 0) {
+                    ok = false;
+                }
+                cc[a] = k;
+            }
+            if (ok) key = cell_bucket(d, rp, g, cc[0], cc[1], cc[2]);
+        }
+        const unsigned same = __match_any_sync(FULL, key);
+        int q0 = 0, csz = 0;
+        if (key >= 0 && (same & lt) == 0u) {
+            const int2 s = cell_range(d, key);
+            q0 = s.x;
+            csz = s.y - s.x;
+        }
+        // the buckets' candidates as one sequence, taken 32 at a time: lane l
+        // takes entry c = base + l, which lies in the bucket of the last lane
+        // whose exclusive prefix of bucket sizes is <= c
+        int pre = csz;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int y = __shfl_up_sync(FULL, pre, o);
+            if (lane >= o) pre += y;
+        }
+        const int total = __shfl_sync(FULL, pre, 31);
+        pre -= csz;
+        q0 -= pre;
+        const float reach = g == CG_NEAR ? Bnear.hi : fminf(Bes.hi, Breq.hi);
+        for (int base = 0; base < total; base += 32) {
+            const int c = base + lane;
             int lo = 0;
 #pragma unroll
             for (int step = 16; step; step >>= 1) {
                 const int pm = __shfl_sync(FULL, pre, lo + step);
-                if (pm <= g) lo += step;
+                if (pm <= c) lo += step;
             }
-            const int q = __shfl_sync(FULL, kq0, lo) + (g - __shfl_sync(FULL, pre, lo));
+            const int q = __shfl_sync(FULL, q0, lo) + c;
             int flags = 0;
             bool qa_free = false;
             int j = -1;
-            if (g < total) {
+            if (c < total) {
                 const float4 f = d.cell_pos[q];
-                j = __float_as_int(f.w);
-                float ddx = f.x - mx, ddy = f.y - my, ddz = f.z - mz;
+                j = __float_as_int(f.w) & ~CELL_CHARGED;
+                const bool es_pair = es_on && __float_as_int(f.w) < 0;
+                float ddx = f.x - me.x, ddy = f.y - me.y, ddz = f.z - me.z;
                 if (periodic) {
                     ddx = min_image_f(ddx, Lx);
                     ddy = min_image_f(ddy, Ly);
                     ddz = min_image_f(ddz, Lz);
                 }
                 const float d2 = ddx * ddx + ddy * ddy + ddz * ddz;
-                if (j != i && d2 <= pre2) {
-                    const int2 cs = d.cell_cs[q];
-                    const int cj = cs.x, sj = cs.y;
+                if (j != i && d2 <= reach) {
+                    const int cj = d.chain[j], sj = d.seq[j];
                     const int df = si > sj ? si - sj : sj - si;
                     if (!(ci == cj && df < 3)) {
-                        bool in_req, pa, es, qa, pd;
-                        if (in_band(Breq, d2) || (pauli_on && in_band(Bpa, d2)) || (es_on && in_band(Bes, d2)) ||
-                            (qa_on && in_band(Bqa, d2)) || (pid_on && in_band(Bpid, d2))) {
-                            const double s2 = periodic ? dist2_exact(bx, pi, pos[j]) : dist2_open(pi, pos[j]);
+                        bool in_req, pa, es, qa, pd, near;
+                        if (in_band(Breq, d2) || in_band(Bnear, d2) || (pauli_on && in_band(Bpa, d2)) ||
+                            (es_pair && in_band(Bes, d2)) || (qa_on && in_band(Bqa, d2)) ||
+                            (pid_on && in_band(Bpid, d2))) {
+                            const double s2 = periodic ? dist2_exact(rp.box, pi, pos[j]) : dist2_open(pi, pos[j]);
                             in_req = s2 < rp.s_req;
+                            near = s2 < rp.s_near;
                             pa = s2 < rp.s_pa;
                             es = s2 < rp.s_es;
                             qa = s2 < rp.s_qa;
                             pd = s2 < rp.s_pid;
                         } else {
                             in_req = d2 < Breq.lo;
+                            near = d2 < Bnear.lo;
                             pa = d2 < Bpa.lo;
                             es = d2 < Bes.lo;
                             qa = d2 < Bqa.lo;
                             pd = d2 < Bpid.lo;
                         }
-                        if (in_req) {
+                        if (in_req && near == (g == CG_NEAR)) {
                             if (pauli_on && pa) flags |= NL_PAULI;
-                            if (es_on && es && qi_w * narrow_f(pos[j].w) != 0.0f) flags |= NL_ES;
+                            if (es_pair && es) flags |= NL_ES;
                             if (pid_on && pd && (d.bflags[j] & (BF_PREV | BF_NEXT)) == (BF_PREV | BF_NEXT))
                                 flags |= NL_PID;
                             qa_free = qa_on && j > i && qa;
@@ -1384,7 +1435,8 @@ __global__ void __launch_bounds__(TL_THREADS, 4) k_nl_tile(Dev d, TermP p, int c
 constexpr int EVAL_FB = 64, EVAL_LPB = 4;
 static size_t force_smem(bool mixed, int mode, int fb, bool qa) {
     if (mode == 0) fb = EVAL_FB;
-    if (mixed) return fb == 32 ? step_smem<float, 32>(qa) : fb == 64 ? step_smem<float, 64>(qa) : step_smem<float, 128>(qa);
+    if (mixed)
+        return fb == 32 ? step_smem<float, 32>(qa) : fb == 64 ? step_smem<float, 64>(qa) : step_smem<float, 128>(qa);
     return fb == 32 ? step_smem<double, 32>(qa) : fb == 64 ? step_smem<double, 64>(qa) : step_smem<double, 128>(qa);
 }
 static int force_blocks(int n, int fb) { return (n + fb - 6) / (fb - 5); }   // step_beads
@@ -1556,7 +1608,6 @@ void Engine::remove_replica(int rep) {
         CK(cudaMemsetAsync(d.go_cnt + b, 0, sizeof(int32_t) * n, stream));
         if (r.nat_len) CK(cudaMemsetAsync(d.nat_on + r.nat_off, 0, r.nat_len, stream));
         if (r.chunk_len) CK(cudaMemsetAsync(d.chunks + r.chunk_off, 0xff, sizeof(int2) * r.chunk_len, stream));
-        if (r.cell_len) CK(cudaMemsetAsync(d.cell_rep + r.cell_off, 0xff, sizeof(int32_t) * r.cell_len, stream));
         CK(cudaMemsetAsync(d.rep + rep, 0, sizeof(RepDev), stream));
         CK(cudaStreamSynchronize(stream));
         for (int i = 0; i < n; ++i) owner_h[b + i] = -1;
@@ -1611,9 +1662,6 @@ void Engine::activate_staged() {
         RepHost &r = reps[st.k];
         CK(cudaMemcpyAsync(d.rep_of + r.begin, st.rep_of.data(), sizeof(int32_t) * r.n, cudaMemcpyHostToDevice,
                            stream));
-        if (!st.cell_rep.empty())
-            CK(cudaMemcpyAsync(d.cell_rep + r.cell_off, st.cell_rep.data(), sizeof(int32_t) * st.cell_rep.size(),
-                               cudaMemcpyHostToDevice, stream));
         CK(cudaMemcpyAsync(d.rep + st.k, &st.rd, sizeof(RepDev), cudaMemcpyHostToDevice, stream));
         for (int i = 0; i < r.n; ++i) owner_h[r.begin + i] = st.k;
         r.staged = false;
@@ -1985,6 +2033,18 @@ void Engine::derive_rep(int ri, RepDev &rd) {
     rd.s_es = sq_below(inv_above(rd.es_min_inv));
     rd.s_qa = sq_below(inv_above(rd.qa_min_inv));
     rd.s_pid = sq_below(inv_above(rd.pid_min_inv));
+    // the near grid's radius: the largest of the terms that act between any
+    // two beads; the far grid's: the electrostatic one
+    auto near_term = [&](double radius, double s) {
+        rd.r_near = std::max(rd.r_near, std::min(radius, rd.req_r));
+        rd.s_near = std::max(rd.s_near, std::min(s, rd.s_req));
+    };
+    if (p.on[XMD_TERM_PAULI]) near_term(1.0 / rd.pauli_min_inv, rd.s_pa);
+    if (p.on[XMD_TERM_QA]) near_term(1.0 / rd.qa_min_inv, rd.s_qa);
+    if (p.on[XMD_TERM_PID]) near_term(1.0 / rd.pid_min_inv, rd.s_pid);
+    if (rd.r_near <= 0.0) rd.r_near = rd.req_r > 0.0 ? rd.req_r : 1.0;
+    rd.far = (p.on[XMD_TERM_CONST_ES] || p.on[XMD_TERM_REL_ES]) && rd.req_r > 0.0;
+    rd.r_far = rd.far ? std::min(1.0 / rd.es_min_inv, rd.req_r) : 1.0;
     rd.s_ss = sq_below(2.0 * p.nat_ss_dist + rd.pad);   // update_nat_ssbonds, native_ss.cpp:15
     rd.noise_sd = std::sqrt(2.0 * 1.0 * r.temperature) * std::sqrt(p.gamma_factor) * 1.0;
     rd.begin = r.begin;
@@ -2033,7 +2093,8 @@ void Engine::allocate() {
     d.N = N;
     d.R = R;
     d.nl_cap = nl_cap;
-    const size_t cells = (size_t)std::max(1, cap.cells);
+    // near grids, then the far grids at half their size
+    const size_t cells = (size_t)std::max(1, cap.cells) / 2 * 3 + 3;
     const size_t NN = (size_t)std::max(1, cap.nat);
     d.pos[0] = (double4_32a *)dalloc(sizeof(double4_32a) * N);
     d.pos[1] = (double4_32a *)dalloc(sizeof(double4_32a) * N);
@@ -2104,15 +2165,14 @@ void Engine::allocate() {
     d.nl_cnt = (int32_t *)dalloc(sizeof(int32_t) * N);
     d.cell_cnt = (int32_t *)dalloc(sizeof(int32_t) * cells);
     d.cell_start = (int32_t *)dalloc(sizeof(int32_t) * cells);
-    d.cell_fill = (int32_t *)dalloc(sizeof(int32_t) * cells);
-    d.cell_items = (int32_t *)dalloc(sizeof(int32_t) * N);
-    d.bead_cell = (int32_t *)dalloc(sizeof(int32_t) * N);
-    d.cell_pos = (float4 *)dalloc(sizeof(float4) * N);
-    d.bead_slot = (int32_t *)dalloc(sizeof(int32_t) * N);
-    d.cell_cs = (int2 *)dalloc(sizeof(int2) * N);
     d.ncells = (int)cells;
-    d.cell_rep = (int32_t *)dalloc(sizeof(int32_t) * cells);
-    CK(cudaMemsetAsync(d.cell_rep, 0xff, sizeof(int32_t) * cells, stream));
+    d.ncells_near = (int)cells / 3 * 2;
+    d.cell_base = (int32_t *)dalloc(sizeof(int32_t) * ((cells + CELL_SCAN - 1) / CELL_SCAN + 1));
+    // both grids' slots, where some replica may use them
+    const size_t slots = cap.cells > 0 ? 2 * (size_t)N : 1;
+    d.cell_items = (int32_t *)dalloc(sizeof(int32_t) * slots);
+    d.cell_key = (int32_t *)dalloc(sizeof(int32_t) * slots);
+    d.cell_pos = (float4 *)dalloc(sizeof(float4) * slots);
     d.rng = (uint64_t *)dalloc(sizeof(uint64_t) * N);
     d.jump = (uint64_t *)dalloc(sizeof(uint64_t) * JUMP_WORDS * R);
     d.rep = (RepDev *)dalloc(sizeof(RepDev) * R);
@@ -2337,7 +2397,7 @@ void Engine::place_pending() {
 
 // static data, lists and state of replica slot k onto the device.  With st
 // (staged placement) every upload goes on the side stream, after the last
-// removal's clears, and the activation data (bead and bucket owners, the
+// removal's clears, and the activation data (bead owners, the
 // replica record) is kept in st for activate_staged().
 void Engine::place(int k, Staged *st) {
     const xmd_params &p = params;
@@ -2475,11 +2535,6 @@ void Engine::place(int k, Staged *st) {
     CK(cudaMemsetAsync(d.nat_on + no, 0, nnat, us));
     CK(cudaMemsetAsync(d.nl_cnt + b, 0, sizeof(int32_t) * n, us));
     CK(cudaMemsetAsync(d.go_cnt + b, 0, sizeof(int32_t) * n, us));
-    if (ncell) {
-        std::vector<int32_t> cr(ncell, k);
-        if (st) st->cell_rep = cr;
-        else up(d.cell_rep + co, cr.data(), sizeof(int32_t) * ncell);
-    }
     std::vector<int2> ch(nchunk);
     for (int c = 0; c < nchunk; ++c) ch[c] = make_int2(k, b + c * TL_CH);
     up(d.chunks + ho, ch.data(), sizeof(int2) * nchunk);
@@ -2898,11 +2953,11 @@ void Engine::launch_rebuild() {
     if (timing) record(ev_rebuild, n_ev_rebuild);
     if (any_cell) {
         const int gb = (d.N + 255) / 256;
-        k_cells<<<d.R, CB, 0, stream>>>(d, cur);
+        k_cells<<<gb, 256, 0, stream>>>(d, cur);
         k_cell_count<<<gb, 256, 0, stream>>>(d, cur);
-        k_cell_scan<<<d.R, CB, 0, stream>>>(d);
+        k_cell_scan<<<(d.ncells + CELL_SCAN - 1) / CELL_SCAN, 256, 0, stream>>>(d);
         k_cell_scatter<<<gb, 256, 0, stream>>>(d);
-        k_cell_finish<<<(d.ncells + CF_WARPS - 1) / CF_WARPS, CF_WARPS * 32, 0, stream>>>(d, cur);
+        k_cell_finish<<<2 * gb, 256, 0, stream>>>(d, cur);
         k_nl_cells<<<(d.N + NC_WARPS - 1) / NC_WARPS, NC_WARPS * 32, 0, stream>>>(d, tp, cur);
     }
     if (any_tile) k_nl_tile<<<tile_grid, TL_THREADS, tile_smem, stream>>>(d, tp, cur, 1);
@@ -3226,19 +3281,19 @@ void Engine::add_rebuild_nodes(cudaGraph_t body, int cn) {
     if (any_cell) {
         cudaKernelNodeParams k1{}, k2{}, kc{}, ks{}, kx{}, kf{};
         k1.func = (void *)k_cells;
-        k1.gridDim = dim3(d.R);
-        k1.blockDim = dim3(CB);
+        const unsigned gb = (unsigned)((d.N + 255) / 256);
+        k1.gridDim = dim3(gb);
+        k1.blockDim = dim3(256);
         k1.kernelParams = a1;
         add(k1);
-        const unsigned gb = (unsigned)((d.N + 255) / 256);
         kc.func = (void *)k_cell_count;
         kc.gridDim = dim3(gb);
         kc.blockDim = dim3(256);
         kc.kernelParams = a1;
         add(kc);
         ks.func = (void *)k_cell_scan;
-        ks.gridDim = dim3(d.R);
-        ks.blockDim = dim3(CB);
+        ks.gridDim = dim3((unsigned)((d.ncells + CELL_SCAN - 1) / CELL_SCAN));
+        ks.blockDim = dim3(256);
         ks.kernelParams = a3;
         add(ks);
         kx.func = (void *)k_cell_scatter;
@@ -3247,8 +3302,8 @@ void Engine::add_rebuild_nodes(cudaGraph_t body, int cn) {
         kx.kernelParams = a3;
         add(kx);
         kf.func = (void *)k_cell_finish;
-        kf.gridDim = dim3((unsigned)((d.ncells + CF_WARPS - 1) / CF_WARPS));
-        kf.blockDim = dim3(CF_WARPS * 32);
+        kf.gridDim = dim3(2 * gb);
+        kf.blockDim = dim3(256);
         kf.kernelParams = a1;
         add(kf);
         k2.func = (void *)k_nl_cells;

@@ -59,11 +59,18 @@ struct RepDev {
     int per[3];
     int per_any;             // some axis is periodic
     float Lh[3], Ll[3], Li[3];   // mixed path: cell as h + l, and its inverse (0 on open axes)
-    int dims[3];             // cells along periodic axes
-    double lo[3], cs[3];     // bounding-box minimum and 1/cell edge along open axes
-    int hashed;              // cells hashed into the bucket budget
+    // cell build, per grid (near: every bead; far: charged beads): radius,
+    // cells along periodic axes, 1/cell edge along open axes, whether cells
+    // are hashed into the bucket budget, whether their coordinates fit the
+    // packed form
+    double r_near, r_far, s_near;   // s < s_near <=> the near grid gives the pair
+    int far;                 // charged beads search the far grid
+    int dims[2][3];
+    double lo[3], cs[2];     // bounding-box minimum along open axes
+    int hashed[2], packed[2];
+    unsigned lo_key[3], hi_key[3];   // bounding box during a build, as ordered integers
+    float near_lo, near_hi;  // FP32 band of r_near
     int tile;                // Verlet build by whole-replica tiles (no cell grid)
-    float pre2;              // squared FP32 pre-filter radius of the Verlet build
     double band_m;           // FP32 distance error bound of the cell build
     float band_lo[5], band_hi[5];   // cell build: FP32 bands of the list radius, r_excl + pad, 2D + pad,
                                     // QA radius + pad, PID cutoff + pad
@@ -127,7 +134,8 @@ struct Dev {
     int N, R, nl_cap;
     double4_32a *pos[2];        // x, y, z, charge; double-buffered
     double *yh;             // [15][N]: y1x y1y y1z y2x ... y5z
-    float4 *spl[2];         // mixed path: positions split per axis, [2 i] = (hx, hy, hz, charge), [2 i + 1] = (lx, ly, lz, 0)
+    // mixed path: positions split per axis, [2 i] = (hx, hy, hz, charge), [2 i + 1] = (lx, ly, lz, 0)
+    float4 *spl[2];
     double4_32a *orig;          // positions at the last list rebuild
     double *F;              // [3N] force output of eval
     double *Vrep;           // [R][XMD_NUM_TERMS] energies of eval
@@ -156,12 +164,12 @@ struct Dev {
     double *act_d;
     int32_t *go_cnt;
     int32_t *nl_row, *nl_cnt;
-    int32_t *cell_cnt, *cell_start, *cell_fill, *cell_items, *bead_cell;
-    float4 *cell_pos;       // bucket-sorted FP32 coordinates (+ bead index bits)
-    int32_t *bead_slot;     // bead -> its slot in cell_pos
-    int2 *cell_cs;          // (chain, sequence index) of each slot of cell_pos
-    int32_t *cell_rep;      // bucket of the pool -> replica owning it (-1: free)
-    int ncells;             // buckets in the pool
+    int32_t *cell_cnt;      // beads per bucket (zero between builds)
+    int32_t *cell_start, *cell_base;   // first slot of a bucket: cell_start[c] + cell_base[c / CELL_SCAN]
+    int32_t *cell_items;    // bucket-sorted beads
+    int32_t *cell_key;      // [2][N] packed cell coordinates of a bead in the near and far grid
+    float4 *cell_pos;       // bucket-sorted FP32 coordinates, bead index (+ charged bit)
+    int ncells, ncells_near;   // buckets in the pool, of the near grids
     uint64_t *rng;          // per-bead generator state
     uint64_t *jump;         // [R][16][16] nibble tables of the GF(2) jump (4 N_r draws)
     RepDev *rep;
@@ -422,11 +430,11 @@ private:
     int qa_bchunk_next = 0;   // next free chunk of the QA re-listing (static contexts)
     std::vector<int32_t> owner_h;              // bead slot -> replica (or -1)
     void allocate();
-    // the staged replicas' activation data: bead -> replica, bucket ->
-    // replica and the replica record, written on the step stream
+    // the staged replicas' activation data: bead -> replica and the replica
+    // record, written on the step stream
     struct Staged {
         int k = 0;
-        std::vector<int32_t> rep_of, cell_rep;
+        std::vector<int32_t> rep_of;
         RepDev rd{};
     };
     std::vector<Staged> staged_reps;
