@@ -13,6 +13,16 @@
 
 namespace xmdg {
 
+// Every kernel of a step starts with this, in every thread: it waits until the
+// kernels before it in the step graph have finished and their writes are
+// visible, and lets the next one be launched, so that a launch overlaps its
+// predecessor's last blocks (programmatic edges of Engine::graph_for; a plain
+// launch waits for nothing here).
+__device__ __forceinline__ void step_order() {
+    cudaGridDependencySynchronize();
+    cudaTriggerProgrammaticLaunchCompletion();
+}
+
 template <class T> struct V3 { T x, y, z; };
 
 template <class T> __device__ __forceinline__ V3<T> v3(T x, T y, T z) { return V3<T>{x, y, z}; }

@@ -183,7 +183,7 @@ struct Dev {
     int nchunks;
     int *work;              // chunks of the replicas flagged at the last skin check
     int *nwork;             // number of entries in `work`
-    int any_cell;           // some replica uses the cell-grid build
+    int any_cell;           // some placed replica uses the cell-grid build
     int qa_on;
     QaDev qa;
     // pseudo-improper dihedral potential: per bead its bundles' forces on
@@ -387,7 +387,7 @@ private:
         return std::max(4 * tile_sms, (ng + QA_SIFT - 1) / QA_SIFT);
     }
     // graphs rebuild with a plain row-build node instead of an IF node
-    bool plain_rebuild() const { return any_tile && !any_cell && !d.qa_on; }
+    bool plain_rebuild() const { return any_tile && !live_cell && !d.qa_on; }
     // graphs without rebuild nodes: a flagged check halts the graph's
     // remaining steps and the host rebuilds (static contexts with cell-path
     // replicas or the quasi-adiabatic term, where the rebuild is a chain of
@@ -415,7 +415,9 @@ private:
     bool auto_grow = true;       // grow Verlet rows instead of failing
     int cond_graphs_left = 0;    // gated contexts: IF-node graphs to run before the next gated one
     cudaGraphExec_t graph_for(int start_cur, bool gated, int len);
-    bool any_cell = false, any_tile = false;   // which Verlet builds the replicas use
+    bool any_tile = false;                     // some replica may use the tile build
+    int live_cell = 0;                         // placed replicas that use the cell build
+    void count_cell(int change);
     size_t tile_smem = 0;                      // dynamic shared memory of k_nl_tile
     int tile_grid = 1;                         // resident blocks of k_nl_tile over all SMs
     void add_rebuild_nodes(cudaGraph_t body, int cn);
