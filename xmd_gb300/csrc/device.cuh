@@ -392,24 +392,6 @@ __device__ __forceinline__ uint64_t rng_next(uint64_t &st) {
     st ^= st >> 18;
     return res;
 }
-// Four draws of one bead (normal_x2 then normal, lang_pc.cpp:15-16)
-__device__ __forceinline__ void noise3(uint64_t st, double *nx, double *ny, double *nz) {
-    const double inv = 1.0 / 4294967296.0;
-    double u1 = (double)(rng_next(st) >> 32) * inv;
-    double u2 = (double)(rng_next(st) >> 32) * inv;
-    double u3 = (double)(rng_next(st) >> 32) * inv;
-    double u4 = (double)(rng_next(st) >> 32) * inv;
-    double r = sqrt(-2.0 * log(u1));
-    if (isnan(r)) r = 0.0;
-    double t = (2.0 * 3.141592653589793) * u2;
-    double s, c;
-    sincos(t, &s, &c);
-    *nx = r * c;
-    *ny = r * s;
-    double r2 = sqrt(-2.0 * log(u3));
-    if (isnan(r2)) r2 = 0.0;
-    *nz = r2 * cos((2.0 * 3.141592653589793) * u4);
-}
 // The same product from 16 nibble tables of 16 entries (entry [q][v] = XOR of
 // the columns 4q..4q+3 selected by the bits of v): 16 lookups instead of 64
 constexpr int JUMP_WORDS = 256;

@@ -2176,6 +2176,18 @@ void Engine::allocate() {
         CK(cudaMemcpyAsync(hdf, tf, sizeof(float) * 9 * 6, cudaMemcpyHostToDevice, stream));
         CK(cudaStreamSynchronize(stream));
         d.heur_ang = ha; d.heur_dih = hd; d.heur_dih_f = hdf;
+        // radius_of: c is the middle of interval j of 128 in [1, 2), halved in
+        // the upper half, 1 beside 1
+        double2 lt[128];
+        for (int j = 0; j < 128; ++j) {
+            const double mid = 1.0 + (j + 0.5) / 128.0;
+            const double inv = j == 0 || j == 127 ? 1.0 : 1.0 / (j < 64 ? mid : 0.5 * mid);
+            lt[j] = make_double2(inv, (double)-logl((long double)inv));
+        }
+        double2 *ltd = (double2 *)dalloc(sizeof lt);
+        CK(cudaMemcpyAsync(ltd, lt, sizeof lt, cudaMemcpyHostToDevice, stream));
+        CK(cudaStreamSynchronize(stream));
+        d.logt = ltd;
     }
     d.nl_row = (int32_t *)dalloc(sizeof(int32_t) * (size_t)nl_cap * N);
     d.nl_cnt = (int32_t *)dalloc(sizeof(int32_t) * N);

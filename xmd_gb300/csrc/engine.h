@@ -171,6 +171,7 @@ struct Dev {
     float4 *cell_pos;       // bucket-sorted FP32 coordinates, bead index (+ charged bit)
     int ncells, ncells_near;   // buckets in the pool, of the near grids
     uint64_t *rng;          // per-bead generator state
+    const double2 *logt;    // [128] (1 / c, log c) of the FP64 noise's logarithm
     uint64_t *jump;         // [R][16][16] nibble tables of the GF(2) jump (4 N_r draws)
     RepDev *rep;
     int *any_rebuild;       // [0]: some replica flagged at the last check; [1..3]: gate

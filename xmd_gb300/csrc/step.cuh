@@ -77,6 +77,82 @@ __device__ __forceinline__ float rsq(float x) {
     return x > 0.0f && y > 0.0f ? z : y;
 }
 
+// ---- noise of the FP64 path -------------------------------------------------------
+// Box-Muller on four 32-bit draws k / 2^32 as noise3 forms them
+// (rand_gen.h:22-58, lang_pc.cpp:15-16), with the reductions done on the
+// integer draws: no FP64 conversion, argument reduction or special-case path
+// (84 FP64 instructions a bead; 150 with the library's log, sincos and cos).
+// Draws and draw order are noise3's, results within a few 2^-53.
+__device__ __forceinline__ double int_to_d(int k) {   // exact, one addition
+    return __dsub_rn(__hiloint2double(0x43300000, (int)((unsigned)k ^ 0x80000000u)), 4503601774854144.0);
+}
+// sqrt(-2 log(k / 2^32)); k = 0 gives infinity, as log(0) does.  k / 2^32 =
+// z 2^e with z in [0.75, 1.5); log z = log c + log1p(z / c - 1) with c from a
+// table of 128 (c = 1 on both sides of 1, so that results near 0 keep their
+// relative accuracy), log1p by its series to the 8th power (|r| <= 2^-7).
+__device__ __forceinline__ double radius_of(unsigned k, const double2 *__restrict__ logt) {
+    const int n = __clz((int)(k | 1u));
+    const unsigned m = k << n;                    // leading one at bit 31
+    const int j = (m >> 24) & 127;
+    const bool up = j >= 64;
+    const double z = __hiloint2double((up ? 0x3fe00000 : 0x3ff00000) | (int)((m & 0x7fffffffu) >> 11), (int)(m << 21));
+    const double2 c = __ldg(logt + j);            // 1 / c, log c
+    const double r = __fma_rn(z, c.x, -1.0);
+    double q = __fma_rn(r, -0.125, 1.0 / 7.0);
+    q = __fma_rn(r, q, -1.0 / 6.0);
+    q = __fma_rn(r, q, 0.2);
+    q = __fma_rn(r, q, -0.25);
+    q = __fma_rn(r, q, 1.0 / 3.0);
+    q = __fma_rn(r, q, -0.5);
+    const double l1 = __fma_rn(__dmul_rn(r, r), q, r);
+    const double e = int_to_d((up ? 0 : -1) - n);
+    const double x = __dmul_rn(-2.0, __dadd_rn(__fma_rn(e, 0.6931471805599453, c.y), l1));
+    const double y = rsqrt(x), w = __dmul_rn(x, y);   // the square root, with one Newton correction
+    return k ? __fma_rn(__fma_rn(-w, w, x), __dmul_rn(0.5, y), w) : __longlong_as_double(0x7ff0000000000000ll);
+}
+// sine and cosine of 2 pi k / 2^32: the quadrant from the top bits, the rest in
+// [-pi/4, pi/4] by Taylor series (remainders below 1e-19)
+__device__ __forceinline__ double sin_series(double x, double x2) {
+    double p = __fma_rn(x2, 2.8114572543455206e-15, -7.647163731819816e-13);
+    p = __fma_rn(x2, p, 1.6059043836821613e-10);
+    p = __fma_rn(x2, p, -2.505210838544172e-08);
+    p = __fma_rn(x2, p, 2.7557319223985893e-06);
+    p = __fma_rn(x2, p, -0.0001984126984126984);
+    p = __fma_rn(x2, p, 0.008333333333333333);
+    p = __fma_rn(x2, p, -0.16666666666666666);
+    return __fma_rn(__dmul_rn(x, x2), p, x);
+}
+__device__ __forceinline__ double cos_series(double x2) {
+    double p = __fma_rn(x2, 4.779477332387385e-14, -1.1470745597729725e-11);
+    p = __fma_rn(x2, p, 2.08767569878681e-09);
+    p = __fma_rn(x2, p, -2.755731922398589e-07);
+    p = __fma_rn(x2, p, 2.48015873015873e-05);
+    p = __fma_rn(x2, p, -0.001388888888888889);
+    p = __fma_rn(x2, p, 0.041666666666666664);
+    p = __fma_rn(x2, p, -0.5);
+    return __fma_rn(x2, p, 1.0);
+}
+__device__ __forceinline__ double turn_rest(unsigned k, unsigned *quad) {
+    *quad = (k + 0x20000000u) >> 30;
+    return __dmul_rn(int_to_d((int)(k - (*quad << 30))), 1.4629180792671596e-09);   // 2 pi / 2^32
+}
+__device__ __forceinline__ double flip(double x, unsigned neg) {
+    return __hiloint2double(__double2hiint(x) ^ (int)(neg << 31), __double2loint(x));
+}
+__device__ __forceinline__ void noise3_turns(uint64_t st, const double2 *logt, double *nx, double *ny, double *nz) {
+    const unsigned k1 = (unsigned)(rng_next(st) >> 32), k2 = (unsigned)(rng_next(st) >> 32);
+    const unsigned k3 = (unsigned)(rng_next(st) >> 32), k4 = (unsigned)(rng_next(st) >> 32);
+    unsigned q;
+    double x = turn_rest(k2, &q), x2 = __dmul_rn(x, x);
+    const double s = sin_series(x, x2), c = cos_series(x2), r = radius_of(k1, logt);
+    // quadrants 0..3: cos = c, -s, -c, s; sin = s, c, -s, -c
+    *nx = __dmul_rn(r, flip(q & 1 ? s : c, (q ^ (q >> 1)) & 1));
+    *ny = __dmul_rn(r, flip(q & 1 ? c : s, q >> 1));
+    x = turn_rest(k4, &q);
+    x2 = __dmul_rn(x, x);
+    *nz = __dmul_rn(radius_of(k3, logt), flip(q & 1 ? sin_series(x, x2) : cos_series(x2), (q ^ (q >> 1)) & 1));
+}
+
 // ---- geometry slots -------------------------------------------------------------
 // FP64: bond e (3), unit cross product u (3), |e|, 1/|e|, 1/|x|.  Bonds, cross
 // products, lengths and units are formed with every operation rounded on its
@@ -367,6 +443,9 @@ template <class FT, int FB> struct StepSh {
     FT f[3][FCAP];                    // pair forces
     FT n[3][FB];                      // noise
     FT e[3][FB];                      // squared skin-test displacement per axis
+    // FP64: electrostatic entries set aside (their charge product, and which)
+    FT ew[MIX ? 1 : FCAP];
+    int eq[MIX ? 1 : FCAP], neq, next_es;
     int off[FB + 4], ng[FB], nl[FB], nat0[FB], rep[FB], state[FB], ws[4], next;
     // followed, in contexts with the quasi-adiabatic term, by the beads'
     // contact slots in ascending order, int [FB][QA_REF_CAP]
@@ -375,10 +454,23 @@ template <class FT, int FB> constexpr size_t step_smem(bool qa) {
     return (sizeof(StepSh<FT, FB>) + 15) / 16 * 16 + (qa ? sizeof(int) * QA_REF_CAP * FB : 0);
 }
 
-// force of pair entry e of the block on its bead
+// Debye-Hueckel force factor: eval_const_es_forces::iter es/const.cpp:13-32,
+// eval_relative_es_forces::iter es/relative.cpp:13-32
+template <class FT>
+__device__ __forceinline__ FT es_factor(const TermP &p, FT vq, FT s2, FT rn, FT *V) {
+    const FT sdi = tpar<FT>(p.es_sdi, p.f.es_sdi);
+    *V = mul_(mul_(vq, exp_(-mul_(mul_(s2, rn), sdi))), mul_(rn, rn));
+    return -mul_(*V, fma_<FT>(p.es_rel ? FT(2) : FT(1), rn, sdi));
+}
+
+// force of pair entry e of the block on its bead.  On the FP64 path the
+// electrostatic part (an exponential, half the pair's FP64 work) is set aside
+// when it is all there is to the pair: *es gets its charge factor and the
+// pair vector is returned, so that whole warps of such pairs do it later
+// instead of every warp that holds one.
 template <class FT, int MODE, int FB>
 __device__ __forceinline__ V3<FT> pair_entry(const Dev &d, const TermP &p, int cur, const StepSh<FT, FB> &s,
-                                             const int (*s_q)[QA_REF_CAP], int i0, int e, Ener<MODE> &en) {
+                                             const int (*s_q)[QA_REF_CAP], int i0, int e, Ener<MODE> &en, FT *es) {
     constexpr bool MIX = sizeof(FT) == 4;
     // the entry's bead: the last one that starts at or before it
     int lo = 0;
@@ -452,13 +544,13 @@ __device__ __forceinline__ V3<FT> pair_entry(const Dev &d, const TermP &p, int c
             }
         }
         if (ent & NL_ES) {
-            // eval_const_es_forces::iter es/const.cpp:13-32,
-            // eval_relative_es_forces::iter es/relative.cpp:13-32
-            const FT sdi = tpar<FT>(p.es_sdi, p.f.es_sdi);
-            const FT V_ = mul_(mul_(mul_(tpar<FT>(p.es_Vf, p.f.es_Vf), mul_(s.p[MIX ? 6 : 3][lo + 3], qj)),
-                                    exp_(-mul_(mul_(s2, rn), sdi))),
-                               mul_(rn, rn));
-            dV = fma_<FT>(-V_, fma_<FT>(p.es_rel ? FT(2) : FT(1), rn, sdi), dV);
+            const FT vq = mul_(tpar<FT>(p.es_Vf, p.f.es_Vf), mul_(s.p[MIX ? 6 : 3][lo + 3], qj));
+            if (!MIX && MODE == 1 && dV == FT(0)) {
+                *es = vq;
+                return r12;
+            }
+            FT V_;
+            dV = add_(dV, es_factor<FT>(p, vq, s2, rn, &V_));
             if (MODE == 0 && i < j) en.add(d, r, p.es_rel ? XMD_TERM_REL_ES : XMD_TERM_CONST_ES, (double)V_);
         }
     }
@@ -476,6 +568,9 @@ __device__ __forceinline__ void force_block(const Dev &d, const TermP &p, int cu
     constexpr int NT = FB * LPB, FBT = step_beads<FB>(), NP = FB + 1, NC = FBT + 3;
     constexpr int TT = (3 * FBT + NT - 1) / NT;   // (axis, bead) tasks per thread
     constexpr int FCAP = StepSh<FT, FB>::FCAP;
+    // first thread of the tasks: with four threads per slot, past the warps of
+    // the geometry and the angles
+    constexpr int W0 = LPB == 4 ? FB : 0;
     using ST = typename StepSum<FT>::T;
     extern __shared__ __align__(16) unsigned char step_mem[];
     StepSh<FT, FB> &s = *reinterpret_cast<StepSh<FT, FB> *>(step_mem);
@@ -519,6 +614,20 @@ __device__ __forceinline__ void force_block(const Dev &d, const TermP &p, int cu
     const bool draws = MODE == 1 && bn >= 0 && bn < FBT && i0 + bn < N;
     uint64_t st0 = 0;
     if (draws) st0 = d.rng[i0 + bn];
+    double y[TT][6], o[TT];
+#pragma unroll
+    for (int u = 0; u < TT; ++u) {
+        const int w = t - W0 + u * NT, a = w / FBT, i = i0 + w - a * FBT;
+        o[u] = 0.0;
+#pragma unroll
+        for (int q = 0; q < 6; ++q) y[u][q] = 0.0;
+        if (MODE == 1 && w >= 0 && w < 3 * FBT && i < N) {
+            y[u][0] = reinterpret_cast<const double *>(d.pos[cur] + i)[a];
+#pragma unroll
+            for (int q = 0; q < 5; ++q) y[u][q + 1] = d.yh[(size_t)(q * 3 + a) * Ns + i];
+            o[u] = reinterpret_cast<const double *>(d.orig + i)[a];
+        }
+    }
     int scan = 0, cnt = 0;
     if (t < FB) {
         const int i = i0 + t;
@@ -542,7 +651,7 @@ __device__ __forceinline__ void force_block(const Dev &d, const TermP &p, int cu
         // a replica that has taken its steps keeps its state
         if (MODE == 0) s.state[t] = r >= 0 ? 1 : -1;
     }
-    if (t == 0) s.next = 0;
+    if (t == 0) s.next = s.neq = s.next_es = 0;
     if (!__syncthreads_or(r >= 0)) return;   // no bead slot of the block is in use
     int T = 0;
 #pragma unroll
@@ -632,7 +741,7 @@ __device__ __forceinline__ void force_block(const Dev &d, const TermP &p, int cu
             // four draws per bead (normal_x2 then normal, lang_pc.cpp:15-16)
             FT a, b, g;
             if constexpr (MIX) noise3m(st0, &a, &b, &g);
-            else noise3(st0, &a, &b, &g);
+            else noise3_turns(st0, d.logt, &a, &b, &g);
             s.n[0][bn] = a; s.n[1][bn] = b; s.n[2][bn] = g;
             const int rb = s.rep[bn];
             s.rng[bn] = rb >= 0 ? gf2_apply_nib(d.jump + JUMP_WORDS * rb, st0) : 0;
@@ -695,8 +804,38 @@ __device__ __forceinline__ void force_block(const Dev &d, const TermP &p, int cu
 
     // ---- E: pair entries, FCAP at a time; between the passes every (axis,
     // bead) thread adds its bead's forces
+    // what the integrator does before the force is known: lang_pc_step::
+    // operator(), lang_pc.cpp:11-37, mass = 1 (main.cpp:156), is linear in the
+    // force, so corrector and predictor (the Taylor shift by repeated
+    // addition) are applied to y1..y5 alone here, beside the other warps'
+    // work, and the force and noise enter with one multiply-add per order at
+    // the end.  The position is rounded where the reference rounds it, once
+    // by the corrector and once by the predictor: a rounding more at its
+    // scale grows to 5e-8 A in 50 steps from a stiff extended start.
+    double err0[TT], sum0[TT];
+    if constexpr (MODE == 1) {
+#pragma unroll
+        for (int u = 0; u < TT; ++u) {
+            err0[u] = sum0[u] = 0.0;
+            if (t < W0) continue;
+            double(&q)[6] = y[u];
+            const double err = __fma_rn(__dmul_rn(p.gamma_factor, __dmul_rn(q[1], p.dt_inv)), p.dt2_half, q[2]);
+            err0[u] = err;
+            q[1] = __fma_rn(-(251.0 / 360.0), err, q[1]);
+            q[2] = __dsub_rn(q[2], err);
+            q[3] = __fma_rn(-(11.0 / 18.0), err, q[3]);
+            q[4] = __fma_rn(-(1.0 / 6.0), err, q[4]);
+            q[5] = __fma_rn(-(1.0 / 60.0), err, q[5]);
+#pragma unroll
+            for (int m = 0; m < 5; ++m) {
+#pragma unroll
+                for (int k = 4; k >= (m ? m : 1); --k) q[k] = __dadd_rn(q[k], q[k + 1]);
+                if (m == 0) sum0[u] = q[1];
+            }
+        }
+    }
+
     ST acc[TT];
-    double y[TT][6], o[TT], sd[TT];
     for (int p0 = 0;; p0 += FCAP) {
         const int pe = min(T - p0, FCAP);
         for (;;) {
@@ -704,29 +843,46 @@ __device__ __forceinline__ void force_block(const Dev &d, const TermP &p, int cu
             if (lane == 0) at = atomicAdd(&s.next, 32);
             at = __shfl_sync(0xffffffffu, at, 0);
             if (at >= pe) break;
+            FT es = FT(0);
             if (at + lane < pe) {
-                const V3<FT> f = pair_entry<FT, MODE, FB>(d, p, cur, s, s_q, i0, p0 + at + lane, en);
+                const V3<FT> f = pair_entry<FT, MODE, FB>(d, p, cur, s, s_q, i0, p0 + at + lane, en, &es);
                 s.f[0][at + lane] = f.x; s.f[1][at + lane] = f.y; s.f[2][at + lane] = f.z;
             }
+            if constexpr (!MIX && MODE == 1) {
+                const unsigned m = __ballot_sync(0xffffffffu, es != FT(0));
+                int to = 0;
+                if (lane == 0 && m) to = atomicAdd(&s.neq, __popc(m));
+                to = __shfl_sync(0xffffffffu, to, 0) + __popc(m & ((1u << lane) - 1u));
+                if (es != FT(0)) {
+                    s.eq[to] = at + lane;
+                    s.ew[to] = es;
+                }
+            }
         }
-        if (MODE == 1 && p0 == 0) {
-            // the integrator's state, on its way while the last entries finish
-#pragma unroll
-            for (int u = 0; u < TT; ++u) {
-                const int w = t + u * NT, a = w / FBT, b = w - a * FBT, i = i0 + b;
-                if (w >= 3 * FBT || i >= N || s.rep[b] < 0) continue;
-                y[u][0] = reinterpret_cast<const double *>(d.pos[cur] + i)[a];
-#pragma unroll
-                for (int q = 0; q < 5; ++q) y[u][q + 1] = d.yh[(size_t)(q * 3 + a) * Ns + i];
-                o[u] = reinterpret_cast<const double *>(d.orig + i)[a];
-                sd[u] = d.rep[s.rep[b]].noise_sd;
+        if constexpr (!MIX && MODE == 1) {
+            // the electrostatic entries set aside
+            __syncthreads();
+            const int ne = s.neq;
+            for (;;) {
+                int at = 0;
+                if (lane == 0) at = atomicAdd(&s.next_es, 32);
+                at = __shfl_sync(0xffffffffu, at, 0);
+                if (at >= ne) break;
+                if (at + lane < ne) {
+                    const int k = s.eq[at + lane];
+                    const V3<FT> r12{s.f[0][k], s.f[1][k], s.f[2][k]};
+                    const FT s2 = fdot(r12, r12), rn = rsq(s2);
+                    FT V_;
+                    const V3<FT> f = fscl<FT>(mul_(es_factor<FT>(p, s.ew[at + lane], s2, rn, &V_), rn), r12);
+                    s.f[0][k] = f.x; s.f[1][k] = f.y; s.f[2][k] = f.z;
+                }
             }
         }
         __syncthreads();
 #pragma unroll
         for (int u = 0; u < TT; ++u) {
-            const int w = t + u * NT, a = w / FBT, b = w - a * FBT;
-            if (w >= 3 * FBT) continue;
+            const int w = t - W0 + u * NT, a = w / FBT, b = w - a * FBT;
+            if (w < 0 || w >= 3 * FBT) continue;
             if (p0 == 0) {
                 const int k = b + 2;   // centre slot of the bead
                 const FT v[9] = {s.c[a][k], -s.c[a][k - 1], s.c[9 + a][k - 1], s.c[6 + a][k], s.c[3 + a][k + 1],
@@ -748,7 +904,7 @@ __device__ __forceinline__ void force_block(const Dev &d, const TermP &p, int cu
         }
         if (p0 + FCAP >= T) break;
         __syncthreads();
-        if (t == 0) s.next = 0;
+        if (t == 0) s.next = s.neq = s.next_es = 0;
         __syncthreads();
     }
 
@@ -758,9 +914,9 @@ __device__ __forceinline__ void force_block(const Dev &d, const TermP &p, int cu
     double F[TT];
 #pragma unroll
     for (int u = 0; u < TT; ++u) {
-        const int w = t + u * NT, a = w / FBT, b = w - a * FBT, i = i0 + b;
+        const int w = t - W0 + u * NT, a = w / FBT, b = w - a * FBT, i = i0 + b;
         F[u] = 0.0;
-        if (w >= 3 * FBT || s.state[b] != 1) continue;
+        if (w < 0 || w >= 3 * FBT || s.state[b] != 1) continue;
         if (p.on[XMD_TERM_NAT_SS]) {
             const int s1 = d.ss_end[i];
             for (int k = d.ss_start[i]; k < s1; ++k) {
@@ -803,31 +959,28 @@ __device__ __forceinline__ void force_block(const Dev &d, const TermP &p, int cu
     if constexpr (MODE == 0) {
         en.flush(d);
     } else {
-        // ---- F: lang_pc_step::operator(), lang_pc.cpp:11-37, mass = 1
-        // (main.cpp:156): Gear-5 corrector, then the predictor's Taylor shift by
-        // repeated addition (15 additions)
+        // ---- F: force and noise into the history.  K[k], k > 0: the
+        // corrector's factors c_m (lang_pc.cpp:24-29) after the predictor's
+        // shift, sum of binomial(m, k) c_m over m >= k; K[0]: their sum over
+        // m >= 1, for the predictor's change of the position
+        constexpr double c0 = 3.0 / 16.0, c1 = 251.0 / 360.0, c2 = 1.0;
+        constexpr double c3 = 11.0 / 18.0, c4 = 1.0 / 6.0, c5 = 1.0 / 60.0;
+        constexpr double K[6] = {c1 + c2 + c3 + c4 + c5, c1 + 2.0 * c2 + 3.0 * c3 + 4.0 * c4 + 5.0 * c5,
+                                 c2 + 3.0 * c3 + 6.0 * c4 + 10.0 * c5, c3 + 4.0 * c4 + 10.0 * c5, c4 + 5.0 * c5, c5};
         __syncthreads();
 #pragma unroll
         for (int u = 0; u < TT; ++u) {
-            const int w = t + u * NT, a = w / FBT, b = w - a * FBT, i = i0 + b;
-            if (w >= 3 * FBT || s.state[b] != 1) continue;
+            const int w = t - W0 + u * NT, a = w / FBT, b = w - a * FBT, i = i0 + b;
+            if (w < 0 || w >= 3 * FBT || s.state[b] != 1) continue;
+            const RepDev &rp = d.rep[s.rep[b]];
             double nz;
             if constexpr (MIX) nz = widen_f(s.n[a][b]);
             else nz = s.n[a][b];
             double(&q)[6] = y[u];
-            const double v = __dmul_rn(q[1], p.dt_inv);
-            const double acl = __fma_rn(sd[u], nz, __fma_rn(-p.gamma_factor, v, F[u]));
-            const double err = __fma_rn(-acl, p.dt2_half, q[2]);
-            q[0] = __fma_rn(-(3.0 / 16.0), err, q[0]);
-            q[1] = __fma_rn(-(251.0 / 360.0), err, q[1]);
-            q[2] = __dsub_rn(q[2], err);
-            q[3] = __fma_rn(-(11.0 / 18.0), err, q[3]);
-            q[4] = __fma_rn(-(1.0 / 6.0), err, q[4]);
-            q[5] = __fma_rn(-(1.0 / 60.0), err, q[5]);
+            const double fh = __dmul_rn(__fma_rn(rp.noise_sd, nz, F[u]), p.dt2_half);
+            q[0] = __dadd_rn(__fma_rn(-c0, __dsub_rn(err0[u], fh), q[0]), __fma_rn(K[0], fh, sum0[u]));
 #pragma unroll
-            for (int m = 0; m < 5; ++m)
-#pragma unroll
-                for (int k = 4; k >= m; --k) q[k] = __dadd_rn(q[k], q[k + 1]);
+            for (int k = 1; k < 6; ++k) q[k] = __fma_rn(K[k], fh, q[k]);
 #pragma unroll
             for (int k = 0; k < 5; ++k) d.yh[(size_t)(k * 3 + a) * Ns + i] = q[k + 1];
             s.F[a][b] = q[0];
@@ -837,7 +990,6 @@ __device__ __forceinline__ void force_block(const Dev &d, const TermP &p, int cu
             // Open axes wrap by exactly zero.  The mixed path squares the FP64
             // difference in FP32.
             double e = __dsub_rn(o[u], q[0]);
-            const RepDev &rp = d.rep[s.rep[b]];
             if (rp.per_any)
                 e = __dsub_rn(e, __dmul_rn(rp.box.cell[a], rint(__dmul_rn(e, rp.box.cell_inv[a]))));
             if constexpr (MIX) {
