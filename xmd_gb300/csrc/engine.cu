@@ -502,14 +502,8 @@ template <class FT, int MODE, int FB, int LPB>
 __global__ void __launch_bounds__(FB * LPB, (force_min_blocks<FT, FB, LPB>())) k_force(Dev d, TermP p, int cur,
                                                                                   int fuse) {
     __shared__ int last_s;
-    static_assert(LPB == 1 || LPB == 2 || LPB == 4, "one, two or four threads per bead");
-    constexpr int FBT = step_beads<FB>();
-    const int i = blockIdx.x * FBT + threadIdx.x;
-    const int r = threadIdx.x < FBT && i < d.N ? d.rep_of[i] : -1;   // no kernel writes it
-    step_order();
-    // uniform: the gate changes between launches
-    if (MODE == 1 && (fuse == FUSE_CHECK_GATE || fuse == FUSE_GATE) && d.gate[0]) return;
-    force_block<FT, MODE, FB, LPB>(d, p, cur, r);
+    static_assert(LPB == 1 || LPB == 2 || LPB == 4 || LPB == 8, "threads per bead slot");
+    if (!force_block<FT, MODE, FB, LPB>(d, p, cur, MODE == 1 && (fuse == FUSE_CHECK_GATE || fuse == FUSE_GATE))) return;
     if (MODE == 1 && (fuse == FUSE_CHECK || fuse == FUSE_CHECK_GATE)) {
         __syncthreads();
         if (threadIdx.x == 0) {
@@ -1441,18 +1435,19 @@ __global__ void __launch_bounds__(TL_THREADS, 4) k_nl_tile(Dev d, TermP p, int c
 constexpr int EVAL_FB = 64, EVAL_LPB = 4;
 static size_t force_smem(bool mixed, int mode, int fb, bool qa) {
     if (mode == 0) fb = EVAL_FB;
-    if (mixed)
-        return fb == 32 ? step_smem<float, 32>(qa) : fb == 64 ? step_smem<float, 64>(qa) : step_smem<float, 128>(qa);
-    return fb == 32 ? step_smem<double, 32>(qa) : fb == 64 ? step_smem<double, 64>(qa) : step_smem<double, 128>(qa);
+#define XMD_SM(B) (mixed ? step_smem<float, B>(qa) : step_smem<double, B>(qa))
+    return fb == 32 ? XMD_SM(32) : fb == 64 ? XMD_SM(64) : XMD_SM(128);
+#undef XMD_SM
 }
 static int force_blocks(int n, int fb) { return (n + fb - 6) / (fb - 5); }   // step_beads
 static void *force_kernel(bool mixed, int mode, int fb, int lpb) {
 #define XMD_FK(M, B, L) (mixed ? (void *)k_force<float, M, B, L> : (void *)k_force<double, M, B, L>)
     if (mode == 0) return XMD_FK(0, EVAL_FB, EVAL_LPB);
-    switch (fb * 8 + lpb) {
+    switch (fb * 8 + lpb) {   // (eight threads per slot: Engine::force_shape)
     case 32 * 8 + 1: return XMD_FK(1, 32, 1);
     case 32 * 8 + 2: return XMD_FK(1, 32, 2);
     case 32 * 8 + 4: return XMD_FK(1, 32, 4);
+    case 32 * 8 + 8: return XMD_FK(1, 32, 8);
     case 64 * 8 + 1: return XMD_FK(1, 64, 1);
     case 64 * 8 + 2: return XMD_FK(1, 64, 2);
     case 64 * 8 + 4: return XMD_FK(1, 64, 4);
@@ -1461,6 +1456,28 @@ static void *force_kernel(bool mixed, int mode, int fb, int lpb) {
     default: return XMD_FK(1, 128, 4);
     }
 #undef XMD_FK
+}
+
+// The step kernel's block as it runs: slots and threads per slot.  With 32-slot
+// blocks so few that a block's own latency is the kernel's time (mixed: all
+// resident at once, four per SM; FP64: one per SM, beyond which the FP64 pipe
+// binds), eight threads per slot instead of four: the pair entries go to twice
+// the warps.  us per MD step, four -> eight: 61 native chains mixed 31 -> 23,
+// 16 x 500 mixed 22 -> 18, 2,992 beads with contacts FP64 67 -> 47; 16 x 500
+// FP64 (297 blocks) 39 -> 44.
+Engine::ForceShape Engine::force_shape() const {
+    const bool mixed = params.precision == XMD_PREC_MIXED;
+    if (tune.fb == 32 && tune.lpb == 4 && force_blocks(d.N, 32) <= (mixed ? 4 : 1) * tile_sms) return ForceShape{32, 8};
+    return ForceShape{tune.fb, tune.lpb};
+}
+// The shape where none was set: 32-slot blocks up to 16 per SM (two waves at
+// four threads per slot), where more and smaller blocks keep the SMs evenly
+// loaded; beyond that 64-slot blocks, whose halo is half as large (5 of 64
+// slots, not of 32).  us per MD step, 32 / 64 slots: 54,744 beads mixed 70.9 /
+// 71.7, 66,007 beads mixed 45.4 / 42.8 and FP64 139.4 / 141.1, 8,000 beads FP64
+// 39 / 44.
+void Engine::default_shape() {
+    if (!tuned) tune.fb = force_blocks(d.N, 32) <= 16 * tile_sms ? 32 : 64;
 }
 
 void Engine::launch_force(int mode, int c) {
@@ -1472,7 +1489,8 @@ void Engine::launch_force(int mode, int c) {
         if (mode == 0) k_pid<0><<<(d.N + 127) / 128, 128, 0, stream>>>(d, tp, c);
         else k_pid<1><<<(d.N + 127) / 128, 128, 0, stream>>>(d, tp, c);
     }
-    const int fb = mode == 0 ? EVAL_FB : tune.fb, lpb = mode == 0 ? EVAL_LPB : tune.lpb;
+    const ForceShape fs = mode == 0 ? ForceShape{EVAL_FB, EVAL_LPB} : force_shape();
+    const int fb = fs.fb, lpb = fs.lpb;
     const int nb = force_blocks(d.N, fb);
     int fuse = FUSE_NONE;
     void *args[] = {&d, &tp, &c, &fuse};
@@ -2244,6 +2262,7 @@ void Engine::allocate() {
         const int k = tune.tile_per_sm > 0 ? std::min(tune.tile_per_sm, tile_max_per_sm) : tile_max_per_sm;
         tile_grid = std::max(1, std::min(d.nchunks, tile_sms * k));
     }
+    default_shape();
 
     // term parameters
     std::memset(&tp, 0, sizeof tp);
@@ -3041,6 +3060,7 @@ void Engine::set_tuning(const Tune &t) {
         throw std::invalid_argument("tuning: steps per graph must be 8, 16, 32 or 64");
     if (t.tile_per_sm < 0) throw std::invalid_argument("tuning: tile blocks per SM must be >= 0");
     tune = t;
+    tuned = true;
     if (finalized) {
         const int k = tune.tile_per_sm > 0 ? std::min(tune.tile_per_sm, tile_max_per_sm) : tile_max_per_sm;
         tile_grid = std::max(1, std::min(d.nchunks, tile_sms * k));
@@ -3174,10 +3194,11 @@ cudaGraphExec_t Engine::graph_for(int start_cur, bool gated, int len) {
     if (gs.exec) return gs.exec;
     cudaGraph_t g;
     CK(cudaGraphCreate(&g, 0));
-    const int nb = force_blocks(d.N, tune.fb);
     const bool mixed = params.precision == XMD_PREC_MIXED;
-    void *fk = force_kernel(mixed, 1, tune.fb, tune.lpb);
-    const size_t fsmem = force_smem(mixed, 1, tune.fb, d.qa_on);
+    const ForceShape fs = force_shape();
+    const int nb = force_blocks(d.N, fs.fb);
+    void *fk = force_kernel(mixed, 1, fs.fb, fs.lpb);
+    const size_t fsmem = force_smem(mixed, 1, fs.fb, d.qa_on);
     if (fsmem > 48 * 1024) CK(cudaFuncSetAttribute(fk, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fsmem));
     // a chain of nodes.  Between two kernels the edge is programmatic: the
     // second is launched while the first one's last blocks run and waits in
@@ -3222,7 +3243,7 @@ cudaGraphExec_t Engine::graph_for(int start_cur, bool gated, int len) {
         void *dargs[] = {&d, &dt, &rcheck};
         if (tp.ext_on) add((void *)k_ext<1>, (d.N + 255) / 256, 256, 0, sargs);   // AFM, walls
         if (tp.on[XMD_TERM_PID]) add((void *)k_pid<1>, (d.N + 127) / 128, 128, 0, sargs);
-        add(fk, nb, tune.fb * tune.lpb, fsmem, fargs);
+        add(fk, nb, fs.fb * fs.lpb, fsmem, fargs);
         if (d.qa_on) {
             add((void *)k_qa_sift, sift_grid(), QA_SIFT, 0, sargs);
             add((void *)k_qa_step, d.R, 1024, 0, sargs);

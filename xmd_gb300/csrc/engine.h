@@ -380,6 +380,10 @@ private:
     bool isolate_faults = false;
     void launch_force(int mode, int c);
     void split_positions();
+    struct ForceShape { int fb, lpb; };
+    ForceShape force_shape() const;
+    void default_shape();
+    bool tuned = false;   // a launch shape was set
     int tile_sms = 1, tile_max_per_sm = 1;     // for the tile build's resident grid
     // the QA sift's fixed grid: four blocks per SM, each taking at most
     // QA_SIFT groups of free-pair slots

@@ -21,12 +21,15 @@
 // quasi-adiabatic contacts, summed in that order after the bonded forces: the
 // trajectory is the same bits for every launch shape.
 //
-// What it measured, 256 chains of 50-800 beads (66,007), us per MD step at 64
-// slots x 4 threads, against a block whose threads kept to one bead each from
-// list loops to integrator (bonded geometry formed per term, a third of the
-// bonded warps with 3 live lanes, noise and skin test on a quarter of the
-// lanes): FP64 456 -> 156 (its FP64 pipe 81 % active), mixed 65 -> 44 (27.5 M
-// -> 11.6 M warp instructions).  One chain of 100 beads in FP64: 55 -> 24.
+// What it measured, us per MD step, against a block whose threads kept to one
+// bead each from list loops to integrator (bonded geometry formed per term, a
+// third of the bonded warps with 3 live lanes, noise and skin test on a quarter
+// of the lanes): 256 chains of 50-800 beads (66,007) FP64 456 -> 139, mixed
+// 65 -> 43; 61 native chains mixed 38 -> 23; 16 x 500 periodic FP64 105 -> 39,
+// mixed 31 -> 18; one chain of 100 beads FP64 55 -> 18.  FP64 is bound by its
+// pipe (81 % active while blocks run) and the tail of the last wave, mixed by
+// latency: index load, position load and arithmetic of a round of entries,
+// the barriers between the phases, 32 warps per SM to hide them.
 #pragma once
 
 namespace xmdg {
@@ -413,11 +416,11 @@ __device__ __forceinline__ void dihedral_chiral(const Dev &d, const TermP &p, co
 // ---- pair vectors -------------------------------------------------------------------
 // mixed: from split positions; the minimum image leaves the short form unless
 // a pair actually lies across the box
-__device__ __forceinline__ V3<float> pair_vec(const RepDev &rp, const F2 (&a)[3], const F2 (&b)[3]) {
+__device__ __forceinline__ V3<float> pair_vec(const RepDev &rp, bool per, const F2 (&a)[3], const F2 (&b)[3]) {
     float v[3];
 #pragma unroll
     for (int k = 0; k < 3; ++k) v[k] = __fadd_rn(__fsub_rn(b[k].h, a[k].h), __fsub_rn(b[k].l, a[k].l));
-    if (rp.per_any) {
+    if (per) {
 #pragma unroll
         for (int k = 0; k < 3; ++k)
             if (rintf(__fmul_rn(v[k], rp.Li[k])) != 0.0f)
@@ -434,7 +437,7 @@ __device__ __forceinline__ void spl_load(const float4 *spl, int j, F2 (&b)[3]) {
 template <class FT, int FB> struct StepSh {
     static constexpr bool MIX = sizeof(FT) == 4;
     // pair forces held at once; a block with more entries takes several passes
-    static constexpr int FCAP = 8 * FB;
+    static constexpr int FCAP = FB <= 32 ? 512 : 8 * FB;
     double F[3][FB];                  // new positions
     uint64_t rng[FB];                 // generator states after the step
     FT p[MIX ? 7 : 4][FB + 4];        // positions; mixed: h, l per axis, charge; FP64: x, y, z, charge
@@ -446,7 +449,7 @@ template <class FT, int FB> struct StepSh {
     // FP64: electrostatic entries set aside (their charge product, and which)
     FT ew[MIX ? 1 : FCAP];
     int eq[MIX ? 1 : FCAP], neq, next_es;
-    int off[FB + 4], ng[FB], nl[FB], nat0[FB], rep[FB], state[FB], ws[4], next;
+    int off[FB + 4], ng[FB], nl[FB], nat0[FB], rep[FB], state[FB], per[FB], ss0[FB], ss1[FB], ws[4], next;
     // followed, in contexts with the quasi-adiabatic term, by the beads'
     // contact slots in ascending order, int [FB][QA_REF_CAP]
 };
@@ -463,39 +466,71 @@ __device__ __forceinline__ FT es_factor(const TermP &p, FT vq, FT s2, FT rn, FT 
     return -mul_(*V, fma_<FT>(p.es_rel ? FT(2) : FT(1), rn, sdi));
 }
 
-// force of pair entry e of the block on its bead.  On the FP64 path the
-// electrostatic part (an exponential, half the pair's FP64 work) is set aside
-// when it is all there is to the pair: *es gets its charge factor and the
-// pair vector is returned, so that whole warps of such pairs do it later
-// instead of every warp that holds one.
-template <class FT, int MODE, int FB>
-__device__ __forceinline__ V3<FT> pair_entry(const Dev &d, const TermP &p, int cur, const StepSh<FT, FB> &s,
-                                             const int (*s_q)[QA_REF_CAP], int i0, int e, Ener<MODE> &en, FT *es) {
-    constexpr bool MIX = sizeof(FT) == 4;
+// a pair entry of the block: its bead's slot, the partner, the row's flags (0:
+// a native contact of length rm), the contact slot (-1: none)
+template <class FT> struct PairRef { int lo, j, ent, slot; FT rm; };
+template <class FT, int FB>
+__device__ __forceinline__ PairRef<FT> pair_fetch(const Dev &d, const TermP &p, const StepSh<FT, FB> &s,
+                                                  const int (*s_q)[QA_REF_CAP], int i0, int e, bool on) {
+    PairRef<FT> q{0, -1, 0, -1, FT(0)};
+    if (!on) return q;
     // the entry's bead: the last one that starts at or before it
     int lo = 0;
 #pragma unroll
     for (int h = FB / 2; h; h >>= 1)
         if (s.off[lo + h] <= e) lo += h;
-    const int i = i0 + lo, ng = s.ng[lo];
-    int m = e - s.off[lo];
-    int j = -1, slot = -1, ent = 0;
-    FT rm = FT(0);
-    if (m < ng) {
-        const int q = s.nat0[lo] + m;
-        j = d.act_j[q];
-        if constexpr (MIX) rm = narrow_f(d.act_d[q]);
-        else rm = d.act_d[q];
-    } else if ((m -= ng) < s.nl[lo]) {
-        ent = d.nl_row[(size_t)m * d.N + i];
-        if (ent & (NL_PAULI | NL_ES)) j = ent & NL_MASK;
-        rm = tpar<FT>(p.pauli_r_excl, p.f.pauli_r_excl);
+    const int i = i0 + lo, m = e - s.off[lo], k = m - s.ng[lo];
+    q.lo = lo;
+    if (k < s.nl[lo]) {
+        // one load for both lists, so that it diverges nowhere
+        const int at = s.nat0[lo] + m;
+        const int32_t *src = k < 0 ? d.act_j + at : d.nl_row + (size_t)k * d.N + i;
+        const int v = *src;
+        if (k < 0) {
+            const double nd = d.act_d[at];
+            if constexpr (sizeof(FT) == 4) q.rm = narrow_f(nd);
+            else q.rm = nd;
+            q.j = v;
+        } else {
+            q.ent = v;
+            q.j = v & (NL_PAULI | NL_ES) ? v & NL_MASK : -1;   // or a PID bundle only
+            q.rm = tpar<FT>(p.pauli_r_excl, p.f.pauli_r_excl);
+        }
     } else {
-        slot = s_q[lo][m - s.nl[lo]];
-        const int x = d.qa.ct_i1[slot];
-        j = x == i ? d.qa.ct_i2[slot] : x;
+        q.slot = s_q[lo][k - s.nl[lo]];
+        const int x = d.qa.ct_i1[q.slot];
+        q.j = x == i ? d.qa.ct_i2[q.slot] : x;
     }
-    if (j < 0) return V3<FT>{FT(0), FT(0), FT(0)};   // a PID bundle only
+    return q;
+}
+// the partner's position, and the pair vector from it
+template <class FT> struct PairPos { double4_32a p; };
+template <> struct PairPos<float> { float4 h, l; };
+template <class FT> __device__ __forceinline__ PairPos<FT> pair_pos(const Dev &d, int cur, int j) {
+    PairPos<FT> x{};
+    if constexpr (sizeof(FT) == 4) {
+        if (j >= 0) {
+            x.h = d.spl[cur][2 * (size_t)j];
+            x.l = d.spl[cur][2 * (size_t)j + 1];
+        }
+    } else {
+        if (j >= 0) x.p = d.pos[cur][j];
+    }
+    return x;
+}
+
+// force of a pair entry on its bead.  On the FP64 path the electrostatic part
+// (an exponential, half the pair's FP64 work) is set aside when it is all
+// there is to the pair: *es gets its charge factor and the pair vector is
+// returned, so that whole warps of such pairs do it later instead of every
+// warp that holds one.
+template <class FT, int MODE, int FB>
+__device__ __forceinline__ V3<FT> pair_entry(const Dev &d, const TermP &p, const StepSh<FT, FB> &s, int i0,
+                                             const PairRef<FT> &e, const PairPos<FT> &x, Ener<MODE> &en, FT *es) {
+    constexpr bool MIX = sizeof(FT) == 4;
+    const int lo = e.lo, i = i0 + lo, j = e.j, ent = e.ent, slot = e.slot;
+    const FT rm = e.rm;
+    if (j < 0) return V3<FT>{FT(0), FT(0), FT(0)};
     const int r = s.rep[lo];
     const RepDev &rp = d.rep[r];
     V3<FT> r12;
@@ -503,15 +538,13 @@ __device__ __forceinline__ V3<FT> pair_entry(const Dev &d, const TermP &p, int c
     if constexpr (MIX) {
         const F2 pa[3] = {{s.p[0][lo + 3], s.p[3][lo + 3]}, {s.p[1][lo + 3], s.p[4][lo + 3]},
                           {s.p[2][lo + 3], s.p[5][lo + 3]}};
-        const float4 h = d.spl[cur][2 * (size_t)j], l = d.spl[cur][2 * (size_t)j + 1];
-        const F2 pb[3] = {{h.x, l.x}, {h.y, l.y}, {h.z, l.z}};
-        r12 = pair_vec(rp, pa, pb);
-        qj = h.w;
+        const F2 pb[3] = {{x.h.x, x.l.x}, {x.h.y, x.l.y}, {x.h.z, x.l.z}};
+        r12 = pair_vec(rp, s.per[lo] != 0, pa, pb);
+        qj = x.h.w;
     } else {
-        const double4_32a pj = d.pos[cur][j];
         const double4_32a pi = make_double4_32a(s.p[0][lo + 3], s.p[1][lo + 3], s.p[2][lo + 3], 0.0);
-        r12 = r_uv_p<double>(rp.box, rp.per_any != 0, pi, pj);
-        qj = pj.w;
+        r12 = r_uv_p<double>(rp.box, s.per[lo] != 0, pi, x.p);
+        qj = x.p.w;
     }
     const FT s2 = fdot(r12, r12), rn = rsq(s2);
     FT dV = FT(0);
@@ -530,10 +563,10 @@ __device__ __forceinline__ V3<FT> pair_entry(const Dev &d, const TermP &p, int c
         // Go (go.cpp:31-46, lj.h:22-30) and Pauli (pauli.cpp:32-48,
         // shifted_lj.h:14-21) have one force law, Pauli inside r_excl only
         const bool go = ent == 0;
-        const FT x = mul_(rn, rm);
-        if (go || ((ent & NL_PAULI) && FT(1) < x)) {
+        const FT w = mul_(rn, rm);
+        if (go || ((ent & NL_PAULI) && FT(1) < w)) {
             const FT depth = go ? tpar<FT>(p.go_depth, p.f.go_depth) : tpar<FT>(p.pauli_depth, p.f.pauli_depth);
-            const FT x2 = mul_(x, x), x3 = mul_(x2, x), s6 = mul_(x3, x3);
+            const FT w2 = mul_(w, w), w3 = mul_(w2, w), s6 = mul_(w3, w3);
             // s6 - s12 = s6 (1 - s6)
             dV = mul_(mul_(mul_(FT(12), depth), rn), mul_(s6, add_(FT(1), -s6)));
             dV = clampv<FT>(dV, FT(-1.0e3), FT(1.0e3));
@@ -561,16 +594,19 @@ __device__ __forceinline__ V3<FT> pair_entry(const Dev &d, const TermP &p, int c
 // MODE 1: forces, then one Langevin predictor-corrector step (lang_pc.cpp:5-41)
 //         writing pos[cur^1], y1..y5, the generator state and the skin-test
 //         displacement (verify.cpp:10-15).
-// r: replica of the block's bead t (threads t < FBT), -1 where there is none.
+// gated: the kernel does nothing while the gate is closed; returns whether it
+// was open.
 template <class FT, int MODE, int FB, int LPB>
-__device__ __forceinline__ void force_block(const Dev &d, const TermP &p, int cur, int r) {
+__device__ __forceinline__ bool force_block(const Dev &d, const TermP &p, int cur, bool gated) {
     constexpr bool MIX = sizeof(FT) == 4;
-    constexpr int NT = FB * LPB, FBT = step_beads<FB>(), NP = FB + 1, NC = FBT + 3;
-    constexpr int TT = (3 * FBT + NT - 1) / NT;   // (axis, bead) tasks per thread
+    constexpr int NT = FB * LPB;
+    constexpr int FBT = step_beads<FB>(), NP = FB + 1, NC = FBT + 3;
     constexpr int FCAP = StepSh<FT, FB>::FCAP;
-    // first thread of the tasks: with four threads per slot, past the warps of
-    // the geometry and the angles
-    constexpr int W0 = LPB == 4 ? FB : 0;
+    // first thread of the (axis, bead) tasks: with four threads per slot or
+    // more, past the warps of the geometry and the angles
+    constexpr int W0 = LPB >= 4 ? FB : 0;
+    constexpr int TT = (3 * FBT + NT - W0 - 1) / (NT - W0);   // tasks per thread
+    static_assert(LPB < 4 || TT == 1, "one task per thread");
     using ST = typename StepSum<FT>::T;
     extern __shared__ __align__(16) unsigned char step_mem[];
     StepSh<FT, FB> &s = *reinterpret_cast<StepSh<FT, FB> *>(step_mem);
@@ -578,25 +614,13 @@ __device__ __forceinline__ void force_block(const Dev &d, const TermP &p, int cu
     const int N = d.N, t = threadIdx.x, i0 = blockIdx.x * FBT, lane = t & 31;
     const size_t Ns = (size_t)N;
     const bool qa = d.qa_on && p.on[XMD_TERM_QA];
+    const unsigned FULL = 0xffffffffu;
 
-    // ---- A: tile and list lengths.  What later phases load from memory
-    // without needing a result is loaded here, so that its latency passes
-    // once: the centre's parameters, the generator state
-    for (int k = t; k < NP; k += NT) {
-        const int idx = i0 - 3 + k;
-        const bool ok = idx >= 0 && idx < N;
-        if constexpr (MIX) {
-            const float4 z = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-            const float4 h = ok ? d.spl[cur][2 * (size_t)idx] : z, l = ok ? d.spl[cur][2 * (size_t)idx + 1] : z;
-            s.p[0][k] = h.x; s.p[1][k] = h.y; s.p[2][k] = h.z;
-            s.p[3][k] = l.x; s.p[4][k] = l.y; s.p[5][k] = l.z;
-            s.p[6][k] = h.w;
-        } else {
-            const double4_32a q = ok ? d.pos[cur][idx] : make_double4_32a(0, 0, 0, 0);
-            s.p[0][k] = q.x; s.p[1][k] = q.y; s.p[2][k] = q.z; s.p[3][k] = q.w;
-        }
-    }
-    const int sc = t & (FB - 1), c = i0 - 2 + sc;   // the thread's centre (t < 2 FB)
+    // ---- A: what no kernel writes is loaded before the kernels before this
+    // one have finished: owners, flags and parameters of the thread's centre,
+    // the native ranges
+    const int r = t < FBT && i0 + t < N ? d.rep_of[i0 + t] : -1;   // replica of bead t
+    const int sc = t & (FB - 1), c = i0 - 2 + sc;                  // the thread's centre (t < 2 FB)
     uint32_t fl = 0;
     CentreP<FT> cp{FT(0), FT(0), FT(0), FT(0), FT(0)};
     if (t < 2 * FB && sc < NC && c >= 0 && c < N) {
@@ -610,10 +634,29 @@ __device__ __forceinline__ void force_block(const Dev &d, const TermP &p, int cu
             if (LPB == 1 || t >= FB) { const double2 q = d.dih_cs[c]; cp.c0 = q.x; cp.s0 = q.y; }
         }
     }
-    const int bn = LPB == 1 ? t : t - FB;           // the bead whose noise this thread draws
+    int nat0 = 0, ss0 = 0, ss1 = 0;
+    if (t < FBT && i0 + t < N) {
+        nat0 = d.nat_start[i0 + t];
+        if (p.on[XMD_TERM_NAT_SS]) {
+            ss0 = d.ss_start[i0 + t];
+            ss1 = d.ss_end[i0 + t];
+        }
+    }
+    step_order();
+    if (gated && d.gate[0]) return false;   // uniform: the gate changes between launches
+
+    // the tile, the list lengths, and what later phases load without needing
+    // a result, so that its latency passes once
+    const int bn = LPB == 1 ? t : t - FB;                          // the bead whose noise this thread draws
     const bool draws = MODE == 1 && bn >= 0 && bn < FBT && i0 + bn < N;
     uint64_t st0 = 0;
     if (draws) st0 = d.rng[i0 + bn];
+    int ng = 0, nl = 0, nq = 0;
+    if (t < FBT && i0 + t < N) {
+        nl = d.nl_cnt[i0 + t];
+        if (p.on[XMD_TERM_GO]) ng = d.go_cnt[i0 + t];
+        if (qa) nq = min(d.qa.ref_cnt[i0 + t], QA_REF_CAP);
+    }
     double y[TT][6], o[TT];
 #pragma unroll
     for (int u = 0; u < TT; ++u) {
@@ -628,40 +671,48 @@ __device__ __forceinline__ void force_block(const Dev &d, const TermP &p, int cu
             o[u] = reinterpret_cast<const double *>(d.orig + i)[a];
         }
     }
+    for (int k = t; k < NP; k += NT) {
+        const int idx = i0 - 3 + k;
+        const bool ok = idx >= 0 && idx < N;
+        if constexpr (MIX) {
+            const float4 z = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            const float4 h = ok ? d.spl[cur][2 * (size_t)idx] : z, l = ok ? d.spl[cur][2 * (size_t)idx + 1] : z;
+            s.p[0][k] = h.x; s.p[1][k] = h.y; s.p[2][k] = h.z;
+            s.p[3][k] = l.x; s.p[4][k] = l.y; s.p[5][k] = l.z;
+            s.p[6][k] = h.w;
+        } else {
+            const double4_32a q = ok ? d.pos[cur][idx] : make_double4_32a(0, 0, 0, 0);
+            s.p[0][k] = q.x; s.p[1][k] = q.y; s.p[2][k] = q.z; s.p[3][k] = q.w;
+        }
+    }
     int scan = 0, cnt = 0;
     if (t < FB) {
-        const int i = i0 + t;
-        int ng = 0, nl = 0, nq = 0, nat0 = 0;
-        if (r >= 0) {
-            nl = d.nl_cnt[i];
-            if (p.on[XMD_TERM_GO]) {
-                nat0 = d.nat_start[i];
-                ng = d.go_cnt[i];
-            }
-            if (qa) nq = min(d.qa.ref_cnt[i], QA_REF_CAP);
-        }
+        if (r < 0) ng = nl = nq = 0;
         scan = cnt = ng + nl + nq;
 #pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const int y = __shfl_up_sync(0xffffffffu, scan, o);
-            if (lane >= o) scan += y;
+        for (int o_ = 1; o_ < 32; o_ <<= 1) {
+            const int x = __shfl_up_sync(FULL, scan, o_);
+            if (lane >= o_) scan += x;
         }
         if (lane == 31) s.ws[t >> 5] = scan;
         s.ng[t] = ng; s.nl[t] = nl; s.nat0[t] = nat0; s.rep[t] = r;
-        // a replica that has taken its steps keeps its state
-        if (MODE == 0) s.state[t] = r >= 0 ? 1 : -1;
+        s.ss0[t] = ss0; s.ss1[t] = r >= 0 ? ss1 : ss0;
     }
     if (t == 0) s.next = s.neq = s.next_es = 0;
-    if (!__syncthreads_or(r >= 0)) return;   // no bead slot of the block is in use
+    if (!__syncthreads_or(r >= 0)) return true;   // no bead slot of the block is in use
     int T = 0;
 #pragma unroll
     for (int k = 0; k < FB / 32; ++k) T += s.ws[k];
+    // a replica that has taken its steps keeps its state (its word is stored
+    // when it is needed, not waited for here)
+    int state = r >= 0 ? 1 : -1;
     if (t < FB) {
         int base = 0;
         for (int k = 0; k < (t >> 5); ++k) base += s.ws[k];
         s.off[t] = base + scan - cnt;
         if (t == FB - 1) s.off[FB] = T;
-        if (MODE == 1) s.state[t] = r < 0 ? -1 : (d.rep[r].steps_left == 0 ? 0 : 1);
+        s.per[t] = r >= 0 ? d.rep[r].per_any : 0;
+        if (MODE == 1 && r >= 0 && d.rep[r].steps_left == 0) state = 0;
     }
     __syncthreads();
     if (qa) {
@@ -682,8 +733,8 @@ __device__ __forceinline__ void force_block(const Dev &d, const TermP &p, int cu
             int x = 0;
 #pragma unroll
             for (int u = 0; u < HOLD; ++u) {
-                const int y = __shfl_sync(qm, v[u], m % LPB, LPB);
-                if (m / LPB == u) x = y;
+                const int w = __shfl_sync(qm, v[u], m % LPB, LPB);
+                if (m / LPB == u) x = w;
             }
 #pragma unroll
             for (int u = 0; u < HOLD; ++u) rk[u] += x < v[u];
@@ -747,7 +798,7 @@ __device__ __forceinline__ void force_block(const Dev &d, const TermP &p, int cu
             s.rng[bn] = rb >= 0 ? gf2_apply_nib(d.jump + JUMP_WORDS * rb, st0) : 0;
         }
         // the geometry is read by the warps of this part only
-        if constexpr (LPB == 4) asm volatile("bar.sync 1, %0;" ::"n"(2 * FB) : "memory");
+        if constexpr (LPB >= 4) asm volatile("bar.sync 1, %0;" ::"n"(2 * FB) : "memory");
         else __syncthreads();
 
         // ---- D: bonded centres
@@ -800,80 +851,92 @@ __device__ __forceinline__ void force_block(const Dev &d, const TermP &p, int cu
             nh[i] = n.x; nh[Ns + i] = n.y; nh[2 * Ns + i] = n.z;
             nh[3 * Ns + i] = h.x; nh[4 * Ns + i] = h.y; nh[5 * Ns + i] = h.z;
         }
+        if (t < FB) s.state[t] = state;
     }
 
     // ---- E: pair entries, FCAP at a time; between the passes every (axis,
-    // bead) thread adds its bead's forces
-    // what the integrator does before the force is known: lang_pc_step::
-    // operator(), lang_pc.cpp:11-37, mass = 1 (main.cpp:156), is linear in the
-    // force, so corrector and predictor (the Taylor shift by repeated
-    // addition) are applied to y1..y5 alone here, beside the other warps'
-    // work, and the force and noise enter with one multiply-add per order at
-    // the end.  The position is rounded where the reference rounds it, once
-    // by the corrector and once by the predictor: a rounding more at its
-    // scale grows to 5e-8 A in 50 steps from a stiff extended start.
-    double err0[TT], sum0[TT];
-    if constexpr (MODE == 1) {
-#pragma unroll
-        for (int u = 0; u < TT; ++u) {
-            err0[u] = sum0[u] = 0.0;
-            if (t < W0) continue;
-            double(&q)[6] = y[u];
-            const double err = __fma_rn(__dmul_rn(p.gamma_factor, __dmul_rn(q[1], p.dt_inv)), p.dt2_half, q[2]);
-            err0[u] = err;
-            q[1] = __fma_rn(-(251.0 / 360.0), err, q[1]);
-            q[2] = __dsub_rn(q[2], err);
-            q[3] = __fma_rn(-(11.0 / 18.0), err, q[3]);
-            q[4] = __fma_rn(-(1.0 / 6.0), err, q[4]);
-            q[5] = __fma_rn(-(1.0 / 60.0), err, q[5]);
-#pragma unroll
-            for (int m = 0; m < 5; ++m) {
-#pragma unroll
-                for (int k = 4; k >= (m ? m : 1); --k) q[k] = __dadd_rn(q[k], q[k + 1]);
-                if (m == 0) sum0[u] = q[1];
-            }
-        }
-    }
-
+    // bead) thread adds its bead's forces.  A warp fetches the index data of
+    // its next 32 entries before it computes the last ones.
+    double err0[TT], sum0[TT], sd[TT];
     ST acc[TT];
     for (int p0 = 0;; p0 += FCAP) {
         const int pe = min(T - p0, FCAP);
-        for (;;) {
+        auto grab = [&]() {
             int at = 0;
             if (lane == 0) at = atomicAdd(&s.next, 32);
-            at = __shfl_sync(0xffffffffu, at, 0);
-            if (at >= pe) break;
+            return __shfl_sync(FULL, at, 0) + lane;
+        };
+        int at = grab();
+        PairRef<FT> ref = pair_fetch<FT, FB>(d, p, s, s_q, i0, p0 + at, at < pe);
+        if (MODE == 1 && p0 == 0) {
+            // what the integrator does before the force is known:
+            // lang_pc_step::operator(), lang_pc.cpp:11-37, mass = 1
+            // (main.cpp:156), is linear in the force, so corrector and
+            // predictor (the Taylor shift by repeated addition) are applied to
+            // y1..y5 alone here, beside the other warps' work, and the force
+            // and noise enter with one multiply-add per order at the end.  The
+            // position is rounded where the reference rounds it, once by the
+            // corrector and once by the predictor: a rounding more at its
+            // scale grows to 5e-8 A in 50 steps from a stiff extended start.
+#pragma unroll
+            for (int u = 0; u < TT; ++u) {
+                err0[u] = sum0[u] = sd[u] = 0.0;
+                const int w = t - W0 + u * NT, b = w % FBT;
+                if (w < 0 || w >= 3 * FBT) continue;
+                if (s.rep[b] >= 0) sd[u] = d.rep[s.rep[b]].noise_sd;
+                double(&q)[6] = y[u];
+                const double err = __fma_rn(__dmul_rn(p.gamma_factor, __dmul_rn(q[1], p.dt_inv)), p.dt2_half, q[2]);
+                err0[u] = err;
+                q[1] = __fma_rn(-(251.0 / 360.0), err, q[1]);
+                q[2] = __dsub_rn(q[2], err);
+                q[3] = __fma_rn(-(11.0 / 18.0), err, q[3]);
+                q[4] = __fma_rn(-(1.0 / 6.0), err, q[4]);
+                q[5] = __fma_rn(-(1.0 / 60.0), err, q[5]);
+#pragma unroll
+                for (int m = 0; m < 5; ++m) {
+#pragma unroll
+                    for (int k = 4; k >= (m ? m : 1); --k) q[k] = __dadd_rn(q[k], q[k + 1]);
+                    if (m == 0) sum0[u] = q[1];
+                }
+            }
+        }
+        while (at - lane < pe) {
+            const PairPos<FT> x = pair_pos<FT>(d, cur, ref.j);
+            const int nx = grab();
+            const PairRef<FT> nref = pair_fetch<FT, FB>(d, p, s, s_q, i0, p0 + nx, nx < pe);
             FT es = FT(0);
-            if (at + lane < pe) {
-                const V3<FT> f = pair_entry<FT, MODE, FB>(d, p, cur, s, s_q, i0, p0 + at + lane, en, &es);
-                s.f[0][at + lane] = f.x; s.f[1][at + lane] = f.y; s.f[2][at + lane] = f.z;
+            if (at < pe) {
+                const V3<FT> f = pair_entry<FT, MODE, FB>(d, p, s, i0, ref, x, en, &es);
+                s.f[0][at] = f.x; s.f[1][at] = f.y; s.f[2][at] = f.z;
             }
             if constexpr (!MIX && MODE == 1) {
-                const unsigned m = __ballot_sync(0xffffffffu, es != FT(0));
+                const unsigned m = __ballot_sync(FULL, es != FT(0));
                 int to = 0;
                 if (lane == 0 && m) to = atomicAdd(&s.neq, __popc(m));
-                to = __shfl_sync(0xffffffffu, to, 0) + __popc(m & ((1u << lane) - 1u));
+                to = __shfl_sync(FULL, to, 0) + __popc(m & ((1u << lane) - 1u));
                 if (es != FT(0)) {
-                    s.eq[to] = at + lane;
+                    s.eq[to] = at;
                     s.ew[to] = es;
                 }
             }
+            at = nx;
+            ref = nref;
         }
         if constexpr (!MIX && MODE == 1) {
             // the electrostatic entries set aside
             __syncthreads();
             const int ne = s.neq;
             for (;;) {
-                int at = 0;
-                if (lane == 0) at = atomicAdd(&s.next_es, 32);
-                at = __shfl_sync(0xffffffffu, at, 0);
-                if (at >= ne) break;
-                if (at + lane < ne) {
-                    const int k = s.eq[at + lane];
+                int k0 = 0;
+                if (lane == 0) k0 = atomicAdd(&s.next_es, 32);
+                k0 = __shfl_sync(FULL, k0, 0);
+                if (k0 >= ne) break;
+                if (k0 + lane < ne) {
+                    const int k = s.eq[k0 + lane];
                     const V3<FT> r12{s.f[0][k], s.f[1][k], s.f[2][k]};
                     const FT s2 = fdot(r12, r12), rn = rsq(s2);
                     FT V_;
-                    const V3<FT> f = fscl<FT>(mul_(es_factor<FT>(p, s.ew[at + lane], s2, rn, &V_), rn), r12);
+                    const V3<FT> f = fscl<FT>(mul_(es_factor<FT>(p, s.ew[k0 + lane], s2, rn, &V_), rn), r12);
                     s.f[0][k] = f.x; s.f[1][k] = f.y; s.f[2][k] = f.z;
                 }
             }
@@ -917,25 +980,22 @@ __device__ __forceinline__ void force_block(const Dev &d, const TermP &p, int cu
         const int w = t - W0 + u * NT, a = w / FBT, b = w - a * FBT, i = i0 + b;
         F[u] = 0.0;
         if (w < 0 || w >= 3 * FBT || s.state[b] != 1) continue;
-        if (p.on[XMD_TERM_NAT_SS]) {
-            const int s1 = d.ss_end[i];
-            for (int k = d.ss_start[i]; k < s1; ++k) {
-                if (!d.ss_on[k]) continue;
-                const int j = d.ss_j[k], rb = s.rep[b];
-                V3<FT> r12;
-                if constexpr (MIX) {
-                    F2 pa[3], pb[3];
-                    spl_load(d.spl[cur], i, pa);
-                    spl_load(d.spl[cur], j, pb);
-                    r12 = pair_vec(d.rep[rb], pa, pb);
-                } else {
-                    r12 = r_uv_p<double>(d.rep[rb].box, d.rep[rb].per_any != 0, d.pos[cur][i], d.pos[cur][j]);
-                }
-                FT V_;
-                const V3<FT> f = ss_pair<FT>(p, r12, &V_);
-                sum_acc(acc[u], a == 0 ? f.x : (a == 1 ? f.y : f.z));
-                if (MODE == 0 && i < j && a == 0) en.add(d, rb, XMD_TERM_NAT_SS, (double)V_);
+        for (int k = s.ss0[b]; k < s.ss1[b]; ++k) {
+            if (!d.ss_on[k]) continue;
+            const int j = d.ss_j[k], rb = s.rep[b];
+            V3<FT> r12;
+            if constexpr (MIX) {
+                F2 pa[3], pb[3];
+                spl_load(d.spl[cur], i, pa);
+                spl_load(d.spl[cur], j, pb);
+                r12 = pair_vec(d.rep[rb], s.per[b] != 0, pa, pb);
+            } else {
+                r12 = r_uv_p<double>(d.rep[rb].box, s.per[b] != 0, d.pos[cur][i], d.pos[cur][j]);
             }
+            FT V_;
+            const V3<FT> f = ss_pair<FT>(p, r12, &V_);
+            sum_acc(acc[u], a == 0 ? f.x : (a == 1 ? f.y : f.z));
+            if (MODE == 0 && i < j && a == 0) en.add(d, rb, XMD_TERM_NAT_SS, (double)V_);
         }
         F[u] = sum_total(acc[u]);
         if (p.ext_on) F[u] += d.fext[3 * (size_t)i + a];
@@ -972,12 +1032,11 @@ __device__ __forceinline__ void force_block(const Dev &d, const TermP &p, int cu
         for (int u = 0; u < TT; ++u) {
             const int w = t - W0 + u * NT, a = w / FBT, b = w - a * FBT, i = i0 + b;
             if (w < 0 || w >= 3 * FBT || s.state[b] != 1) continue;
-            const RepDev &rp = d.rep[s.rep[b]];
             double nz;
             if constexpr (MIX) nz = widen_f(s.n[a][b]);
             else nz = s.n[a][b];
             double(&q)[6] = y[u];
-            const double fh = __dmul_rn(__fma_rn(rp.noise_sd, nz, F[u]), p.dt2_half);
+            const double fh = __dmul_rn(__fma_rn(sd[u], nz, F[u]), p.dt2_half);
             q[0] = __dadd_rn(__fma_rn(-c0, __dsub_rn(err0[u], fh), q[0]), __fma_rn(K[0], fh, sum0[u]));
 #pragma unroll
             for (int k = 1; k < 6; ++k) q[k] = __fma_rn(K[k], fh, q[k]);
@@ -990,8 +1049,10 @@ __device__ __forceinline__ void force_block(const Dev &d, const TermP &p, int cu
             // Open axes wrap by exactly zero.  The mixed path squares the FP64
             // difference in FP32.
             double e = __dsub_rn(o[u], q[0]);
-            if (rp.per_any)
-                e = __dsub_rn(e, __dmul_rn(rp.box.cell[a], rint(__dmul_rn(e, rp.box.cell_inv[a]))));
+            if (s.per[b]) {
+                const BoxD &bx = d.rep[s.rep[b]].box;
+                e = __dsub_rn(e, __dmul_rn(bx.cell[a], rint(__dmul_rn(e, bx.cell_inv[a]))));
+            }
             if constexpr (MIX) {
                 const float ef = narrow_f(e);
                 s.e[a][b] = __fmul_rn(ef, ef);
@@ -1030,11 +1091,11 @@ __device__ __forceinline__ void force_block(const Dev &d, const TermP &p, int cu
                 d.rng[i] = s.rng[t];
             }
             // one atomic per warp where its beads are of one replica
-            const unsigned act = __ballot_sync(0xffffffffu, st == 1);
+            const unsigned act = __ballot_sync(FULL, st == 1);
             if (act) {
-                const int r0 = __shfl_sync(0xffffffffu, r, __ffs(act) - 1);
+                const int r0 = __shfl_sync(FULL, r, __ffs(act) - 1);
                 const unsigned long long db = (unsigned long long)__double_as_longlong(disp);
-                if (__all_sync(0xffffffffu, st != 1 || r == r0)) {
+                if (__all_sync(FULL, st != 1 || r == r0)) {
                     const unsigned long long m = warp_max_bits(db);
                     if (lane == 0) atomicMax(&d.rep[r0].maxdisp, m);
                 } else if (st == 1) {
@@ -1043,6 +1104,7 @@ __device__ __forceinline__ void force_block(const Dev &d, const TermP &p, int cu
             }
         }
     }
+    return true;
 }
 
 }  // namespace xmdg
