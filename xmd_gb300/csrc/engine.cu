@@ -1502,7 +1502,7 @@ void Engine::launch_force(int mode, int c) {
 }
 
 void Engine::split_positions() {
-    if (params.precision != XMD_PREC_MIXED) return;
+    if (params.precision != XMD_PREC_MIXED && !d.qa_on) return;
     k_split<<<(d.N + 255) / 256, 256, 0, stream>>>(d, cur);
     ++launches;
 }
@@ -2346,7 +2346,7 @@ void Engine::allocate() {
         // quasi-adiabatic state (tables of main.cpp:681-700, lj_variants.cpp:59-62)
         d.qa_on = 1;
         QaDev &q = d.qa;
-        q.nh = (float *)dalloc(sizeof(float) * 6 * (size_t)N);
+        q.nh = (float4 *)dalloc(2 * sizeof(float4) * (size_t)N);
         q.sync = (int32_t *)dalloc(sizeof(int32_t) * N);
         q.ref_cnt = (int32_t *)dalloc(sizeof(int32_t) * N);
         q.ref = (int32_t *)dalloc(sizeof(int32_t) * QA_REF_CAP * (size_t)N);

@@ -100,7 +100,7 @@ constexpr int QA_BCHUNK = 1024;      // beads per chunk of the free-pair re-list
 
 // device record of the quasi-adiabatic state
 struct QaDev {
-    float *nh;                   // [6][N]: n then h (precompute_nh.cpp:12-20) to FP32 accuracy
+    float4 *nh;                  // [N][2]: n, h (precompute_nh.cpp:12-20) to FP32 accuracy
     int32_t *sync;               // [N] packed int8 x4: back | side_all | side_polar | side_hydrophobic
     int32_t *ref_cnt, *ref;      // [N], [QA_REF_CAP][N] contact slots per bead
     int32_t *tmp_cnt, *tmp;      // [N], [QA_TMP_CAP][N] partners collected at a rebuild
@@ -134,7 +134,7 @@ struct Dev {
     int N, R, nl_cap;
     double4_32a *pos[2];        // x, y, z, charge; double-buffered
     double *yh;             // [15][N]: y1x y1y y1z y2x ... y5z
-    // mixed path: positions split per axis, [2 i] = (hx, hy, hz, charge), [2 i + 1] = (lx, ly, lz, 0)
+    // mixed path, and the contacts' sift: positions split per axis, [2 i] = (hx, hy, hz, charge), [2 i + 1] = (lx, ly, lz, 0)
     float4 *spl[2];
     double4_32a *orig;          // positions at the last list rebuild
     double *F;              // [3N] force output of eval

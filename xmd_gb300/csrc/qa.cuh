@@ -14,6 +14,26 @@
 
 namespace xmdg {
 
+// ---- pair vectors -------------------------------------------------------------------
+// mixed: from split positions; the minimum image leaves the short form unless
+// a pair actually lies across the box
+__device__ __forceinline__ V3<float> pair_vec(const RepDev &rp, bool per, const F2 (&a)[3], const F2 (&b)[3]) {
+    float v[3];
+#pragma unroll
+    for (int k = 0; k < 3; ++k) v[k] = __fadd_rn(__fsub_rn(b[k].h, a[k].h), __fsub_rn(b[k].l, a[k].l));
+    if (per) {
+#pragma unroll
+        for (int k = 0; k < 3; ++k)
+            if (rintf(__fmul_rn(v[k], rp.Li[k])) != 0.0f)
+                v[k] = mi_axis(a[k], b[k], rp.Lh[k], rp.Ll[k], rp.Li[k], true);
+    }
+    return V3<float>{v[0], v[1], v[2]};
+}
+__device__ __forceinline__ void spl_load(const float4 *spl, int j, F2 (&b)[3]) {
+    const float4 h = spl[2 * (size_t)j], l = spl[2 * (size_t)j + 1];
+    b[0] = F2{h.x, l.x}; b[1] = F2{h.y, l.y}; b[2] = F2{h.z, l.z};
+}
+
 enum : int { QA_FORMING = 0, QA_BREAKING = 1 };
 
 // ---- exactly rounded vector helpers (no FMA contraction) -------------------
@@ -158,9 +178,6 @@ __device__ __noinline__ int qa_sift_fp64(const Dev &d, const RepDev &rp, int i1,
     return type;
 }
 
-__device__ __forceinline__ V3<float> nh_f(const QaDev &q, size_t N, int i, int off) {
-    return V3<float>{q.nh[(off + 0) * N + i], q.nh[(off + 1) * N + i], q.nh[(off + 2) * N + i]};
-}
 // x > T (or, with less, x < T) decided in FP32; *unsure when x is within
 // the band of T
 __device__ __forceinline__ bool cmp_band(float x, float T, bool less, bool *unsure) {
@@ -183,19 +200,22 @@ __device__ __forceinline__ void qa_sift_group(const Dev &d, const TermP &p, int 
     if (live && !q.fp_vac[slot]) {
         i1 = q.fp_i1[slot];
         i2 = q.fp_i2[slot];
-        const double4_32a *pos = d.pos[cur];
-        const bool per = (rp.per[0] | rp.per[1] | rp.per[2]) != 0;
-        const PairGeo<float> geo(rp.box, per, pos[i1]);
-        const V3<float> r12 = geo.to(pos[i2]);
+        // positions as the step kernel split them (splitting both beads of
+        // every pair here was half of the sift's instructions)
+        F2 pa[3], pb[3];
+        spl_load(d.spl[cur], i1, pa);
+        spl_load(d.spl[cur], i2, pb);
+        const V3<float> r12 = pair_vec(rp, rp.per_any != 0, pa, pb);
         const float d2 = r12.x * r12.x + r12.y * r12.y + r12.z * r12.z;
         // beyond every type's formation distance no pair is a candidate (the
         // widened FP32 gate keeps every pair the FP64 gate keeps)
         if (d2 <= q.req_out2_f) {
-            const float rn = 1.0f / sqrtf(d2);
+            const float rn = rsq(d2);
             const V3<float> u{r12.x * rn, r12.y * rn, r12.z * rn};
-            const size_t N = d.N;
-            const V3<float> n1 = nh_f(q, N, i1, 0), n2 = nh_f(q, N, i2, 0);
-            const V3<float> h1 = nh_f(q, N, i1, 3), h2 = nh_f(q, N, i2, 3);
+            const float4 f1 = q.nh[2 * (size_t)i1], g1 = q.nh[2 * (size_t)i1 + 1];
+            const float4 f2 = q.nh[2 * (size_t)i2], g2 = q.nh[2 * (size_t)i2 + 1];
+            const V3<float> n1{f1.x, f1.y, f1.z}, h1{g1.x, g1.y, g1.z};
+            const V3<float> n2{f2.x, f2.y, f2.z}, h2{g2.x, g2.y, g2.z};
             bool unsure = false;
             const bool back1 = cmp_band(fabsf(dot(h1, u)), q.min_cos_hr_f, false, &unsure);
             const bool back2 = cmp_band(fabsf(dot(h2, u)), q.min_cos_hr_f, false, &unsure);

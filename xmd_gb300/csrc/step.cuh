@@ -69,17 +69,6 @@ template <class T> __device__ __forceinline__ V3<T> fscl(T s, V3<T> a) {
     return V3<T>{mul_(s, a.x), mul_(s, a.y), mul_(s, a.z)};
 }
 
-// 1 / sqrt(x).  FP32: the hardware estimate and one Newton step (3
-// instructions, within 1 ulp), where 1 / sqrtf(x) takes about twenty; zero
-// and infinity as the estimate gives them.
-__device__ __forceinline__ double rsq(double x) { return rsqrt(x); }
-__device__ __forceinline__ float rsq(float x) {
-    const float y = rsqrtf(x);
-    const float r = __fmaf_rn(-__fmul_rn(x, y), y, 1.0f);
-    const float z = __fmaf_rn(__fmul_rn(0.5f, y), r, y);
-    return x > 0.0f && y > 0.0f ? z : y;
-}
-
 // ---- noise of the FP64 path -------------------------------------------------------
 // Box-Muller on four 32-bit draws k / 2^32 as noise3 forms them
 // (rand_gen.h:22-58, lang_pc.cpp:15-16), with the reductions done on the
@@ -411,26 +400,6 @@ __device__ __forceinline__ void dihedral_chiral(const Dev &d, const TermP &p, co
         for (int k = 0; k < 4; ++k) q[k] = q[k] + h[k];
         if (MODE == 0 && own) en.add(d, rc, XMD_TERM_CHIR, Vch);
     }
-}
-
-// ---- pair vectors -------------------------------------------------------------------
-// mixed: from split positions; the minimum image leaves the short form unless
-// a pair actually lies across the box
-__device__ __forceinline__ V3<float> pair_vec(const RepDev &rp, bool per, const F2 (&a)[3], const F2 (&b)[3]) {
-    float v[3];
-#pragma unroll
-    for (int k = 0; k < 3; ++k) v[k] = __fadd_rn(__fsub_rn(b[k].h, a[k].h), __fsub_rn(b[k].l, a[k].l));
-    if (per) {
-#pragma unroll
-        for (int k = 0; k < 3; ++k)
-            if (rintf(__fmul_rn(v[k], rp.Li[k])) != 0.0f)
-                v[k] = mi_axis(a[k], b[k], rp.Lh[k], rp.Ll[k], rp.Li[k], true);
-    }
-    return V3<float>{v[0], v[1], v[2]};
-}
-__device__ __forceinline__ void spl_load(const float4 *spl, int j, F2 (&b)[3]) {
-    const float4 h = spl[2 * (size_t)j], l = spl[2 * (size_t)j + 1];
-    b[0] = F2{h.x, l.x}; b[1] = F2{h.y, l.y}; b[2] = F2{h.z, l.z};
 }
 
 // ---- the block ----------------------------------------------------------------------
@@ -847,9 +816,8 @@ __device__ __forceinline__ bool force_block(const Dev &d, const TermP &p, int cu
                     h = V3<float>{-narrow_f(s.g[GU][s2]), -narrow_f(s.g[GU + 1][s2]), -narrow_f(s.g[GU + 2][s2])};
                 }
             }
-            float *nh = d.qa.nh;
-            nh[i] = n.x; nh[Ns + i] = n.y; nh[2 * Ns + i] = n.z;
-            nh[3 * Ns + i] = h.x; nh[4 * Ns + i] = h.y; nh[5 * Ns + i] = h.z;
+            d.qa.nh[2 * (size_t)i] = make_float4(n.x, n.y, n.z, 0.0f);
+            d.qa.nh[2 * (size_t)i + 1] = make_float4(h.x, h.y, h.z, 0.0f);
         }
         if (t < FB) s.state[t] = state;
     }
@@ -1070,18 +1038,20 @@ __device__ __forceinline__ bool force_block(const Dev &d, const TermP &p, int cu
                 // the replica has taken its steps, or the bead keeps its state
                 if (st == 2) d.rep[r].fault = 1;
                 d.pos[cur ^ 1][i] = d.pos[cur][i];
-                if constexpr (MIX) {
+                if (MIX || qa) {
                     d.spl[cur ^ 1][2 * (size_t)i] = d.spl[cur][2 * (size_t)i];
                     d.spl[cur ^ 1][2 * (size_t)i + 1] = d.spl[cur][2 * (size_t)i + 1];
                 }
             } else if (st == 1) {
                 const FT q = s.p[MIX ? 6 : 3][t + 3];
                 double4_32a pn = make_double4_32a(s.F[0][t], s.F[1][t], s.F[2][t], 0.0);
-                if constexpr (MIX) {
+                if (MIX || qa) {   // (the sift reads them too)
                     const P2 x = split_p(pn);
-                    pn.w = widen_f(q);
-                    d.spl[cur ^ 1][2 * (size_t)i] = make_float4(x.x.h, x.y.h, x.z.h, q);
+                    d.spl[cur ^ 1][2 * (size_t)i] = make_float4(x.x.h, x.y.h, x.z.h, MIX ? (float)q : narrow_f((double)q));
                     d.spl[cur ^ 1][2 * (size_t)i + 1] = make_float4(x.x.l, x.y.l, x.z.l, 0.0f);
+                }
+                if constexpr (MIX) {
+                    pn.w = widen_f(q);
                     disp = widen_f(__fadd_rn(__fadd_rn(s.e[0][t], s.e[1][t]), s.e[2][t]));
                 } else {
                     pn.w = q;
