@@ -868,6 +868,43 @@ __global__ void k_go_lists(Dev d, int b, int n) {
     d.go_cnt[i] = at - n0;
 }
 
+// One bead's partners put in ascending order by the warp that collected them:
+// a bitonic sort of 32 U register entries (distinct beads, padded with the
+// largest int).  Ranking every entry against every other took two thirds of
+// k_nl_cells' instructions (3470 a bead at about 60 partners).
+template <int U> __device__ __noinline__ void sort_row(int32_t *row, int m, int lane) {
+    static_assert(32 * U <= QA_TMP_CAP, "a row holds the padded entries' slots");
+    int v[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) v[u] = u * 32 + lane < m ? row[u * 32 + lane] : INT_MAX;
+#pragma unroll
+    for (int k = 2; k <= 32 * U; k <<= 1)
+#pragma unroll
+        for (int j = k >> 1; j; j >>= 1) {
+            if (j >= 32) {
+#pragma unroll
+                for (int u = 0; u < U; ++u) {
+                    const int w = u ^ (j >> 5);
+                    if (w < u) continue;
+                    const int lo = min(v[u], v[w]), hi = max(v[u], v[w]);
+                    const bool up = ((u * 32) & k) == 0;
+                    v[u] = up ? lo : hi;
+                    v[w] = up ? hi : lo;
+                }
+            } else {
+#pragma unroll
+                for (int u = 0; u < U; ++u) {
+                    const int o = __shfl_xor_sync(0xffffffffu, v[u], j);
+                    const bool up = ((u * 32 + lane) & k) == 0;
+                    v[u] = up == ((lane & j) == 0) ? min(v[u], o) : max(v[u], o);
+                }
+            }
+        }
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+        if (u * 32 + lane < m) row[u * 32 + lane] = v[u];
+}
+
 constexpr int NC_WARPS = 8;
 __global__ void __launch_bounds__(NC_WARPS * 32, 4) k_nl_cells(Dev d, TermP p, int cur) {
     const int lane = threadIdx.x & 31;
@@ -933,7 +970,12 @@ __global__ void __launch_bounds__(NC_WARPS * 32, 4) k_nl_cells(Dev d, TermP p, i
     }
     const int cap = d.nl_cap;
     int cnt = 0, tcnt = 0;
+    // candidates within reach (one in six of those in the buckets), in order;
+    // the tests behind the distance run on 32 of them at a time
+    __shared__ int2 s_queue[NC_WARPS][64];
+    int2 *queue = s_queue[threadIdx.x >> 5];
     for (int g = 0; g < 2; ++g) {
+        int qn = 0;
         if (g == CG_NEAR ? rp.s_near <= 0.0 : !(es_on && rp.far)) continue;
         // neighbouring buckets: lane l < 27 takes offsets (l % 3, l / 3 % 3, l / 9) - 1,
         // the first lane of each bucket its range of slots
@@ -992,21 +1034,35 @@ __global__ void __launch_bounds__(NC_WARPS * 32, 4) k_nl_cells(Dev d, TermP p, i
                 if (pm <= c) lo += step;
             }
             const int q = __shfl_sync(FULL, q0, lo) + c;
-            int flags = 0;
-            bool qa_free = false;
-            int j = -1;
+            bool in = false;
+            int jw = 0;
+            float dj = 0.0f;
             if (c < total) {
                 const float4 f = d.cell_pos[q];
-                j = __float_as_int(f.w) & ~CELL_CHARGED;
-                const bool es_pair = es_on && __float_as_int(f.w) < 0;
+                jw = __float_as_int(f.w);
                 float ddx = f.x - me.x, ddy = f.y - me.y, ddz = f.z - me.z;
                 if (periodic) {
                     ddx = min_image_f(ddx, Lx);
                     ddy = min_image_f(ddy, Ly);
                     ddz = min_image_f(ddz, Lz);
                 }
-                const float d2 = ddx * ddx + ddy * ddy + ddz * ddz;
-                if (j != i && d2 <= reach) {
+                dj = ddx * ddx + ddy * ddy + ddz * ddz;
+                in = (jw & ~CELL_CHARGED) != i && dj <= reach;
+            }
+            const unsigned im = __ballot_sync(FULL, in);
+            if (in) queue[qn + __popc(im & lt)] = make_int2(jw, __float_as_int(dj));
+            qn += __popc(im);
+            const bool last = base + 32 >= total;
+            while (qn >= 32 || (last && qn)) {
+                __syncwarp();
+                int flags = 0;
+                bool qa_free = false;
+                int j = -1;
+                if (lane < qn) {
+                    const int2 e = queue[lane];
+                    j = e.x & ~CELL_CHARGED;
+                    const bool es_pair = es_on && e.x < 0;
+                    const float d2 = __int_as_float(e.y);
                     const int cj = d.chain[j], sj = d.seq[j];
                     const int df = si > sj ? si - sj : sj - si;
                     if (!(ci == cj && df < 3)) {
@@ -1038,77 +1094,63 @@ __global__ void __launch_bounds__(NC_WARPS * 32, 4) k_nl_cells(Dev d, TermP p, i
                         }
                     }
                 }
-            }
-            // a native contact leaves every list (natives leave only with
-            // native contacts enabled, main.cpp:504-530); a pair in contact
-            // is no free pair.  The bead's natives and contact partners are
-            // held one per lane and broadcast.
-            if (go_on && __any_sync(FULL, flags != 0 || qa_free)) {
-                if (nnat <= 32) {
-                    for (int k = 0; k < nnat; ++k)
-                        if (__shfl_sync(FULL, my_nat, k) == j) { flags = 0; qa_free = false; }
-                } else {
-                    for (int k = n0; k < n1; ++k)
-                        if (d.nat_j[k] == j) { flags = 0; qa_free = false; }
+                // a native contact leaves every list (natives leave only with
+                // native contacts enabled, main.cpp:504-530); a pair in contact
+                // is no free pair.  The bead's natives and contact partners are
+                // held one per lane and broadcast.
+                if (go_on && __any_sync(FULL, flags != 0 || qa_free)) {
+                    if (nnat <= 32) {
+                        for (int k = 0; k < nnat; ++k)
+                            if (__shfl_sync(FULL, my_nat, k) == j) { flags = 0; qa_free = false; }
+                    } else {
+                        for (int k = n0; k < n1; ++k)
+                            if (d.nat_j[k] == j) { flags = 0; qa_free = false; }
+                    }
                 }
-            }
-            if (qa_on && __any_sync(FULL, qa_free))
-                for (int k = 0; k < nref; ++k)
-                    if (__shfl_sync(FULL, my_qa, k) == j) qa_free = false;
-            // a native disulfide is in no non-native list (main.cpp:579-580)
-            if (nss && __any_sync(FULL, flags != 0 || qa_free)) {
-                if (nss <= 32) {
-                    for (int k = 0; k < nss; ++k)
-                        if (__shfl_sync(FULL, my_ss, k) == j) { flags = 0; qa_free = false; }
-                } else {
-                    for (int k = ss0; k < ss1; ++k)
-                        if (d.ss_j[k] == j) { flags = 0; qa_free = false; }
+                if (qa_on && __any_sync(FULL, qa_free))
+                    for (int k = 0; k < nref; ++k)
+                        if (__shfl_sync(FULL, my_qa, k) == j) qa_free = false;
+                // a native disulfide is in no non-native list (main.cpp:579-580)
+                if (nss && __any_sync(FULL, flags != 0 || qa_free)) {
+                    if (nss <= 32) {
+                        for (int k = 0; k < nss; ++k)
+                            if (__shfl_sync(FULL, my_ss, k) == j) { flags = 0; qa_free = false; }
+                    } else {
+                        for (int k = ss0; k < ss1; ++k)
+                            if (d.ss_j[k] == j) { flags = 0; qa_free = false; }
+                    }
                 }
-            }
-            const unsigned km = __ballot_sync(FULL, flags != 0);
-            if (flags) {
-                const int at = cnt + __popc(km & lt);
-                if (at < cap) d.nl_row[(size_t)at * d.N + i] = j | flags;
-            }
-            cnt += __popc(km);
-            if (qa_on) {
-                const unsigned qm = __ballot_sync(FULL, qa_free);
-                if (qa_free) {
-                    const int at = tcnt + __popc(qm & lt);
-                    if (at < QA_TMP_CAP) d.qa.tmp[(size_t)at * d.N + i] = j;
+                const unsigned km = __ballot_sync(FULL, flags != 0);
+                if (flags) {
+                    const int at = cnt + __popc(km & lt);
+                    if (at < cap) d.nl_row[(size_t)at * d.N + i] = j | flags;
                 }
-                tcnt += __popc(qm);
+                cnt += __popc(km);
+                if (qa_on) {
+                    const unsigned qm = __ballot_sync(FULL, qa_free);
+                    if (qa_free) {
+                        const int at = tcnt + __popc(qm & lt);
+                        if (at < QA_TMP_CAP) d.qa.tmp[(size_t)i * QA_TMP_CAP + at] = j;
+                    }
+                    tcnt += __popc(qm);
+                }
+                // what is left (fewer than 32) moves to the front
+                const int2 left = queue[32 + lane];
+                __syncwarp();
+                queue[lane] = left;
+                __syncwarp();
+                qn = max(qn - 32, 0);
             }
         }
     }
     if (qa_on && tcnt > 1) {
-        // order the partners by j: each entry's rank is the number of smaller
-        // ones (partners are distinct beads)
         const int m = min(tcnt, QA_TMP_CAP);
+        int32_t *row = d.qa.tmp + (size_t)i * QA_TMP_CAP;
         __syncwarp();
-        int vals[QA_TMP_CAP / 32];
-#pragma unroll
-        for (int u = 0; u < QA_TMP_CAP / 32; ++u) {
-            const int k = u * 32 + lane;
-            vals[u] = k < m ? d.qa.tmp[(size_t)k * d.N + i] : 0x7fffffff;
-        }
-        int rank[QA_TMP_CAP / 32];
-#pragma unroll
-        for (int u = 0; u < QA_TMP_CAP / 32; ++u) rank[u] = 0;
-        for (int k = 0; k < m; ++k) {
-            int v = 0;
-#pragma unroll
-            for (int u = 0; u < QA_TMP_CAP / 32; ++u)
-                if (k / 32 == u) v = __shfl_sync(FULL, vals[u], k & 31);
-#pragma unroll
-            for (int u = 0; u < QA_TMP_CAP / 32; ++u) rank[u] += v < vals[u];
-        }
-        __syncwarp();
-#pragma unroll
-        for (int u = 0; u < QA_TMP_CAP / 32; ++u) {
-            const int k = u * 32 + lane;
-            if (k < m) d.qa.tmp[(size_t)rank[u] * d.N + i] = vals[u];
-        }
+        if (m <= 32) sort_row<1>(row, m, lane);
+        else if (m <= 64) sort_row<2>(row, m, lane);
+        else if (m <= 128) sort_row<4>(row, m, lane);
+        else sort_row<8>(row, m, lane);
     }
     if (lane == 0) {
         atomicMax(&d.ctr[1], (unsigned long long)cnt);   // longest row needed
@@ -1394,7 +1436,7 @@ __device__ __forceinline__ void tl_chunk(const Dev &d, const TermP &p, int cur, 
                 const unsigned qm = __ballot_sync(0xffffffffu, qa_free);
                 if (qa_free) {
                     const int at = tcnt + __popc(qm & lt);
-                    if (at < QA_TMP_CAP) d.qa.tmp[(size_t)at * d.N + i] = b + lj;
+                    if (at < QA_TMP_CAP) d.qa.tmp[(size_t)i * QA_TMP_CAP + at] = b + lj;
                 }
                 tcnt += __popc(qm);
             }
@@ -2357,7 +2399,6 @@ void Engine::allocate() {
         q.bchunk = (int2 *)dalloc(sizeof(int2) * q.nbchunk);
         CK(cudaMemsetAsync(q.bchunk, 0, sizeof(int2) * q.nbchunk, stream));
         q.bcsum = (int32_t *)dalloc(sizeof(int32_t) * q.nbchunk);
-        q.bcbase = (int32_t *)dalloc(sizeof(int32_t) * q.nbchunk);
         qa_bchunk_next = 0;
         const int fp_total = std::max(1, cap.fp), ct_total = std::max(1, cap.ct);
         q.fp_total = fp_total;
@@ -3011,8 +3052,7 @@ void Engine::launch_rebuild() {
     if (any_tile) k_nl_tile<<<tile_grid, TL_THREADS, tile_smem, stream>>>(d, tp, cur, 1);
     if (d.qa_on) {
         k_qa_fp_scan<<<d.qa.nbchunk, QA_BCHUNK, 0, stream>>>(d);
-        k_qa_fp_base<<<d.R, 1024, 0, stream>>>(d);
-        k_qa_fp_fill<<<d.qa.nbchunk, QA_BCHUNK, 0, stream>>>(d);
+        k_qa_fp_fill<<<dim3(d.qa.nbchunk, QA_FG), 256, 0, stream>>>(d);
         k_qa_compact<<<d.R, 1024, 0, stream>>>(d);
     }
     if (timing) record(ev_rebuild, n_ev_rebuild);
@@ -3333,20 +3373,15 @@ void Engine::add_rebuild_nodes(cudaGraph_t body, int cn) {
         add(kt);
     }
     if (d.qa_on) {
-        cudaKernelNodeParams k3{}, k4{}, k5{}, k6{};
+        cudaKernelNodeParams k3{}, k5{}, k6{};
         k3.func = (void *)k_qa_fp_scan;
         k3.gridDim = dim3(d.qa.nbchunk);
         k3.blockDim = dim3(QA_BCHUNK);
         k3.kernelParams = a3;
         add(k3);
-        k4.func = (void *)k_qa_fp_base;
-        k4.gridDim = dim3(d.R);
-        k4.blockDim = dim3(1024);
-        k4.kernelParams = a3;
-        add(k4);
         k5.func = (void *)k_qa_fp_fill;
-        k5.gridDim = dim3(d.qa.nbchunk);
-        k5.blockDim = dim3(QA_BCHUNK);
+        k5.gridDim = dim3(d.qa.nbchunk, QA_FG);
+        k5.blockDim = dim3(256);
         k5.kernelParams = a3;
         add(k5);
         k6.func = (void *)k_qa_compact;

@@ -96,6 +96,7 @@ constexpr int QA_TMP_CAP = 256;  // free-pair partners j > i per bead at a rebui
 constexpr int QA_FP_PER_BEAD = 96;   // free-pair slots per bead of a replica (+256)
 constexpr int QA_CT_PER_BEAD = 8;    // contact slots per bead of a replica (+256)
 constexpr int QA_SIFT = 256;         // free-pair slots per block of the candidate sift
+constexpr int QA_FG = 16;        // blocks that list one chunk's partners
 constexpr int QA_BCHUNK = 1024;      // beads per chunk of the free-pair re-listing
 
 // device record of the quasi-adiabatic state
@@ -103,10 +104,10 @@ struct QaDev {
     float4 *nh;                  // [N][2]: n, h (precompute_nh.cpp:12-20) to FP32 accuracy
     int32_t *sync;               // [N] packed int8 x4: back | side_all | side_polar | side_hydrophobic
     int32_t *ref_cnt, *ref;      // [N], [QA_REF_CAP][N] contact slots per bead
-    int32_t *tmp_cnt, *tmp;      // [N], [QA_TMP_CAP][N] partners collected at a rebuild
+    int32_t *tmp_cnt, *tmp;      // [N], [N][QA_TMP_CAP] partners collected at a rebuild
     int32_t *tmp_off;            // [N] offset of a bead's partners within its chunk
     int2 *bchunk;                // (replica, first bead) of each chunk of QA_BCHUNK beads
-    int32_t *bcsum, *bcbase;     // per chunk: partners, first free-pair slot
+    int32_t *bcsum;              // partners per chunk
     int nbchunk;
     int32_t *fp_i1, *fp_i2, *fp_rep;   // free-pair slots
     uint8_t *fp_vac;

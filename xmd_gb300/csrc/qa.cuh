@@ -576,46 +576,41 @@ __global__ void __launch_bounds__(QA_BCHUNK) k_qa_fp_scan(Dev d) {
     if (i < end) q.tmp_off[i] = pos;
     if (threadIdx.x == 0) q.bcsum[blockIdx.x] = total;
 }
-__global__ void __launch_bounds__(1024) k_qa_fp_base(Dev d) {
-    const int r = blockIdx.x, t = threadIdx.x;
-    RepDev &rp = d.rep[r];
-    if (!rp.active || !rp.rebuild) return;
+// QA_FG blocks per chunk, a warp per bead: a bead's row and its slots are both
+// contiguous (one thread per bead wrote single words: 33 us for 30720 beads'
+// list, a block's 1024 threads each walking a row).  A block sums the earlier
+// chunks of its replica itself.
+__global__ void __launch_bounds__(256) k_qa_fp_fill(Dev d) {
     const QaDev &q = d.qa;
-    __shared__ int s_warp[33];
-    __shared__ int s_run;
-    if (t == 0) s_run = 0;
+    const int c = blockIdx.x, t = threadIdx.x, lane = t & 31, w = t >> 5;
+    const int2 ch = q.bchunk[c];
+    RepDev &rp = d.rep[ch.x];
+    if (!rp.active || !rp.rebuild) return;
+    __shared__ int s_sum[8];
+    const int off = rp.qa_bchunk_off, cap = rp.fp_cap;
+    int sum = 0;
+    for (int k = off + t; k < c; k += 256) sum += q.bcsum[k];
+    sum = __reduce_add_sync(0xffffffffu, sum);
+    if (lane == 0) s_sum[w] = sum;
     __syncthreads();
-    const int off = rp.qa_bchunk_off, nb = rp.qa_nbchunk;
-    for (int base = 0; base < nb; base += 1024) {
-        const int c = base + t;
-        const int v = c < nb ? q.bcsum[off + c] : 0;
-        int pos;
-        const int total = block_exscan(v, &pos, s_warp);
-        if (c < nb) q.bcbase[off + c] = s_run + pos;
-        __syncthreads();
-        if (t == 0) s_run += total;
-        __syncthreads();
+    int base = 0;
+#pragma unroll
+    for (int k = 0; k < 8; ++k) base += s_sum[k];
+    if (t == 0 && blockIdx.y == 0 && c - off == rp.qa_nbchunk - 1) {
+        const int all = base + q.bcsum[c];
+        if (all > cap) atomicOr(d.status, 4);
+        rp.fp_n = min(all, cap);
     }
-    if (t == 0) {
-        if (s_run > rp.fp_cap) atomicOr(d.status, 4);
-        rp.fp_n = min(s_run, rp.fp_cap);
-    }
-}
-__global__ void __launch_bounds__(QA_BCHUNK) k_qa_fp_fill(Dev d) {
-    const QaDev &q = d.qa;
-    const int2 ch = q.bchunk[blockIdx.x];
-    const RepDev &rp = d.rep[ch.x];
-    if (!rp.active || !rp.rebuild) return;
-    const int i = ch.y + threadIdx.x;
-    if (i >= rp.begin + rp.n) return;
-    const int cnt = min(q.tmp_cnt[i], QA_TMP_CAP);
-    const int o0 = q.bcbase[blockIdx.x] + q.tmp_off[i];
-    for (int k = 0; k < cnt; ++k) {
-        const int o = o0 + k;
-        if (o < rp.fp_cap) {
-            q.fp_i1[rp.fp_off + o] = i;
-            q.fp_i2[rp.fp_off + o] = q.tmp[(size_t)k * d.N + i];
-            q.fp_vac[rp.fp_off + o] = 0;
+    constexpr int PER = QA_BCHUNK / QA_FG;
+    const int b0 = ch.y + blockIdx.y * PER, b1 = min(b0 + PER, rp.begin + rp.n);
+    for (int i = b0 + w; i < b1; i += 8) {
+        const int cnt = min(q.tmp_cnt[i], QA_TMP_CAP);
+        const int o0 = base + q.tmp_off[i];
+        for (int k = lane; k < cnt && o0 + k < cap; k += 32) {
+            const size_t o = (size_t)rp.fp_off + o0 + k;
+            q.fp_i1[o] = i;
+            q.fp_i2[o] = q.tmp[(size_t)i * QA_TMP_CAP + k];
+            q.fp_vac[o] = 0;
         }
     }
 }
