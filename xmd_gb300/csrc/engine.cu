@@ -1560,7 +1560,68 @@ Engine::Engine(const xmd_params &p) : params(p) {
     CK(cudaStreamCreateWithFlags(&ustream, cudaStreamNonBlocking));
     CK(cudaEventCreateWithFlags(&ev_staged, cudaEventDisableTiming));
     CK(cudaEventCreateWithFlags(&ev_removed, cudaEventDisableTiming));
-    CK(cudaMallocHost(&h_any, sizeof(int) * 4));
+    CK(cudaMallocHost(&h_any, sizeof(int) * 16 + sizeof(double) * XMD_NUM_TERMS));
+    for (auto &e : down_ev) CK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+    ring.s = stream;
+    uring.s = ustream;
+}
+
+char *Engine::HostRing::take(size_t bytes) {
+    bytes = (bytes + 15) & ~(size_t)15;
+    if (bytes > HALF) throw std::logic_error("engine: copy larger than its staging memory");
+    if (!h) {
+        CK(cudaMallocHost(&h, 2 * HALF));
+        for (auto &e : ev) CK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+    }
+    if (off + bytes > HALF) {
+        CK(cudaEventRecord(ev[cur], s));
+        cur ^= 1;
+        CK(cudaEventSynchronize(ev[cur]));
+        off = 0;
+    }
+    char *p = h + cur * HALF + off;
+    off += bytes;
+    return p;
+}
+
+void Engine::HostRing::up(void *dst, const void *src, size_t bytes) {
+    for (size_t o = 0; o < bytes; o += HALF) {
+        const size_t m = std::min(HALF, bytes - o);
+        char *p = take(m);
+        std::memcpy(p, (const char *)src + o, m);
+        CK(cudaMemcpyAsync((char *)dst + o, p, m, cudaMemcpyHostToDevice, s));
+    }
+}
+
+Engine::HostRing::~HostRing() {
+    if (h) cudaFreeHost(h);
+    for (auto &e : ev)
+        if (e) cudaEventDestroy(e);
+}
+
+void Engine::fetch_words() {
+    CK(cudaMemcpyAsync(h_any, d.any_rebuild, sizeof(int) * 16, cudaMemcpyDeviceToHost, stream));
+    CK(cudaStreamSynchronize(stream));
+}
+
+void Engine::down(void *dst, const void *src, size_t bytes) {
+    constexpr size_t PIECE = HostRing::HALF / 2 + 16;   // two pieces never share a half
+    char *p[2] = {nullptr, nullptr};
+    size_t len[2] = {0, 0}, at = 0;
+    for (size_t o = 0, k = 0; o < bytes + PIECE; o += PIECE, ++k) {
+        if (o < bytes) {
+            len[k & 1] = std::min(PIECE, bytes - o);
+            p[k & 1] = ring.take(len[k & 1]);
+            CK(cudaMemcpyAsync(p[k & 1], (const char *)src + o, len[k & 1], cudaMemcpyDeviceToHost, stream));
+            CK(cudaEventRecord(down_ev[k & 1], stream));
+        }
+        if (k && at < bytes) {
+            const int q = (k - 1) & 1;
+            CK(cudaEventSynchronize(down_ev[q]));
+            std::memcpy((char *)dst + at, p[q], len[q]);
+            at += len[q];
+        }
+    }
 }
 
 Engine::~Engine() {
@@ -1573,6 +1634,8 @@ Engine::~Engine() {
     for (auto e : ev_rebuild) cudaEventDestroy(e);
     release();
     if (h_any) cudaFreeHost(h_any);
+    for (auto e : down_ev)
+        if (e) cudaEventDestroy(e);
     if (ev_staged) cudaEventDestroy(ev_staged);
     if (ev_removed) cudaEventDestroy(ev_removed);
     if (ustream) cudaStreamDestroy(ustream);
@@ -1735,9 +1798,8 @@ void Engine::activate_staged() {
     CK(cudaStreamWaitEvent(stream, ev_staged, 0));
     for (Staged &st : staged_reps) {
         RepHost &r = reps[st.k];
-        CK(cudaMemcpyAsync(d.rep_of + r.begin, st.rep_of.data(), sizeof(int32_t) * r.n, cudaMemcpyHostToDevice,
-                           stream));
-        CK(cudaMemcpyAsync(d.rep + st.k, &st.rd, sizeof(RepDev), cudaMemcpyHostToDevice, stream));
+        ring.up(d.rep_of + r.begin, st.rep_of.data(), sizeof(int32_t) * r.n);
+        ring.up(d.rep + st.k, &st.rd, sizeof(RepDev));
         for (int i = 0; i < r.n; ++i) owner_h[r.begin + i] = st.k;
         r.staged = false;
         r.placed = true;
@@ -2264,10 +2326,29 @@ void Engine::allocate() {
     d.rng = (uint64_t *)dalloc(sizeof(uint64_t) * N);
     d.jump = (uint64_t *)dalloc(sizeof(uint64_t) * JUMP_WORDS * R);
     d.rep = (RepDev *)dalloc(sizeof(RepDev) * R);
-    d.any_rebuild = (int *)dalloc(sizeof(int) * 4);
+    d.any_rebuild = (int *)dalloc(sizeof(int) * 16);   // one block: the host reads it with one copy
     d.gate = d.any_rebuild + 1;
-    d.status = (int *)dalloc(sizeof(int) * 4);
-    d.ctr = (unsigned long long *)dalloc(sizeof(unsigned long long) * 4);
+    d.status = d.any_rebuild + 4;
+    d.ctr = (unsigned long long *)(d.any_rebuild + 8);
+    // jumps of the generator by 4 2^l draws (bead i starts 4 i draws after the
+    // seed), as nibble tables: entry [q][v] = XOR of the columns 4q + b for
+    // the bits b of v
+    rng_levels = 1;
+    while (N >> rng_levels) ++rng_levels;
+    rng_pow = (uint64_t *)dalloc(sizeof(uint64_t) * JUMP_WORDS * rng_levels);
+    std::vector<uint64_t> jt((size_t)JUMP_WORDS * rng_levels);
+    GF2 jm = gf2_jump(4);
+    for (int l = 0; l < rng_levels; ++l) {
+        for (int q = 0; q < 16; ++q)
+            for (int v = 0; v < 16; ++v) {
+                uint64_t e = 0;
+                for (int bb = 0; bb < 4; ++bb)
+                    if ((v >> bb) & 1) e ^= jm[4 * q + bb];
+                jt[(size_t)JUMP_WORDS * l + 16 * q + v] = e;
+            }
+        jm = gf2_mul(jm, jm);
+    }
+    ring.up(rng_pow, jt.data(), sizeof(uint64_t) * jt.size());
     d.nchunks = std::max(1, cap.chunks);
     d.chunks = (int2 *)dalloc(sizeof(int2) * d.nchunks);
     d.work = (int *)dalloc(sizeof(int) * d.nchunks);
@@ -2483,6 +2564,15 @@ void Engine::place_pending() {
         }
 }
 
+// the jump table of replica slot k: 4 n draws, the bits of n applied in turn
+__global__ void k_jump(Dev d, int k, const uint64_t *__restrict__ pw, unsigned n) {
+    const int t = threadIdx.x;
+    uint64_t x = (uint64_t)(t & 15) << (4 * (t >> 4));
+    for (int l = 0; n >> l; ++l)
+        if ((n >> l) & 1u) x = gf2_apply_nib(pw + (size_t)JUMP_WORDS * l, x);
+    d.jump[(size_t)JUMP_WORDS * k + t] = x;
+}
+
 // static data, lists and state of replica slot k onto the device.  With st
 // (staged placement) every upload goes on the side stream, after the last
 // removal's clears, and the activation data (bead owners, the
@@ -2490,6 +2580,7 @@ void Engine::place_pending() {
 void Engine::place(int k, Staged *st) {
     const xmd_params &p = params;
     cudaStream_t us = st ? ustream : stream;
+    HostRing &ring_ = st ? uring : ring;
     if (st) CK(cudaStreamWaitEvent(ustream, ev_removed, 0));
     RepHost &r = reps[k];
     const int n = r.n;
@@ -2564,11 +2655,8 @@ void Engine::place(int k, Staged *st) {
         for (auto &e : nat[i]) { nj.push_back(e.first); nd.push_back(e.second); }
         ne[i] = no + (int)nj.size();
     }
-    // (pageable sources: each copy returns once the driver has taken the
-    // data, so the host vectors may go out of scope)
-    auto up = [&](void *dst, const void *src, size_t bytes_) {
-        if (bytes_) CK(cudaMemcpyAsync(dst, src, bytes_, cudaMemcpyHostToDevice, us));
-    };
+    // (the ring has taken the data when a call returns)
+    auto up = [&](void *dst, const void *src, size_t bytes_) { ring_.up(dst, src, bytes_); };
     if (st) st->rep_of = rep_of;
     else up(d.rep_of + b, rep_of.data(), sizeof(int32_t) * n);
     up(d.chain + b, chain.data(), sizeof(int32_t) * n);
@@ -2686,21 +2774,11 @@ void Engine::place(int k, Staged *st) {
         CK(cudaMemsetAsync(d.qa.ref_cnt + b, 0, sizeof(int32_t) * n, us));
     }
     if (!st) up(d.rep + k, &rd, sizeof(RepDev));
-    GF2 j = gf2_jump(4ull * (uint64_t)n);
-    std::vector<uint64_t> jt(JUMP_WORDS);
-    // nibble tables: entry [q][v] = XOR of the columns 4q+b for the bits b of v
-    for (int q = 0; q < 16; ++q)
-        for (int v = 0; v < 16; ++v) {
-            uint64_t e = 0;
-            for (int bb = 0; bb < 4; ++bb)
-                if ((v >> bb) & 1) e ^= j[4 * q + bb];
-            jt[16 * q + v] = e;
-        }
-    up(d.jump + (size_t)JUMP_WORDS * k, jt.data(), sizeof(uint64_t) * JUMP_WORDS);
+    k_jump<<<1, JUMP_WORDS, 0, us>>>(d, k, rng_pow, (unsigned)n);
     if (st) {
         // the state (upload_state's data) on the side stream too; the record
         // starts as upload_state leaves it: t = 0, first list build pending
-        upload_state_data(k, us);
+        upload_state_data(k, ring_, false);
         rd.t = 0.0;
         rd.first = 1;
         rd.maxdisp = 0;
@@ -2710,53 +2788,101 @@ void Engine::place(int k, Staged *st) {
         r.staged = true;
         return;
     }
-    CK(cudaStreamSynchronize(stream));
     for (int i = 0; i < n; ++i) owner_h[b + i] = k;
     r.placed = true;
     if (r.cell_len) count_cell(1);
     upload_state(k);
 }
 
-// positions, history (y1 = v dt, y2..y5 = 0) and generator states of a
-// replica, uploaded on stream us
-void Engine::upload_state_data(int k, cudaStream_t us) {
-    RepHost &r = reps[k];
-    int n = r.n, b = r.begin;
-    std::vector<double4_32a> pos(n);
-    for (int i = 0; i < n; ++i) {
-        double q = params.charge[r.atype[i]];
-        pos[i] = make_double4_32a(r.r[3 * i], r.r[3 * i + 1], r.r[3 * i + 2], q);
+// A replica's state from the host: positions, history (y1 = v dt, y2..y5 = 0)
+// and generator states of beads i0 .. i0 + m of replica slot k, read from
+// pinned memory (r, then v), a block's rows in one sweep.  The generator of
+// bead i is the seed 4 i draws on, by the bits of i (the host's chain over the
+// beads and 18 pageable copies took 0.96 ms for 54744 beads).  With `record`
+// the slot starts over: t = 0, first list build pending; a new state thaws a
+// frozen replica.
+struct ChargeP { double q[XMD_NUM_AA]; };
+constexpr int ST_TB = 256, ST_PIECE = 16384;   // beads per block, per piece of staging memory
+__global__ void __launch_bounds__(ST_TB) k_set_state(Dev d, int cur, int k, int b, int i0, int m,
+                                                     const double *__restrict__ in, ChargeP c, double dt,
+                                                     uint64_t seed, const uint64_t *__restrict__ pw, int record,
+                                                     long long steps_left) {
+    __shared__ double s_in[6 * ST_TB];
+    const int t = threadIdx.x, base = blockIdx.x * ST_TB, cnt = min(ST_TB, m - base);
+    for (int q = t; q < 3 * cnt; q += ST_TB) {
+        s_in[q] = in[3 * (size_t)base + q];
+        s_in[3 * ST_TB + q] = in[3 * (size_t)(m + base) + q];
     }
-    CK(cudaMemcpyAsync(d.pos[cur] + b, pos.data(), sizeof(double4_32a) * n, cudaMemcpyHostToDevice, us));
-    std::vector<double> col(n);
-    for (int k2 = 0; k2 < 15; ++k2) {
-        for (int i = 0; i < n; ++i) col[i] = k2 < 3 ? r.v[3 * i + k2] * params.dt : 0.0;
-        CK(cudaMemcpyAsync(d.yh + (size_t)k2 * d.N + b, col.data(), sizeof(double) * n,
-                           cudaMemcpyHostToDevice, us));
+    __syncthreads();
+    if (t < cnt) {
+        const int i = i0 + base + t;
+        const size_t g = (size_t)b + i, N = d.N;
+        const double *x = s_in + 3 * t, *v = x + 3 * ST_TB;
+        d.pos[cur][g] = make_double4_32a(x[0], x[1], x[2], c.q[d.atype[g]]);
+        for (int a = 0; a < 15; ++a) d.yh[a * N + g] = a < 3 ? __dmul_rn(v[a], dt) : 0.0;
+        uint64_t s = seed;
+        for (int l = 0; i >> l; ++l)
+            if ((i >> l) & 1) s = gf2_apply_nib(pw + (size_t)JUMP_WORDS * l, s);
+        d.rng[g] = s;
     }
-    std::vector<uint64_t> st(n);
-    uint64_t s = r.seed;
-    for (int i = 0; i < n; ++i) {
-        st[i] = s;
-        for (int q = 0; q < 4; ++q) s = xs_step(s);
+    if (record && blockIdx.x == 0 && t == 0) {
+        RepDev &rp = d.rep[k];
+        rp.t = 0.0;
+        rp.first = 1;
+        rp.maxdisp = 0;
+        if (rp.fault) {
+            rp.fault = 0;
+            rp.steps_left = steps_left;
+        }
     }
-    CK(cudaMemcpyAsync(d.rng + b, st.data(), sizeof(uint64_t) * n, cudaMemcpyHostToDevice, us));
+}
+// positions, velocities (y1 / dt) and time the other way
+__global__ void __launch_bounds__(ST_TB) k_get_state(Dev d, int cur, int k, int b, int i0, int m, double dt_inv,
+                                                     double *__restrict__ out, double *__restrict__ t_out) {
+    __shared__ double s_out[6 * ST_TB];
+    const int t = threadIdx.x, base = blockIdx.x * ST_TB, cnt = min(ST_TB, m - base);
+    if (t < cnt) {
+        const size_t g = (size_t)b + i0 + base + t, N = d.N;
+        const double4_32a p = d.pos[cur][g];
+        double *x = s_out + 3 * t, *v = x + 3 * ST_TB;
+        x[0] = p.x; x[1] = p.y; x[2] = p.z;
+        for (int a = 0; a < 3; ++a) v[a] = __dmul_rn(d.yh[a * N + g], dt_inv);
+    }
+    __syncthreads();
+    for (int q = t; q < 3 * cnt; q += ST_TB) {
+        out[3 * (size_t)base + q] = s_out[q];
+        out[3 * (size_t)(m + base) + q] = s_out[3 * ST_TB + q];
+    }
+    if (blockIdx.x == 0 && t == 0) *t_out = d.rep[k].t;
 }
 
-void Engine::upload_state(int k) {
-    upload_state_data(k, stream);
-    RepDev rd;
-    CK(cudaMemcpyAsync(&rd, d.rep + k, sizeof(RepDev), cudaMemcpyDeviceToHost, stream));
-    CK(cudaStreamSynchronize(stream));
-    rd.t = 0.0;
-    rd.first = 1;
-    rd.maxdisp = 0;
-    if (rd.fault) {   // a new state thaws a frozen replica
-        rd.fault = 0;
-        rd.steps_left = reps[k].steps_left;
+void Engine::upload_state_data(int k, HostRing &up, bool record) {
+    const RepHost &r = reps[k];
+    ChargeP c;
+    for (int a = 0; a < XMD_NUM_AA; ++a) c.q[a] = params.charge[a];
+    for (int i0 = 0; i0 < r.n; i0 += ST_PIECE) {
+        const int m = std::min(ST_PIECE, r.n - i0);
+        double *in = (double *)up.take(sizeof(double) * 6 * m);
+        std::memcpy(in, r.r.data() + 3 * (size_t)i0, sizeof(double) * 3 * m);
+        std::memcpy(in + 3 * (size_t)m, r.v.data() + 3 * (size_t)i0, sizeof(double) * 3 * m);
+        k_set_state<<<(m + ST_TB - 1) / ST_TB, ST_TB, 0, up.s>>>(d, cur, k, r.begin, i0, m, in, c, params.dt, r.seed,
+                                                                 rng_pow, record && i0 == 0, r.steps_left);
+        CK(cudaGetLastError());
     }
-    CK(cudaMemcpyAsync(d.rep + k, &rd, sizeof(RepDev), cudaMemcpyHostToDevice, stream));
-    CK(cudaStreamSynchronize(stream));
+}
+
+void Engine::upload_state(int k) { upload_state_data(k, ring, true); }
+
+// (no early way out: the test vectorises)
+static bool all_finite(const double *x, size_t n) {
+    const uint64_t EXP = 0x7ffull << 52;
+    uint64_t bad = 0;
+    for (size_t k = 0; k < n; ++k) {
+        uint64_t u;
+        std::memcpy(&u, x + k, 8);
+        bad |= (uint64_t)((u & EXP) == EXP);
+    }
+    return bad == 0;
 }
 
 void Engine::set_state(int rep, const double *r, const double *v) {
@@ -2766,7 +2892,7 @@ void Engine::set_state(int rep, const double *r, const double *v) {
     h.r.assign(r, r + 3 * (size_t)h.n);
     if (v) h.v.assign(v, v + 3 * (size_t)h.n);
     else h.v.assign(3 * (size_t)h.n, 0.0);
-    for (double x : h.r) if (!std::isfinite(x)) throw std::invalid_argument("non-finite position");
+    if (!all_finite(h.r.data(), h.r.size())) throw std::invalid_argument("non-finite position");
     h.have_state = true;
     if (h.placed) upload_state(rep);
 }
@@ -2813,24 +2939,31 @@ void Engine::get_state(int rep, double *r, double *v, double *t) {
     check_rep(reps, rep);
     ready();
     const RepHost &h = reps[rep];
-    int n = h.n, b = h.begin;
-    std::vector<double4_32a> pos(n);
-    CK(cudaMemcpyAsync(pos.data(), d.pos[cur] + b, sizeof(double4_32a) * n, cudaMemcpyDeviceToHost, stream));
-    std::vector<double> y1(3 * (size_t)n);
-    for (int a = 0; a < 3; ++a)
-        CK(cudaMemcpyAsync(y1.data() + (size_t)a * n, d.yh + (size_t)a * d.N + b, sizeof(double) * n,
-                           cudaMemcpyDeviceToHost, stream));
-    RepDev rd;
-    CK(cudaMemcpyAsync(&rd, d.rep + rep, sizeof(RepDev), cudaMemcpyDeviceToHost, stream));
-    CK(cudaStreamSynchronize(stream));
     const double dt_inv = 1.0 / params.dt;
-    for (int i = 0; i < n; ++i) {
-        if (r) { r[3 * i] = pos[i].x; r[3 * i + 1] = pos[i].y; r[3 * i + 2] = pos[i].z; }
-        if (v) for (int a = 0; a < 3; ++a) v[3 * i + a] = y1[(size_t)a * n + i] * dt_inv;
+    // pieces of staging memory (more than half a half each, so that a piece
+    // waits only for one already handed over), the last copied out while the
+    // next is filled
+    static_assert(2 * (48 * ST_PIECE + 8) > HostRing::HALF && 48 * ST_PIECE + 8 <= HostRing::HALF, "pieces");
+    double *p[2] = {nullptr, nullptr};
+    for (int i0 = 0, c = 0; i0 < h.n + ST_PIECE; i0 += ST_PIECE, ++c) {
+        if (i0 < h.n) {
+            const int m = std::min(ST_PIECE, h.n - i0);
+            p[c & 1] = (double *)ring.take(sizeof(double) * (6 * (size_t)m + 1));
+            k_get_state<<<(m + ST_TB - 1) / ST_TB, ST_TB, 0, stream>>>(d, cur, rep, h.begin, i0, m, dt_inv, p[c & 1],
+                                                                       p[c & 1] + 6 * (size_t)m);
+            CK(cudaGetLastError());
+            CK(cudaEventRecord(down_ev[c & 1], stream));
+        }
+        if (c && i0 - ST_PIECE < h.n) {
+            const int j0 = i0 - ST_PIECE, m = std::min(ST_PIECE, h.n - j0);
+            const double *q = p[(c - 1) & 1];
+            CK(cudaEventSynchronize(down_ev[(c - 1) & 1]));
+            if (r) std::memcpy(r + 3 * (size_t)j0, q, sizeof(double) * 3 * m);
+            if (v) std::memcpy(v + 3 * (size_t)j0, q + 3 * (size_t)m, sizeof(double) * 3 * m);
+            if (t) *t = q[6 * (size_t)m];
+        }
     }
-    if (t) *t = rd.t;
 }
-
 // ---- snapshots: the replica's whole mutable device state -----------------------
 // The reference's store (include/xmd/store/store.h; main.cpp's make_saved
 // items) keeps positions, the Gear history, time, the pair lists and the QA
@@ -3062,9 +3195,7 @@ void Engine::launch_rebuild() {
 // reaches `frac` of the capacity.  Returns true when the rows were
 // reallocated (lists must then be rebuilt; captured graphs are dropped).
 bool Engine::grow_rows(double frac) {
-    unsigned long long need = 0;
-    CK(cudaMemcpyAsync(&need, d.ctr + 1, sizeof(need), cudaMemcpyDeviceToHost, stream));
-    CK(cudaStreamSynchronize(stream));
+    const unsigned long long need = ((const unsigned long long *)(h_any + 8))[1];
     if ((double)need < frac * nl_cap) return false;
     resize_rows((int)(2 * need + 16));
     return true;
@@ -3183,12 +3314,12 @@ void Engine::ensure_nl() {
     for (int attempt = 0; attempt < 3; ++attempt) {
         k_nl_check<<<1, 1024, 0, stream>>>(d, 0, 0.0, (cudaGraphConditionalHandle)0, 0);
         ++launches;
-        CK(cudaMemcpyAsync(h_any, d.any_rebuild, sizeof(int), cudaMemcpyDeviceToHost, stream));
-        CK(cudaStreamSynchronize(stream));
-        if (*h_any) launch_rebuild();
-        int st = 0;
-        CK(cudaMemcpyAsync(&st, d.status, sizeof(int), cudaMemcpyDeviceToHost, stream));
-        CK(cudaStreamSynchronize(stream));
+        fetch_words();
+        if (h_any[0]) {
+            launch_rebuild();
+            fetch_words();
+        }
+        const int st = h_any[4];
         if (!(st & ST_CAPACITY) || !auto_grow) {
             if (auto_grow) grow_rows(0.6);   // keep headroom for the run ahead
             return;
@@ -3393,9 +3524,8 @@ void Engine::add_rebuild_nodes(cudaGraph_t body, int cn) {
 }
 
 void Engine::check_status(const char *where) {
-    int st = 0;
-    CK(cudaMemcpyAsync(&st, d.status, sizeof(int), cudaMemcpyDeviceToHost, stream));
-    CK(cudaStreamSynchronize(stream));
+    fetch_words();
+    const int st = h_any[4];
     CK(cudaGetLastError());
     if (st & ST_CAPACITY)
         throw std::length_error(std::string(where) + ": Verlet row capacity exceeded (raise `engine: nl capacity`)");
@@ -3423,10 +3553,11 @@ void Engine::eval_forces(int rep, double *F, double *V) {
         Ft.resize(3 * (size_t)h.n);
         Fh = Ft.data();
     }
-    CK(cudaMemcpyAsync(Fh, d.F + 3 * (size_t)h.begin, sizeof(double) * 3 * h.n, cudaMemcpyDeviceToHost, stream));
-    if (V) CK(cudaMemcpyAsync(V, d.Vrep + (size_t)rep * XMD_NUM_TERMS, sizeof(double) * XMD_NUM_TERMS,
+    double *Vh = (double *)(h_any + 16);
+    if (V) CK(cudaMemcpyAsync(Vh, d.Vrep + (size_t)rep * XMD_NUM_TERMS, sizeof(double) * XMD_NUM_TERMS,
                               cudaMemcpyDeviceToHost, stream));
-    CK(cudaStreamSynchronize(stream));
+    down(Fh, d.F + 3 * (size_t)h.begin, sizeof(double) * 3 * h.n);
+    if (V) std::memcpy(V, Vh, sizeof(double) * XMD_NUM_TERMS);
     // only this replica's forces decide: a replica frozen by a non-finite
     // force does not fail the evaluation of the others
     const bool iso = isolate_faults;
@@ -3438,8 +3569,7 @@ void Engine::eval_forces(int rep, double *F, double *V) {
         throw;
     }
     isolate_faults = iso;
-    for (size_t k = 0; k < 3 * (size_t)h.n; ++k)
-        if (!std::isfinite(Fh[k])) throw std::domain_error("eval_forces: non-finite force");
+    if (!all_finite(Fh, 3 * (size_t)h.n)) throw std::domain_error("eval_forces: non-finite force");
 }
 
 void Engine::step(int nsteps) {

@@ -373,7 +373,29 @@ private:
     cudaStream_t stream = nullptr;
     std::vector<void *> allocs;
     size_t alloc_bytes = 0;   // device memory held by this context
-    int *h_any = nullptr;        // pinned
+    // pinned: [0..3] any_rebuild and the gate, [4] status, [8..15] ctr as last
+    // fetched; the rest receives a replica's energies
+    int *h_any = nullptr;
+    // Host copies go through pinned memory (a pageable copy occupies the host
+    // for its whole length and synchronises): two halves taken in turn, a half
+    // reused once the copies issued from it are done.  One ring per stream.
+    struct HostRing {
+        static constexpr size_t HALF = 1 << 20;
+        char *h = nullptr;
+        cudaStream_t s = nullptr;
+        cudaEvent_t ev[2] = {nullptr, nullptr};
+        int cur = 0;
+        size_t off = 0;
+        char *take(size_t bytes);   // at most HALF, 16-byte aligned
+        void up(void *dst, const void *src, size_t bytes);
+        ~HostRing();
+    };
+    HostRing ring, uring;
+    cudaEvent_t down_ev[2] = {nullptr, nullptr};
+    void fetch_words();           // any_rebuild .. ctr into h_any (synchronises)
+    void down(void *dst, const void *src, size_t bytes);   // device to host (synchronises)
+    uint64_t *rng_pow = nullptr;  // [levels][256] nibble tables: 4 2^l draws
+    int rng_levels = 0;
     TermP tp{};
     int64_t launches = 0, md_steps = 0;
     double *staging = nullptr;   // packed host-layout buffer [18 N]
@@ -427,7 +449,7 @@ private:
     size_t tile_smem = 0;                      // dynamic shared memory of k_nl_tile
     int tile_grid = 1;                         // resident blocks of k_nl_tile over all SMs
     void add_rebuild_nodes(cudaGraph_t body, int cn);
-    bool grow_rows(double frac);
+    bool grow_rows(double frac);   // from the longest row last fetched
     void drop_graphs();
 
     struct Caps {
@@ -460,7 +482,7 @@ private:
     void launch_rebuild();
     void check_status(const char *where);
     void upload_state(int rep);
-    void upload_state_data(int rep, cudaStream_t us);
+    void upload_state_data(int rep, HostRing &up, bool record);
 };
 
 std::string &last_error();

@@ -104,7 +104,7 @@ class Engine:
 
     def eval_forces(self, rep: int = 0):
         n = self.sizes[rep]
-        F = np.zeros(3 * n)
+        F = np.empty(3 * n)
         V = np.zeros(abi.NUM_TERMS)
         check(self.lib.xmd_gpu_eval_forces(self.h, rep, dptr(F), dptr(V)))
         return F.reshape(n, 3), V
@@ -114,7 +114,7 @@ class Engine:
 
     def get_state(self, rep: int = 0):
         n = self.sizes[rep]
-        r, v, t = np.zeros(3 * n), np.zeros(3 * n), C.c_double()
+        r, v, t = np.empty(3 * n), np.empty(3 * n), C.c_double()
         check(self.lib.xmd_gpu_get_state(self.h, rep, dptr(r), dptr(v), C.byref(t)))
         return r.reshape(n, 3), v.reshape(n, 3), t.value
 

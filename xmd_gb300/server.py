@@ -93,7 +93,7 @@ class Server:
     def result(self, rid: int):
         """Wait for a request: final positions, velocities [n, 3], time, latency (s)."""
         n = self.sizes.pop(rid)
-        r, v = np.zeros(3 * n), np.zeros(3 * n)
+        r, v = np.empty(3 * n), np.empty(3 * n)
         t, lat = C.c_double(), C.c_double()
         check(self.lib.xmd_gpu_server_result(self.h, int(rid), dptr(r), dptr(v), C.byref(t), C.byref(lat)))
         return r.reshape(n, 3), v.reshape(n, 3), t.value, lat.value
