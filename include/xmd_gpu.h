@@ -411,7 +411,7 @@ int xmd_gpu_server_destroy(xmd_gpu_server *srv);
  * device synchronisation.  Every input and output is a device pointer the
  * caller owns; the function calls no cudaMalloc, cudaFree or allocating
  * library routine.  Its scratch is a file-scope __device__ array of about
- * 1.75 MiB that every GPU which loads the library holds until exit, sized for
+ * 10 MiB that every GPU which loads the library holds until exit, sized for
  * XMD_NOALLOC_MAX_BEADS beads; larger n is rejected with XMD_ERR_CAPACITY.
  *
  * Computes, on `stream` (a cudaStream_t; NULL = legacy default stream), the

@@ -48,6 +48,7 @@ CASES = [
     (1025, 20, (20, 0, 20), 3.1, 1.0, 20.0, None),
     (700, 8, (5, 8, 11), 4.9, 1.0, 0.0, None),        # one cell, one cell, two cells
     (700, 12, (7, 12, 0), 3.4, 1.0, -36.0, 5000),     # two, three, open; cap inside the list
+    (900, 10, (0, 0, 0), 3.2, 1.0, 0.0, 30003),       # rows around 32 and 64 partners, kept and not; cap inside
     (1500, 6, (0, 0, 0), 20.0, 1.0, 0.0, None),       # every pair: rows beyond shared memory
     (1500, 6, (9, 9, 9), 4.0, 1.0, 0.0, 300001),      # long rows, cap inside one
     (900, 20, (20, 20, 20), 3.1, 1e-3, 0.0, None),

@@ -9,7 +9,7 @@
 // xmd_gpu_verlet_pairs_noalloc() takes device buffers for all inputs and
 // outputs and keeps the scratch of its cell list (bucket counts, starts and
 // fills, bucket-sorted bead indices, per-bead row counts and offsets) in the
-// file-scope array below: about 1.75 MiB that every GPU which loads the
+// file-scope array below: about 10 MiB that every GPU which loads the
 // library holds until the process exits.
 //
 // The search itself is the one the engine runs at every Verlet rebuild:
@@ -25,13 +25,16 @@
 // rounds instead of one candidate after another.  A candidate is decided in
 // FP32 unless its distance lies in the FP32 error band around the cutoff,
 // where the FP64 test decides (GB300 runs an FP64 warp instruction over 16
-// cycles; FP64 throughout would make the search FP64-bound).  A row of up to
-// NA_ROW partners is put in order by rank in shared memory; a longer one by
-// insertion in global memory, O(m^2) for m partners (a periodic box under two
-// cutoffs wide, a cluster much denser than a protein).
+// cycles; FP64 throughout would make the search FP64-bound).  The count keeps
+// rows of up to NA_KEEP partners, put in order in registers, so that writing
+// them is a copy; a longer row is searched again and put in order by rank in
+// shared memory up to NA_ROW partners, beyond that by insertion in global
+// memory, O(m^2) for m partners (a periodic box under two cutoffs wide, a
+// cluster much denser than a protein).
 //
-// 30,720 beads at 1e-3 A^-3, cutoff 20 A: 3,200 us -> 122 us (one block for
-// the grid took 250 us of it, and one thread per row, twice, 1,500 us each).
+// 30,720 beads at 1e-3 A^-3, cutoff 20 A: 3,200 us -> 110 us (one block for
+// the grid took 250 us of it, and one thread per row, twice, 1,500 us each;
+// searching every row twice 12 us).
 #include <cuda_runtime.h>
 
 #include <climits>
@@ -47,9 +50,11 @@ namespace xmdg {
 namespace {
 
 constexpr int NA_MAX = XMD_NOALLOC_MAX_BEADS;   // beads, and buckets
+static_assert(NA_MAX <= 65536, "kept partners are 16 bits wide");
 constexpr int NA_SCAN = 1024;                   // elements per scan block
 constexpr int NA_PARTS = NA_MAX / NA_SCAN;
 constexpr int NA_ROW = 512;                     // partners of a row ordered in shared memory
+constexpr int NA_KEEP = 64;                     // partners of a row that the count keeps for the output
 constexpr int NA_WARPS = 8;
 constexpr int NA_PACK = 1023;                   // cell coordinates that fit the packed form
 
@@ -58,6 +63,7 @@ struct __align__(16) NaScratch {
     int row[NA_MAX];       // sort cursors per bucket; then row counts, then row offsets within their scan block
     float4 items[NA_MAX];  // beads in bucket order: FP32 coordinates and the bead's index
     int cell[NA_MAX];      // packed cell coordinates of each bead (or its bucket, when they do not fit)
+    uint16_t kept[NA_MAX][NA_KEEP];   // rows of up to NA_KEEP partners, in order (an index is below NA_MAX)
     int start_base[NA_PARTS], row_base[NA_PARTS], part[NA_PARTS];
     unsigned long long lo_key[3], hi_key[3];
     unsigned done[3];
@@ -289,9 +295,37 @@ __global__ void __launch_bounds__(256) k_na_sort(NaScratch *s, const double *__r
     s->items[at] = make_float4(f[0], f[1], f[2], __int_as_float(i));
 }
 
-// partners j > i, one warp per bead; pass 0 counts, pass 1 writes the row in
-// order of j (its m smallest partners, m = what fits below cap, so that the
-// output is always the (i, j)-ordered prefix of the full list)
+// 32 U register entries in ascending order over a warp (bitonic)
+template <int U> __device__ __forceinline__ void na_sort(int (&v)[U], int lane) {
+#pragma unroll
+    for (int k = 2; k <= 32 * U; k <<= 1)
+#pragma unroll
+        for (int j = k >> 1; j; j >>= 1) {
+            if (j >= 32) {
+#pragma unroll
+                for (int u = 0; u < U; ++u) {
+                    const int w = u ^ (j >> 5);
+                    if (w < u) continue;
+                    const int lo = min(v[u], v[w]), hi = max(v[u], v[w]);
+                    v[u] = ((u * 32) & k) == 0 ? lo : hi;
+                    v[w] = ((u * 32) & k) == 0 ? hi : lo;
+                }
+            } else {
+#pragma unroll
+                for (int u = 0; u < U; ++u) {
+                    const int o = __shfl_xor_sync(0xffffffffu, v[u], j);
+                    const bool up = ((u * 32 + lane) & k) == 0;
+                    v[u] = up == ((lane & j) == 0) ? min(v[u], o) : max(v[u], o);
+                }
+            }
+        }
+}
+
+// partners j > i, one warp per bead; pass 0 counts (and keeps rows of up to
+// NA_KEEP partners in order), pass 1 writes the row in order of j (its m
+// smallest partners, m = what fits below cap, so that the output is always
+// the (i, j)-ordered prefix of the full list), searching again only for longer
+// rows
 template <int PASS>
 __global__ void __launch_bounds__(NA_WARPS * 32) k_na_rows(NaScratch *s, const double *__restrict__ r,
                                                            const int32_t *__restrict__ chain,
@@ -301,7 +335,8 @@ __global__ void __launch_bounds__(NA_WARPS * 32) k_na_rows(NaScratch *s, const d
     const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5;
     const int slot = blockIdx.x * NA_WARPS + wp;
     if (slot >= n) return;   // warp-uniform exits
-    __shared__ int buf[PASS ? NA_WARPS : 1][PASS ? NA_ROW : 1];
+    __shared__ int buf[NA_WARPS][PASS ? NA_ROW : NA_KEEP];
+    __shared__ int s_queue[NA_WARPS][64];
     const float4 me = s->items[slot];
     const int i = __float_as_int(me.w);
     int base = 0, m = 0, rows = 0;
@@ -310,6 +345,14 @@ __global__ void __launch_bounds__(NA_WARPS * 32) k_na_rows(NaScratch *s, const d
         rows = (i + 1 < n ? s->row[i + 1] + s->row_base[(i + 1) / NA_SCAN] : *count) - base;
         m = min(rows, max(0, cap - base));
         if (m == 0) return;
+        if (rows <= NA_KEEP) {
+            int32_t *const out = pairs + 2 * (size_t)base;
+            for (int k = lane; k < m; k += 32) {
+                out[2 * k] = i;
+                out[2 * k + 1] = s->kept[i][k];
+            }
+            return;
+        }
     }
     const bool per = (s->per[0] | s->per[1] | s->per[2]) != 0;
     const float Lx = s->L[0], Ly = s->L[1], Lz = s->L[2];
@@ -358,7 +401,11 @@ __global__ void __launch_bounds__(NA_WARPS * 32) k_na_rows(NaScratch *s, const d
     const int ci = chain[i], si = seq[i];
     int32_t *const row = pairs + 2 * (size_t)base;
     const bool long_row = PASS && rows > NA_ROW;
-    int cnt = 0, kept = 0;
+    // candidates within reach with j > i (one in a dozen), 32 of them to a test
+    // of the chain distance and, inside the error band, of the FP64 distance
+    constexpr int EXACT = 1 << 30;
+    int *const queue = s_queue[wp];
+    int cnt = 0, kept = 0, qn = 0;
     for (int g0 = 0; g0 < total; g0 += 32) {
         // candidate g lies in the bucket of the last lane that starts at or before it
         const int g = g0 + lane;
@@ -369,48 +416,79 @@ __global__ void __launch_bounds__(NA_WARPS * 32) k_na_rows(NaScratch *s, const d
             if (pm <= g) lo += h;
         }
         const int q = __shfl_sync(FULL, q0, lo) + g;
-        bool hit = false;
-        int j = -1;
+        bool in = false;
+        int e = 0;
         if (g < total) {
             const float4 f = s->items[q];
-            j = __float_as_int(f.w);
-            if (j > i) {
-                float dx = f.x - me.x, dy = f.y - me.y, dz = f.z - me.z;
-                if (per) {
-                    dx = na_image(dx, Lx);
-                    dy = na_image(dy, Ly);
-                    dz = na_image(dz, Lz);
-                }
-                const float d2 = dx * dx + dy * dy + dz * dz;
-                if (!(d2 > bhi)) {
-                    const int sj = seq[j], df = si > sj ? si - sj : sj - si;
-                    if (!(chain[j] == ci && df < 3)) hit = d2 < blo || na_dist(*s, r, i, j) < cutoff;
-                }
+            e = __float_as_int(f.w);
+            float dx = f.x - me.x, dy = f.y - me.y, dz = f.z - me.z;
+            if (per) {
+                dx = na_image(dx, Lx);
+                dy = na_image(dy, Ly);
+                dz = na_image(dz, Lz);
             }
+            const float d2 = dx * dx + dy * dy + dz * dz;
+            in = e > i && !(d2 > bhi);
+            if (!(d2 < blo)) e |= EXACT;
         }
-        unsigned bm = __ballot_sync(FULL, hit);
-        if (PASS && !long_row) {
-            if (hit) buf[wp][cnt + __popc(bm & ((1u << lane) - 1u))] = j;
-        } else if (PASS) {
-            // insertion, the row's m smallest kept in order
-            for (; bm; bm &= bm - 1) {
-                const int jj = __shfl_sync(FULL, j, __ffs(bm) - 1);
-                if (lane != 0) continue;
-                if (kept == m && jj >= row[2 * (m - 1) + 1]) continue;
-                int y = kept < m ? kept : m - 1;
-                while (y > 0 && row[2 * (y - 1) + 1] > jj) {
-                    row[2 * y + 1] = row[2 * (y - 1) + 1];
-                    --y;
-                }
-                row[2 * y + 1] = jj;
-                if (kept < m) ++kept;
+        const unsigned im = __ballot_sync(FULL, in);
+        if (in) queue[qn + __popc(im & ((1u << lane) - 1u))] = e;
+        qn += __popc(im);
+        const bool last = g0 + 32 >= total;
+        while (qn >= 32 || (last && qn)) {
+            __syncwarp();
+            bool hit = false;
+            int j = -1;
+            if (lane < qn) {
+                const int e2 = queue[lane];
+                j = e2 & ~EXACT;
+                const int sj = seq[j], df = si > sj ? si - sj : sj - si;
+                if (!(chain[j] == ci && df < 3)) hit = !(e2 & EXACT) || na_dist(*s, r, i, j) < cutoff;
             }
-            continue;
+            const int left = queue[32 + lane];
+            __syncwarp();
+            queue[lane] = left;
+            __syncwarp();
+            qn = max(qn - 32, 0);
+            unsigned bm = __ballot_sync(FULL, hit);
+            if (!PASS) {
+                const int at = cnt + __popc(bm & ((1u << lane) - 1u));
+                if (hit && at < NA_KEEP) buf[wp][at] = j;
+            }
+            if (PASS && !long_row) {
+                if (hit) buf[wp][cnt + __popc(bm & ((1u << lane) - 1u))] = j;
+            } else if (PASS) {
+                // insertion, the row's m smallest kept in order
+                for (; bm; bm &= bm - 1) {
+                    const int jj = __shfl_sync(FULL, j, __ffs(bm) - 1);
+                    if (lane != 0) continue;
+                    if (kept == m && jj >= row[2 * (m - 1) + 1]) continue;
+                    int y = kept < m ? kept : m - 1;
+                    while (y > 0 && row[2 * (y - 1) + 1] > jj) {
+                        row[2 * y + 1] = row[2 * (y - 1) + 1];
+                        --y;
+                    }
+                    row[2 * y + 1] = jj;
+                    if (kept < m) ++kept;
+                }
+                continue;
+            }
+            cnt += __popc(bm);
         }
-        cnt += __popc(bm);
     }
     if (!PASS) {
         if (lane == 0) s->row[i] = cnt;
+        __syncwarp();
+        if (cnt <= 32) {
+            int v[1] = {lane < cnt ? buf[wp][lane] : INT_MAX};
+            na_sort(v, lane);
+            if (lane < cnt) s->kept[i][lane] = (uint16_t)v[0];
+        } else if (cnt <= NA_KEEP) {
+            int v[2] = {buf[wp][lane], lane + 32 < cnt ? buf[wp][lane + 32] : INT_MAX};
+            na_sort(v, lane);
+            s->kept[i][lane] = (uint16_t)v[0];
+            if (lane + 32 < cnt) s->kept[i][lane + 32] = (uint16_t)v[1];
+        }
         return;
     }
     __syncwarp();
