@@ -1475,6 +1475,11 @@ __global__ void __launch_bounds__(TL_THREADS, 4) k_nl_tile(Dev d, TermP p, int c
 // threads per bead, the shapes the autotuner chooses from); the evaluation
 // pass has one shape
 constexpr int EVAL_FB = 64, EVAL_LPB = 4;
+// The limit belongs to the kernel, not to a context: always the largest any
+// context uses, so that a later context does not lower it for an earlier one.
+static void allow_smem(const void *kernel, size_t most) {
+    CK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most));
+}
 static size_t force_smem(bool mixed, int mode, int fb, bool qa) {
     if (mode == 0) fb = EVAL_FB;
 #define XMD_SM(B) (mixed ? step_smem<float, B>(qa) : step_smem<double, B>(qa))
@@ -1539,7 +1544,7 @@ void Engine::launch_force(int mode, int c) {
     const bool mixed = params.precision == XMD_PREC_MIXED;
     void *fk = force_kernel(mixed, mode, fb, lpb);
     const size_t smem = force_smem(mixed, mode, fb, d.qa_on);
-    if (smem > 48 * 1024) CK(cudaFuncSetAttribute(fk, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    if (smem > 48 * 1024) allow_smem(fk, force_smem(mixed, mode, fb, true));
     CK(cudaLaunchKernel(fk, dim3(nb), dim3(fb * lpb), args, smem, stream));
 }
 
@@ -2349,6 +2354,7 @@ void Engine::allocate() {
         jm = gf2_mul(jm, jm);
     }
     ring.up(rng_pow, jt.data(), sizeof(uint64_t) * jt.size());
+    if (dynamic) uring.take(0);   // both rings exist before the first step
     d.nchunks = std::max(1, cap.chunks);
     d.chunks = (int2 *)dalloc(sizeof(int2) * d.nchunks);
     d.work = (int *)dalloc(sizeof(int) * d.nchunks);
@@ -2373,7 +2379,7 @@ void Engine::allocate() {
         if (r.in_use && r.n <= TILE_MAX) tile_smem = std::max(tile_smem, tile_bytes(r.n));
     if (dynamic) tile_smem = tile_bytes(std::min(TILE_MAX, cap.beads));
     if (tile_smem > 48 * 1024)
-        CK(cudaFuncSetAttribute(k_nl_tile, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tile_smem));
+        allow_smem((const void *)k_nl_tile, tile_bytes(TILE_MAX));
     {
         // the tile build runs as many blocks as are resident at once (or the
         // tuned number per SM); they take the work list's chunks in turn
@@ -3370,7 +3376,7 @@ cudaGraphExec_t Engine::graph_for(int start_cur, bool gated, int len) {
     const int nb = force_blocks(d.N, fs.fb);
     void *fk = force_kernel(mixed, 1, fs.fb, fs.lpb);
     const size_t fsmem = force_smem(mixed, 1, fs.fb, d.qa_on);
-    if (fsmem > 48 * 1024) CK(cudaFuncSetAttribute(fk, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fsmem));
+    if (fsmem > 48 * 1024) allow_smem(fk, force_smem(mixed, 1, fs.fb, true));
     // a chain of nodes.  Between two kernels the edge is programmatic: the
     // second is launched while the first one's last blocks run and waits in
     // step_order(); a conditional node takes and gives full edges.
