@@ -58,3 +58,18 @@ def test_block_edges(kind, prec):
             want = got
         for a, b in zip(got, want):
             assert np.array_equal(a, b), shape
+
+
+def test_extended_start_mixed_force():
+    """Extended starts hold triples straight to ~1e-6 rad, whose dihedral
+    forces (1 / sin theta) are the largest of a replica: the mixed bar of
+    1e-5 of the largest force holds there for every chain."""
+    ss = [synth.make_system([90 + 7 * k], 300 + k, temperature=0.35) for k in range(40)]
+    F = {}
+    for prec in ("fp64", "mixed"):
+        with Engine(synth.yaml_for("c4", prec)) as e:
+            for s in ss:
+                e.add_system(s)
+            F[prec] = [e.eval_forces(k)[0] for k in range(len(ss))]
+    for m, f in zip(F["mixed"], F["fp64"]):
+        assert np.abs(m - f).max() <= 1e-5 * np.abs(f).max()

@@ -327,10 +327,27 @@ __device__ __forceinline__ void dihedral_chiral(const Dev &d, const TermP &p, co
         } else if (p.on[XMD_TERM_CND]) {
             const FT c0 = cp.c0, s0 = cp.s0;
             const FT CDA = tpar<FT>(p.cnd_CDA, p.f.cnd_CDA), CDB = tpar<FT>(p.cnd_CDB, p.f.cnd_CDB);
-            const FT sd = fma_<FT>(sphi, c0, -mul_(cphi, s0));
-            const FT sd2 = mul_(sd, sd);
+            FT sd = fma_<FT>(sphi, c0, -mul_(cphi, s0));
+            FT s3, sd2;
             // sin 3x = sin x (3 - 4 sin^2 x), cos 3x = cos x (1 - 4 sin^2 x)
-            const FT s3 = mul_(sd, fma_<FT>(FT(-4), sd2, FT(3)));
+            if constexpr (MIX) {
+                // sine and cosine brought back to the unit circle (their FP32
+                // factors err by some 3e-7, which the sine of 3x takes ninefold
+                // where the cosine is small), and the smaller one squared: the
+                // force of near-straight quads, 1 / sin theta large, cancels
+                // between the two harmonics (3.5e-5 of it lost without this)
+                float cd = __fmaf_rn(cphi, c0, __fmul_rn(sphi, s0));
+                const float c2 = __fmul_rn(cd, cd), c2l = __fmaf_rn(cd, cd, -c2);
+                const float m = -0.5f * __fadd_rn(__fmaf_rn(sd, sd, __fadd_rn(c2, -1.0f)), c2l);
+                sd = __fmaf_rn(m, sd, sd);
+                cd = __fmaf_rn(m, cd, cd);
+                sd2 = __fmul_rn(sd, sd);
+                s3 = __fmul_rn(sd, fabsf(sd) > fabsf(cd) ? __fmaf_rn(4.0f, __fmul_rn(cd, cd), -1.0f)
+                                                         : __fmaf_rn(-4.0f, sd2, 3.0f));
+            } else {
+                sd2 = mul_(sd, sd);
+                s3 = mul_(sd, fma_<FT>(FT(-4), sd2, FT(3)));
+            }
             dV = fma_<FT>(mul_(FT(3), CDB), s3, mul_(CDA, sd));
             if (MODE == 0) {
                 const FT cd = fma_<FT>(cphi, c0, mul_(sphi, s0));
