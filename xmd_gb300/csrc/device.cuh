@@ -345,6 +345,103 @@ __device__ __forceinline__ void chiral_mixed(const TermP &p, V3<float> r12, V3<f
     f[3] = -(g * x12_23);
 }
 
+// ---- bonded terms of the mixed path -------------------------------------------
+// The reference formulation (acos of a clamped cosine; cross products of bond
+// vectors) loses all accuracy in FP32 near straight triples, where the stiff
+// starting chains live: the reference's own FP32 build misses by ~1e-3.  Here
+// the bond vectors, their cross products and the dihedral's triple product are
+// formed in float-float and the angles are taken with atan2 in FP32:
+//   theta = atan2(|r12 x r23|, -r12.r23)                    (= acos of the cosine)
+//   phi   = atan2(|r23| (x12_23 . r34), x12_23 . x23_34)    (= +-acos, sign of
+//            x12_23 . r34 as in complex_native.cpp:27-28)
+// after which every FP32 operation is well conditioned.  Force expressions are
+// those of angle/native.cpp:25-38 and dihedral/complex_native.cpp:37-48.
+// The rounding of these expressions and of the pair terms below is part of what
+// a mixed run returns: the dynamics amplifies one FP32 rounding to 1e-3 of a
+// single bead's velocity within 128 steps, so any other form of them, a more
+// exact one too, gives other trajectories.
+
+// tether from the narrowed bond vector r12 = r2 - r1, its length and 1 / length
+__device__ __forceinline__ V3<float> tether_mixed(const TermP &p, V3<float> r12, float r12_n, float inv,
+                                                  float nat_dist, float *V) {
+    float dr = r12_n - nat_dist, dr2 = dr * dr;
+    float H1 = p.f.tether_H1, H2 = p.f.tether_H2;
+    float V_ = 0.5f * dr2 * (H1 + H2 * dr2);
+    float dV_dr = dr * (H1 + 2.0f * H2 * dr2);
+    *V = clampv<float>(V_, -1.0e3f, 1.0e3f);
+    dV_dr = clampv<float>(dV_dr, -1.0e3f, 1.0e3f);
+    return dV_dr * V3<float>{r12.x * inv, r12.y * inv, r12.z * inv};
+}
+
+// r12, r23: narrowed bond vectors with their inverse lengths; x12_23: their
+// narrowed cross product, x_n its length.
+// hc: heuristic angle coefficients (or null); their polynomial, whose terms
+// cancel to ~1e-5 of their size, is summed in FP64
+__device__ __forceinline__ void angle_mixed(const TermP &p, V3<float> r12, V3<float> r23, V3<float> x12_23,
+                                            float r12_rn, float r23_rn, float x_n, float nat_theta, const double *hc,
+                                            V3<float> *f1, V3<float> *f2, V3<float> *f3, float *V) {
+    V3<float> d1 = r12_rn * unit(cross(r12, x12_23));
+    V3<float> d3 = r23_rn * unit(cross(r23, x12_23));
+    V3<float> d2 = (-d1) - d3;
+    float theta = atan2f(x_n, -dot(r12, r23));
+    float dV;
+    if (hc) {
+        const double2 vd = heur_poly_nl(hc, (double)theta);
+        *V = (float)vd.x;
+        dV = (float)vd.y;
+    } else {
+        float dtheta = theta - nat_theta;
+        float k = p.f.nat_ang_k;
+        *V = 0.5f * k * dtheta * dtheta;
+        dV = k * dtheta;
+    }
+    *f1 = -(dV * d1);
+    *f2 = -(dV * d2);
+    *f3 = -(dV * d3);
+}
+
+// narrowed bond vectors and cross products, |r23|, 1 / |x12_23| and
+// 1 / |x23_34|; X = x12_23 . x23_34, T = x12_23 . r34 (hc: heuristic dihedral
+// coefficients or null)
+__device__ __forceinline__ void dihedral_mixed(const TermP &p, V3<float> r12, V3<float> r23, V3<float> r34,
+                                               V3<float> x12_23, V3<float> x23_34, float r23_n, float x12_23_rn,
+                                               float x23_34_rn, float X, float T, float nat_phi, bool cnd, bool snd,
+                                               const float *hc, V3<float> *f, float *Vc, float *Vs) {
+    float phi = atan2f(r23_n * T, X);
+    float diff_ = phi - nat_phi;
+    float dV = 0.0f;
+    *Vc = 0.0f;
+    *Vs = 0.0f;
+    if (hc) {
+        float sp, cp;
+        sincosf(phi, &sp, &cp);
+        heur_dih_nl<float>(hc, sp, cp, Vc, &dV);
+    } else if (cnd) {
+        float s1, c1, s3, c3;
+        sincosf(diff_, &s1, &c1);
+        sincosf(3.0f * diff_, &s3, &c3);
+        float CDA = p.f.cnd_CDA, CDB = p.f.cnd_CDB;
+        *Vc = CDA * (1.0f - c1) + CDB * (1.0f - c3);
+        dV += CDA * s1 + CDB * 3.0f * s3;
+    }
+    if (snd && !hc) {
+        float CDH = p.f.snd_CDH;
+        *Vs = 0.5f * CDH * diff_ * diff_;
+        dV += CDH * diff_;
+    }
+    V3<float> x12_23_u = x12_23_rn * x12_23, x23_34_u = x23_34_rn * x23_34;
+    V3<float> d1 = x12_23_rn * (r23_n * (-x12_23_u));
+    V3<float> d4 = x23_34_rn * (r23_n * x23_34_u);
+    float k1 = dot(r12, r23), k4 = dot(r23, r34), den = r23_n * r23_n;
+    V3<float> df{(-d1.x * k1 + d4.x * k4) / den, (-d1.y * k1 + d4.y * k4) / den, (-d1.z * k1 + d4.z * k4) / den};
+    V3<float> d2 = (-d1) + df;
+    V3<float> d3 = (-d4) - df;
+    f[0] = -(dV * d1);
+    f[1] = -(dV * d2);
+    f[2] = -(dV * d3);
+    f[3] = -(dV * d4);
+}
+
 // ---- pair terms: force on the first bead of r12 = r_uv(r_i, r_j) ------------
 
 // lj::operator(): primitives/lj.h:22-30
@@ -355,6 +452,26 @@ __device__ __forceinline__ void lj_eval(T depth, T r_min, T r_inv, T *V, T *dV) 
     T dV_dr = T(12) * depth * r_inv * (s6 - s12);
     *V = clampv<T>(V_, T(-1.0e3), T(1.0e3));
     *dV = clampv<T>(dV_dr, T(-1.0e3), T(1.0e3));
+}
+
+// Go contact (eval_go_forces::iter go.cpp:31-46, lj::operator() lj.h:22-30;
+// shift 0) and, inside r_excl, Pauli exclusion (pauli.cpp:32-48,
+// shifted_lj.h:14-21; shift 1) of the mixed path: energy and dV/dr
+__device__ __forceinline__ void lj_mixed(float depth, float r_min, float r_inv, float shift, float *V, float *dV) {
+    float s = r_inv * r_min, s6 = ipow6(s), s12 = s6 * s6;
+    float V_ = depth * (s12 - 2.0f * s6 + shift);
+    float dV_dr = 12.0f * depth * r_inv * (s6 - s12);
+    *V = clampv<float>(V_, -1.0e3f, 1.0e3f);
+    *dV = clampv<float>(dV_dr, -1.0e3f, 1.0e3f);
+}
+
+// Debye-Hueckel on the mixed path: eval_const_es_forces::iter es/const.cpp:13-32
+// and eval_relative_es_forces::iter es/relative.cpp:13-32
+__device__ __forceinline__ float es_mixed(const TermP &p, float r, float r_inv, float q1_x_q2, float *V) {
+    float sdi = p.f.es_sdi;
+    float Vij = p.f.es_Vf * q1_x_q2 * exp_(-r * sdi) * r_inv * r_inv;
+    *V = Vij;
+    return p.es_rel ? -Vij * (sdi + 2.0f * r_inv) : -Vij * (sdi + r_inv);
 }
 
 // native disulfide: eval_nat_ssbond_forces::iter native_ss.cpp:27-40,

@@ -2136,14 +2136,17 @@ void Engine::derive_rep(int ri, RepDev &rd) {
         rd.box.cell_inv[a] = r.cell[a] != 0.0 ? 1.0 / r.cell[a] : 0.0;   // box.h:12-22
         rd.per[a] = r.cell[a] != 0.0;
         rd.per_any |= rd.per[a];
-        // the length as h + l, h truncated as split_d's
-        uint64_t u;
-        std::memcpy(&u, &r.cell[a], 8);
-        u &= ~0x1fffffffull;
-        double h;
-        std::memcpy(&h, &u, 8);
+        // the length as h + l, both truncated as split_d's
+        auto leading = [](double x) {
+            uint64_t u;
+            std::memcpy(&u, &x, 8);
+            u &= ~0x1fffffffull;
+            std::memcpy(&x, &u, 8);
+            return x;
+        };
+        const double h = leading(r.cell[a]);
         rd.Lh[a] = (float)h;
-        rd.Ll[a] = (float)(r.cell[a] - h);
+        rd.Ll[a] = (float)leading(r.cell[a] - h);
         rd.Li[a] = (float)rd.box.cell_inv[a];
     }
     // max_cutoff: main.cpp:500, 545-551, 628-630, 642-644, 742-746
@@ -2706,7 +2709,7 @@ void Engine::place(int k, Staged *st) {
     std::vector<double2> dcs(n);
     for (int i = 0; i < n; ++i) {
         dcs[i] = make_double2(std::cos(dr[i]), std::sin(dr[i]));
-        bf[i] = make_float4(0.0f, (float)ar[i], (float)dcs[i].x, (float)dcs[i].y);
+        bf[i] = make_float4((float)tr[i], (float)ar[i], (float)dr[i], 0.0f);
     }
     up(d.dih_cs + b, dcs.data(), sizeof(double2) * n);
     up(d.bond_f + b, bf.data(), sizeof(float4) * n);

@@ -157,7 +157,7 @@ struct Dev {
     double *fext;           // [3N] external force of the step (k_ext: AFM, walls)
     int32_t *ss_start, *ss_end, *ss_j;   // native disulfide partners per bead (CSR, both directions)
     uint8_t *ss_on;         // in the list of the last rebuild (update_nat_ssbonds, native_ss.cpp:8-19)
-    float4 *bond_f;         // (0, theta0, cos phi0, sin phi0) in FP32 for the mixed path
+    float4 *bond_f;         // (r0, theta0, phi0, 0) in FP32 for the mixed path
     int32_t *nat_start, *nat_end, *nat_j;   // natives of bead i: [nat_start[i], nat_end[i])
     double *nat_d;
     uint8_t *nat_on;        // in the Go list of the last rebuild (update_go_contacts, go.cpp:11-22)

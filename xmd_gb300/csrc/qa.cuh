@@ -15,17 +15,21 @@
 namespace xmdg {
 
 // ---- pair vectors -------------------------------------------------------------------
-// mixed: from split positions; the minimum image leaves the short form unless
-// a pair actually lies across the box
+// mixed: from split positions.  A pair across the box takes mi_axis; any other
+// has the float-float difference's high part, which is what mi_axis gives it
+// (it subtracts zero).
 __device__ __forceinline__ V3<float> pair_vec(const RepDev &rp, bool per, const F2 (&a)[3], const F2 (&b)[3]) {
     float v[3];
-#pragma unroll
-    for (int k = 0; k < 3; ++k) v[k] = __fadd_rn(__fsub_rn(b[k].h, a[k].h), __fsub_rn(b[k].l, a[k].l));
     if (per) {
 #pragma unroll
-        for (int k = 0; k < 3; ++k)
+        for (int k = 0; k < 3; ++k) {
+            v[k] = ff_diff(a[k], b[k]).h;
             if (rintf(__fmul_rn(v[k], rp.Li[k])) != 0.0f)
                 v[k] = mi_axis(a[k], b[k], rp.Lh[k], rp.Ll[k], rp.Li[k], true);
+        }
+    } else {
+#pragma unroll
+        for (int k = 0; k < 3; ++k) v[k] = mi_axis(a[k], b[k], 0.0f, 0.0f, 0.0f, false);
     }
     return V3<float>{v[0], v[1], v[2]};
 }

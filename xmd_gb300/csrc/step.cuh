@@ -151,9 +151,9 @@ __device__ __forceinline__ void noise3_turns(uint64_t st, const double2 *logt, d
 // own, as the reference's uncontracted build forms them: on extended starts
 // triples are straight to ~1e-6 rad, where a contracted cross product moves
 // a dihedral force by 1e-10 of itself.
-// Mixed: bond and cross product in float-float (6 + 6), 1/|e|, 1/|x|.
+// Mixed: bond and cross product in float-float (6 + 6), 1/|e|, 1/|x|, |e|, |x|.
 enum : int { GE = 0, GU = 3, GLEN = 6, GRN = 7, GRX = 8, GN64 = 9 };
-enum : int { MEH = 0, MEL = 3, MXH = 6, MXL = 9, MRN = 12, MRX = 13, GN32 = 16 };
+enum : int { MEH = 0, MEL = 3, MXH = 6, MXL = 9, MRN = 12, MRX = 13, MLEN = 14, MLX = 15, GN32 = 16 };
 
 // energies of the evaluation pass: per thread for the block's first replica,
 // reduced over the warp at the end; other replicas at once
@@ -193,9 +193,10 @@ template <> struct Ener<0> {
 };
 
 // ---- bonded centres ----------------------------------------------------------------
-// a centre's parameters: bond length (mixed: with its low part), angle, cosine
-// and sine of the dihedral
-template <class FT> struct CentreP { FT r0, t0, c0, s0, r0l; };
+// a centre's parameters: bond length, angle, cosine and sine of the dihedral
+// (mixed: the dihedral itself)
+template <class FT> struct CentreP { FT r0, t0, c0, s0; };
+template <> struct CentreP<float> { float r0, t0, p0; };
 
 // sp: the centre's position slot.  g: geometry slots [.][FB].
 
@@ -213,60 +214,48 @@ __device__ __forceinline__ void bond_angle(const Dev &d, const TermP &p, const F
     const FT rn1 = g[MIX ? MRN : GRN][sp - 1], rn2 = g[MIX ? MRN : GRN][sp];
     if ((fl & BF_TETH) && p.on[XMD_TERM_TETHER]) {
         // eval_tether_forces::iter tether.cpp:21-36, harmonic.h:18-25
-        FT dr;
+        FT V_;
         if constexpr (MIX) {
-            // the bond length in float-float: its stiffness (2500 eps per unit
-            // squared) makes an FP32 length the largest error of the force
-            const FF px = two_prod(e2.x, e2.x), py = two_prod(e2.y, e2.y), pz = two_prod(e2.z, e2.z);
-            const FF s1 = two_sum(px.h, py.h), s2 = two_sum(s1.h, pz.h);
-            float low = __fadd_rn(__fadd_rn(px.l, py.l), __fadd_rn(pz.l, __fadd_rn(s1.l, s2.l)));
-            const V3<float> el{g[MEL][sp], g[MEL + 1][sp], g[MEL + 2][sp]};
-            low = __fmaf_rn(2.0f, fdot(e2, el), low);
-            const float l0 = __fmul_rn(s2.h, rn2);
-            const float rest = __fadd_rn(__fmaf_rn(-l0, l0, s2.h), low);
-            dr = __fadd_rn(__fsub_rn(l0, cp.r0), __fmaf_rn(__fmul_rn(0.5f, rn2), rest, -cp.r0l));
+            *ft = tether_mixed(p, e2, g[MLEN][sp], rn2, cp.r0, &V_);
         } else {
-            dr = g[GLEN][sp] - cp.r0;
+            const double dr = g[GLEN][sp] - cp.r0, dr2 = mul_(dr, dr);
+            double dV = mul_(dr, fma_<double>(mul_(2.0, p.tether_H2), dr2, p.tether_H1));
+            dV = clampv<double>(dV, -1.0e3, 1.0e3);
+            *ft = fscl<double>(mul_(dV, rn2), e2);
+            V_ = clampv<double>(mul_(mul_(0.5, dr2), fma_<double>(p.tether_H2, dr2, p.tether_H1)), -1.0e3, 1.0e3);
         }
-        const FT dr2 = mul_(dr, dr);
-        const FT H1 = tpar<FT>(p.tether_H1, p.f.tether_H1), H2 = tpar<FT>(p.tether_H2, p.f.tether_H2);
-        FT dV = mul_(dr, fma_<FT>(mul_(FT(2), H2), dr2, H1));
-        dV = clampv<FT>(dV, FT(-1.0e3), FT(1.0e3));
-        *ft = fscl<FT>(mul_(dV, rn2), e2);
-        if (MODE == 0 && own)
-            en.add(d, rc, XMD_TERM_TETHER,
-                   (double)clampv<FT>(mul_(mul_(FT(0.5), dr2), fma_<FT>(H2, dr2, H1)), FT(-1.0e3), FT(1.0e3)));
+        if (MODE == 0 && own) en.add(d, rc, XMD_TERM_TETHER, (double)V_);
     }
     if (do_ang) {
-        // eval_native_angle_forces::iter angle/native.cpp:13-39.  The cross
-        // products of the bonds with the plane's normal have lengths |r12| and
-        // |r23| (the bonds lie in the plane), so the reference's unit vectors
-        // along them need no further square root.
-        V3<FT> u;   // the plane's unit normal
+        // eval_native_angle_forces::iter angle/native.cpp:13-39
         double V_ = 0.0;
-        FT dV, theta;
         if constexpr (MIX) {
             const V3<float> x{g[MXH][sp], g[MXH + 1][sp], g[MXH + 2][sp]};
-            u = fscl<float>(g[MRX][sp], x);
-            theta = atan2f(__fmul_rn(fdot(x, x), g[MRX][sp]), -fdot(e1, e2));
+            float Vf;
+            angle_mixed(p, e1, e2, x, rn1, rn2, g[MLX][sp], cp.t0, hac, a1, a2, a3, &Vf);
+            V_ = (double)Vf;
         } else {
-            u = V3<double>{g[GU][sp], g[GU + 1][sp], g[GU + 2][sp]};
+            // the cross products of the bonds with the plane's unit normal have
+            // lengths |r12| and |r23| (the bonds lie in the plane), so the
+            // reference's unit vectors along them need no further square root
+            const V3<double> u{g[GU][sp], g[GU + 1][sp], g[GU + 2][sp]};
             const V3<DN> b1{e1.x, e1.y, e1.z}, b2{e2.x, e2.y, e2.z};
-            theta = acos_c<DN>(-dot(b1, b2) * DN(rn1) * DN(rn2)).v;
-        }
-        if (hac) {
-            const double2 vd = heur_poly_nl(hac, (double)theta);
-            V_ = vd.x;
-            dV = (FT)vd.y;
-        } else {
-            const FT dt = theta - cp.t0;
-            dV = mul_(tpar<FT>(p.nat_ang_k, p.f.nat_ang_k), dt);
-            if (MODE == 0) V_ = (double)mul_(FT(0.5), mul_(dV, dt));
+            const double theta = acos_c<DN>(-dot(b1, b2) * DN(rn1) * DN(rn2)).v;
+            double dV;
+            if (hac) {
+                const double2 vd = heur_poly_nl(hac, theta);
+                V_ = vd.x;
+                dV = vd.y;
+            } else {
+                const double dt = theta - cp.t0;
+                dV = mul_(p.nat_ang_k, dt);
+                if (MODE == 0) V_ = mul_(0.5, mul_(dV, dt));
+            }
+            *a1 = fscl<double>(-mul_(dV, mul_(rn1, rn1)), fcross(e1, u));
+            *a3 = fscl<double>(-mul_(dV, mul_(rn2, rn2)), fcross(e2, u));
+            *a2 = V3<double>{-add_(a1->x, a3->x), -add_(a1->y, a3->y), -add_(a1->z, a3->z)};
         }
         if (MODE == 0 && own) en.add(d, rc, h_ang ? XMD_TERM_HEUR_ANG : XMD_TERM_NAT_ANG, V_);
-        *a1 = fscl<FT>(-mul_(dV, mul_(rn1, rn1)), fcross(e1, u));
-        *a3 = fscl<FT>(-mul_(dV, mul_(rn2, rn2)), fcross(e2, u));
-        *a2 = V3<FT>{-add_(a1->x, a3->x), -add_(a1->y, a3->y), -add_(a1->z, a3->z)};
     }
 }
 
@@ -283,96 +272,70 @@ __device__ __forceinline__ void dihedral_chiral(const Dev &d, const TermP &p, co
         e3{g[0][sp + 1], g[1][sp + 1], g[2][sp + 1]};
     if (do_dih) {
         // eval_cnd_forces::iter dihedral/complex_native.cpp:13-49,
-        // eval_snd_forces::iter dihedral/simple_native.cpp:13-45.  Sine and
-        // cosine of phi come from the geometry, those of phi - phi0 and
-        // 3 (phi - phi0) by the addition theorems: no arc cosine and no
-        // sine of an angle, except for the terms that need phi itself.
-        V3<FT> u1, u2;
-        FT rx1, rx2, rn2, len2, cphi, sphi, tsign;
+        // eval_snd_forces::iter dihedral/simple_native.cpp:13-45
+        double Vc = 0.0, Vs = 0.0;
         if constexpr (MIX) {
-            rx1 = g[MRX][sp]; rx2 = g[MRX][sp + 1]; rn2 = g[MRN][sp];
             const V3<float> x1{g[MXH][sp], g[MXH + 1][sp], g[MXH + 2][sp]},
                 x2{g[MXH][sp + 1], g[MXH + 1][sp + 1], g[MXH + 2][sp + 1]};
-            u1 = fscl<float>(rx1, x1);
-            u2 = fscl<float>(rx2, x2);
-            len2 = __fmul_rn(fdot(e2, e2), rn2);
-            // the triple product in float-float: small against its factors
-            // for flat quads
+            // the triple product in float-float: small against its factors for
+            // flat quads
             const V3<FF> xf{FF{x1.x, g[MXL][sp]}, FF{x1.y, g[MXL + 1][sp]}, FF{x1.z, g[MXL + 2][sp]}};
             const V3<FF> ef{FF{e3.x, g[MEL][sp + 1]}, FF{e3.y, g[MEL + 1][sp + 1]}, FF{e3.z, g[MEL + 2][sp + 1]}};
-            tsign = ff_dot(xf, ef).h;
-            sphi = __fmul_rn(__fmul_rn(__fmul_rn(len2, tsign), rx1), rx2);
-            cphi = __fmul_rn(__fmul_rn(fdot(x1, x2), rx1), rx2);
+            float Vcf, Vsf;
+            dihedral_mixed(p, e1, e2, e3, x1, x2, g[MLEN][sp], g[MRX][sp], g[MRX][sp + 1], dot(x1, x2),
+                           ff_dot(xf, ef).h, cp.p0, p.on[XMD_TERM_CND] != 0, p.on[XMD_TERM_SND] != 0,
+                           h_dih ? d.heur_dih_f + 6 * hdt : nullptr, q, &Vcf, &Vsf);
+            Vc = (double)Vcf;
+            Vs = (double)Vsf;
         } else {
-            rx1 = g[GRX][sp]; rx2 = g[GRX][sp + 1]; rn2 = g[GRN][sp];
-            len2 = g[GLEN][sp];
-            u1 = V3<double>{g[GU][sp], g[GU + 1][sp], g[GU + 2][sp]};
-            u2 = V3<double>{g[GU][sp + 1], g[GU + 1][sp + 1], g[GU + 2][sp + 1]};
+            // sine and cosine of phi come from the geometry, those of
+            // phi - phi0 and 3 (phi - phi0) by the addition theorems: no arc
+            // cosine and no sine of an angle, except for the terms that need
+            // phi itself
+            const double rx1 = g[GRX][sp], rx2 = g[GRX][sp + 1], rn2 = g[GRN][sp], len2 = g[GLEN][sp];
+            const V3<double> u1{g[GU][sp], g[GU + 1][sp], g[GU + 2][sp]},
+                u2{g[GU][sp + 1], g[GU + 1][sp + 1], g[GU + 2][sp + 1]};
             // the cosine as the reference rounds it, clamped; the sine of its
             // arc cosine is sqrt((1 - c)(1 + c))
             const V3<DN> a{u1.x, u1.y, u1.z}, b{u2.x, u2.y, u2.z};
-            cphi = clampv<double>(dot(a, b).v, -1.0, 1.0);
+            const double cphi = clampv<double>(dot(a, b).v, -1.0, 1.0);
             const double s2 = __dmul_rn(__dsub_rn(1.0, cphi), __dadd_rn(1.0, cphi));
-            sphi = s2 > 0.0 ? __dmul_rn(s2, rsqrt(s2)) : s2;
-            tsign = fdot(u1, e3);
+            double sphi = s2 > 0.0 ? __dmul_rn(s2, rsqrt(s2)) : s2;
+            const double tsign = fdot(u1, e3);
             if (tsign < 0.0) sphi = -sphi;
-        }
-        FT dV = FT(0);
-        double Vc = 0.0, Vs = 0.0;
-        if (h_dih) {
-            FT V_;
-            if constexpr (MIX) heur_dih_nl<float>(d.heur_dih_f + 6 * hdt, sphi, cphi, &V_, &dV);
-            else heur_dih_nl<double>(d.heur_dih + 6 * hdt, sphi, cphi, &V_, &dV);
-            Vc = (double)V_;
-        } else if (p.on[XMD_TERM_CND]) {
-            const FT c0 = cp.c0, s0 = cp.s0;
-            const FT CDA = tpar<FT>(p.cnd_CDA, p.f.cnd_CDA), CDB = tpar<FT>(p.cnd_CDB, p.f.cnd_CDB);
-            FT sd = fma_<FT>(sphi, c0, -mul_(cphi, s0));
-            FT s3, sd2;
-            // sin 3x = sin x (3 - 4 sin^2 x), cos 3x = cos x (1 - 4 sin^2 x)
-            if constexpr (MIX) {
-                // sine and cosine brought back to the unit circle (their FP32
-                // factors err by some 3e-7, which the sine of 3x takes ninefold
-                // where the cosine is small), and the smaller one squared: the
-                // force of near-straight quads, 1 / sin theta large, cancels
-                // between the two harmonics (3.5e-5 of it lost without this)
-                float cd = __fmaf_rn(cphi, c0, __fmul_rn(sphi, s0));
-                const float c2 = __fmul_rn(cd, cd), c2l = __fmaf_rn(cd, cd, -c2);
-                const float m = -0.5f * __fadd_rn(__fmaf_rn(sd, sd, __fadd_rn(c2, -1.0f)), c2l);
-                sd = __fmaf_rn(m, sd, sd);
-                cd = __fmaf_rn(m, cd, cd);
-                sd2 = __fmul_rn(sd, sd);
-                s3 = __fmul_rn(sd, fabsf(sd) > fabsf(cd) ? __fmaf_rn(4.0f, __fmul_rn(cd, cd), -1.0f)
-                                                         : __fmaf_rn(-4.0f, sd2, 3.0f));
-            } else {
-                sd2 = mul_(sd, sd);
-                s3 = mul_(sd, fma_<FT>(FT(-4), sd2, FT(3)));
+            double dV = 0.0;
+            if (h_dih) {
+                heur_dih_nl<double>(d.heur_dih + 6 * hdt, sphi, cphi, &Vc, &dV);
+            } else if (p.on[XMD_TERM_CND]) {
+                const double c0 = cp.c0, s0 = cp.s0, CDA = p.cnd_CDA, CDB = p.cnd_CDB;
+                const double sd = fma_<double>(sphi, c0, -mul_(cphi, s0));
+                // sin 3x = sin x (3 - 4 sin^2 x), cos 3x = cos x (1 - 4 sin^2 x)
+                const double sd2 = mul_(sd, sd), s3 = mul_(sd, fma_<double>(-4.0, sd2, 3.0));
+                dV = fma_<double>(mul_(3.0, CDB), s3, mul_(CDA, sd));
+                if (MODE == 0) {
+                    const double cd = fma_<double>(cphi, c0, mul_(sphi, s0));
+                    const double c3 = mul_(cd, fma_<double>(-4.0, sd2, 1.0));
+                    // 1 - cos x = sin^2 x / (1 + cos x), without cancellation at the minimum
+                    const double v1 = cd > 0.0 ? sd2 / (1.0 + cd) : 1.0 - cd;
+                    const double v3 = c3 > 0.0 ? s3 * s3 / (1.0 + c3) : 1.0 - c3;
+                    Vc = CDA * v1 + CDB * v3;
+                }
             }
-            dV = fma_<FT>(mul_(FT(3), CDB), s3, mul_(CDA, sd));
-            if (MODE == 0) {
-                const FT cd = fma_<FT>(cphi, c0, mul_(sphi, s0));
-                const FT c3 = mul_(cd, fma_<FT>(FT(-4), sd2, FT(1)));
-                // 1 - cos x = sin^2 x / (1 + cos x), without cancellation at the minimum
-                const FT v1 = cd > FT(0) ? sd2 / (FT(1) + cd) : FT(1) - cd;
-                const FT v3 = c3 > FT(0) ? s3 * s3 / (FT(1) + c3) : FT(1) - c3;
-                Vc = (double)(CDA * v1 + CDB * v3);
-            }
-        }
-        if (p.on[XMD_TERM_SND] && !h_dih) {
-            FT phi, CDH, p0;
-            if constexpr (MIX) {
-                phi = atan2f(sphi, cphi);
-                CDH = p.f.snd_CDH;
-                p0 = narrow_f(d.dih_p0[c]);
-            } else {
-                phi = acos(cphi);
+            if (p.on[XMD_TERM_SND] && !h_dih) {
+                double phi = acos(cphi);
                 if (tsign < 0.0) phi = -phi;
-                CDH = p.snd_CDH;
-                p0 = d.dih_p0[c];
+                const double df = phi - d.dih_p0[c];
+                dV = fma_<double>(p.snd_CDH, df, dV);
+                Vs = 0.5 * p.snd_CDH * df * df;
             }
-            const FT df = phi - p0;
-            dV = fma_<FT>(CDH, df, dV);
-            Vs = 0.5 * (double)CDH * (double)df * (double)df;
+            const double k = mul_(dV, len2), iden = mul_(rn2, rn2);
+            q[0] = fscl<double>(mul_(k, rx1), u1);
+            q[3] = fscl<double>(-mul_(k, rx2), u2);
+            const double k1 = mul_(fdot(e1, e2), iden), k4 = mul_(fdot(e2, e3), iden);
+            const V3<double> w{fma_<double>(q[0].x, k1, -mul_(q[3].x, k4)), fma_<double>(q[0].y, k1, -mul_(q[3].y, k4)),
+                               fma_<double>(q[0].z, k1, -mul_(q[3].z, k4))};
+            q[1] = V3<double>{-add_(q[0].x, w.x), -add_(q[0].y, w.y), -add_(q[0].z, w.z)};
+            q[2] = V3<double>{add_(w.x, -q[3].x), add_(w.y, -q[3].y), add_(w.z, -q[3].z)};
         }
         if (MODE == 0 && own) {
             if (h_dih) en.add(d, rc, XMD_TERM_HEUR_DIH, Vc);
@@ -381,14 +344,6 @@ __device__ __forceinline__ void dihedral_chiral(const Dev &d, const TermP &p, co
                 if (p.on[XMD_TERM_SND]) en.add(d, rc, XMD_TERM_SND, Vs);
             }
         }
-        const FT k = mul_(dV, len2), iden = mul_(rn2, rn2);
-        q[0] = fscl<FT>(mul_(k, rx1), u1);
-        q[3] = fscl<FT>(-mul_(k, rx2), u2);
-        const FT k1 = mul_(fdot(e1, e2), iden), k4 = mul_(fdot(e2, e3), iden);
-        const V3<FT> w{fma_<FT>(q[0].x, k1, -mul_(q[3].x, k4)), fma_<FT>(q[0].y, k1, -mul_(q[3].y, k4)),
-                       fma_<FT>(q[0].z, k1, -mul_(q[3].z, k4))};
-        q[1] = V3<FT>{-add_(q[0].x, w.x), -add_(q[0].y, w.y), -add_(q[0].z, w.z)};
-        q[2] = V3<FT>{add_(w.x, -q[3].x), add_(w.y, -q[3].y), add_(w.z, -q[3].z)};
     }
     if ((fl & BF_CHIR) && p.on[XMD_TERM_CHIR]) {
         // eval_chiral_forces::iter chiral.cpp:15-37
@@ -430,8 +385,11 @@ template <class FT, int FB> struct StepSh {
     FT g[MIX ? (int)GN32 : (int)GN64][FB];   // geometry
     FT c[24][FB];                     // centre forces: tether, angle on c-1, c, c+1, dihedral on c-1 .. c+2
     FT f[3][FCAP];                    // pair forces
+    // mixed: the second force of entries with two, and which those are
+    FT f2[3][MIX ? FCAP : 1];
+    unsigned two[MIX ? FCAP / 32 : 1];
     FT n[3][FB];                      // noise
-    FT e[3][FB];                      // squared skin-test displacement per axis
+    FT e[3][FB];                      // skin-test displacement per axis (FP64: squared)
     // FP64: electrostatic entries set aside (their charge product, and which)
     FT ew[MIX ? 1 : FCAP];
     int eq[MIX ? 1 : FCAP], neq, next_es;
@@ -443,13 +401,11 @@ template <class FT, int FB> constexpr size_t step_smem(bool qa) {
     return (sizeof(StepSh<FT, FB>) + 15) / 16 * 16 + (qa ? sizeof(int) * QA_REF_CAP * FB : 0);
 }
 
-// Debye-Hueckel force factor: eval_const_es_forces::iter es/const.cpp:13-32,
-// eval_relative_es_forces::iter es/relative.cpp:13-32
-template <class FT>
-__device__ __forceinline__ FT es_factor(const TermP &p, FT vq, FT s2, FT rn, FT *V) {
-    const FT sdi = tpar<FT>(p.es_sdi, p.f.es_sdi);
-    *V = mul_(mul_(vq, exp_(-mul_(mul_(s2, rn), sdi))), mul_(rn, rn));
-    return -mul_(*V, fma_<FT>(p.es_rel ? FT(2) : FT(1), rn, sdi));
+// Debye-Hueckel force factor of the FP64 path: eval_const_es_forces::iter
+// es/const.cpp:13-32, eval_relative_es_forces::iter es/relative.cpp:13-32
+__device__ __forceinline__ double es_factor(const TermP &p, double vq, double len, double rn, double *V) {
+    *V = mul_(mul_(vq, exp_(-mul_(len, p.es_sdi))), mul_(rn, rn));
+    return -mul_(*V, fma_<double>(p.es_rel ? 2.0 : 1.0, rn, p.es_sdi));
 }
 
 // a pair entry of the block: its bead's slot, the partner, the row's flags (0:
@@ -505,34 +461,44 @@ template <class FT> __device__ __forceinline__ PairPos<FT> pair_pos(const Dev &d
     return x;
 }
 
-// force of a pair entry on its bead.  On the FP64 path the electrostatic part
-// (an exponential, half the pair's FP64 work) is set aside when it is all
-// there is to the pair: *es gets its charge factor and the pair vector is
-// returned, so that whole warps of such pairs do it later instead of every
-// warp that holds one.
+// force of a pair entry on its bead.
+// Mixed: a pair on both the Pauli and the electrostatic list has two forces,
+// which enter the bead's sum one after the other: the second one goes to *two
+// and the entry says so.
+// FP64: the electrostatic part (an exponential, half the pair's FP64 work) is
+// set aside when it is all there is to the pair: *es gets its charge factor
+// and the pair vector is returned, so that whole warps of such pairs do it
+// later instead of every warp that holds one.
+enum : int { PE_DONE = 0, PE_TWO = 1 };
 template <class FT, int MODE, int FB>
-__device__ __forceinline__ V3<FT> pair_entry(const Dev &d, const TermP &p, const StepSh<FT, FB> &s, int i0,
-                                             const PairRef<FT> &e, const PairPos<FT> &x, Ener<MODE> &en, FT *es) {
+__device__ __forceinline__ int pair_entry(const Dev &d, const TermP &p, const StepSh<FT, FB> &s, int i0,
+                                          const PairRef<FT> &e, const PairPos<FT> &x, Ener<MODE> &en, V3<FT> *f,
+                                          V3<FT> *two, FT *es) {
     constexpr bool MIX = sizeof(FT) == 4;
     const int lo = e.lo, i = i0 + lo, j = e.j, ent = e.ent, slot = e.slot;
     const FT rm = e.rm;
-    if (j < 0) return V3<FT>{FT(0), FT(0), FT(0)};
+    *f = V3<FT>{FT(0), FT(0), FT(0)};
+    if (j < 0) return PE_DONE;
     const int r = s.rep[lo];
     const RepDev &rp = d.rep[r];
     V3<FT> r12;
-    FT qj;
+    FT qj, rn, len;
     if constexpr (MIX) {
         const F2 pa[3] = {{s.p[0][lo + 3], s.p[3][lo + 3]}, {s.p[1][lo + 3], s.p[4][lo + 3]},
                           {s.p[2][lo + 3], s.p[5][lo + 3]}};
         const F2 pb[3] = {{x.h.x, x.l.x}, {x.h.y, x.l.y}, {x.h.z, x.l.z}};
         r12 = pair_vec(rp, s.per[lo] != 0, pa, pb);
         qj = x.h.w;
+        len = norm(r12);
+        rn = 1.0f / len;
     } else {
         const double4_32a pi = make_double4_32a(s.p[0][lo + 3], s.p[1][lo + 3], s.p[2][lo + 3], 0.0);
         r12 = r_uv_p<double>(rp.box, s.per[lo] != 0, pi, x.p);
         qj = x.p.w;
+        const double s2 = fdot(r12, r12);
+        rn = rsqrt(s2);
+        len = mul_(rn, s2);
     }
-    const FT s2 = fdot(r12, r12), rn = rsq(s2);
     FT dV = FT(0);
     if (slot >= 0) {
         // quasi-adiabatic contact: the force part of process_contacts::iter
@@ -542,7 +508,8 @@ __device__ __forceinline__ V3<FT> pair_entry(const Dev &d, const TermP &p, const
         double depth, rmin, rmax;
         qa_lj(p, d.qa, d.qa.ct_type[slot], &depth, &rmin, &rmax);
         FT V_, dq;
-        sink_lj_eval<FT>((FT)depth, (FT)rmin, (FT)rmax, mul_(rn, s2), rn, &V_, &dq);
+        if constexpr (MIX) len = rn * nsq(r12);
+        sink_lj_eval<FT>((FT)depth, (FT)rmin, (FT)rmax, len, rn, &V_, &dq);
         dV = mul_((FT)sat, dq);
         if (MODE == 0 && i < j) en.add(d, r, XMD_TERM_QA, sat * (double)V_);
     } else {
@@ -550,30 +517,49 @@ __device__ __forceinline__ V3<FT> pair_entry(const Dev &d, const TermP &p, const
         // shifted_lj.h:14-21) have one force law, Pauli inside r_excl only
         const bool go = ent == 0;
         const FT w = mul_(rn, rm);
-        if (go || ((ent & NL_PAULI) && FT(1) < w)) {
+        const bool lj = go || ((ent & NL_PAULI) && FT(1) < w);
+        if (lj) {
             const FT depth = go ? tpar<FT>(p.go_depth, p.f.go_depth) : tpar<FT>(p.pauli_depth, p.f.pauli_depth);
-            const FT w2 = mul_(w, w), w3 = mul_(w2, w), s6 = mul_(w3, w3);
-            // s6 - s12 = s6 (1 - s6)
-            dV = mul_(mul_(mul_(FT(12), depth), rn), mul_(s6, add_(FT(1), -s6)));
-            dV = clampv<FT>(dV, FT(-1.0e3), FT(1.0e3));
-            if (MODE == 0 && i < j) {
-                FT V_ = mul_(depth, add_(mul_(s6, add_(s6, FT(-2))), go ? FT(0) : FT(1)));
-                V_ = clampv<FT>(V_, FT(-1.0e3), FT(1.0e3));
-                en.add(d, r, go ? XMD_TERM_GO : XMD_TERM_PAULI, (double)V_);
+            FT V_;
+            if constexpr (MIX) {
+                lj_mixed(depth, rm, rn, go ? 0.0f : 1.0f, &V_, &dV);
+            } else {
+                const double w2 = mul_(w, w), w3 = mul_(w2, w), s6 = mul_(w3, w3);
+                // s6 - s12 = s6 (1 - s6)
+                dV = mul_(mul_(mul_(12.0, depth), rn), mul_(s6, add_(1.0, -s6)));
+                dV = clampv<double>(dV, -1.0e3, 1.0e3);
+                V_ = mul_(depth, add_(mul_(s6, add_(s6, -2.0)), go ? 0.0 : 1.0));
+                V_ = clampv<double>(V_, -1.0e3, 1.0e3);
             }
+            if (MODE == 0 && i < j) en.add(d, r, go ? XMD_TERM_GO : XMD_TERM_PAULI, (double)V_);
         }
         if (ent & NL_ES) {
-            const FT vq = mul_(tpar<FT>(p.es_Vf, p.f.es_Vf), mul_(s.p[MIX ? 6 : 3][lo + 3], qj));
-            if (!MIX && MODE == 1 && dV == FT(0)) {
-                *es = vq;
-                return r12;
-            }
             FT V_;
-            dV = add_(dV, es_factor<FT>(p, vq, s2, rn, &V_));
-            if (MODE == 0 && i < j) en.add(d, r, p.es_rel ? XMD_TERM_REL_ES : XMD_TERM_CONST_ES, (double)V_);
+            if constexpr (MIX) {
+                const float dE = es_mixed(p, len, rn, __fmul_rn(s.p[6][lo + 3], qj), &V_);
+                if (MODE == 0 && i < j) en.add(d, r, p.es_rel ? XMD_TERM_REL_ES : XMD_TERM_CONST_ES, (double)V_);
+                if (lj) {
+                    const V3<float> u = rn * r12;
+                    *f = dV * u;
+                    *two = dE * u;
+                    return PE_TWO;
+                }
+                dV = dE;
+            } else {
+                const double vq = mul_(p.es_Vf, mul_(s.p[3][lo + 3], qj));
+                if (MODE == 1 && dV == 0.0) {
+                    *es = vq;
+                    *f = r12;
+                    return PE_DONE;
+                }
+                dV = add_(dV, es_factor(p, vq, len, rn, &V_));
+                if (MODE == 0 && i < j) en.add(d, r, p.es_rel ? XMD_TERM_REL_ES : XMD_TERM_CONST_ES, V_);
+            }
         }
     }
-    return fscl<FT>(mul_(dV, rn), r12);
+    if constexpr (MIX) *f = dV * (rn * r12);
+    else *f = fscl<double>(mul_(dV, rn), r12);
+    return PE_DONE;
 }
 
 // MODE 0: forces and per-term energies at pos[cur] (eval).
@@ -608,13 +594,12 @@ __device__ __forceinline__ bool force_block(const Dev &d, const TermP &p, int cu
     const int r = t < FBT && i0 + t < N ? d.rep_of[i0 + t] : -1;   // replica of bead t
     const int sc = t & (FB - 1), c = i0 - 2 + sc;                  // the thread's centre (t < 2 FB)
     uint32_t fl = 0;
-    CentreP<FT> cp{FT(0), FT(0), FT(0), FT(0), FT(0)};
+    CentreP<FT> cp{};
     if (t < 2 * FB && sc < NC && c >= 0 && c < N) {
         fl = d.bflags[c];
         if constexpr (MIX) {
             const float4 q = d.bond_f[c];
-            const F2 r0 = split_d(d.teth_r0[c]);
-            cp = CentreP<float>{r0.h, q.y, q.z, q.w, r0.l};
+            cp = CentreP<float>{q.x, q.y, q.z};
         } else {
             if (LPB == 1 || t < FB) { cp.r0 = d.teth_r0[c]; cp.t0 = d.ang_t0[c]; }
             if (LPB == 1 || t >= FB) { const double2 q = d.dih_cs[c]; cp.c0 = q.x; cp.s0 = q.y; }
@@ -748,13 +733,17 @@ __device__ __forceinline__ bool force_block(const Dev &d, const TermP &p, int cu
                 s.g[MEH][k] = e.x.h; s.g[MEH + 1][k] = e.y.h; s.g[MEH + 2][k] = e.z.h;
                 s.g[MEL][k] = e.x.l; s.g[MEL + 1][k] = e.y.l; s.g[MEL + 2][k] = e.z.l;
                 const V3<float> ef{e.x.h, e.y.h, e.z.h};
-                s.g[MRN][k] = rsq(fdot(ef, ef));
+                const float len = norm(ef);
+                s.g[MLEN][k] = len;
+                s.g[MRN][k] = 1.0f / len;
                 if (k > 0) {
                     const V3<FF> x = ff_cross(bond(k - 1), e);
                     s.g[MXH][k] = x.x.h; s.g[MXH + 1][k] = x.y.h; s.g[MXH + 2][k] = x.z.h;
                     s.g[MXL][k] = x.x.l; s.g[MXL + 1][k] = x.y.l; s.g[MXL + 2][k] = x.z.l;
                     const V3<float> xf{x.x.h, x.y.h, x.z.h};
-                    s.g[MRX][k] = rsq(fdot(xf, xf));
+                    const float lx = norm(xf);
+                    s.g[MLX][k] = lx;
+                    s.g[MRX][k] = 1.0f / lx;
                 }
             } else {
                 auto bond = [&](int a) {
@@ -890,11 +879,17 @@ __device__ __forceinline__ bool force_block(const Dev &d, const TermP &p, int cu
             const int nx = grab();
             const PairRef<FT> nref = pair_fetch<FT, FB>(d, p, s, s_q, i0, p0 + nx, nx < pe);
             FT es = FT(0);
+            int kind = PE_DONE;
             if (at < pe) {
-                const V3<FT> f = pair_entry<FT, MODE, FB>(d, p, s, i0, ref, x, en, &es);
+                V3<FT> f, two;
+                kind = pair_entry<FT, MODE, FB>(d, p, s, i0, ref, x, en, &f, &two, &es);
                 s.f[0][at] = f.x; s.f[1][at] = f.y; s.f[2][at] = f.z;
+                if (MIX && kind == PE_TWO) { s.f2[0][at] = two.x; s.f2[1][at] = two.y; s.f2[2][at] = two.z; }
             }
-            if constexpr (!MIX && MODE == 1) {
+            if constexpr (MIX) {
+                const unsigned m = __ballot_sync(FULL, kind == PE_TWO);
+                if (lane == 0) s.two[at >> 5] = m;
+            } else if constexpr (MODE == 1) {
                 const unsigned m = __ballot_sync(FULL, es != FT(0));
                 int to = 0;
                 if (lane == 0 && m) to = atomicAdd(&s.neq, __popc(m));
@@ -919,9 +914,9 @@ __device__ __forceinline__ bool force_block(const Dev &d, const TermP &p, int cu
                 if (k0 + lane < ne) {
                     const int k = s.eq[k0 + lane];
                     const V3<FT> r12{s.f[0][k], s.f[1][k], s.f[2][k]};
-                    const FT s2 = fdot(r12, r12), rn = rsq(s2);
-                    FT V_;
-                    const V3<FT> f = fscl<FT>(mul_(es_factor<FT>(p, s.ew[k0 + lane], s2, rn, &V_), rn), r12);
+                    const double s2 = fdot(r12, r12), rn = rsqrt(s2);
+                    double V_;
+                    const V3<double> f = fscl<double>(mul_(es_factor(p, s.ew[k0 + lane], mul_(s2, rn), rn, &V_), rn), r12);
                     s.f[0][k] = f.x; s.f[1][k] = f.y; s.f[2][k] = f.z;
                 }
             }
@@ -947,8 +942,24 @@ __device__ __forceinline__ bool force_block(const Dev &d, const TermP &p, int cu
                     for (int q = 0; q < 9; ++q) sum_acc(acc[u], v[q]);
                 }
             }
-            const int e1 = min(s.off[b + 1] - p0, FCAP);
-            for (int q = max(s.off[b] - p0, 0); q < e1; ++q) sum_acc(acc[u], s.f[a][q]);
+            const int e0 = max(s.off[b] - p0, 0), e1 = min(s.off[b + 1] - p0, FCAP);
+            bool two = false;
+            if constexpr (MIX) {
+                for (int q = e0 & ~31; q < e1; q += 32) {
+                    unsigned m = s.two[q >> 5];
+                    if (q < e0) m &= ~0u << (e0 - q);
+                    if (q + 32 > e1) m &= ~0u >> (q + 32 - e1);
+                    two |= m != 0u;
+                }
+            }
+            if (!two) {
+                for (int q = e0; q < e1; ++q) sum_acc(acc[u], s.f[a][q]);
+            } else if constexpr (MIX) {
+                for (int q = e0; q < e1; ++q) {
+                    sum_acc(acc[u], s.f[a][q]);
+                    if ((s.two[q >> 5] >> (q & 31)) & 1u) sum_acc(acc[u], s.f2[a][q]);
+                }
+            }
         }
         if (p0 + FCAP >= T) break;
         __syncthreads();
@@ -1031,17 +1042,17 @@ __device__ __forceinline__ bool force_block(const Dev &d, const TermP &p, int cu
             // skin test: norm(box->r_uv(r_, orig_r_)), verify.cpp:12-14, squared;
             // the check takes one square root of the maximum (sqrt is monotone
             // and correctly rounded, so that equals the max of the norms).
-            // Open axes wrap by exactly zero.  The mixed path squares the FP64
-            // difference in FP32.
-            double e = __dsub_rn(o[u], q[0]);
-            if (s.per[b]) {
-                const BoxD &bx = d.rep[s.rep[b]].box;
-                e = __dsub_rn(e, __dmul_rn(bx.cell[a], rint(__dmul_rn(e, bx.cell_inv[a]))));
-            }
+            // Open axes wrap by exactly zero.  The mixed path takes the
+            // displacement from split positions and squares it in FP32.
             if constexpr (MIX) {
-                const float ef = narrow_f(e);
-                s.e[a][b] = __fmul_rn(ef, ef);
+                const RepDev &rp = d.rep[s.rep[b]];
+                s.e[a][b] = mi_axis(split_d(o[u]), split_d(q[0]), rp.Lh[a], rp.Ll[a], rp.Li[a], s.per[b] != 0);
             } else {
+                double e = __dsub_rn(o[u], q[0]);
+                if (s.per[b]) {
+                    const BoxD &bx = d.rep[s.rep[b]].box;
+                    e = __dsub_rn(e, __dmul_rn(bx.cell[a], rint(__dmul_rn(e, bx.cell_inv[a]))));
+                }
                 s.e[a][b] = __dmul_rn(e, e);
             }
         }
@@ -1069,7 +1080,7 @@ __device__ __forceinline__ bool force_block(const Dev &d, const TermP &p, int cu
                 }
                 if constexpr (MIX) {
                     pn.w = widen_f(q);
-                    disp = widen_f(__fadd_rn(__fadd_rn(s.e[0][t], s.e[1][t]), s.e[2][t]));
+                    disp = widen_f(nsq(V3<float>{s.e[0][t], s.e[1][t], s.e[2][t]}));
                 } else {
                     pn.w = q;
                     disp = __dadd_rn(__dadd_rn(s.e[0][t], s.e[1][t]), s.e[2][t]);
