@@ -1,0 +1,46 @@
+"""Contexts with reserved capacity while replicas come and go.  A replica's
+trajectory does not depend on what the context held before it: the same bits as
+alone in a fresh one."""
+import numpy as np
+import pytest
+
+from xmd_gb300 import Engine, synth
+
+pytestmark = pytest.mark.gpu
+
+
+def yaml(prec="fp64", build="auto"):
+    return synth.yaml_for("c4", prec) + f"  nl build: {build}\n"
+
+
+def system(n, seed, start="saw"):
+    return synth.make_system([n], seed, temperature=0.45, start=start)
+
+
+def run_alone(y, s, steps):
+    with Engine(y) as e:
+        e.reserve(2000, 4, 16000)
+        rep = e.add_system(s)
+        e.step(steps)
+        return e.get_history(rep)[0], e.stats()["rebuilds"]
+
+
+@pytest.mark.parametrize("prec", ["fp64", "mixed"])
+@pytest.mark.parametrize("build", ["auto", "cell", "tile"])
+@pytest.mark.parametrize("emptied", [False, True])
+def test_steps_of_an_empty_context(prec, build, emptied):
+    # steps while nothing is placed (before the first replica, or after the last
+    # one left), then a run over several list rebuilds with the same graphs
+    y, s = yaml(prec, build), system(120, 6)
+    want, rebuilds = run_alone(y, s, 96)
+    assert rebuilds >= 3
+    with Engine(y) as e:
+        e.reserve(2000, 4, 16000)
+        if emptied:
+            k = e.add_system(system(70, 7))
+            e.step(2)
+            e.remove_replica(k)
+        e.step(96)
+        rep = e.add_system(s)
+        e.step(96)
+        assert np.array_equal(e.get_history(rep)[0], want)

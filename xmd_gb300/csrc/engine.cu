@@ -3469,7 +3469,9 @@ void Engine::add_rebuild_nodes(cudaGraph_t body, int cn) {
     void *a3[] = {&d};
     int one = 1;
     void *a4[] = {&d, &tp, &cn, &one};
-    if (live_cell) {
+    // (by the context's capacity, not by what is placed now: the graph is kept
+    // while replicas come and go, and a kernel without a flagged replica returns)
+    if (cap.cells > 0) {
         cudaKernelNodeParams k1{}, k2{}, kc{}, ks{}, kx{}, kf{};
         k1.func = (void *)k_cells;
         const unsigned gb = (unsigned)((d.N + 255) / 256);
