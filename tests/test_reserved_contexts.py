@@ -1,6 +1,8 @@
 """Contexts with reserved capacity while replicas come and go.  A replica's
 trajectory does not depend on what the context held before it: the same bits as
 alone in a fresh one."""
+import time
+
 import numpy as np
 import pytest
 
@@ -44,3 +46,33 @@ def test_steps_of_an_empty_context(prec, build, emptied):
         rep = e.add_system(s)
         e.step(96)
         assert np.array_equal(e.get_history(rep)[0], want)
+
+
+@pytest.mark.parametrize("prec", ["fp64", "mixed"])
+def test_finished_replicas_cost_no_step(prec):
+    # once every replica has taken its steps, a step kernel only carries the
+    # positions over: 48 chains of 500 beads, where a step's arithmetic is most
+    # of its time (well over half in both precisions)
+    one = system(500, 8, "native")
+    with Engine(yaml(prec)) as e:
+        for k in range(48):
+            e.add_system(one, seed=k + 1)
+
+        def seconds():
+            best = 1e9
+            for _ in range(5):
+                t0 = time.perf_counter()
+                e.step(64)
+                best = min(best, time.perf_counter() - t0)
+            return best
+
+        e.step(64)
+        running = seconds()
+        for k in range(48):
+            e.set_steps(k, 0)
+        before = [e.get_history(k)[0] for k in (0, 47)]
+        e.step(64)
+        done = seconds()
+        for k, y in zip((0, 47), before):
+            assert np.array_equal(e.get_history(k)[0], y)
+    assert done < 0.7 * running, (done, running)

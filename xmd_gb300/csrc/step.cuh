@@ -623,7 +623,9 @@ __device__ __forceinline__ bool force_block(const Dev &d, const TermP &p, int cu
     uint64_t st0 = 0;
     if (draws) st0 = d.rng[i0 + bn];
     int ng = 0, nl = 0, nq = 0;
+    long long left = -1;
     if (t < FBT && i0 + t < N) {
+        if (MODE == 1) left = d.rep[max(r, 0)].steps_left;
         nl = d.nl_cnt[i0 + t];
         if (p.on[XMD_TERM_GO]) ng = d.go_cnt[i0 + t];
         if (qa) nq = min(d.qa.ref_cnt[i0 + t], QA_REF_CAP);
@@ -656,9 +658,12 @@ __device__ __forceinline__ bool force_block(const Dev &d, const TermP &p, int cu
             s.p[0][k] = q.x; s.p[1][k] = q.y; s.p[2][k] = q.z; s.p[3][k] = q.w;
         }
     }
+    // 1: the bead steps, 0: its replica has taken its steps (or is frozen) and
+    // keeps its state, -1: free slot
+    const int state = r < 0 ? -1 : left != 0;
     int scan = 0, cnt = 0;
     if (t < FB) {
-        if (r < 0) ng = nl = nq = 0;
+        if (state != 1) ng = nl = nq = 0;
         scan = cnt = ng + nl + nq;
 #pragma unroll
         for (int o_ = 1; o_ < 32; o_ <<= 1) {
@@ -668,22 +673,28 @@ __device__ __forceinline__ bool force_block(const Dev &d, const TermP &p, int cu
         if (lane == 31) s.ws[t >> 5] = scan;
         s.ng[t] = ng; s.nl[t] = nl; s.nat0[t] = nat0; s.rep[t] = r;
         s.ss0[t] = ss0; s.ss1[t] = r >= 0 ? ss1 : ss0;
+        s.state[t] = state;
     }
     if (t == 0) s.next = s.neq = s.next_es = 0;
-    if (!__syncthreads_or(r >= 0)) return true;   // no bead slot of the block is in use
+    if (!__syncthreads_or(state == 1)) {   // no bead of the block steps
+        if (MODE == 1 && state == 0) {
+            d.pos[cur ^ 1][i0 + t] = d.pos[cur][i0 + t];
+            if (MIX || qa) {
+                d.spl[cur ^ 1][2 * (size_t)(i0 + t)] = d.spl[cur][2 * (size_t)(i0 + t)];
+                d.spl[cur ^ 1][2 * (size_t)(i0 + t) + 1] = d.spl[cur][2 * (size_t)(i0 + t) + 1];
+            }
+        }
+        return true;
+    }
     int T = 0;
 #pragma unroll
     for (int k = 0; k < FB / 32; ++k) T += s.ws[k];
-    // a replica that has taken its steps keeps its state (its word is stored
-    // when it is needed, not waited for here)
-    int state = r >= 0 ? 1 : -1;
     if (t < FB) {
         int base = 0;
         for (int k = 0; k < (t >> 5); ++k) base += s.ws[k];
         s.off[t] = base + scan - cnt;
         if (t == FB - 1) s.off[FB] = T;
         s.per[t] = r >= 0 ? d.rep[r].per_any : 0;
-        if (MODE == 1 && r >= 0 && d.rep[r].steps_left == 0) state = 0;
     }
     __syncthreads();
     if (qa) {
@@ -796,7 +807,7 @@ __device__ __forceinline__ bool force_block(const Dev &d, const TermP &p, int cu
                 s.c[12 + 3 * k][sc] = q[k].x; s.c[13 + 3 * k][sc] = q[k].y; s.c[14 + 3 * k][sc] = q[k].z;
             }
         }
-        if (MODE == 1 && qa && t < FBT && r >= 0) {
+        if (MODE == 1 && qa && t < FBT && state == 1) {
             // n and h at this step's positions (precompute_nh.cpp:12-20) to
             // FP32 accuracy, for the sift's FP32 decisions (which recompute
             // them in FP64 near a threshold)
@@ -825,7 +836,6 @@ __device__ __forceinline__ bool force_block(const Dev &d, const TermP &p, int cu
             d.qa.nh[2 * (size_t)i] = make_float4(n.x, n.y, n.z, 0.0f);
             d.qa.nh[2 * (size_t)i + 1] = make_float4(h.x, h.y, h.z, 0.0f);
         }
-        if (t < FB) s.state[t] = state;
     }
 
     // ---- E: pair entries, FCAP at a time; between the passes every (axis,
