@@ -469,7 +469,8 @@ template <class FT> __device__ __forceinline__ PairPos<FT> pair_pos(const Dev &d
 // set aside when it is all there is to the pair: *es gets its charge factor
 // and the pair vector is returned, so that whole warps of such pairs do it
 // later instead of every warp that holds one.
-enum : int { PE_DONE = 0, PE_TWO = 1 };
+// Returns what became of it.
+enum : int { PE_DONE = 0, PE_TWO = 1, PE_ES = 2 };
 template <class FT, int MODE, int FB>
 __device__ __forceinline__ int pair_entry(const Dev &d, const TermP &p, const StepSh<FT, FB> &s, int i0,
                                           const PairRef<FT> &e, const PairPos<FT> &x, Ener<MODE> &en, V3<FT> *f,
@@ -550,7 +551,7 @@ __device__ __forceinline__ int pair_entry(const Dev &d, const TermP &p, const St
                 if (MODE == 1 && dV == 0.0) {
                     *es = vq;
                     *f = r12;
-                    return PE_DONE;
+                    return PE_ES;
                 }
                 dV = add_(dV, es_factor(p, vq, len, rn, &V_));
                 if (MODE == 0 && i < j) en.add(d, r, p.es_rel ? XMD_TERM_REL_ES : XMD_TERM_CONST_ES, V_);
@@ -900,11 +901,11 @@ __device__ __forceinline__ bool force_block(const Dev &d, const TermP &p, int cu
                 const unsigned m = __ballot_sync(FULL, kind == PE_TWO);
                 if (lane == 0) s.two[at >> 5] = m;
             } else if constexpr (MODE == 1) {
-                const unsigned m = __ballot_sync(FULL, es != FT(0));
+                const unsigned m = __ballot_sync(FULL, kind == PE_ES);
                 int to = 0;
                 if (lane == 0 && m) to = atomicAdd(&s.neq, __popc(m));
                 to = __shfl_sync(FULL, to, 0) + __popc(m & ((1u << lane) - 1u));
-                if (es != FT(0)) {
+                if (kind == PE_ES) {
                     s.eq[to] = at;
                     s.ew[to] = es;
                 }
