@@ -6,7 +6,7 @@ import time
 import numpy as np
 import pytest
 
-from xmd_gb300 import Engine, synth
+from xmd_gb300 import Engine, Server, synth
 
 pytestmark = pytest.mark.gpu
 
@@ -76,3 +76,13 @@ def test_finished_replicas_cost_no_step(prec):
         for k, y in zip((0, 47), before):
             assert np.array_equal(e.get_history(k)[0], y)
     assert done < 0.7 * running, (done, running)
+
+
+def test_split_positions_only_where_they_are_read():
+    # two float4 per bead and buffer hold the mixed path's split positions (and
+    # the contacts' sift's): an FP64 context without contacts has none
+    per_bead = {}
+    for prec in ("fp64", "mixed"):
+        with Server(yaml(prec), hbm_budget=64 << 20, max_beads=4000) as srv:
+            per_bead[prec] = srv.stats()["bytes_per_bead"]
+    assert per_bead["mixed"] - per_bead["fp64"] == pytest.approx(64.0, abs=0.5)

@@ -2244,8 +2244,8 @@ void Engine::allocate() {
     const size_t NN = (size_t)std::max(1, cap.nat);
     d.pos[0] = (double4_32a *)dalloc(sizeof(double4_32a) * N);
     d.pos[1] = (double4_32a *)dalloc(sizeof(double4_32a) * N);
-    d.spl[0] = (float4 *)dalloc(2 * sizeof(float4) * N);
-    d.spl[1] = (float4 *)dalloc(2 * sizeof(float4) * N);
+    if (p.precision == XMD_PREC_MIXED || p.on[XMD_TERM_QA])   // (nothing else reads split positions)
+        for (auto &x : d.spl) x = (float4 *)dalloc(2 * sizeof(float4) * N);
     d.yh = (double *)dalloc(sizeof(double) * 15 * (size_t)N);
     d.orig = (double4_32a *)dalloc(sizeof(double4_32a) * N);
     d.F = (double *)dalloc(sizeof(double) * 3 * (size_t)N);
