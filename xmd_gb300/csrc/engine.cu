@@ -612,8 +612,8 @@ __device__ __forceinline__ float f_of_key(unsigned k) { return __uint_as_float((
 // only the origin of the cells and of the FP32 coordinates, and coordinates
 // below it fall into cell 0); the last block then sets the grids and FP32
 // bands of the flagged replicas.  One block per replica took 138 us for one of
-// 54,744 beads.
-__global__ void __launch_bounds__(256) k_cells(Dev d, int cur) {
+// beads.  `count`: the launches of the pass, for the statistics.
+__global__ void __launch_bounds__(256) k_cells(Dev d, int cur, int count) {
     const int i = blockIdx.x * 256 + threadIdx.x;
     __shared__ int last_s;
     const int r = i < d.N ? d.rep_of[i] : -1;
@@ -643,7 +643,7 @@ __global__ void __launch_bounds__(256) k_cells(Dev d, int cur) {
     __threadfence();
     if (threadIdx.x == 0) {
         d.ctr[3] = 0ull;
-        atomicAdd(d.ctr, 1ull);
+        atomicAdd(d.ctr, (unsigned long long)count);
     }
     for (int k = threadIdx.x; k < d.R; k += 256) {
         if (!cell_flagged(d, k)) continue;
@@ -1457,12 +1457,12 @@ __device__ __forceinline__ void tl_chunk(const Dev &d, const TermP &p, int cur, 
     }
 }
 
-// `count`: a pass with work adds to the pass counter (launches that run
-// every step, with or without work, are counted where they are issued)
+// `count`: the launches of a pass that has no cell build (0: counted elsewhere;
+// launches that run every step, with or without work, where they are issued)
 __global__ void __launch_bounds__(TL_THREADS, 4) k_nl_tile(Dev d, TermP p, int cur, int count) {
     step_order();
     const int nw = *d.nwork;
-    if (count && blockIdx.x == 0 && threadIdx.x == 0 && !d.any_cell && nw > 0) atomicAdd(d.ctr, 1ull);
+    if (count && blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(d.ctr, (unsigned long long)count);
     for (int w = blockIdx.x; w < nw; w += gridDim.x) {
         tl_chunk(d, p, cur, d.chunks[d.work[w]]);
         __syncthreads();   // the next chunk overwrites the shared tile
@@ -1744,7 +1744,7 @@ void Engine::remove_replica(int rep) {
         if (r.chunk_len) CK(cudaMemsetAsync(d.chunks + r.chunk_off, 0xff, sizeof(int2) * r.chunk_len, stream));
         CK(cudaMemsetAsync(d.rep + rep, 0, sizeof(RepDev), stream));
         CK(cudaStreamSynchronize(stream));
-        if (r.cell_len) count_cell(-1);
+        if (r.cell_len) --live_cell;
         for (int i = 0; i < n; ++i) owner_h[b + i] = -1;
         a_beads.release(b, n);
         a_nat.release(r.nat_off, r.nat_len);
@@ -1788,14 +1788,6 @@ void Engine::stage(int rep) {
     staged_reps.push_back(std::move(st));
 }
 
-// replicas above the tile build's size come and go in a dynamic context: while
-// none is placed, its steps run in plain graphs (no conditional node, no
-// separate skin check: 12 requests of 1-8 chains, 256 steps, 14.0 -> 11.1 ms)
-void Engine::count_cell(int change) {
-    live_cell += change;
-    d.any_cell = live_cell > 0;
-}
-
 void Engine::activate_staged() {
     if (staged_reps.empty()) return;
     use_device();
@@ -1808,7 +1800,7 @@ void Engine::activate_staged() {
         for (int i = 0; i < r.n; ++i) owner_h[r.begin + i] = st.k;
         r.staged = false;
         r.placed = true;
-        if (r.cell_len) count_cell(1);
+        if (r.cell_len) ++live_cell;
     }
     staged_reps.clear();
 }
@@ -2376,7 +2368,6 @@ void Engine::allocate() {
     a_ct.init(cap.ct);
     any_tile = cap.chunks > 0;
     live_cell = 0;
-    d.any_cell = 0;
     tile_smem = 0;
     for (auto &r : reps)
         if (r.in_use && r.n <= TILE_MAX) tile_smem = std::max(tile_smem, tile_bytes(r.n));
@@ -2799,7 +2790,7 @@ void Engine::place(int k, Staged *st) {
     }
     for (int i = 0; i < n; ++i) owner_h[b + i] = k;
     r.placed = true;
-    if (r.cell_len) count_cell(1);
+    if (r.cell_len) ++live_cell;
     upload_state(k);
 }
 
@@ -3184,14 +3175,14 @@ void Engine::launch_rebuild() {
     if (timing) record(ev_rebuild, n_ev_rebuild);
     if (live_cell) {
         const int gb = (d.N + 255) / 256;
-        k_cells<<<gb, 256, 0, stream>>>(d, cur);
+        k_cells<<<gb, 256, 0, stream>>>(d, cur, pass_launches(true));
         k_cell_count<<<gb, 256, 0, stream>>>(d, cur);
         k_cell_scan<<<(d.ncells + CELL_SCAN - 1) / CELL_SCAN, 256, 0, stream>>>(d);
         k_cell_scatter<<<gb, 256, 0, stream>>>(d);
         k_cell_finish<<<2 * gb, 256, 0, stream>>>(d, cur);
         k_nl_cells<<<(d.N + NC_WARPS - 1) / NC_WARPS, NC_WARPS * 32, 0, stream>>>(d, tp, cur);
     }
-    if (any_tile) k_nl_tile<<<tile_grid, TL_THREADS, tile_smem, stream>>>(d, tp, cur, 1);
+    if (any_tile) k_nl_tile<<<tile_grid, TL_THREADS, tile_smem, stream>>>(d, tp, cur, live_cell ? 0 : pass_launches(false));
     if (d.qa_on) {
         k_qa_fp_scan<<<d.qa.nbchunk, QA_BCHUNK, 0, stream>>>(d);
         k_qa_fp_fill<<<dim3(d.qa.nbchunk, QA_FG), 256, 0, stream>>>(d);
@@ -3467,17 +3458,19 @@ void Engine::add_rebuild_nodes(cudaGraph_t body, int cn) {
     void *a1[] = {&d, &cn};
     void *a2[] = {&d, &tp, &cn};
     void *a3[] = {&d};
-    int one = 1;
-    void *a4[] = {&d, &tp, &cn, &one};
+    const bool cells = cap.cells > 0;
+    int in_cells = pass_launches(cells), in_tile = cells ? 0 : in_cells;
+    void *ac[] = {&d, &cn, &in_cells};
+    void *a4[] = {&d, &tp, &cn, &in_tile};
     // (by the context's capacity, not by what is placed now: the graph is kept
     // while replicas come and go, and a kernel without a flagged replica returns)
-    if (cap.cells > 0) {
+    if (cells) {
         cudaKernelNodeParams k1{}, k2{}, kc{}, ks{}, kx{}, kf{};
         k1.func = (void *)k_cells;
         const unsigned gb = (unsigned)((d.N + 255) / 256);
         k1.gridDim = dim3(gb);
         k1.blockDim = dim3(256);
-        k1.kernelParams = a1;
+        k1.kernelParams = ac;
         add(k1);
         kc.func = (void *)k_cell_count;
         kc.gridDim = dim3(gb);
@@ -3680,10 +3673,10 @@ void Engine::stats(int64_t *out) {
     std::vector<RepDev> rd(d.R);
     CK(cudaMemcpyAsync(rd.data(), d.rep, sizeof(RepDev) * d.R, cudaMemcpyDeviceToHost, stream));
     CK(cudaStreamSynchronize(stream));
-    unsigned long long passes = 0;
-    CK(cudaMemcpyAsync(&passes, d.ctr, sizeof(passes), cudaMemcpyDeviceToHost, stream));
+    unsigned long long in_passes = 0;   // launches of the rebuild passes so far
+    CK(cudaMemcpyAsync(&in_passes, d.ctr, sizeof(in_passes), cudaMemcpyDeviceToHost, stream));
     CK(cudaStreamSynchronize(stream));
-    out[XMD_STAT_LAUNCHES] = launches + (int64_t)((live_cell ? 6 : 0) + (any_tile ? 1 : 0) + (d.qa_on ? 4 : 0)) * (int64_t)passes;
+    out[XMD_STAT_LAUNCHES] = launches + (int64_t)in_passes;
     for (int i = 0; i < d.N; ++i)
         if (owner_h[i] >= 0) out[XMD_STAT_NL_ENTRIES] += cnt[i];
     for (int k = 0; k < nn; ++k) out[XMD_STAT_GO_ACTIVE] += on[k];
