@@ -608,10 +608,12 @@ __device__ __forceinline__ unsigned f_key(float x) {
 }
 __device__ __forceinline__ float f_of_key(unsigned k) { return __uint_as_float((k >> 31) ? k & 0x7fffffffu : ~k); }
 
-// Bounding boxes along open axes, over the whole grid (in FP32: the minimum is
-// only the origin of the cells and of the FP32 coordinates, and coordinates
-// below it fall into cell 0); the last block then sets the grids and FP32
-// bands of the flagged replicas.  One block per replica took 138 us for one of
+// Bounding boxes along open axes, over the whole grid (in FP32, rounded
+// outwards: no coordinate lies below the minimum, which is the origin of the
+// cells and of the FP32 coordinates, and none is larger than the span that
+// their error bound is taken from, however far from the origin the replica
+// lies); the last block then sets the grids and FP32 bands of the flagged
+// replicas.  One block per replica took 138 us for one of
 // beads.  `count`: the launches of the pass, for the statistics.
 __global__ void __launch_bounds__(256) k_cells(Dev d, int cur, int count) {
     const int i = blockIdx.x * 256 + threadIdx.x;
@@ -623,10 +625,11 @@ __global__ void __launch_bounds__(256) k_cells(Dev d, int cur, int count) {
         const double4_32a q = d.pos[cur][i];
         const unsigned m = __match_any_sync(act, r);
         const bool lead = (threadIdx.x & 31) == __ffs(m) - 1;
-        const float x[3] = {narrow_f(q.x), narrow_f(q.y), narrow_f(q.z)};
+        const double x[3] = {q.x, q.y, q.z};
 #pragma unroll
         for (int a = 0; a < 3; ++a) {
-            const unsigned lo = __reduce_min_sync(m, f_key(x[a])), hi = __reduce_max_sync(m, f_key(x[a]));
+            const unsigned lo = __reduce_min_sync(m, f_key(__double2float_rd(x[a])));
+            const unsigned hi = __reduce_max_sync(m, f_key(__double2float_ru(x[a])));
             if (lead) {
                 atomicMin(&d.rep[r].lo_key[a], lo);
                 atomicMax(&d.rep[r].hi_key[a], hi);
