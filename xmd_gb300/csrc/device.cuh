@@ -40,11 +40,8 @@ template <class T> __device__ __forceinline__ V3<T> cross(V3<T> a, V3<T> b) {
 __device__ __forceinline__ double sqrt_(double x) { return sqrt(x); }
 __device__ __forceinline__ float sqrt_(float x) { return sqrtf(x); }
 __device__ __forceinline__ double acos_(double x) { return acos(x); }
-__device__ __forceinline__ float acos_(float x) { return acosf(x); }
 __device__ __forceinline__ double exp_(double x) { return exp(x); }
 __device__ __forceinline__ float exp_(float x) { return expf(x); }
-__device__ __forceinline__ void sincos_(double x, double *s, double *c) { sincos(x, s, c); }
-__device__ __forceinline__ void sincos_(float x, float *s, float *c) { sincosf(x, s, c); }
 
 template <class T> __device__ __forceinline__ T norm(V3<T> a) { return sqrt_(nsq(a)); }
 template <class T> __device__ __forceinline__ T ninv(V3<T> a) { return T(1) / norm(a); }
@@ -86,16 +83,13 @@ __device__ __forceinline__ bool operator<(DN a, DN b) { return a.v < b.v; }
 __device__ __forceinline__ bool operator>(DN a, DN b) { return a.v > b.v; }
 __device__ __forceinline__ DN sqrt_(DN x) { return DN(__dsqrt_rn(x.v)); }
 __device__ __forceinline__ DN acos_(DN x) { return DN(acos(x.v)); }
-__device__ __forceinline__ DN exp_(DN x) { return DN(exp(x.v)); }
 __device__ __forceinline__ DN sin(DN x) { return DN(::sin(x.v)); }
 __device__ __forceinline__ DN dn_cos(DN x) { return DN(::cos(x.v)); }
 __device__ __forceinline__ DN dn_fabs(DN x) { return DN(::fabs(x.v)); }
 __device__ __forceinline__ DN dn_rint(DN x) { return DN(::rint(x.v)); }
-__device__ __forceinline__ void sincos_(DN x, DN *s, DN *c) { sincos(x.v, &s->v, &c->v); }
 template <> __host__ __device__ __forceinline__ DN tpar<DN>(double d, float) { return DN(d); }
 __device__ __forceinline__ float ldg_(const float *p) { return __ldg(p); }
 __device__ __forceinline__ double ldg_(const double *p) { return __ldg(p); }
-__device__ __forceinline__ DN ldg_(const DN *p) { return DN(__ldg(&p->v)); }
 template <class T> __device__ __forceinline__ V3<double> v3d(V3<T> a) {
     return V3<double>{(double)a.x, (double)a.y, (double)a.z};
 }
@@ -220,14 +214,6 @@ __device__ __forceinline__ FF ff_dot(const V3<FF> &a, const V3<FF> &b) {
 // position of a bead split per axis (mixed path)
 struct P2 { F2 x, y, z; };
 __device__ __forceinline__ P2 split_p(double4_32a p) { return P2{split_d(p.x), split_d(p.y), split_d(p.z)}; }
-
-// FP64 difference, narrowed to FT
-template <class T>
-__device__ __forceinline__ V3<T> diff(double4_32a u, double4_32a w) {
-    return V3<T>{T(w.x - u.x), T(w.y - u.y), T(w.z - u.z)};
-}
-
-
 
 // box::r_uv: box.h:36-49.  The wrap is done in FP64 before narrowing.
 template <class T>
@@ -540,14 +526,6 @@ __device__ __forceinline__ void noise3m(uint64_t st, float *nx, float *ny, float
     const float r2 = sqrtf(-2.0f * __logf(u3));
     *nz = r2 * __cosf(two_pi * u4 - 3.141592653589793f);
 }
-// 64x64 GF(2) matrix (columns) times state: the xorshift jump-ahead
-__device__ __forceinline__ uint64_t gf2_apply(const uint64_t *__restrict__ col, uint64_t x) {
-    uint64_t y = 0;
-#pragma unroll 16
-    for (int k = 0; k < 64; ++k) y ^= col[k] & (0ull - ((x >> k) & 1ull));
-    return y;
-}
-
 // ---- pair geometry of the mixed path ------------------------------------------
 // Pair vectors from split positions in FP32 (the minimum image subtracted in
 // float-float), with no FP64 instruction per pair.
@@ -593,9 +571,6 @@ template <> struct PairGeo<float> {
                          mi_axis(u.z, w.z, Lh[2], Ll[2], Li[2], per)};
     }
     __device__ __forceinline__ V3<float> to(double4_32a pj) const { return diff2(si, split_p(pj)); }
-    __device__ __forceinline__ V3<float> between(double4_32a a, double4_32a b) const {
-        return diff2(split_p(a), split_p(b));
-    }
 };
 
 }  // namespace xmdg

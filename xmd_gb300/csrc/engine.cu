@@ -491,9 +491,9 @@ __global__ void __launch_bounds__(1024) k_qa_refree(Dev d, double dt, int check)
 // while the gate is closed; FUSE_GATE, no decision (a later kernel of the step
 // takes it), and the kernel returns at once while the gate is closed.  The
 // kernel holds no device-side graph call, so profilers see it in graphs.
-// resident blocks the register allocation leaves room for: 16 warps per SM
-// (at most 128 registers) with one or two threads per bead, 28 (at most 73)
-// with four
+// Resident blocks that the register allocation leaves room for: at most 64
+// registers a thread in mixed precision (32 warps per SM), 80 in FP64 (25 warps),
+// whatever the threads per slot
 template <class FT, int FB, int LPB> constexpr int force_min_blocks() {
     return 65536 / (FB * LPB * (sizeof(FT) == 4 ? 64 : 80)) > 0 ? 65536 / (FB * LPB * (sizeof(FT) == 4 ? 64 : 80)) : 1;
 }

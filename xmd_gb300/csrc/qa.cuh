@@ -90,22 +90,12 @@ __device__ __forceinline__ void qa_nh(double4_32a rp, double4_32a rc, double4_32
     *n = d3unit(d3sub(v2, v1));
     *h = d3unit(d3cross(v2, v1));
 }
-// the same to FP32 accuracy: bond vectors, their difference and their cross
-// product in float-float from split positions (within ~2^-44 of the exact
-// values however straight the chain), normalised in FP32; each component
-// is within ~3e-7 of the FP64 unit vector's
+// a unit vector to FP32 accuracy (n and h of the step kernel, from the bonds'
+// difference and cross product it holds in float-float or FP64: each component
+// within ~3e-7 of the FP64 unit vector's, however straight the chain)
 __device__ __forceinline__ V3<float> unit_f(V3<float> a) {
     const float s = 1.0f / sqrtf(a.x * a.x + a.y * a.y + a.z * a.z);
     return V3<float>{a.x * s, a.y * s, a.z * s};
-}
-__device__ __forceinline__ void qa_nh_f(double4_32a rp, double4_32a rc, double4_32a rn, V3<float> *n, V3<float> *h) {
-    const P2 sp = split_p(rp), sc = split_p(rc), sn = split_p(rn);
-    const V3<FF> v1{ff_diff(sp.x, sc.x), ff_diff(sp.y, sc.y), ff_diff(sp.z, sc.z)};
-    const V3<FF> v2{ff_diff(sc.x, sn.x), ff_diff(sc.y, sn.y), ff_diff(sc.z, sn.z)};
-    const V3<FF> dv{ff_sub(v2.x, v1.x), ff_sub(v2.y, v1.y), ff_sub(v2.z, v1.z)};
-    const V3<FF> x = ff_cross(v2, v1);
-    *n = unit_f(V3<float>{dv.x.h, dv.y.h, dv.z.h});
-    *h = unit_f(V3<float>{x.x.h, x.y.h, x.z.h});
 }
 
 // ---- block-wide helpers (blockDim.x == 1024) ------------------------------------
@@ -143,8 +133,8 @@ __device__ __forceinline__ int block_exscan(int v, int *out, int *s_warp) {
 //
 // The decisions are taken in FP32 where they are certain: the pair vector
 // from split positions (float-float differences, error <= 2^-24 of each
-// component), its unit vector, and n, h to FP32 accuracy (qa_nh_f, written by
-// the step kernel); every dot product of unit vectors is then within 2e-6 of
+// component), its unit vector, and n, h to FP32 accuracy (written by the step
+// kernel); every dot product of unit vectors is then within 2e-6 of
 // its FP64 value and the squared distance within 1e-6 of it (relative).  A pair whose value lies
 // within QA_BAND of any threshold it is tested against is decided again from
 // scratch in FP64 with explicit rounding (the reference's operations), so the

@@ -70,11 +70,12 @@ template <class T> __device__ __forceinline__ V3<T> fscl(T s, V3<T> a) {
 }
 
 // ---- noise of the FP64 path -------------------------------------------------------
-// Box-Muller on four 32-bit draws k / 2^32 as noise3 forms them
-// (rand_gen.h:22-58, lang_pc.cpp:15-16), with the reductions done on the
+// Box-Muller on the bead's next four 32-bit draws k / 2^32, in the order radius
+// and angle of x and y, radius and angle of z (normal_x2 then normal,
+// rand_gen.h:22-58, lang_pc.cpp:15-16), with the reductions done on the
 // integer draws: no FP64 conversion, argument reduction or special-case path
 // (84 FP64 instructions a bead; 150 with the library's log, sincos and cos).
-// Draws and draw order are noise3's, results within a few 2^-53.
+// Results are within a few 2^-53 of the library's.
 __device__ __forceinline__ double int_to_d(int k) {   // exact, one addition
     return __dsub_rn(__hiloint2double(0x43300000, (int)((unsigned)k ^ 0x80000000u)), 4503601774854144.0);
 }
