@@ -1553,6 +1553,10 @@ void Engine::launch_force(int mode, int c) {
 
 void Engine::split_positions() {
     if (params.precision != XMD_PREC_MIXED && !d.qa_on) return;
+    // a context that was FP64 until now allocates them here (an allocation
+    // enqueues the array's clearing on the step stream)
+    for (auto &x : d.spl)
+        if (!x) x = (float4 *)dalloc(2 * sizeof(float4) * (size_t)d.N);
     k_split<<<(d.N + 255) / 256, 256, 0, stream>>>(d, cur);
     ++launches;
 }
@@ -2239,7 +2243,9 @@ void Engine::allocate() {
     const size_t NN = (size_t)std::max(1, cap.nat);
     d.pos[0] = (double4_32a *)dalloc(sizeof(double4_32a) * N);
     d.pos[1] = (double4_32a *)dalloc(sizeof(double4_32a) * N);
-    if (p.precision == XMD_PREC_MIXED || p.on[XMD_TERM_QA])   // (nothing else reads split positions)
+    // nothing else reads split positions (a later change of the precision:
+    // split_positions)
+    if (p.precision == XMD_PREC_MIXED || p.on[XMD_TERM_QA])
         for (auto &x : d.spl) x = (float4 *)dalloc(2 * sizeof(float4) * N);
     d.yh = (double *)dalloc(sizeof(double) * 15 * (size_t)N);
     d.orig = (double4_32a *)dalloc(sizeof(double4_32a) * N);
