@@ -325,9 +325,13 @@ int xmd_gpu_set_kernel_timing(xmd_gpu_ctx *ctx, int on);
 
 /* ---- launch shapes and the autotuner ------------------------------------------
  * No counterpart in the reference (its OpenMP loop has no launch shape).
- * shape[4] = {beads per step-kernel block (32, 64, 128), resident tile-build
- * blocks per SM (0 = as many as fit), steps per captured graph (8, 16, 32, 64),
- * threads per bead in the step kernel (1, 2, 4)}.
+ * shape[4] = {bead slots per step-kernel block (32, 64, 128; five of them hold
+ * neighbours' beads), resident tile-build blocks per SM (0 = as many as fit),
+ * steps per captured graph (8, 16, 32, 64), threads per slot in the step kernel
+ * (1, 2, 4)}.  (32, 4) runs with eight threads per slot in contexts so small that
+ * every block is resident at once; the shape still reads 4.  Without a shape
+ * set, slots per block follow the context's capacity: 32, or 64 beyond 16
+ * blocks of 32 slots per SM.
  * Results never depend on the shape.  xmd_gpu_autotune times every candidate
  * on a clone of the context (same replicas, same starting state; the
  * context's own state is untouched), keeps the fastest and returns it with

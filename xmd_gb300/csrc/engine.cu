@@ -613,8 +613,8 @@ __device__ __forceinline__ float f_of_key(unsigned k) { return __uint_as_float((
 // cells and of the FP32 coordinates, and none is larger than the span that
 // their error bound is taken from, however far from the origin the replica
 // lies); the last block then sets the grids and FP32 bands of the flagged
-// replicas.  One block per replica took 138 us for one of
-// beads.  `count`: the launches of the pass, for the statistics.
+// replicas.  One block per replica took 138 us for one of 54,744 beads.
+// `count`: the launches of the pass, for the statistics.
 __global__ void __launch_bounds__(256) k_cells(Dev d, int cur, int count) {
     const int i = blockIdx.x * 256 + threadIdx.x;
     __shared__ int last_s;
@@ -1512,9 +1512,9 @@ static void *force_kernel(bool mixed, int mode, int fb, int lpb) {
 // blocks so few that a block's own latency is the kernel's time (mixed: all
 // resident at once, four per SM; FP64: one per SM, beyond which the FP64 pipe
 // binds), eight threads per slot instead of four: the pair entries go to twice
-// the warps.  us per MD step, four -> eight: 61 native chains mixed 31 -> 23,
-// 16 x 500 mixed 22 -> 18, 2,992 beads with contacts FP64 67 -> 47; 16 x 500
-// FP64 (297 blocks) 39 -> 44.
+// the warps.  us per MD step, four -> eight: 61 native chains mixed 26.8 -> 21.5,
+// 16 x 500 mixed 20.0 -> 17.2, 67 short chains with contacts FP64 52 -> 47;
+// 16 x 500 FP64 (297 blocks) 39 -> 44.
 Engine::ForceShape Engine::force_shape() const {
     const bool mixed = params.precision == XMD_PREC_MIXED;
     if (tune.fb == 32 && tune.lpb == 4 && force_blocks(d.N, 32) <= (mixed ? 4 : 1) * tile_sms) return ForceShape{32, 8};
@@ -1523,9 +1523,10 @@ Engine::ForceShape Engine::force_shape() const {
 // The shape where none was set: 32-slot blocks up to 16 per SM (two waves at
 // four threads per slot), where more and smaller blocks keep the SMs evenly
 // loaded; beyond that 64-slot blocks, whose halo is half as large (5 of 64
-// slots, not of 32).  us per MD step, 32 / 64 slots: 54,744 beads mixed 70.9 /
-// 71.7, 66,007 beads mixed 45.4 / 42.8 and FP64 139.4 / 141.1, 8,000 beads FP64
-// 39 / 44.
+// slots, not of 32).  us per MD step, 32 / 64 slots: 8,000 beads mixed 17.2 /
+// 22.0 and FP64 35.1 / 42.7, 54,744 beads mixed 35.4 / 35.9, 66,007 beads mixed
+// 44.0 / 42.0; FP64 hardly minds there (141.8 / 143.7), so the line lies where
+// mixed turns.
 void Engine::default_shape() {
     if (!tuned) tune.fb = force_blocks(d.N, 32) <= 16 * tile_sms ? 32 : 64;
 }

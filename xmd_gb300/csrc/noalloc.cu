@@ -32,7 +32,7 @@
 // memory, O(m^2) for m partners (a periodic box under two cutoffs wide, a
 // cluster much denser than a protein).
 //
-// 30,720 beads at 1e-3 A^-3, cutoff 20 A: 3,200 us -> 110 us (one block for
+// 30,720 beads at 1e-3 A^-3, cutoff 20 A: 3,200 us -> 96 us (one block for
 // the grid took 250 us of it, and one thread per row, twice, 1,500 us each;
 // searching every row twice 12 us).
 #include <cuda_runtime.h>

@@ -24,9 +24,9 @@
 // What it measured, us per MD step, against a block whose threads kept to one
 // bead each from list loops to integrator (bonded geometry formed per term, a
 // third of the bonded warps with 3 live lanes, noise and skin test on a quarter
-// of the lanes): 256 chains of 50-800 beads (66,007) FP64 456 -> 139, mixed
-// 65 -> 43; 61 native chains mixed 38 -> 23; 16 x 500 periodic FP64 105 -> 39,
-// mixed 31 -> 18; one chain of 100 beads FP64 55 -> 18.  FP64 is bound by its
+// of the lanes): 256 chains of 50-800 beads (66,007) FP64 458 -> 141, mixed
+// 66 -> 44; 61 native chains mixed 38 -> 24; 16 x 500 periodic FP64 111 -> 40,
+// mixed 32 -> 20; one chain of 100 beads FP64 54 -> 17.  FP64 is bound by its
 // pipe (81 % active while blocks run) and the tail of the last wave, mixed by
 // latency: index load, position load and arithmetic of a round of entries,
 // the barriers between the phases, 32 warps per SM to hide them.
